@@ -154,6 +154,7 @@ int imps_ctx_destroy(imps_ctx* h) {
   }
   for (auto e : c.event_pool) cudaEventDestroy(e);
   c.scratch.clear();
+  c.optional.clear();
   c.red.release();
   if (c.host_pinned) cudaFreeHost(c.host_pinned);
   if (c.dev_info) cudaFree(c.dev_info);
@@ -204,6 +205,10 @@ int imps_ctx_set_wait_limit(imps_ctx* h, int64_t cycles) {
 int imps_ctx_set_workspace_limit(imps_ctx* h, int64_t bytes) {
   if (!h || bytes < 0) return IMPS_INVALID_ARG;
   h->c.workspace_limit = (size_t)bytes;
+  if (bytes > 0) {
+    cudaSetDevice(h->c.device);
+    h->c.release_optional();
+  }
   return IMPS_OK;
 }
 
@@ -211,6 +216,7 @@ int imps_ctx_workspace_bytes(imps_ctx* h, int64_t* bytes) {
   if (!h || !bytes) return IMPS_INVALID_ARG;
   size_t total = 0;
   for (const auto& kv : h->c.scratch) total += kv.second.bytes;
+  for (const auto& kv : h->c.optional) total += kv.second.bytes;
   *bytes = (int64_t)total;
   return IMPS_OK;
 }

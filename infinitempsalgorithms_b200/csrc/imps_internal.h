@@ -157,8 +157,37 @@ struct Context {
         throw Error(IMPS_OOM, "workspace limit of " + std::to_string(workspace_limit) + " bytes reached (buffer '" +
                                   name + "' needs " + std::to_string(bytes) + " bytes)");
     }
-    b.ensure(bytes);
+    try {
+      b.ensure(bytes);
+    } catch (const Error& e) {
+      if (e.status != IMPS_OOM || optional.empty()) throw;
+      cudaGetLastError();
+      release_optional();
+      b.ensure(bytes);
+    }
     return b;
+  }
+  // Scratch that only makes a call faster (partial tiles, residue planes): nullptr when it
+  // is not to be had -- a workspace cap is set, the call may not allocate, or the device is
+  // out of memory -- and the caller then takes its path without it.  Kept between calls;
+  // given back when a cap is set or a required buffer does not fit.
+  std::map<std::string, DevBuf> optional;
+  int no_scratch = 0;   // > 0: a call that must not allocate is running
+  void* optional_buf(const char* name, size_t bytes) {
+    if (no_scratch > 0 || workspace_limit > 0) return nullptr;
+    DevBuf& b = optional[name];
+    try {
+      b.ensure(bytes);
+    } catch (const Error& e) {
+      if (e.status != IMPS_OOM) throw;
+      cudaGetLastError();   // a failed cudaMalloc leaves no sticky error
+      return nullptr;
+    }
+    return b.ptr;
+  }
+  void release_optional() {
+    cudaStreamSynchronize(stream);
+    optional.clear();
   }
   double* pinned(size_t bytes);
 };
@@ -243,6 +272,12 @@ struct MaxSlicesScope {
   int old;
   MaxSlicesScope(Context* c, int s) : ctx(c), old(c->max_adaptive_slices) { ctx->max_adaptive_slices = s; }
   ~MaxSlicesScope() { ctx->max_adaptive_slices = old; }
+};
+// No optional scratch while alive.
+struct NoScratchScope {
+  Context* ctx;
+  explicit NoScratchScope(Context* c) : ctx(c) { ctx->no_scratch++; }
+  ~NoScratchScope() { ctx->no_scratch--; }
 };
 // Sets the accuracy the split GEMMs must meet while alive.
 struct TolScope {

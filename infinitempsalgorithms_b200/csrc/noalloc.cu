@@ -112,6 +112,7 @@ void ac_apply_noalloc(Context* ctx, int Dl, int d, int Dr, int m, int n, const c
   dcplx* T1 = reinterpret_cast<dcplx*>(base + kNoAllocWBytes);
   dcplx* T2 = T1 + t1;
   IMPS_CUDA(cudaMemcpyAsync(Wd, W_host, wbytes, cudaMemcpyHostToDevice, ctx->stream));
+  NoScratchScope ns(ctx);
   zgemm_fp64(ctx, OP_N, OP_N, Dl * m, d * Dr, Dl, 1.0, GL, (int64_t)Dl * m, 0, x, Dl, 0, 0.0, T1, (int64_t)Dl * m, 0, 1);
   // right levels without any block read as zero (the array keeps the previous call's data)
   for (int q = 0; q < n; ++q)

@@ -8,8 +8,9 @@
 #include "imps_internal.h"
 #include "split_gemm.h"
 
-#include <atomic>
+#include <algorithm>
 #include <cmath>
+#include <type_traits>
 
 namespace imps {
 namespace {
@@ -126,25 +127,27 @@ __global__ void __launch_bounds__(NT, 2)
 }
 
 // ---------------------------------------------------------------------------
-// FP64 tensor-core variant: mma.sync m8n8k4 f64 (DMMA).  128 x 64 complex output
-// tile per CTA of 8 warps (4 x 2 warps of 32 x 32), K stage of 16 complex, a
-// 3-stage cp.async ring (zero-filled at the matrix edges).  A complex product is
-// four real DMMAs per 8 x 8 block: re += ar br - ai bi, im += ar bi + ai br; the
-// conjugate of an operand only flips the sign of its imaginary fragment.
-// Shared tiles are k-major rows of double2 with one element of padding.
+// FP64 tensor-core variant: mma.sync m8n8k4 f64 (DMMA).  64 x 64 complex output tile per
+// CTA of 8 warps (2 x 4 warps of 32 x 16), two CTAs per SM, a K stage of 16 complex, a
+// 3-stage cp.async ring (zero-filled at the matrix edges).  A complex product is four real
+// DMMAs per 8 x 8 block: re += ar br - ai bi, im += ar bi + ai br; the conjugate of an
+// operand only flips the sign of its imaginary fragment.
+// Shared tiles are k-major rows of double2.  A fragment read takes 4 k x 2 m (or n)
+// consecutive elements per 8-lane phase, so a row stride of 2 mod 8 elements is free of
+// bank conflicts; the loads of a transposed operand walk 4 k x 2 m per phase for the same
+// reason.  Bound by the FP64 tensor pipe: four warps a scheduler (two CTAs) hide the
+// fragment reads and the stage barriers behind the MMAs.  Measured (B200, N x N):
+// 6144 x 4096 x 1024 6.50 ms and 4096 x 1024 x 6144 6.57 ms, 31.5 TFLOP/s (6.88 and 7.81 ms
+// with 128 x 64 tiles of 32 x 32 warps and 2-way conflicts in the fragment reads); with the
+// K stages shared (split_k) 502 x 251 x 1255 55 us (was 239) and 256 x 256 x 1024 (C x N)
+// 32 us (was 210).
 // ---------------------------------------------------------------------------
-// Tile shapes of the DMMA engine: TM = 128 (8 warps, one CTA per SM by registers and
-// shared memory) for large grids; TM = 64 (4 warps, two CTAs per SM) for grids that would
-// not fill the SMs twice over with 128-row tiles (the skinny products of the blocked QR).
 namespace dm {
-constexpr int BN = 64, BK = 16, STAGES = 3;
-template <int TM>
-struct Tile {
-  static constexpr int BM = TM, NT = 2 * TM, WM = TM / 32;
-  static constexpr int LDA = BM + 1, LDB = BN + 1;
-  static constexpr int A_ELEMS = BK * LDA, B_ELEMS = BK * LDB;
-  static constexpr int SMEM = STAGES * (A_ELEMS + B_ELEMS) * 16;
-};
+constexpr int BM = 64, BN = 64, BK = 16, STAGES = 3, NT = 256;
+constexpr int LD = BM + 2;
+constexpr int TILE = BK * LD;                    // elements of one operand's stage
+constexpr int SMEM = STAGES * 2 * TILE * 16;
+constexpr int SMEM_ALONE = 120 * 1024;           // keeps a second CTA off the SM
 }  // namespace dm
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
@@ -160,149 +163,213 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
-template <int OPA, int OPB, bool BETA, int TM>
-__global__ void __launch_bounds__(2 * TM, 128 / TM)
+// SPLITK: nsplit CTAs (along x) share one output tile, each summing its part of the K
+// stages; CTA r writes its plain partial sums to part[r] (M x N each), which
+// k_sum_split adds in order (so the result does not depend on timing).
+template <int OPA, int OPB, bool BETA, bool SPLITK>
+__global__ void __launch_bounds__(dm::NT, 2)
     k_zgemm_dmma(int M, int N, int K, double2 alpha, const double2* __restrict__ A, int64_t lda, int64_t sA,
                  const double2* __restrict__ B, int64_t ldb, int64_t sB, double2 beta, double2* __restrict__ C,
-                 int64_t ldc, int64_t sC) {
-  using T = dm::Tile<TM>;
-  extern __shared__ __align__(16) double2 smem_dm[];
-  double2* As = smem_dm;                             // [STAGES][BK][LDA]
-  double2* Bs = smem_dm + dm::STAGES * T::A_ELEMS;   // [STAGES][BK][LDB]
+                 int64_t ldc, int64_t sC, int nsplit, double2* __restrict__ part) {
+  extern __shared__ __align__(16) double2 smem_dm[];   // [STAGES][A tile, B tile][BK][LD]
   const int bz = blockIdx.z;
   A += sA * bz;
   B += sB * bz;
   C += sC * bz;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp % T::WM, wn = warp / T::WM;  // warp tile origin (32 * wm, 32 * wn)
-  const int m0 = blockIdx.x * T::BM, n0 = blockIdx.y * dm::BN;
+  const int wm = warp & 1, wn = warp >> 1;  // warp tile origin (32 wm, 16 wn)
+  const int rank = SPLITK ? (int)(blockIdx.x % nsplit) : 0;
+  const int m0 = (int)(SPLITK ? blockIdx.x / nsplit : blockIdx.x) * dm::BM, n0 = blockIdx.y * dm::BN;
   const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dm));
 
-  auto issue = [&](int stage, int k0) {
-    // A tile: BM x BK complex, 8 per thread (NT = 2 BM)
-    static_assert(dm::BN == 64 && dm::BK == 16 && (TM == 64 || TM == 128), "load mapping assumes these tiles");
+  // Load coordinates.  An operand whose line index (m or n) is contiguous: line tid % 64,
+  // k = tid / 64 + 4 r; one contiguous in k: k from bits 0, 1, 3, 4 of tid, line from bit 2
+  // and the warp, + 16 r.
+  constexpr bool AK = OPA != OP_N, BKc = OPB == OP_N;   // contiguous along k
+  const int kc = (tid & 3) | ((tid >> 1) & 12), lc = ((tid >> 2) & 1) | (warp << 1);
+  const int ll = tid & 63, kl = tid >> 6;
+  const int am = AK ? lc : ll, ak = AK ? kc : kl;
+  const int bn = BKc ? lc : ll, bk = BKc ? kc : kl;
+  const int64_t a_r = AK ? 16 * lda : 4 * lda, b_r = BKc ? 16 * ldb : 4 * ldb;         // step of r
+  const int64_t a_s = AK ? dm::BK : dm::BK * lda, b_s = BKc ? dm::BK : dm::BK * ldb;   // step of a stage
+  // this CTA's K stages
+  const int kall = (K + dm::BK - 1) / dm::BK;
+  const int kt0 = SPLITK ? (int)((int64_t)kall * rank / nsplit) : 0;
+  const int ktiles = (SPLITK ? (int)((int64_t)kall * (rank + 1) / nsplit) : kall) - kt0;
+  const double2* pa = A + (AK ? ak + lda * (int64_t)(m0 + am) : (m0 + am) + lda * (int64_t)ak) + a_s * kt0;
+  const double2* pb = B + (BKc ? bk + ldb * (int64_t)(n0 + bn) : (n0 + bn) + ldb * (int64_t)bk) + b_s * kt0;
+  const uint32_t da = sbase + 16u * (ak * dm::LD + am), db = sbase + 16u * (dm::TILE + bk * dm::LD + bn);
+  constexpr uint32_t DA_R = 16u * (AK ? 16 : 4 * dm::LD), DB_R = 16u * (BKc ? 16 : 4 * dm::LD);
+
+  auto issue = [&](int stage, int kt) {
+    const int k0 = (kt0 + kt) * dm::BK;
+    const double2* qa = pa + a_s * kt;
+    const double2* qb = pb + b_s * kt;
+    const uint32_t so = 16u * (uint32_t)(stage * 2 * dm::TILE);
 #pragma unroll
-    for (int r = 0; r < 8; ++r) {
-      int m, k;
-      if (OPA == OP_N) { m = tid & (TM - 1); k = (tid / TM) + 2 * r; }
-      else { k = tid & 15; m = (tid >> 4) + (T::NT / 16) * r; }
-      const int gm = m0 + m, gk = k0 + k;
-      const bool ok = gm < M && gk < K;
-      const double2* src = ok ? ((OPA == OP_N) ? A + gm + lda * (int64_t)gk : A + gk + lda * (int64_t)gm) : A;
-      cp_async16(sbase + 16u * (stage * T::A_ELEMS + k * T::LDA + m), src, ok ? 16 : 0);
+    for (int r = 0; r < 4; ++r) {
+      const bool ok = AK ? (m0 + am + 16 * r < M && k0 + ak < K) : (m0 + am < M && k0 + ak + 4 * r < K);
+      cp_async16(da + so + DA_R * r, ok ? qa + a_r * r : A, ok ? 16 : 0);
     }
-    // B tile: BK x BN complex, 1024 / NT per thread
 #pragma unroll
-    for (int r = 0; r < 1024 / T::NT; ++r) {
-      int n, k;
-      if (OPB == OP_N) { k = tid & 15; n = (tid >> 4) + (T::NT / 16) * r; }
-      else { n = tid & 63; k = (tid >> 6) + (T::NT / 64) * r; }
-      const int gn = n0 + n, gk = k0 + k;
-      const bool ok = gn < N && gk < K;
-      const double2* src = ok ? ((OPB == OP_N) ? B + gk + ldb * (int64_t)gn : B + gn + ldb * (int64_t)gk) : B;
-      cp_async16(sbase + 16u * (dm::STAGES * T::A_ELEMS + stage * T::B_ELEMS + k * T::LDB + n), src, ok ? 16 : 0);
+    for (int r = 0; r < 4; ++r) {
+      const bool ok = BKc ? (n0 + bn + 16 * r < N && k0 + bk < K) : (n0 + bn < N && k0 + bk + 4 * r < K);
+      cp_async16(db + so + DB_R * r, ok ? qb + b_r * r : B, ok ? 16 : 0);
     }
   };
 
-  double cre[4][4][2], cim[4][4][2];
+  double cre[4][2][2], cim[4][2][2];
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) cre[i][j][0] = cre[i][j][1] = cim[i][j][0] = cim[i][j][1] = 0.0;
+    for (int j = 0; j < 2; ++j) cre[i][j][0] = cre[i][j][1] = cim[i][j][0] = cim[i][j][1] = 0.0;
 
-  const int ktiles = (K + dm::BK - 1) / dm::BK;
 #pragma unroll
   for (int st = 0; st < dm::STAGES - 1; ++st) {
-    if (st < ktiles) issue(st, st * dm::BK);
+    if (st < ktiles) issue(st, st);
     cp_async_commit();
   }
   const int fr = lane >> 2, fk = lane & 3;  // fragment row/col (A: row m, col k; B: col n, row k)
+  const int fa = fk * dm::LD + 32 * wm + fr, fb = dm::TILE + fk * dm::LD + 16 * wn + fr;
+  int stage = 0, nstage = dm::STAGES - 1;
   for (int kt = 0; kt < ktiles; ++kt) {
     cp_async_wait<dm::STAGES - 2>();
     __syncthreads();
-    {
-      const int nk = kt + dm::STAGES - 1;
-      if (nk < ktiles) issue(nk % dm::STAGES, nk * dm::BK);
-      cp_async_commit();
-    }
-    const double2* as = As + (kt % dm::STAGES) * T::A_ELEMS;
-    const double2* bs = Bs + (kt % dm::STAGES) * T::B_ELEMS;
+    if (kt + dm::STAGES - 1 < ktiles) issue(nstage, kt + dm::STAGES - 1);
+    cp_async_commit();
+    const double2* ss = smem_dm + stage * 2 * dm::TILE;
 #pragma unroll
     for (int kb = 0; kb < dm::BK; kb += 4) {
-      double ar[4], ai[4], nai[4], br[4], bi[4];
+      double ar[4], ai[4], br[2], bi[2];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const double2 v = as[(kb + fk) * T::LDA + 32 * wm + 8 * i + fr];
+        const double2 v = ss[kb * dm::LD + fa + 8 * i];
         ar[i] = v.x;
         ai[i] = (OPA == OP_C) ? -v.y : v.y;
-        nai[i] = -ai[i];
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const double2 v = bs[(kb + fk) * T::LDB + 32 * wn + 8 * j + fr];
+      for (int j = 0; j < 2; ++j) {
+        const double2 v = ss[kb * dm::LD + fb + 8 * j];
         br[j] = v.x;
         bi[j] = (OPB == OP_C) ? -v.y : v.y;
       }
-      // the two updates of one accumulator are 32 MMAs apart
+      // the two updates of one accumulator are 16 MMAs apart
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < 2; ++j) {
           dmma(cre[i][j][0], cre[i][j][1], ar[i], br[j]);
           dmma(cim[i][j][0], cim[i][j][1], ar[i], bi[j]);
         }
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          dmma(cre[i][j][0], cre[i][j][1], nai[i], bi[j]);
+        for (int j = 0; j < 2; ++j) {
+          dmma(cre[i][j][0], cre[i][j][1], -ai[i], bi[j]);
           dmma(cim[i][j][0], cim[i][j][1], ai[i], br[j]);
         }
     }
+    stage = stage + 1 == dm::STAGES ? 0 : stage + 1;
+    nstage = nstage + 1 == dm::STAGES ? 0 : nstage + 1;
   }
   cp_async_wait<0>();
   // D fragment: row = lane >> 2, cols 2 (lane & 3) + {0, 1} of each 8 x 8 block
+  double2* P = SPLITK ? part + ((int64_t)bz * nsplit + rank) * M * (int64_t)N : nullptr;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     const int gm = m0 + 32 * wm + 8 * i + fr;
     if (gm >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 2; ++j)
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
-        const int gn = n0 + 32 * wn + 8 * j + 2 * fk + e;
+        const int gn = n0 + 16 * wn + 8 * j + 2 * fk + e;
         if (gn >= N) continue;
         const double vr = cre[i][j][e], vi = cim[i][j][e];
+        if (SPLITK) {
+          P[gm + M * (int64_t)gn] = make_double2(vr, vi);
+          continue;
+        }
         double2 o = make_double2(alpha.x * vr - alpha.y * vi, alpha.x * vi + alpha.y * vr);
+        double2* p = C + gm + ldc * (int64_t)gn;
         if (BETA) {
-          const double2 c = C[gm + ldc * (int64_t)gn];
+          const double2 c = *p;
           o.x += beta.x * c.x - beta.y * c.y;
           o.y += beta.x * c.y + beta.y * c.x;
         }
-        C[gm + ldc * (int64_t)gn] = o;
+        *p = o;
       }
-    }
   }
 }
 
-template <int OPA, int OPB, int TM>
-void launch_dmma(Context* ctx, int M, int N, int K, double2 alpha, const dcplx* A, int64_t lda, int64_t sA,
-                 const dcplx* B, int64_t ldb, int64_t sB, double2 beta, dcplx* C, int64_t ldc, int64_t sC, int batch,
-                 bool use_beta) {
-  using T = dm::Tile<TM>;
-  // the dynamic shared-memory opt-in is per device and per kernel instance; setting it
-  // twice (two host threads racing here) is harmless
-  static std::atomic<uint64_t> attr_set[2];
-  auto kern = use_beta ? k_zgemm_dmma<OPA, OPB, true, TM> : k_zgemm_dmma<OPA, OPB, false, TM>;
-  const uint64_t bit = 1ull << (ctx->device & 63);
-  std::atomic<uint64_t>& done = attr_set[use_beta ? 1 : 0];
-  if (!(done.load() & bit)) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM);
-    if (e != cudaSuccess) throw Error(IMPS_CUDA_ERROR, std::string("zgemm smem opt-in: ") + cudaGetErrorString(e));
-    done.fetch_or(bit);
+// C = alpha sum_r part[r] + beta C, the nsplit partial products of each batch entry in order
+template <bool BETA>
+__global__ void __launch_bounds__(256) k_sum_split(int M, int N, int nsplit, const double2* __restrict__ part,
+                                                   double2 alpha, double2 beta, double2* __restrict__ C, int64_t ldc,
+                                                   int64_t sC) {
+  const int64_t len = (int64_t)M * N;
+  part += (int64_t)blockIdx.y * nsplit * len;
+  C += sC * blockIdx.y;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < len; i += (int64_t)gridDim.x * blockDim.x) {
+    double vr = 0.0, vi = 0.0;
+    int q = 0;
+    for (; q + 4 <= nsplit; q += 4) {  // four loads in flight
+      double2 v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = __ldg(&part[i + len * (q + u)]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        vr += v[u].x;
+        vi += v[u].y;
+      }
+    }
+    for (; q < nsplit; ++q) {
+      const double2 v = __ldg(&part[i + len * q]);
+      vr += v.x;
+      vi += v.y;
+    }
+    double2 o = make_double2(alpha.x * vr - alpha.y * vi, alpha.x * vi + alpha.y * vr);
+    double2* p = C + i % M + ldc * (i / M);
+    if (BETA) {
+      const double2 c = *p;
+      o.x += beta.x * c.x - beta.y * c.y;
+      o.y += beta.x * c.y + beta.y * c.x;
+    }
+    *p = o;
   }
-  dim3 grid((M + T::BM - 1) / T::BM, (N + dm::BN - 1) / dm::BN, batch);
-  kern<<<grid, T::NT, T::SMEM, ctx->stream>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC);
+}
+
+template <int OPA, int OPB, bool BETA, bool SPLITK>
+void launch_dmma(Context* ctx, int nsplit, double2* part, int M, int N, int K, double2 alpha, const dcplx* A,
+                 int64_t lda, int64_t sA, const dcplx* B, int64_t ldb, int64_t sB, double2 beta, dcplx* C, int64_t ldc,
+                 int64_t sC, int batch) {
+  auto kern = k_zgemm_dmma<OPA, OPB, BETA, SPLITK>;
+  static DeviceOnce attr;  // the dynamic shared-memory opt-in
+  attr.run(ctx->device, [&] {
+    IMPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dm::SMEM));
+  });
+  const dim3 grid((M + dm::BM - 1) / dm::BM * nsplit, (N + dm::BN - 1) / dm::BN, batch);
+  kern<<<grid, dm::NT, dm::SMEM, ctx->stream>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, nsplit, part);
+}
+
+// CTAs that share one 64 x 64 output tile (1: none): the smallest time of a model of the
+// grid.  Measured on a B200: a K stage of one CTA takes 3.3 us alone on its SM and 2.46 us
+// of the SM when others run beside it; the partial products cost one more launch (4 us) and
+// their bytes at 3 TB/s.
+int split_k(const Context* ctx, int64_t tiles, int K) {
+  const int kall = (K + dm::BK - 1) / dm::BK;
+  int best = 1;
+  double tbest = 1e300;
+  for (int s = 1; s <= kall && s <= 64; ++s) {
+    const int64_t per_sm = (tiles * s + ctx->num_sms - 1) / ctx->num_sms;
+    double t = ((kall + s - 1) / s) * (per_sm == 1 ? 3.3 : 2.46 * (double)per_sm);
+    if (s > 1) t += 4.0 + (double)tiles * s * (dm::BM * dm::BN * 16 / 3e6);
+    if (t < tbest) {
+      tbest = t;
+      best = s;
+    }
+  }
+  return best;
 }
 
 template <int OPA, int OPB>
@@ -318,12 +385,26 @@ void launch(Context* ctx, int M, int N, int K, double2 alpha, const dcplx* A, in
                                                               sC);
     return;
   }
-  // 128-row tiles unless they would give fewer than two CTAs per SM; then 64-row tiles,
-  // two of which fit an SM
-  const int64_t tiles128 = (int64_t)((M + 127) / 128) * ((N + dm::BN - 1) / dm::BN) * batch;
-  if (tiles128 >= 2 * 148) launch_dmma<OPA, OPB, 128>(ctx, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC,
-                                                       batch, use_beta);
-  else launch_dmma<OPA, OPB, 64>(ctx, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch, use_beta);
+  auto go = [&](auto beta_tag) {
+    constexpr bool BETA = decltype(beta_tag)::value;
+    // the K stages of a tile are shared by several CTAs where the tiles alone would leave
+    // SMs idle (the long-K products of the pushes and of the QR, every product of a small state)
+    const int64_t tiles = (int64_t)((M + dm::BM - 1) / dm::BM) * ((N + dm::BN - 1) / dm::BN) * batch;
+    const int s = split_k(ctx, tiles, K);
+    const int64_t len = (int64_t)M * N;
+    double2* part = nullptr;
+    if (s > 1) part = static_cast<double2*>(ctx->optional_buf("gemm_part", (size_t)len * s * batch * sizeof(double2)));
+    if (!part) {
+      launch_dmma<OPA, OPB, BETA, false>(ctx, 1, nullptr, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
+      return;
+    }
+    launch_dmma<OPA, OPB, BETA, true>(ctx, s, part, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
+    const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((len + 255) / 256, ctx->num_sms * 8 / batch));
+    k_sum_split<BETA><<<dim3(g, batch), 256, 0, ctx->stream>>>(M, N, s, part, alpha, beta, C, ldc, sC);
+    ctx->n_kernels++;
+  };
+  if (use_beta) go(std::true_type{});
+  else go(std::false_type{});
 }
 
 }  // namespace
