@@ -42,7 +42,8 @@ enum {
 
 /* Precision modes of the Heff / transfer contractions. */
 enum {
-  IMPS_PREC_FP64 = 0,       /* plain method: FP64 end to end                       */
+  IMPS_PREC_FP64 = 0,       /* plain method: FP64 results; large products through
+                               exact residue arithmetic, no less accurate          */
   IMPS_PREC_SPLIT_I8 = 1    /* int8 split products on tcgen05, exact int32 sums    */
 };
 
@@ -108,7 +109,8 @@ int imps_ctx_set_stream(imps_ctx* ctx, void* cuda_stream);
  * (up to 6; a tolerance that needs more runs the FP64 engine). */
 int imps_ctx_set_precision(imps_ctx* ctx, int mode, int nslices);
 int imps_ctx_synchronize(imps_ctx* ctx);
-/* Bound of each pipeline wait inside the split GEMM kernel, in SM clock cycles
+/* Bound of each pipeline wait inside the tensor-core GEMM kernels (the split products and
+ * the large FP64 products in residue arithmetic), in SM clock cycles
  * (0 restores the default 2e9, about 1 s).  A wait that runs out sets a device
  * error flag and the kernel returns early; the flag is read at the context's next
  * host synchronisation (at the latest when the entry point returns) and the call

@@ -689,24 +689,25 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
   return fn;
 }
 
-// 3D map over int8 planes: dims (Kp bytes, rows, planes), box (KB, box_rows, 1), 64B swizzle
-CUtensorMap make_map(const int8_t* base, int64_t Kp, int64_t rows, int planes, int box_rows) {
+int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
+
+}  // namespace
+
+CUtensorMap plane_map(const int8_t* base, int64_t Kp, int64_t rows, int planes, int box_k, int box_rows,
+                      int64_t plane_bytes) {
   CUtensorMap m;
   std::memset(&m, 0, sizeof(m));
   cuuint64_t dims[3] = {(cuuint64_t)Kp, (cuuint64_t)rows, (cuuint64_t)planes};
-  cuuint64_t strides[2] = {(cuuint64_t)Kp, (cuuint64_t)(Kp * rows)};
-  cuuint32_t box[3] = {(cuuint32_t)KB, (cuuint32_t)box_rows, 1};
+  cuuint64_t strides[2] = {(cuuint64_t)Kp, (cuuint64_t)(plane_bytes > 0 ? plane_bytes : Kp * rows)};
+  cuuint32_t box[3] = {(cuuint32_t)box_k, (cuuint32_t)box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = get_encode()(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t*>(base), dims, strides, box, estr,
-                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            box_k == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   IMPS_REQUIRE(r == CUDA_SUCCESS, IMPS_CUDA_ERROR, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
   return m;
 }
-
-int64_t round_up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
-
-}  // namespace
 
 // ---------------------------------------------------------------------------
 void split_operand_a(Context* ctx, SplitOperand& S, Op op, int M, int K, const dcplx* A, int64_t lda, int s) {
@@ -793,8 +794,8 @@ void split_gemm(Context* ctx, const SplitOperand& A, const SplitOperand& B, int 
   // 80 for 6, 64 otherwise.  The B planes are padded to 128 rows; a 96- or 80-row box
   // that reaches past them reads TMA's zero fill (and still delivers its full byte count).
   const int bn = (s >= 2 && s <= 6) ? bn_for(s) : 64;
-  const CUtensorMap mapA = make_map(static_cast<const int8_t*>(A.data.ptr), A.Kp, A.Rp, A.s, BM);
-  const CUtensorMap mapB = make_map(static_cast<const int8_t*>(B.data.ptr), B.Kp, B.Rp, B.s, bn);
+  const CUtensorMap mapA = plane_map(static_cast<const int8_t*>(A.data.ptr), A.Kp, A.Rp, A.s, KB, BM);
+  const CUtensorMap mapB = plane_map(static_cast<const int8_t*>(B.data.ptr), B.Kp, B.Rp, B.s, KB, bn);
   GemmArgs g;
   g.num_m = (int)(A.Rp / BM);
   g.num_n = (B.rows + bn - 1) / bn;

@@ -1,0 +1,797 @@
+// FP64 complex GEMM by residue arithmetic on the 5th-generation tensor cores
+// (tcgen05 kind::i8): the Ozaki scheme II idea (Ozaki, Uchino, Imamura,
+// arXiv:2504.08009) for complex operands.
+//
+//  1. Every row a_i of op(A) and column b_j of op(B) is scaled by a power of two and
+//     rounded to Gaussian integers with ||a'_i||_2, ||b'_j||_2 <= 2^58.  By Cauchy-Schwarz
+//     the real and imaginary parts of c'_ij = sum_k a'_ik b'_kj are below 2^116, so c' is
+//     determined by its residues modulo P = product of the 16 moduli below (2^117.7).
+//  2. Each modulus p has a square root of -1, iota: u = x + iota y and v = x - iota y map
+//     the Gaussian integers mod p onto two copies of the integers mod p, in which the
+//     complex product is two real ones (not four).  All residues are int8, the sums over K
+//     exact in int32: 32 real int8 GEMMs of M x N x K.
+//  3. The 32 residues of an output give Re c' / P and Im c' / P as fractions modulo 1
+//     (Chinese remainder theorem), then the product with P and the power-of-two scales.
+//
+// Accuracy: the only errors are the roundings of step 1, below 2^-58 of the row's (column's)
+// 2-norm per element, and those of the final conversion (2^-52 relative).  An element of
+// C is off by about 3e-18 ||a_i|| ||b_j||; an FP64 sum over K random terms is off by
+// 0.3 sqrt(K) 2^-53 of its result, i.e. by more for every K here.  Rows or columns with a
+// NaN or an Inf are recognised and their elements computed by a plain FP64 loop.
+//
+// The four kernels: partial row norms, residue planes, the int8 GEMMs, the reconstruction.
+// Measured (B200): 6144 x 4096 x 1024 1.21 ms = 33 + 141 + 651 + 375 us (6.50 ms on the FP64
+// tensor cores), 4096 x 1024 x 6144 1.09 ms = 90 + 405 + 524 + 69 us (6.57 ms), i.e. 171 and
+// 188 TFLOP/s of FP64 products; error against 80-bit sums 1e-16 .. 3e-16 of the result's norm
+// for K = 256 .. 8192 (FP64 tensor cores 8e-16 .. 6e-15).
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "gemm_modular.h"
+#include "split_gemm.h"
+
+namespace imps {
+namespace {
+
+constexpr int NMOD = 16;
+constexpr int NPL = 2 * NMOD;    // residue planes: u of every modulus, then v
+constexpr int BETA_BITS = 58;    // the integer operands' lines have 2-norm <= 2^58
+constexpr int EXP_NONFINITE = 1 << 20;
+
+// odd, pairwise coprime, at most 241, each with a square root of -1 (all prime factors 1 mod 4)
+constexpr int kMod[NMOD] = {241, 233, 229, 221, 205, 197, 193, 181, 173, 157, 149, 137, 113, 109, 101, 97};
+
+struct ModTables {
+  // residue of a 64-bit integer: dp4a weights 256^j and iota 256^j mod p of its 8 bytes
+  int wa_lo[NMOD], wa_hi[NMOD], wb_lo[NMOD], wb_hi[NMOD];
+  // constants that take out the 2^62 bias of both integers (off_v relative to off_u), or the
+  // 2^31 bias of an int32 sum; off_u and off_s carry the 1.5 2^23 of mod_byte
+  int off_u[NMOD], off_v[NMOD], off_s[NMOD];
+  int p[NMOD];
+  float inv[NMOD];
+  // CRT weights as fractions of P: the first 32 bits as an integer, the next 40 as a double;
+  // re multiplies u + v, im multiplies u - v
+  unsigned re1[NMOD], im1[NMOD];
+  double re2[NMOD], im2[NMOD];
+  unsigned re1_0, im1_0;           // -256 times the sums of the weights (see k_mod_join)
+  double re2_0, im2_0;
+  double P;
+};
+
+constexpr int mod_pow(int b, int e, int p) {
+  int r = 1;
+  for (int i = 0; i < e; ++i) r = r * b % p;
+  return r;
+}
+constexpr int mod_inv(int a, int p) {
+  for (int x = 1; x < p; ++x)
+    if (a * x % p == 1) return x;
+  return 0;
+}
+constexpr int mod_iota(int p) {
+  for (int x = 1; x < p; ++x)
+    if ((x * x + 1) % p == 0) return x;
+  return 0;
+}
+constexpr int kMagicBits = 0x4B400000;   // 1.5 2^23 as a float: its mantissa holds an integer
+constexpr int centred(int x, int p) { return x > p / 2 ? x - p : x; }
+
+// The part of g / p below 2^-32, to 2^-72: sums of 16 of them times 9-bit integers are exact
+// in a double (so that vanishing residues give a zero), and what is dropped is 2^-8 of the
+// rounding of the operands.
+constexpr double low_weight(int g, int p) {
+  const unsigned long long rem = ((unsigned long long)g << 32) % (unsigned)p;
+  return (double)((((rem << 41) / (unsigned)p) + 1) >> 1) / 4722366482869645213696.0;   // 2^72
+}
+
+constexpr ModTables make_tables() {
+  ModTables t{};
+  unsigned __int128 P = 1;
+  for (int i = 0; i < NMOD; ++i) P *= (unsigned)kMod[i];
+  t.P = (double)(P >> 32) * 4294967296.0;   // the dropped 32 of 118 bits are below 2^-85 of it
+  for (int i = 0; i < NMOD; ++i) {
+    const int p = kMod[i], io = mod_iota(p);
+    unsigned w[4] = {0, 0, 0, 0};
+    for (int j = 0; j < 8; ++j) {
+      const int a = mod_pow(256 % p, j, p), b = a * io % p;
+      w[j / 4] |= (unsigned)(centred(a, p) & 255) << (8 * (j % 4));
+      w[2 + j / 4] |= (unsigned)(centred(b, p) & 255) << (8 * (j % 4));
+    }
+    t.wa_lo[i] = (int)w[0];
+    t.wa_hi[i] = (int)w[1];
+    t.wb_lo[i] = (int)w[2];
+    t.wb_hi[i] = (int)w[3];
+    const int bias = mod_pow(2, 62, p), ib = bias * io % p;
+    const int ou = centred((2 * p - bias - ib) % p, p), ov = centred((p - bias + ib) % p, p);
+    t.off_u[i] = ou + kMagicBits;
+    t.off_v[i] = ov - ou;
+    t.off_s[i] = centred(p - mod_pow(2, 31, p), p) + kMagicBits;
+    t.p[i] = p;
+    t.inv[i] = 1.0f / (float)p;
+    // (P / p)^-1 / 2 and (P / p)^-1 / (2 iota) mod p, as fractions of p
+    int q = 1;
+    for (int j = 0; j < NMOD; ++j)
+      if (j != i) q = q * (kMod[j] % p) % p;
+    const int g = mod_inv(q * 2 % p, p), h = mod_inv(q * 2 % p * io % p, p);
+    t.re1[i] = (unsigned)(((unsigned long long)g << 32) / (unsigned)p);
+    t.im1[i] = (unsigned)(((unsigned long long)h << 32) / (unsigned)p);
+    t.re2[i] = low_weight(g, p);
+    t.im2[i] = low_weight(h, p);
+    t.re1_0 -= 256u * t.re1[i];
+    t.im1_0 -= 256u * t.im1[i];
+    t.re2_0 -= 256.0 * t.re2[i];
+    t.im2_0 -= 256.0 * t.im2[i];
+  }
+  return t;
+}
+__constant__ ModTables kTab = make_tables();
+
+// ---------------------------------------------------------------------------
+// Operands
+// ---------------------------------------------------------------------------
+// One side of the product: `lines` rows of op(A) or columns of op(B), each of K elements.
+struct ModOperand {
+  const double2* X;
+  int64_t ld;
+  int lines, K;
+  int kcontig;        // element (l, k) at X[k + ld l], else at X[l + ld k]
+  int conj;
+  int8_t* planes;     // NPL planes of lines x Kp
+  int64_t Kp;
+  double* part;       // per K chunk and line: sum of squares, then max |re|, |im|
+  int nchunk, kchunk;
+  int* expo;          // per line: the scale's exponent
+  int nblocks_norm, nblocks_split;
+};
+
+__device__ __forceinline__ double2 load_elem(const ModOperand& o, int l, int k) {
+  double2 v = o.kcontig ? o.X[k + o.ld * l] : o.X[l + o.ld * k];
+  if (o.conj) v.y = -v.y;
+  return v;
+}
+
+// Partial sums of squares and maxima of every line over the K chunks (a fixed order, so
+// that the scales do not depend on timing).  Blocks [0, a.nblocks_norm) serve a.
+__global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const ModOperand b) {
+  __shared__ double ss[4][64], sm[4][64];
+  const bool first = (int)blockIdx.x < a.nblocks_norm;
+  const ModOperand& o = first ? a : b;
+  const int blk = first ? blockIdx.x : blockIdx.x - a.nblocks_norm;
+  const int chunk = blk % o.nchunk, grp = blk / o.nchunk;
+  const int k0 = chunk * o.kchunk, k1 = min(o.K, k0 + o.kchunk);
+  double* psum = o.part + (int64_t)chunk * o.lines;
+  double* pmax = o.part + (int64_t)(o.nchunk + chunk) * o.lines;
+  double s = 0.0, m = 0.0;
+  auto add = [&](double2 v) {
+    s = fma(v.x, v.x, fma(v.y, v.y, s));
+    m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
+  };
+  if (o.kcontig) {
+    // eight lanes a line, 32 lines a block
+    const int l = grp * 32 + (threadIdx.x >> 3);
+    if (l < o.lines)
+      for (int k = k0 + (threadIdx.x & 7); k < k1; k += 8) add(o.X[k + o.ld * l]);
+#pragma unroll
+    for (int d = 4; d >= 1; d >>= 1) {
+      s += __shfl_xor_sync(0xffffffffu, s, d);
+      m = fmax(m, __shfl_xor_sync(0xffffffffu, m, d));
+    }
+    if (l < o.lines && (threadIdx.x & 7) == 0) {
+      psum[l] = s;
+      pmax[l] = m;
+    }
+  } else {
+    const int tl = threadIdx.x & 63, tk = threadIdx.x >> 6, l = grp * 64 + tl;
+    if (l < o.lines)
+      for (int k = k0 + tk; k < k1; k += 4) add(o.X[l + o.ld * k]);
+    ss[tk][tl] = s;
+    sm[tk][tl] = m;
+    __syncthreads();
+    if (tk == 0 && l < o.lines) {
+      psum[l] = (ss[0][tl] + ss[1][tl]) + (ss[2][tl] + ss[3][tl]);
+      pmax[l] = fmax(fmax(sm[0][tl], sm[1][tl]), fmax(sm[2][tl], sm[3][tl]));
+    }
+  }
+}
+
+// 2^e in the double range
+__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+
+// The scale exponent of a line: x 2^e rounds to integers of 2-norm <= 2^58 (the rounding
+// adds at most sqrt(K / 2), far below the 2^0.6 that 2^116 leaves under P / 2).
+__device__ int line_exponent(const ModOperand& o, int l) {
+  double s = 0.0, m = 0.0;
+  for (int c = 0; c < o.nchunk; ++c) {
+    s += o.part[(int64_t)c * o.lines + l];
+    m = fmax(m, o.part[(int64_t)(o.nchunk + c) * o.lines + l]);
+  }
+  // a NaN does not pass fmax but does reach the sum of squares
+  if (isnan(s) || isinf(m)) return EXP_NONFINITE;
+  if (m == 0.0) return 0;
+  int e;
+  if (s > 1e-280 && s < 1e280) {
+    frexp(sqrt(s) * (1.0 + 1e-12), &e);
+  } else {  // squares that left the range: bound the norm by the largest element
+    int e2;
+    frexp(m, &e);
+    frexp(sqrt(2.0 * o.K), &e2);
+    e += e2;
+  }
+  return BETA_BITS - e;
+}
+
+__device__ __forceinline__ int dp4a_us(unsigned a, int b, int c) {
+  int d;
+  asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+// The residue of s mod p nearest zero (in [-p/2 - 1, p/2 + 1]) in the low byte of the
+// result; sb = s + kMagicBits, |s| < 2^22.  (kMagicBits is 0 mod 256, so it needs no care.)
+__device__ __forceinline__ int mod_byte(int sb, int p, float inv) {
+  const float f = __int_as_float(sb) - 12582912.0f;
+  return sb - __float_as_int(fmaf(f, inv, 12582912.0f)) * p;
+}
+// low bytes of four words
+__device__ __forceinline__ unsigned pack4(int r0, int r1, int r2, int r3) {
+  return __byte_perm(__byte_perm(r0, r1, 0x0040), __byte_perm(r2, r3, 0x0040), 0x5410);
+}
+
+// Residue planes.  A block covers 32 lines x 64 k of the padded extent, transposed through
+// shared memory; a thread turns 8 consecutive k of a line into 8 bytes of each plane.
+// Bound by its integer instructions (about 300 a complex element) and the 32 plane bytes.
+__global__ void __launch_bounds__(256, 4) k_mod_split(const ModOperand a, const ModOperand b) {
+  __shared__ double2 tile[32][65];
+  __shared__ int ex[32];
+  const bool first = (int)blockIdx.x < a.nblocks_split;
+  const ModOperand& o = first ? a : b;
+  const int blk = first ? blockIdx.x : blockIdx.x - a.nblocks_split;
+  const int nk = (int)(o.Kp / 64);
+  const int k0 = (blk % nk) * 64, l0 = (blk / nk) * 32;
+  const int tid = threadIdx.x;
+  if (tid < 32) {
+    const int e = l0 + tid < o.lines ? line_exponent(o, l0 + tid) : 0;
+    ex[tid] = e == EXP_NONFINITE ? 0 : e;
+    if (k0 == 0 && l0 + tid < o.lines) o.expo[l0 + tid] = e;
+  }
+  if (o.kcontig) {
+    const int kx = tid & 63, ly = tid >> 6;
+#pragma unroll
+    for (int r = 0; r < 32; r += 4) {
+      const int l = l0 + r + ly, k = k0 + kx;
+      tile[r + ly][kx] = (l < o.lines && k < o.K) ? o.X[k + o.ld * l] : make_double2(0.0, 0.0);
+    }
+  } else {
+    const int lx = tid & 31, ky = tid >> 5;
+#pragma unroll
+    for (int r = 0; r < 64; r += 8) {
+      const int l = l0 + lx, k = k0 + r + ky;
+      tile[lx][r + ky] = (l < o.lines && k < o.K) ? o.X[l + o.ld * k] : make_double2(0.0, 0.0);
+    }
+  }
+  __syncthreads();
+  const int ll = tid >> 3, kq = tid & 7;
+  if (l0 + ll >= o.lines) return;
+  const int e = ex[ll], eh = e / 2;
+  const double s1 = pow2(eh), s2 = pow2(e - eh);
+  unsigned xlo[8], xhi[8], ylo[8], yhi[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const double2 v = tile[ll][8 * kq + c];
+    const unsigned long long nx = (unsigned long long)__double2ll_rn(v.x * s1 * s2) + (1ull << 62);
+    const unsigned long long ny = (unsigned long long)__double2ll_rn((o.conj ? -v.y : v.y) * s1 * s2) + (1ull << 62);
+    xlo[c] = (unsigned)nx;
+    xhi[c] = (unsigned)(nx >> 32);
+    ylo[c] = (unsigned)ny;
+    yhi[c] = (unsigned)(ny >> 32);
+  }
+  int8_t* out = o.planes + (int64_t)(l0 + ll) * o.Kp + k0 + 8 * kq;
+  const int64_t plane = (int64_t)o.lines * o.Kp;
+#pragma unroll
+  for (int i = 0; i < NMOD; ++i) {
+    int u[8], v[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const int sx = dp4a_us(xhi[c], kTab.wa_hi[i], dp4a_us(xlo[c], kTab.wa_lo[i], kTab.off_u[i]));
+      const int sy = dp4a_us(yhi[c], kTab.wb_hi[i], dp4a_us(ylo[c], kTab.wb_lo[i], 0));
+      u[c] = mod_byte(sx + sy, kTab.p[i], kTab.inv[i]);
+      v[c] = mod_byte(sx - sy + kTab.off_v[i], kTab.p[i], kTab.inv[i]);
+    }
+    *reinterpret_cast<uint2*>(out + plane * i) =
+        make_uint2(pack4(u[0], u[1], u[2], u[3]), pack4(u[4], u[5], u[6], u[7]));
+    *reinterpret_cast<uint2*>(out + plane * (NMOD + i)) =
+        make_uint2(pack4(v[0], v[1], v[2], v[3]), pack4(v[4], v[5], v[6], v[7]));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// The int8 GEMMs: CTA pairs (cta_group::2) on 256 x 256 tiles
+// ---------------------------------------------------------------------------
+// A tile's A rows and B rows are split over the two CTAs (128 each), so a K stage of 128
+// bytes brings 32 KB into each SM for 2 x 128 x 256 x 128 multiply-adds: 64 bytes a clock at
+// the full int8 rate, half of what 128 x 128 tiles of single CTAs need from L2.  Warp 0
+// loads (TMA, no multicast; both CTAs' bytes arrive at the leader's barrier), warp 1 of the
+// leader issues the MMAs and warps 2-17 of both reduce the int32 sums modulo p and write
+// them as bytes (blocks of 16 columns, so that a warp's rows are contiguous) while the next
+// tile's MMAs run into the other TMEM buffer.
+constexpr int GT = 256;                    // tile rows and columns
+constexpr int HALF = 128;                  // rows of A and of B in each CTA
+constexpr int GKB = 128;                   // K bytes a stage
+constexpr int GSTAGES = 6;
+constexpr int GSTAGE_BYTES = 2 * HALF * GKB;
+constexpr int GBUF = 2;
+constexpr int GEPI = 16;
+constexpr int GTHREADS = 32 * (2 + GEPI);
+constexpr int GSMEM = GSTAGES * GSTAGE_BYTES + 1024 + 512;
+constexpr long long GDRAIN = 2000000000LL;
+
+struct ModGemmArgs {
+  int num_m, num_n, kblocks;
+  int M;                // rows written
+  int64_t ldo;          // columns of the output planes (a multiple of 32, >= N)
+  uint8_t* out;         // NPL planes of ldo / 16 column blocks of M rows of 16 bytes
+  int* err;
+  long long wait_cycles;
+};
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
+}
+__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// bounded: false (and the error flag raised) after `limit` cycles
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* err, long long limit) {
+  if (mbar_try(bar, parity)) return true;
+  const long long t0 = clock64();
+  unsigned spins = 0;
+  while (!mbar_try(bar, parity)) {
+    ++spins;
+    if (spins != 1u && (spins & 255u) != 0u) continue;
+    if (spins != 1u && *err) return false;
+    if (clock64() - t0 > limit) {
+      atomicExch((int*)err, 1);
+      return false;
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+  const long long t0 = clock64();
+  while (!mbar_try(bar, parity) && clock64() - t0 < GDRAIN) {
+  }
+}
+// the leader's copy of a barrier, as a shared::cluster address
+__device__ __forceinline__ uint32_t leader_addr(const void* p) {
+  uint32_t a;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(smem_u32(p)));
+  return a;
+}
+__device__ __forceinline__ void tma_load_pair(void* dst, const CUtensorMap* map, uint32_t bar, int x, int y, int z) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(dst)),
+      "l"(map), "r"(bar), "r"(x), "r"(y), "r"(z)
+      : "memory");
+}
+// K-major shared-memory descriptor, 128B swizzle, 8-row groups 1024 B apart
+__device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+  d |= (uint64_t)1 << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
+// kind::i8: s32 = s8 x s8, both K-major, M = N = 256 over the pair
+constexpr uint32_t GIDESC = (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(GT >> 3) << 17) | ((uint32_t)(GT >> 4) << 24);
+
+__device__ __forceinline__ void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+      " tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+      "l"(a), "l"(b), "r"(GIDESC), "r"(acc));
+}
+// arrives at the barrier of both CTAs when the MMAs issued so far have retired
+__device__ __forceinline__ void commit_pair(uint64_t* bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
+          smem_u32(bar)),
+      "h"((uint16_t)3)
+      : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+        "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+      : "r"(taddr));
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GTHREADS, 1)
+    k_mod_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, const ModGemmArgs g) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + GSTAGES * GSTAGE_BYTES);
+  uint64_t* full = bars;                               // leader: both CTAs' bytes of a stage
+  uint64_t* empty = bars + GSTAGES;                    // each CTA: the stage's MMAs have retired
+  uint64_t* tfull = bars + 2 * GSTAGES;                // each CTA: a tile's sums are in TMEM
+  uint64_t* tempty = bars + 2 * GSTAGES + GBUF;        // leader: both CTAs have read them
+  uint64_t* drain = bars + 2 * GSTAGES + 2 * GBUF;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * GSTAGES + 2 * GBUF + 1);
+  volatile int* err = g.err;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < GSTAGES; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    for (int b = 0; b < GBUF; ++b) {
+      mbar_init(&tfull[b], 1);
+      mbar_init(&tempty[b], 2 * GEPI);
+    }
+    mbar_init(drain, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(tmem_slot)));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_sync();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  const int per = g.num_m * g.num_n, ntiles = per * NPL;
+  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      int issued[GSTAGES];
+      for (int s = 0; s < GSTAGES; ++s) issued[s] = -1;
+      for (int t = pair; t < ntiles && ok; t += npairs) {
+        const int pl = t / per, mb = (t % per) % g.num_m, nb = (t % per) / g.num_m;
+        for (int kb = 0; kb < g.kblocks && ok; ++kb) {
+          ok = mbar_wait(&empty[stage], phase ^ 1, err, g.wait_cycles);
+          if (!ok) break;
+          uint8_t* base = smem + stage * GSTAGE_BYTES;
+          if (rank == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&full[stage])),
+                         "r"((uint32_t)(2 * GSTAGE_BYTES))
+                         : "memory");
+          const uint32_t bar = leader_addr(&full[stage]);
+          tma_load_pair(base, &mapA, bar, kb * GKB, mb * GT + (int)rank * HALF, pl);
+          tma_load_pair(base + HALF * GKB, &mapB, bar, kb * GKB, nb * GT + (int)rank * HALF, pl);
+          issued[stage] = (int)phase;
+          if (++stage == GSTAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+      // both CTAs' copies must land before either leaves (the leader's barriers count both;
+      // the cluster barrier at the end holds the other CTA until then)
+      if (rank == 0)
+        for (int s = 0; s < GSTAGES; ++s)
+          if (issued[s] >= 0) mbar_drain(&full[s], (uint32_t)issued[s]);
+    }
+  } else if (warp == 1) {
+    if (rank == 0 && lane == 0) {
+      int stage = 0, n = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int t = pair; t < ntiles && ok; t += npairs, ++n) {
+        const int buf = n % GBUF;
+        ok = mbar_wait(&tempty[buf], ((n / GBUF) & 1) ^ 1, err, g.wait_cycles);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        for (int kb = 0; kb < g.kblocks && ok; ++kb) {
+          ok = mbar_wait(&full[stage], phase, err, g.wait_cycles);
+          if (!ok) break;
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          const uint32_t a0 = smem_u32(smem + stage * GSTAGE_BYTES);
+          const uint64_t da = make_desc(a0), db = make_desc(a0 + HALF * GKB);
+#pragma unroll
+          for (int kk = 0; kk < GKB / 32; ++kk)
+            mma_pair(tmem + (uint32_t)(buf * GT), da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2),
+                     (kb == 0 && kk == 0) ? 0u : 1u);
+          commit_pair(&empty[stage]);
+          if (++stage == GSTAGES) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        if (!ok) break;
+        commit_pair(&tfull[buf]);
+      }
+      commit_pair(drain);
+      mbar_drain(drain, 0);
+    }
+  } else {
+    constexpr int ECOLS = GT / (GEPI / 4);   // columns of a warp
+    const int q = warp & 3, h = (warp - 2) / 4;
+    int n = 0;
+    for (int t = pair; t < ntiles; t += npairs, ++n) {
+      const int pl = t / per, mb = (t % per) % g.num_m, nb = (t % per) / g.num_m;
+      const int mi = pl % NMOD;
+      const int p = kTab.p[mi], wgt = kTab.wa_lo[mi], off = kTab.off_s[mi];
+      const float inv = kTab.inv[mi];
+      const int buf = n % GBUF;
+      if (!mbar_wait(&tfull[buf], (n / GBUF) & 1, err, g.wait_cycles)) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const int row = mb * GT + (int)rank * HALF + q * 32 + lane;
+      uint8_t* orow = g.out + (int64_t)pl * g.M * g.ldo + (int64_t)row * 16;
+#pragma unroll 1
+      for (int ch = 0; ch < ECOLS / 32; ++ch) {
+        uint32_t r[32];
+        tmem_ld32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * GT + h * ECOLS + ch * 32), r);
+        if (ch == ECOLS / 32 - 1) {
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_addr(&tempty[buf]))
+                         : "memory");
+        }
+        const int col = nb * GT + h * ECOLS + ch * 32;
+        if (row < g.M && col < g.ldo) {
+          uint32_t w[8];
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            r[j] = (uint32_t)mod_byte(dp4a_us(r[j] ^ 0x80000000u, wgt, off), p, inv);
+#pragma unroll
+          for (int j = 0; j < 8; ++j)   // stored with an offset of 128
+            w[j] = pack4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]) ^ 0x80808080u;
+          uint8_t* o = orow + (int64_t)col * g.M;   // column block col / 16
+          *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
+          *reinterpret_cast<uint4*>(o + (int64_t)16 * g.M) = make_uint4(w[4], w[5], w[6], w[7]);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  // no CTA leaves, and no TMEM is released, while the pair's MMAs or copies are in flight
+  cluster_sync();
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem));
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Reconstruction
+// ---------------------------------------------------------------------------
+struct ModJoinArgs {
+  int M, N, K;
+  int64_t ldo;
+  const uint8_t* res;
+  const int* ea;
+  const int* eb;
+  double2 alpha, beta;
+  double2* C;
+  int64_t ldc;
+};
+
+// A block joins a 64 x 16 tile of C: a thread reads 4 columns of a row from the 32 planes
+// and sums the CRT fractions of its 4 elements, modulo 1 in 32-bit integers for their
+// leading bits, in FP64 below; the tile goes through shared memory so that C is written
+// along its columns.  The stored bytes are residues + 128, so u + v and u - v + 256 exceed
+// the sums meant by 256 each, which the accumulators' starting values take out.  Per
+// element: 32 integer and 32 double multiply-adds, 32 conversions by exponent trick and
+// 48 bytes of memory traffic.
+template <bool BETA>
+__global__ void __launch_bounds__(256, 3) k_mod_join(const ModJoinArgs g, const ModOperand a, const ModOperand b) {
+  __shared__ double2 tile[16][65];
+  const int tid = threadIdx.x;
+  const int r = tid >> 2, c4 = (tid & 3) * 4;
+  const int m0 = blockIdx.x * 64, n0 = blockIdx.y * 16;
+  const int row = m0 + r;
+  if (row < g.M) {
+    const uint8_t* src = g.res + (int64_t)n0 * g.M + (int64_t)row * 16 + c4;
+    const int64_t plane = (int64_t)g.M * g.ldo;
+    unsigned x1[4], y1[4];
+    double x2[4], y2[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      x1[e] = kTab.re1_0;
+      y1[e] = kTab.im1_0;
+      x2[e] = kTab.re2_0;
+      y2[e] = kTab.im2_0;
+    }
+    // all 32 loads in flight before the first use
+    unsigned wu[NMOD], wv[NMOD];
+#pragma unroll
+    for (int i = 0; i < NMOD; ++i) {
+      wu[i] = __ldcs(reinterpret_cast<const unsigned*>(src + plane * i));
+      wv[i] = __ldcs(reinterpret_cast<const unsigned*>(src + plane * (NMOD + i)));
+    }
+#pragma unroll
+    for (int i = 0; i < NMOD; ++i) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const unsigned u = __byte_perm(wu[i], 0, 0x4440 + e), v = __byte_perm(wv[i], 0, 0x4440 + e);
+        const unsigned sp = u + v, sm = u - v + 256u;
+        x1[e] += sp * kTab.re1[i];
+        y1[e] += sm * kTab.im1[i];
+        x2[e] = fma(__hiloint2double(0x43300000, (int)sp) - 4503599627370496.0, kTab.re2[i], x2[e]);
+        y2[e] = fma(__hiloint2double(0x43300000, (int)sm) - 4503599627370496.0, kTab.im2[i], y2[e]);
+      }
+    }
+    const int ea = g.ea[row];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int col = n0 + c4 + e;
+      if (col >= g.N) continue;
+      const int eb = g.eb[col];
+      double2 v;
+      if (ea == EXP_NONFINITE || eb == EXP_NONFINITE) {
+        v = make_double2(0.0, 0.0);
+        for (int k = 0; k < g.K; ++k) {
+          const double2 x = load_elem(a, row, k), y = load_elem(b, col, k);
+          v.x = fma(-x.y, y.y, fma(x.x, y.x, v.x));
+          v.y = fma(x.y, y.x, fma(x.x, y.y, v.y));
+        }
+      } else {
+        const int t = max(-(ea + eb), -2000), th = t / 2;
+        const double s1 = pow2(th), s2 = pow2(t - th);
+        v.x = fma((double)(int)x1[e], 0x1p-32, x2[e]) * kTab.P * s1 * s2;
+        v.y = fma((double)(int)y1[e], 0x1p-32, y2[e]) * kTab.P * s1 * s2;
+      }
+      tile[c4 + e][r] = v;
+    }
+  }
+  __syncthreads();
+  const int tr = tid & 63;
+  if (m0 + tr >= g.M) return;
+#pragma unroll
+  for (int c = tid >> 6; c < 16; c += 4) {
+    if (n0 + c >= g.N) break;
+    const double2 v = tile[c][tr];
+    double2 o = make_double2(g.alpha.x * v.x - g.alpha.y * v.y, g.alpha.x * v.y + g.alpha.y * v.x);
+    double2* p = g.C + (m0 + tr) + g.ldc * (int64_t)(n0 + c);
+    if (BETA) {
+      const double2 z = *p;
+      o.x += g.beta.x * z.x - g.beta.y * z.y;
+      o.y += g.beta.x * z.y + g.beta.y * z.x;
+    }
+    *p = o;
+  }
+}
+
+int64_t up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
+
+}  // namespace
+
+bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha, const dcplx* A, int64_t lda,
+                   const dcplx* B, int64_t ldb, cplx beta, dcplx* C, int64_t ldc, double t_fp64) {
+  // int32 sums of K products of residues <= 122 stay below 2^31; the planes within 2 GiB a side
+  if (M < 64 || N < 64 || K < 64 || K > 131072) return false;
+  // Modelled times in us, fitted to both engines on a B200: 16 for the four launches, the
+  // operands' and outputs' elements, and the waves of tiles (2.7 of epilogue at least).  The
+  // lines cross near 0.6 GFLOP for square products (256 x 1024 x 256: 29 here and there;
+  // 502 x 251 x 1255: 41 against 55 on the FP64 tensor cores, 1255 x 502 x 251: 46 against
+  // 63) and far later for a short K, whose outputs dominate (4096 x 960 x 64: 165 against 75).
+  const int64_t tiles = (int64_t)((M + GT - 1) / GT) * ((N + GT - 1) / GT) * NPL, npair = ctx->num_sms / 2;
+  const double t_here = 16.0 + 15.4e-6 * ((double)M + N) * K + 14.8e-6 * M * (double)N +
+                        (double)((tiles + npair - 1) / npair) * std::max(2.7, 3.2 / 1024 * K);
+  if (t_here > 0.9 * t_fp64) return false;
+  if (ctx->capturing()) return false;   // its error flag needs a synchronisation
+  const int64_t Kp = up(K, GKB);
+  const size_t pa = (size_t)NPL * M * Kp, pb = (size_t)NPL * N * Kp;
+  if (pa > ((size_t)2 << 30) || pb > ((size_t)2 << 30)) return false;
+  // the output's residues of one column panel within 1 GiB (panels that stay in L2 were no
+  // faster: 1.47 ms against 1.21 ms for 6144 x 4096 x 1024, the GEMMs' last waves)
+  int64_t np = ((int64_t)1 << 30) / ((int64_t)NPL * M) / GT * GT;
+  if (np < GT) return false;
+  np = std::min<int64_t>(np, N);
+  const int64_t ldo = up(np, 32);
+  const size_t pc = (size_t)NPL * M * ldo;
+  const int nchunk = std::max(1, std::min(16, K / 64));
+  const size_t tail = (size_t)(M + N) * (2 * nchunk * sizeof(double) + sizeof(int));
+  auto at = [](size_t x) { return (x + 1023) / 1024 * 1024; };
+  uint8_t* base = static_cast<uint8_t*>(ctx->optional_buf("gemm_modular", at(pa) + at(pb) + at(pc) + tail + 4096));
+  if (!base) return false;
+  int8_t* planesA = reinterpret_cast<int8_t*>(base);
+  int8_t* planesB = reinterpret_cast<int8_t*>(base + at(pa));
+  uint8_t* res = base + at(pa) + at(pb);
+  double* part = reinterpret_cast<double*>(res + at(pc));
+  int* expo = reinterpret_cast<int*>(part + (size_t)(M + N) * 2 * nchunk);
+
+  ModOperand a{}, b{};
+  a.X = A;
+  a.ld = lda;
+  a.lines = M;
+  a.kcontig = opA != OP_N;
+  a.conj = opA == OP_C;
+  a.planes = planesA;
+  a.part = part;
+  a.expo = expo;
+  b.X = B;
+  b.ld = ldb;
+  b.lines = N;
+  b.kcontig = opB == OP_N;
+  b.conj = opB == OP_C;
+  b.planes = planesB;
+  b.part = part + (size_t)M * 2 * nchunk;
+  b.expo = expo + M;
+  for (ModOperand* o : {&a, &b}) {
+    o->K = K;
+    o->Kp = Kp;
+    o->nchunk = nchunk;
+    o->kchunk = (K + nchunk - 1) / nchunk;
+    o->nblocks_norm = (o->lines + (o->kcontig ? 31 : 63)) / (o->kcontig ? 32 : 64) * nchunk;
+    o->nblocks_split = (int)(Kp / 64) * ((o->lines + 31) / 32);
+  }
+  ScopedTimer tm(ctx, "zgemm_modular", 8.0 * M * (double)N * K);
+  k_mod_norms<<<a.nblocks_norm + b.nblocks_norm, 256, 0, ctx->stream>>>(a, b);
+  k_mod_split<<<a.nblocks_split + b.nblocks_split, 256, 0, ctx->stream>>>(a, b);
+  static DeviceOnce attr;
+  attr.run(ctx->device, [] {
+    IMPS_CUDA(cudaFuncSetAttribute(k_mod_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, GSMEM));
+  });
+  const CUtensorMap mapA = plane_map(planesA, Kp, M, NPL, GKB, HALF);
+  ctx->n_kernels += 2;
+  for (int64_t n0 = 0; n0 < N; n0 += np) {
+    const int nn = (int)std::min<int64_t>(np, N - n0);
+    const CUtensorMap mapB = plane_map(planesB + n0 * Kp, Kp, nn, NPL, GKB, HALF, (int64_t)N * Kp);
+    ModGemmArgs g;
+    g.num_m = (M + GT - 1) / GT;
+    g.num_n = (nn + GT - 1) / GT;
+    g.kblocks = (int)(Kp / GKB);
+    g.M = M;
+    g.ldo = ldo;
+    g.out = res;
+    g.err = ctx->err_dev;
+    g.wait_cycles = ctx->wait_cycles;
+    const int pairs = std::min(g.num_m * g.num_n * NPL, ctx->num_sms / 2);
+    k_mod_gemm<<<2 * pairs, GTHREADS, GSMEM, ctx->stream>>>(mapA, mapB, g);
+    ModJoinArgs j;
+    j.M = M;
+    j.N = nn;
+    j.K = K;
+    j.ldo = ldo;
+    j.res = res;
+    j.ea = a.expo;
+    j.eb = b.expo + n0;
+    j.alpha = make_double2(alpha.real(), alpha.imag());
+    j.beta = make_double2(beta.real(), beta.imag());
+    j.C = C + ldc * n0;
+    j.ldc = ldc;
+    ModOperand bj = b;
+    bj.X = b.kcontig ? B + ldb * n0 : B + n0;
+    const dim3 grid((M + 63) / 64, (nn + 15) / 16);
+    if (beta != cplx(0.0, 0.0)) k_mod_join<true><<<grid, 256, 0, ctx->stream>>>(j, a, bj);
+    else k_mod_join<false><<<grid, 256, 0, ctx->stream>>>(j, a, bj);
+    ctx->n_kernels += 2;
+  }
+  IMPS_CUDA(cudaPeekAtLastError());
+  ctx->n_gemm++;
+  ctx->err_armed = true;   // the bounded waits' flag is read at the next synchronisation
+  return true;
+}
+
+}  // namespace imps

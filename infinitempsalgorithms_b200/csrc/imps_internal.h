@@ -167,6 +167,12 @@ struct Context {
     }
     return b;
   }
+  // Whether FP64 sums keep one order (k ascending) whatever the grid.  The split engine
+  // truncates its operands at 2^-7s of a line's scale, so in split mode a last-bit change of
+  // FP64 data moves a truncation and with it the result by that much (the first iteration of
+  // a Hubbard D = 384 run by 5e-2 at its solver tolerances; 1e-11 in FP64 mode): a split-mode
+  // trajectory keeps the plain order, so that it does not depend on how a product was cut up.
+  bool ordered_sums() const { return precision == PREC_SPLIT_I8; }
   // Scratch that only makes a call faster (partial tiles, residue planes): nullptr when it
   // is not to be had -- a workspace cap is set, the call may not allocate, or the device is
   // out of memory -- and the caller then takes its path without it.  Kept between calls;
@@ -176,6 +182,7 @@ struct Context {
   void* optional_buf(const char* name, size_t bytes) {
     if (no_scratch > 0 || workspace_limit > 0) return nullptr;
     DevBuf& b = optional[name];
+    if (bytes > b.bytes && capturing()) return nullptr;   // no allocation inside a graph capture
     try {
       b.ensure(bytes);
     } catch (const Error& e) {
@@ -184,6 +191,13 @@ struct Context {
       return nullptr;
     }
     return b.ptr;
+  }
+  // whether the stream's work is being captured into a graph (also when that cannot be told)
+  bool capturing() const {
+    cudaStreamCaptureStatus st;
+    if (cudaStreamIsCapturing(stream, &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
   }
   void release_optional() {
     cudaStreamSynchronize(stream);

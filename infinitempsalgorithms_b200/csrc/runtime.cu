@@ -476,7 +476,7 @@ static void err_after_sync(Context* ctx) {
   if (ctx->err_host[0] != 0) {
     ctx->err_host[0] = 0;
     IMPS_CUDA(cudaMemsetAsync(ctx->err_dev, 0, sizeof(int), ctx->stream));
-    throw Error(IMPS_TIMEOUT, "a bounded device wait of the split GEMM pipeline ran out");
+    throw Error(IMPS_TIMEOUT, "a bounded device wait of a GEMM pipeline ran out");
   }
 }
 void check_device_errors(Context* ctx) {

@@ -1,5 +1,7 @@
 // int8 split-precision complex GEMM on tcgen05 (see gemm_i8.cu).
 #pragma once
+#include <cuda.h>
+
 #include "imps_internal.h"
 
 namespace imps {
@@ -23,6 +25,11 @@ void split_operand_b(Context* ctx, SplitOperand& S, Op op, int K, int N, const d
 // C (complex, ldc) = alpha * op(A) op(B) (+ C when accumulate) using `s` slice diagonals
 void split_gemm(Context* ctx, const SplitOperand& A, const SplitOperand& B, int s, double alpha, bool accumulate,
                 dcplx* C, int64_t ldc);
+
+// 3D tensor map over int8 planes (Kp bytes, rows, planes), box (box_k, box_rows, 1), swizzled
+// over box_k = 64 or 128 bytes; plane_bytes: stride of the planes, 0 for rows x Kp
+CUtensorMap plane_map(const int8_t* base, int64_t Kp, int64_t rows, int planes, int box_k, int box_rows,
+                      int64_t plane_bytes = 0);
 
 // Slices needed for a requested relative accuracy `tol` (clamped to 2..8).
 int slices_for_tol(double tol);

@@ -5,6 +5,7 @@
 // accumulators per thread (strided by 16 so shared-memory reads of a warp hit
 // consecutive addresses), K tile of 8 staged through shared memory with a
 // register prefetch of the next tile.  Each complex MAC is 4 DFMA.
+#include "gemm_modular.h"
 #include "imps_internal.h"
 #include "split_gemm.h"
 
@@ -356,7 +357,12 @@ void launch_dmma(Context* ctx, int nsplit, double2* part, int M, int N, int K, d
 // grid.  Measured on a B200: a K stage of one CTA takes 3.3 us alone on its SM and 2.46 us
 // of the SM when others run beside it; the partial products cost one more launch (4 us) and
 // their bytes at 3 TB/s.
-int split_k(const Context* ctx, int64_t tiles, int K) {
+struct SplitK {
+  int n;       // CTAs per tile
+  double us;   // modelled time of the product
+};
+SplitK split_k(const Context* ctx, int M, int N, int K, int batch) {
+  const int64_t tiles = (int64_t)((M + dm::BM - 1) / dm::BM) * ((N + dm::BN - 1) / dm::BN) * batch;
   const int kall = (K + dm::BK - 1) / dm::BK;
   int best = 1;
   double tbest = 1e300;
@@ -369,7 +375,7 @@ int split_k(const Context* ctx, int64_t tiles, int K) {
       best = s;
     }
   }
-  return best;
+  return {best, tbest};
 }
 
 template <int OPA, int OPB>
@@ -389,8 +395,7 @@ void launch(Context* ctx, int M, int N, int K, double2 alpha, const dcplx* A, in
     constexpr bool BETA = decltype(beta_tag)::value;
     // the K stages of a tile are shared by several CTAs where the tiles alone would leave
     // SMs idle (the long-K products of the pushes and of the QR, every product of a small state)
-    const int64_t tiles = (int64_t)((M + dm::BM - 1) / dm::BM) * ((N + dm::BN - 1) / dm::BN) * batch;
-    const int s = split_k(ctx, tiles, K);
+    const int s = ctx->ordered_sums() ? 1 : split_k(ctx, M, N, K, batch).n;
     const int64_t len = (int64_t)M * N;
     double2* part = nullptr;
     if (s > 1) part = static_cast<double2*>(ctx->optional_buf("gemm_part", (size_t)len * s * batch * sizeof(double2)));
@@ -425,6 +430,10 @@ void zgemm_fp64(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha, c
     }
     return;
   }
+  // products large enough: residue arithmetic on the int8 tensor cores
+  if (batch == 1 && ctx->fp64_engine == 0 && !ctx->ordered_sums() &&
+      zgemm_modular(ctx, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, split_k(ctx, M, N, K, 1).us))
+    return;
   double2 a = make_double2(alpha.real(), alpha.imag()), bt = make_double2(beta.real(), beta.imag());
   bool use_beta = beta != cplx(0.0, 0.0);
   ScopedTimer t(ctx, "zgemm_fp64", 8.0 * M * (double)N * K * batch);
