@@ -9,10 +9,9 @@
 // the final phase fix Q[:, i] *= ph_i, R[i, :] *= conj(ph_i), ph_i = R_ii / |R_ii|.
 //
 // Two-level blocked right-looking algorithm:
-//  * k_qr_panel: one thread-block cluster of QR_CL CTAs factors the panel
-//    A[p:m, p:p+b] (b <= 16), the panel rows staged in shared memory.  Per column a
-//    single cluster reduction (distributed shared memory after one cluster barrier)
-//    gives ||x||^2, the inner products with the trailing panel columns and those with
+//  * k_qr_panel: one CTA or thread-block cluster (up to QR_CL CTAs, by the rows) factors
+//    the panel A[p:m, p:p+b] (b <= 16), the panel rows held in registers.  Per column a
+//    single reduction (distributed shared memory after one cluster barrier) gives ||x||^2, the inner products with the trailing panel columns and those with
 //    the earlier reflectors needed for the compact-WY factor T (LAPACK zlarft,
 //    T[0:c, c] = -tau_c T[0:c, 0:c] V^H v_c).  The kernel writes R (upper part of A),
 //    V (explicit, unit diagonal, zeros above), tau and T.
@@ -34,12 +33,11 @@ void scale_q_r(Context* ctx, int m, int n, int k, dcplx* Q, int64_t ldq, dcplx* 
 
 namespace {
 
-constexpr int QR_CL = 8;     // CTAs per cluster (portable cluster size)
+constexpr int QR_CL = 8;     // most CTAs per cluster (portable cluster size)
 constexpr int QR_NT = 512;   // threads per CTA
 constexpr int QR_G = QR_CL * QR_NT;
 constexpr int QR_NBMAX = 16;
 constexpr int QR_NBO = 64;   // outer block: columns per compact-WY trailing update
-constexpr size_t QR_PANEL_SMEM = (size_t)QR_NBMAX * QR_NT * sizeof(dcplx);  // NB RPT = 16 for every panel kind
 constexpr int QR_MAXCHUNK = 32;  // most row chunks of a split-K X^H V product
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
@@ -95,179 +93,274 @@ __device__ __forceinline__ double warp_reduce_scatter(double (&val)[NV], int lan
   return r;
 }
 
-// Householder factorization of the panel A[0:R, 0:b] (lda), b <= NB.  Row il of the
-// panel belongs to cluster thread g = rank * QR_NT + tid with il = g + k QR_G, k < RPT,
-// and lives in shared memory (NB RPT QR_NT complex = 128 KiB per CTA).
-// One cluster reduction per column: ||x_c below||^2, d_j = x_c^H x_j (j > c, trailing
-// panel columns) and e_l = V_l^H x_c (l < c, for T), all over the rows below c, together
-// with row c of the panel (held by thread c of CTA 0).  With v = [1; scale x_c below]:
+// Householder factorization of the panel A[0:R, 0:b] (lda), b <= NB, by a cluster of CL
+// CTAs of NT threads.  Row il of the panel belongs to cluster thread g = rank * NT + tid with
+// il = g + k CL NT, k < RPT, and lives in that thread's registers (NB RPT = 16 complex).
+// The columns rotate through them: at column c register column q holds panel column
+// (c + q) mod NB, so position 0 is the current one, the next ones the trailing columns and
+// the last c the finished reflectors, and the column loop needs no unrolling.
+// One reduction per column: ||x_c below||^2, d_j = x_c^H x_j (j > c, trailing panel columns)
+// and e_l = V_l^H x_c (l < c, for T), all over the rows below c, together with row c of the
+// panel (held by thread c of CTA 0).  With v = [1; scale x_c below]:
 //   v^H x_j = x_j[c] + conj(scale) d_j,   V_l^H v = conj(V_l[c]) + scale e_l.
+// Warp 0 alone takes the reflector's square root and divisions and the NB - 1 inner
+// products; the last warp extends T while the others update their rows.
+// The sums run over the 16 warps of every 512 rows in order, then over these groups, however
+// the rows are spread (CTAs of fewer threads push their warps' sums themselves), so a
+// panel's result does not depend on CL and NT.
+// Bound by latency: a column costs one CTA of 512 rows about 2.9 us (its instructions about
+// 1.9 us, the rest the reflector's divisions and the barriers), a cluster barrier 0.65 us
+// more; so up to 256 rows take one CTA, more rows eight CTAs of as few threads as hold them.
+// 16 columns of 512 rows: 66 us with eight CTAs of 512 threads and the rows in shared memory,
+// 48 us on one CTA with the rows in registers, 38 us on eight CTAs of 64 threads; 2048 rows
+// 69 us, 58 us (four CTAs of 512) and 45 us (eight of 256).
 // Outputs: A (R above/on the diagonal, v below), V (R x b, ldv: v with unit diagonal and
 // zeros above; the zabove rows before row 0 are zeroed too), tau[0:b], T (b x b, ldt).
-template <int NB, int RPT>
-__global__ void __cluster_dims__(QR_CL, 1, 1) __launch_bounds__(QR_NT, 1)
+template <int NB, int RPT, int CL, int NT>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT, 1)
     k_qr_panel(int R, int b, int zabove, dcplx* __restrict__ A, int64_t lda, dcplx* __restrict__ V, int64_t ldv,
                dcplx* __restrict__ tau, dcplx* __restrict__ T, int ldt) {
-  constexpr int NV = 2 * NB;       // reduction slots: [0] ||x||^2, [1 + 2s, 2 + 2s] complex slot s
-  constexpr int SPL = 32 / NV;     // lanes per slot after the reduce-scatter
-  extern __shared__ dcplx xs[];    // xs[(k NB + j) QR_NT + tid]
-  __shared__ double wsum[QR_NT / 32][NV];
-  __shared__ double red[2][QR_CL][NV];   // partials pushed by every CTA of the cluster
-  __shared__ double rowc[2][2 * NB];     // row c of the panel, pushed by CTA 0
-  __shared__ double fin[NV + 2 * NB];
+  constexpr int NV = 2 * NB;             // reduction slots: [0] ||x||^2, [2q - 1, 2q] position q
+  constexpr int NW = NT / 32;
+  constexpr bool WARPS = CL > 1 && NT < QR_NT;   // the warps' sums travel, not the CTAs'
+  constexpr int NGRP = WARPS ? CL * NT / QR_NT : 1, GW = QR_NT / 32;   // groups of 512 rows, their warps
+  static_assert(!WARPS || CL * NT % QR_NT == 0, "whole groups");
+  constexpr int HV = NV > 16 ? 16 : NV;  // slots reduced at a time (registers)
+  constexpr int SPL = 32 / HV;           // lanes per slot after the reduce-scatter
+  constexpr int G = CL * NT;
+  __shared__ double wsum[NW][NV];
+  __shared__ double red[2][WARPS ? 1 : CL][NV];   // partials pushed by every CTA of the cluster
+  __shared__ double redw[2][NGRP][WARPS ? GW : 1][NV];   // or by every warp
+  __shared__ dcplx rowl[NB];             // row c of the panel, written by its thread
+  __shared__ double rowc[2][2 * NB];     // the same, pushed by CTA 0
+  __shared__ dcplx sc[3];                // conj(tau), scale, beta
+  __shared__ dcplx wv[NB], zs[NB];
   __shared__ dcplx Tsh[NB][NB + 1];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const uint32_t rank = cluster_rank();
-  const int g = (int)rank * QR_NT + tid;
-#define XS(k, j) xs[((k) * NB + (j)) * QR_NT + tid]
+  const uint32_t rank = CL > 1 ? cluster_rank() : 0u;
+  const int g = (int)rank * NT + tid;
 
+  dcplx x[RPT][NB];
 #pragma unroll
   for (int k = 0; k < RPT; ++k) {
-    const int il = g + k * QR_G;
+    const int il = g + k * G;
 #pragma unroll
-    for (int j = 0; j < NB; ++j) XS(k, j) = (il < R && j < b) ? A[il + lda * (int64_t)j] : make_double2(0.0, 0.0);
+    for (int j = 0; j < NB; ++j) x[k][j] = (il < R && j < b) ? A[il + lda * (int64_t)j] : make_double2(0.0, 0.0);
   }
   if (rank == 0)
-    for (int e = tid; e < NB * (NB + 1); e += QR_NT) Tsh[e / (NB + 1)][e % (NB + 1)] = make_double2(0.0, 0.0);
+    for (int e = tid; e < NB * (NB + 1); e += NT) Tsh[e / (NB + 1)][e % (NB + 1)] = make_double2(0.0, 0.0);
 
+#pragma unroll 1
   for (int c = 0; c < b; ++c) {
     const int par = c & 1;
-    double val[NV];
+    const int nt = NB - c;   // positions below nt are trailing columns, the others reflectors
 #pragma unroll
-    for (int s = 0; s < NV; ++s) val[s] = 0.0;
+    for (int h = 0; h < NV / HV; ++h) {
+      double val[HV];
 #pragma unroll
-    for (int k = 0; k < RPT; ++k) {
-      const int il = g + k * QR_G;
-      if (il > c && il < R) {
-        const dcplx xc = XS(k, c);
-        val[0] = fma(xc.x, xc.x, fma(xc.y, xc.y, val[0]));
+      for (int s = 0; s < HV; ++s) val[s] = 0.0;
 #pragma unroll
-        for (int s = 0; s < NB - 1; ++s) {
-          dcplx p = make_double2(0.0, 0.0);
-          if (s < c) p = cmulc(XS(k, s), xc);                // e_s
-          else if (s + 1 < b) p = cmulc(xc, XS(k, s + 1));   // d_{s+1}
-          val[1 + 2 * s] += p.x;
-          val[2 + 2 * s] += p.y;
+      for (int k = 0; k < RPT; ++k) {
+        const int il = g + k * G;
+        if (il > c && il < R) {
+          const dcplx xc = x[k][0];
+          if (h == 0) val[0] = k == 0 ? fma(xc.x, xc.x, xc.y * xc.y) : fma(xc.x, xc.x, fma(xc.y, xc.y, val[0]));
+#pragma unroll
+          for (int s = 0; s < HV; ++s) {
+            const int slot = h * HV + s, q = (slot + 1) >> 1;
+            if (slot == 0) continue;
+            const dcplx y = x[k][q];
+            double p;
+            if (slot & 1) p = fma(xc.x, y.x, xc.y * y.y);
+            else p = q < nt ? fma(xc.x, y.y, -xc.y * y.x) : fma(y.x, xc.y, -y.y * xc.x);
+            val[s] = k == 0 ? p : val[s] + p;
+          }
         }
       }
-    }
-    const double wv = warp_reduce_scatter<NV>(val, lane);
-    if (lane % SPL == 0) wsum[warp][lane / SPL] = wv;
-    __syncthreads();
-    // push this CTA's partials (and, from CTA 0, row c of the panel: thread c's row
-    // in shared memory) into every CTA of the cluster; no remote loads
-    if (tid < NV) {
-      double t = 0.0;
-      for (int q = 0; q < QR_NT / 32; ++q) t += wsum[q][tid];
+      const double wvl = warp_reduce_scatter<HV>(val, lane);
+      if constexpr (WARPS) {
+        // the lanes of a slot share the peers
+        const int wg = (int)rank * NW + warp;
 #pragma unroll
-      for (uint32_t q = 0; q < QR_CL; ++q) st_peer(&red[par][rank][tid], q, t);
-    } else if (rank == 0 && tid < NV + 2 * NB * QR_CL) {
-      const int e = tid - NV, slot = e % (2 * NB), dst = e / (2 * NB);
-      const dcplx x = xs[(slot >> 1) * QR_NT + c];   // XS(0, slot / 2) of thread c
-      st_peer(&rowc[par][slot], (uint32_t)dst, (slot & 1) ? x.y : x.x);
+        for (int q = 0; q < CL; q += SPL)
+          st_peer(&redw[par][wg / GW][wg % GW][h * HV + lane / SPL], (uint32_t)(q + lane % SPL), wvl);
+      } else if (lane % SPL == 0) {
+        wsum[warp][h * HV + lane / SPL] = wvl;
+      }
     }
-    cluster_sync();
-    if (tid < NV) {
-      double t = 0.0;
+    if (rank == 0 && tid == c) {
 #pragma unroll
-      for (int q = 0; q < QR_CL; ++q) t += red[par][q][tid];
-      fin[tid] = t;
-    } else if (tid < NV + 2 * NB) {
-      fin[tid] = rowc[par][tid - NV];
+      for (int q = 0; q < NB; ++q) rowl[q] = x[0][q];
     }
-    __syncthreads();
-    // the reflector (LAPACK zlarfg), computed identically by every thread
-    const double xsq = fin[0];
-    const dcplx al = make_double2(fin[NV + 2 * c], fin[NV + 2 * c + 1]);
-    dcplx tc, scale;
-    double beta;
-    if (xsq == 0.0 && al.y == 0.0) {
-      tc = make_double2(0.0, 0.0);
-      scale = make_double2(0.0, 0.0);
-      beta = al.x;
+    if constexpr (WARPS) {
+      if (rank == 0 && warp == 0) {   // row c to every CTA, a component a lane
+        __syncwarp();
+        if (lane < 2 * NB) {
+          const dcplx y = rowl[lane >> 1];
+#pragma unroll
+          for (uint32_t q = 0; q < CL; ++q) st_peer(&rowc[par][lane], q, (lane & 1) ? y.y : y.x);
+        }
+      }
+      cluster_sync();
     } else {
-      beta = -copysign(sqrt(al.x * al.x + al.y * al.y + xsq), al.x);
-      tc = make_double2((beta - al.x) / beta, -al.y / beta);
-      const double dr = al.x - beta, di = al.y, den = dr * dr + di * di;
-      scale = make_double2(dr / den, -di / den);   // 1 / (alpha - beta)
+      __syncthreads();
     }
-    const dcplx ctc = make_double2(tc.x, -tc.y), cs = make_double2(scale.x, -scale.y);
-    // v into column c, R diagonal, trailing panel columns x_j -= conj(tau) v (v^H x_j)
+    if constexpr (CL > 1 && !WARPS) {
+      // push this CTA's partials (and, from CTA 0, row c) into every CTA; no remote loads
+      if (tid < NV) {
+        double t = 0.0;
+        for (int q = 0; q < NW; ++q) t += wsum[q][tid];
 #pragma unroll
-    for (int k = 0; k < RPT; ++k) {
-      const int il = g + k * QR_G;
-      if (il < c || il >= R) continue;
-      dcplx v;
-      if (il == c) {
-        v = make_double2(1.0, 0.0);
-        XS(k, c) = make_double2(beta, 0.0);
-      } else {
-        v = cmul(XS(k, c), scale);
-        XS(k, c) = v;
+        for (uint32_t q = 0; q < CL; ++q) st_peer(&red[par][rank][tid], q, t);
+      } else if (rank == 0 && tid < NV + 2 * NB * CL) {
+        const int e = tid - NV, slot = e % (2 * NB), dst = e / (2 * NB);
+        const dcplx y = rowl[slot >> 1];
+        st_peer(&rowc[par][slot], (uint32_t)dst, (slot & 1) ? y.y : y.x);
       }
-      const dcplx cv = cmul(ctc, v);
+      cluster_sync();
+    }
+    if (warp == 0) {
+      double t = 0.0;
+      if (lane < NV) {
+        if constexpr (WARPS) {
+          double tg[NGRP];
 #pragma unroll
-      for (int j = 1; j < NB; ++j) {
-        if (j > c && j < b) {
-          const dcplx dj = make_double2(fin[1 + 2 * (j - 1)], fin[2 + 2 * (j - 1)]);
-          const dcplx rj = make_double2(fin[NV + 2 * j], fin[NV + 2 * j + 1]);
-          const dcplx t = cmul(cs, dj);
-          const dcplx w = make_double2(rj.x + t.x, rj.y + t.y);
-          const dcplx p = cmul(cv, w);
-          dcplx x = XS(k, j);
-          x.x -= p.x;
-          x.y -= p.y;
-          XS(k, j) = x;
+          for (int q = 0; q < NGRP; ++q) tg[q] = 0.0;
+#pragma unroll
+          for (int w = 0; w < GW; ++w)
+#pragma unroll
+            for (int q = 0; q < NGRP; ++q) tg[q] += redw[par][q][w][lane];
+#pragma unroll
+          for (int q = 0; q < NGRP; ++q) t += tg[q];
+        } else if constexpr (CL > 1) {
+#pragma unroll
+          for (int q = 0; q < CL; ++q) t += red[par][q][lane];
+        } else {
+#pragma unroll
+          for (int q = 0; q < NW; ++q) t += wsum[q][lane];
         }
+      }
+      // lane q serves position q
+      const int q = lane < NB ? lane : 0;
+      const double xsq = __shfl_sync(0xffffffffu, t, 0);
+      const double dx = __shfl_sync(0xffffffffu, t, (2 * q - 1) & 31), dy = __shfl_sync(0xffffffffu, t, 2 * q);
+      dcplx al, rq;
+      if constexpr (CL > 1) {
+        al = make_double2(rowc[par][0], rowc[par][1]);
+        rq = make_double2(rowc[par][2 * q], rowc[par][2 * q + 1]);
+      } else {
+        al = rowl[0];
+        rq = rowl[q];
+      }
+      // the reflector (LAPACK zlarfg); the four quotients of tau = (beta - alpha) / beta and
+      // scale = 1 / (alpha - beta) in one division, a lane each
+      dcplx tc, scale;
+      double beta;
+      if (xsq == 0.0 && al.y == 0.0) {
+        tc = make_double2(0.0, 0.0);
+        scale = make_double2(0.0, 0.0);
+        beta = al.x;
+      } else {
+        beta = -copysign(sqrt(al.x * al.x + al.y * al.y + xsq), al.x);
+        const double dr = al.x - beta, di = al.y, den = dr * dr + di * di;
+        const int w = lane & 3;
+        const double num = w == 0 ? beta - al.x : (w == 1 ? -al.y : (w == 2 ? dr : -di));
+        const double quot = num / (w < 2 ? beta : den);
+        tc = make_double2(__shfl_sync(0xffffffffu, quot, 0), __shfl_sync(0xffffffffu, quot, 1));
+        scale = make_double2(__shfl_sync(0xffffffffu, quot, 2), __shfl_sync(0xffffffffu, quot, 3));
+      }
+      const dcplx dq = make_double2(dx, dy);
+      if (lane >= 1 && lane < NB) {
+        if (lane < nt) {
+          const dcplx p = cmul(make_double2(scale.x, -scale.y), dq);
+          wv[lane] = make_double2(rq.x + p.x, rq.y + p.y);
+        } else {
+          const dcplx se = cmul(scale, dq);
+          zs[lane - nt] = make_double2(rq.x + se.x, -rq.y + se.y);
+        }
+      }
+      if (lane == 0) {
+        sc[0] = make_double2(tc.x, -tc.y);
+        sc[1] = scale;
+        sc[2] = make_double2(beta, 0.0);
+        if (rank == 0) tau[c] = tc;
+      }
+    }
+    __syncthreads();
+    // v into column c, R diagonal, trailing panel columns x_j -= conj(tau) v (v^H x_j); every
+    // column moves one position down, column c to the last
+    {
+      const dcplx ctc = sc[0], scale = sc[1];
+#pragma unroll
+      for (int k = 0; k < RPT; ++k) {
+        const int il = g + k * G;
+        dcplx v = x[k][0], keep = x[k][0];
+        const bool live = il >= c && il < R;
+        if (il == c) {
+          v = make_double2(1.0, 0.0);
+          keep = sc[2];
+        } else if (live) {
+          v = cmul(v, scale);
+          keep = v;
+        }
+        const dcplx cv = cmul(ctc, v);
+#pragma unroll
+        for (int q = 1; q < NB; ++q) {
+          dcplx y = x[k][q];
+          if (live && q < nt) {
+            const dcplx p = cmul(cv, wv[q]);
+            y.x -= p.x;
+            y.y -= p.y;
+          }
+          x[k][q - 1] = y;
+        }
+        x[k][NB - 1] = keep;
       }
     }
     // T[0:c, c] = -tau T[0:c, 0:c] z with z_l = V_l^H v = conj(V_l[c]) + scale e_l (LAPACK zlarft)
-    if (rank == 0) {
-      if (tid < c) {
+    if (rank == 0 && warp == NW - 1) {
+      const dcplx tc = make_double2(sc[0].x, -sc[0].y);
+      if (lane < c) {
         dcplx sacc = make_double2(0.0, 0.0);
-        for (int l = tid; l < c; ++l) {
-          const dcplx el = make_double2(fin[1 + 2 * l], fin[2 + 2 * l]);
-          const dcplx se = cmul(scale, el);
-          const dcplx z = make_double2(fin[NV + 2 * l] + se.x, -fin[NV + 2 * l + 1] + se.y);
-          const dcplx p = cmul(Tsh[tid][l], z);
+        for (int l = lane; l < c; ++l) {
+          const dcplx p = cmul(Tsh[lane][l], zs[l]);
           sacc.x += p.x;
           sacc.y += p.y;
         }
         const dcplx t = cmul(tc, sacc);
-        Tsh[tid][c] = make_double2(-t.x, -t.y);
+        Tsh[lane][c] = make_double2(-t.x, -t.y);
       }
-      if (tid == 0) {
-        Tsh[c][c] = tc;
-        tau[c] = tc;
-      }
+      if (lane == 0) Tsh[c][c] = tc;
+      __syncwarp();
     }
   }
-  // write back: the panel (R above the diagonal, v below) and the explicit V
+  // write back: the panel (R above the diagonal, v below) and the explicit V; column j is at
+  // position j + NB - b
 #pragma unroll
   for (int k = 0; k < RPT; ++k) {
-    const int il = g + k * QR_G;
+    const int il = g + k * G;
     if (il >= R) continue;
 #pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      if (j < b) {
-        const dcplx x = XS(k, j);
-        A[il + lda * (int64_t)j] = x;
-        V[il + ldv * (int64_t)j] = il > j ? x : (il == j ? make_double2(1.0, 0.0) : make_double2(0.0, 0.0));
+    for (int q = 0; q < NB; ++q) {
+      const int j = q - (NB - b);
+      if (j >= 0) {
+        const dcplx y = x[k][q];
+        A[il + lda * (int64_t)j] = y;
+        V[il + ldv * (int64_t)j] = il > j ? y : (il == j ? make_double2(1.0, 0.0) : make_double2(0.0, 0.0));
       }
     }
   }
-#undef XS
-  for (int r = g; r < zabove; r += QR_G)
+  for (int r = g; r < zabove; r += G)
     for (int j = 0; j < b; ++j) V[(int64_t)(r - zabove) + ldv * (int64_t)j] = make_double2(0.0, 0.0);
   if (rank == 0) {
     __syncthreads();
-    for (int e = tid; e < b * b; e += QR_NT) {
+    for (int e = tid; e < b * b; e += NT) {
       const int i = e % b, j = e / b;
       T[i + (int64_t)ldt * j] = Tsh[i][j];
     }
   }
-  // no CTA may leave while a peer can still read its shared memory
-  cluster_sync();
+  // no CTA may leave while a peer can still write its shared memory
+  if constexpr (CL > 1) cluster_sync();
 }
 
 // Compact-WY factor of an outer block from the factors of its inner panels (LAPACK
@@ -279,16 +372,19 @@ struct PanelList {
   short w[QR_NBO / 2];
 };
 
-// T, G and the panels' products live in shared memory for the whole merge (one CTA).
-constexpr size_t QR_MERGE_SMEM = (size_t)2 * QR_NBO * (QR_NBO + 1) * sizeof(dcplx);
+// T, G and the panels' products live in shared memory for the whole merge (one CTA), T and G
+// in one array: the block of G above a panel's factor is read in that panel's step and then
+// replaced by T's.  Bound by the latency of the sums' chains.
+constexpr size_t QR_MERGE_SMEM = (size_t)QR_NBO * (QR_NBO + 1) * sizeof(dcplx);
 
-__global__ void __launch_bounds__(256) k_merge_t(int bo, PanelList pl, const dcplx* __restrict__ Tin,
+constexpr int QR_MERGE_NT = 1024;   // one thread per output of a panel's step: 18 us (31 us with 256 threads)
+
+__global__ void __launch_bounds__(QR_MERGE_NT) k_merge_t(int bo, PanelList pl, const dcplx* __restrict__ Tin,
                                                  const dcplx* __restrict__ G, dcplx* __restrict__ Tb) {
   extern __shared__ __align__(16) dcplx msm[];
   const int ld = bo + 1;
   dcplx* Ts = msm;                            // Ts[r + ld c]
-  dcplx* Gs = msm + (size_t)QR_NBO * (QR_NBO + 1);
-  __shared__ dcplx Xs[QR_NBO][QR_NBMAX];
+  __shared__ dcplx Xs[QR_NBO][QR_NBMAX + 1];   // odd stride: no bank conflicts along r
   const int tid = threadIdx.x;
   for (int e = tid; e < bo * bo; e += blockDim.x) {
     const int r = e % bo, c = e / bo;
@@ -297,18 +393,18 @@ __global__ void __launch_bounds__(256) k_merge_t(int bo, PanelList pl, const dcp
     const int o = pl.off[t];
     dcplx v = make_double2(0.0, 0.0);
     if (r >= o && r < o + pl.w[t]) v = Tin[(size_t)t * QR_NBMAX * QR_NBMAX + (r - o) + QR_NBMAX * (c - o)];
+    else if (r < o) v = G[r + (int64_t)bo * c];
     Ts[r + ld * c] = v;
-    if (pl.n > 1) Gs[r + ld * c] = G[r + (int64_t)bo * c];
   }
   __syncthreads();
   for (int t = 1; t < pl.n; ++t) {
     const int c0 = pl.off[t], bt = pl.w[t];
-    const dcplx* Tt = Tin + (size_t)t * QR_NBMAX * QR_NBMAX;
+    const dcplx* Tt = Ts + c0 + ld * c0;   // the panel's own factor: Tt[v + ld u]
     for (int e = tid; e < c0 * bt; e += blockDim.x) {
       const int r = e % c0, u = e / c0;
       dcplx sacc = make_double2(0.0, 0.0);
       for (int l = r; l < c0; ++l) {
-        const dcplx p = cmul(Ts[r + ld * l], Gs[l + ld * (c0 + u)]);
+        const dcplx p = cmul(Ts[r + ld * l], Ts[l + ld * (c0 + u)]);
         sacc.x += p.x;
         sacc.y += p.y;
       }
@@ -319,7 +415,7 @@ __global__ void __launch_bounds__(256) k_merge_t(int bo, PanelList pl, const dcp
       const int r = e % c0, u = e / c0;
       dcplx sacc = make_double2(0.0, 0.0);
       for (int v = 0; v <= u; ++v) {
-        const dcplx p = cmul(Xs[r][v], Tt[v + QR_NBMAX * u]);
+        const dcplx p = cmul(Xs[r][v], Tt[v + ld * u]);
         sacc.x += p.x;
         sacc.y += p.y;
       }
@@ -358,16 +454,11 @@ __global__ void k_sum_partials(int64_t len, int nc, const dcplx* __restrict__ pa
   }
 }
 
-template <int NB, int RPT>
+template <int NB, int RPT, int CL, int NT>
 void launch_panel(Context* ctx, int R, int b, int zabove, dcplx* A, int64_t lda, dcplx* V, int64_t ldv, dcplx* tau,
                   dcplx* T, int ldt) {
-  static_assert(NB * RPT == QR_NBMAX, "panel shared-memory size");
-  static DeviceOnce attr;
-  attr.run(ctx->device, [] {
-    IMPS_CUDA(cudaFuncSetAttribute(k_qr_panel<NB, RPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)QR_PANEL_SMEM));
-  });
-  k_qr_panel<NB, RPT><<<QR_CL, QR_NT, QR_PANEL_SMEM, ctx->stream>>>(R, b, zabove, A, lda, V, ldv, tau, T, ldt);
+  static_assert(NB * RPT == QR_NBMAX, "a thread holds 16 complex numbers");
+  k_qr_panel<NB, RPT, CL, NT><<<CL, NT, 0, ctx->stream>>>(R, b, zabove, A, lda, V, ldv, tau, T, ldt);
   ctx->n_kernels++;
   cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess) throw Error(IMPS_CUDA_ERROR, std::string("qr panel launch: ") + cudaGetErrorString(e));
@@ -386,62 +477,72 @@ int panel_width(int R) {
 // kernel forms the long-K product and a second applies it.
 constexpr int XS_NT = 256;   // threads of the X^H V kernel
 constexpr int XS_ROWS = 64;  // rows staged in shared memory per step (one step per CTA)
-constexpr int XS_MAXO = 16;  // outputs per thread: N b <= 4096
+constexpr int XS_COLS = 16;  // columns of X per CTA, one output (n, l) per thread
 constexpr int XS_LD = XS_ROWS + 1;
 
 // Wh (N x b, ld N) = X^H V over K rows, X (K x N) and V (K x b) with leading dimension ld.
-// CTA g sums rows [g kc, (g + 1) kc) into part[g]; the last CTA to finish (counter) adds
-// the partials in CTA order, so the result does not depend on scheduling, resets the
-// counter and, when T is given, forms Z (b x N, ld b) = op(T) Wh^H (op = C or N).
+// CTA (g, h) sums rows [g kc, (g + 1) kc) of columns [16 h, 16 h + 16) into part[g]; the last
+// CTA of a column group to finish (counter[h]) adds the partials in CTA order, so the result
+// does not depend on scheduling, resets the counter and, when T is given, forms its columns
+// of Z (b x N, ld b) = op(T) Wh^H (op = C or N).  Bound by latency and shared-memory reads:
+// column groups of 16 give three times the CTAs of one group of all columns (48 x 16 outputs
+// over 512 rows: 8 us, 17 us in one group).
 __global__ void __launch_bounds__(XS_NT) k_xhv_small(int K, int N, int b, int kc, const dcplx* __restrict__ X,
                                                       const dcplx* __restrict__ Vm, int64_t ld,
                                                       dcplx* __restrict__ part, unsigned* __restrict__ counter,
                                                       dcplx* __restrict__ Wh, const dcplx* __restrict__ T, int ldt,
                                                       int conjT, dcplx* __restrict__ Z) {
-  extern __shared__ dcplx sh[];  // [N + b columns][XS_LD rows], later the summed Wh
+  __shared__ dcplx sh[(XS_COLS + QR_NBMAX) * XS_LD];  // [16 columns of X, b of V][XS_LD rows], later the summed Wh
+  __shared__ dcplx Ts[QR_NBMAX][QR_NBMAX + 1];
   __shared__ bool last;
-  const int nb = N * b, W = N + b, tid = threadIdx.x;
+  const int nb = N * b, tid = threadIdx.x;
+  const int n0 = blockIdx.y * XS_COLS, nn = min(XS_COLS, N - n0);
   const int k0 = blockIdx.x * kc, k1 = min(K, k0 + kc);
-  dcplx acc[XS_MAXO];
-#pragma unroll
-  for (int i = 0; i < XS_MAXO; ++i) acc[i] = make_double2(0.0, 0.0);
+  const int nl = tid % XS_COLS, l = tid / XS_COLS;
+  const bool live = nl < nn && l < b;
+  dcplx acc = make_double2(0.0, 0.0);
+  if (Z && tid < b * b) {   // op(T), read while the rows are on their way
+    const int i = tid % b, j = tid / b;
+    dcplx t = conjT ? T[j + (int64_t)ldt * i] : T[i + (int64_t)ldt * j];
+    if (conjT) t.y = -t.y;
+    Ts[i][j] = t;
+  }
   for (int r0 = k0; r0 < k1; r0 += XS_ROWS) {
     const int nr = min(XS_ROWS, k1 - r0);
     __syncthreads();
-    for (int e = tid; e < XS_ROWS * W; e += XS_NT) {
+#pragma unroll
+    for (int e = tid; e < XS_ROWS * (XS_COLS + QR_NBMAX); e += XS_NT) {
       const int r = e % XS_ROWS, col = e / XS_ROWS;  // consecutive threads walk rows: coalesced
       dcplx v = make_double2(0.0, 0.0);
-      if (r < nr) v = (col < N) ? X[(int64_t)(r0 + r) + ld * col] : Vm[(int64_t)(r0 + r) + ld * (col - N)];
+      if (r < nr) {
+        if (col < XS_COLS) {
+          if (col < nn) v = X[(int64_t)(r0 + r) + ld * (n0 + col)];
+        } else if (col - XS_COLS < b) {
+          v = Vm[(int64_t)(r0 + r) + ld * (col - XS_COLS)];
+        }
+      }
       sh[r + XS_LD * col] = v;
     }
     __syncthreads();
-#pragma unroll
-    for (int i = 0; i < XS_MAXO; ++i) {
-      const int o = tid + XS_NT * i;
-      if (o < nb) {
-        const dcplx* xc = sh + XS_LD * (o % N);
-        const dcplx* vc = sh + XS_LD * (N + o / N);
-        for (int r = 0; r < nr; ++r) {
-          const dcplx x = xc[r], v = vc[r];
-          acc[i].x = fma(x.x, v.x, fma(x.y, v.y, acc[i].x));
-          acc[i].y = fma(x.x, v.y, fma(-x.y, v.x, acc[i].y));
-        }
+    if (live) {
+      const dcplx* xc = sh + XS_LD * nl;
+      const dcplx* vc = sh + XS_LD * (XS_COLS + l);
+      for (int r = 0; r < nr; ++r) {
+        const dcplx x = xc[r], v = vc[r];
+        acc.x = fma(x.x, v.x, fma(x.y, v.y, acc.x));
+        acc.y = fma(x.x, v.y, fma(-x.y, v.x, acc.y));
       }
     }
   }
-#pragma unroll
-  for (int i = 0; i < XS_MAXO; ++i) {
-    const int o = tid + XS_NT * i;
-    if (o < nb) part[(int64_t)blockIdx.x * nb + o] = acc[i];
-  }
+  const int o = n0 + nl + N * l;
+  if (live) part[(int64_t)blockIdx.x * nb + o] = acc;
   __threadfence();
   __syncthreads();
-  if (tid == 0) last = (atomicAdd(counter, 1u) == gridDim.x - 1);
+  if (tid == 0) last = (atomicAdd(&counter[blockIdx.y], 1u) == gridDim.x - 1);
   __syncthreads();
   if (!last) return;
   __threadfence();
-  __syncthreads();
-  for (int o = tid; o < nb; o += XS_NT) {
+  if (live) {
     dcplx t = make_double2(0.0, 0.0);
     int g = 0;
     for (; g + 4 <= (int)gridDim.x; g += 4) {  // four loads in flight, added in CTA order
@@ -458,28 +559,28 @@ __global__ void __launch_bounds__(XS_NT) k_xhv_small(int K, int N, int b, int kc
       t.y += v.y;
     }
     Wh[o] = t;
-    sh[o] = t;  // nb <= XS_LD * (N + b)
+    sh[nl + XS_COLS * l] = t;
   }
-  if (tid == 0) *counter = 0u;
+  if (tid == 0) counter[blockIdx.y] = 0u;
   if (!Z) return;
   __syncthreads();
   // Z[i, n] = sum_l op(T)[i, l] conj(Wh[n, l])
-  for (int e = tid; e < nb; e += XS_NT) {
-    const int i = e % b, n = e / b;
+  const int i = tid % QR_NBMAX, n = tid / QR_NBMAX;
+  if (i < b && n < nn) {
     dcplx z = make_double2(0.0, 0.0);
-    for (int l = 0; l < b; ++l) {
-      dcplx t = conjT ? T[l + (int64_t)ldt * i] : T[i + (int64_t)ldt * l];
-      if (conjT) t.y = -t.y;
-      const dcplx w = sh[n + N * l];  // conj(w) below
+    for (int q = 0; q < b; ++q) {
+      const dcplx t = Ts[i][q], w = sh[n + XS_COLS * q];  // conj(w) below
       z.x += t.x * w.x + t.y * w.y;
       z.y += t.y * w.x - t.x * w.y;
     }
-    Z[e] = z;
+    Z[i + b * (n0 + n)] = z;
   }
 }
 
 // A2 (R x N, lda) -= V (R x b, ldv) Z (b x N), b <= 16, N <= 64: a thread per element,
-// 64 rows x 4 columns per CTA (row loads coalesced, V rows shared through L1).
+// 64 rows x 4 columns per CTA (row loads coalesced, V rows shared through L1).  FULL: b = 16,
+// all loads issued ahead of the sum.
+template <bool FULL>
 __global__ void __launch_bounds__(256) k_apply_small(int R, int N, int b, const dcplx* __restrict__ Vm, int64_t ldv,
                                                      const dcplx* __restrict__ Z, dcplx* __restrict__ A2,
                                                      int64_t lda) {
@@ -487,12 +588,16 @@ __global__ void __launch_bounds__(256) k_apply_small(int R, int N, int b, const 
   const int n = blockIdx.y * 4 + (threadIdx.x >> 6);
   if (r >= R || n >= N) return;
   dcplx a = A2[r + lda * n];
+  dcplx v[QR_NBMAX];
+#pragma unroll
+  for (int i = 0; i < QR_NBMAX; ++i)
+    if (FULL || i < b) v[i] = Vm[r + ldv * i];
 #pragma unroll
   for (int i = 0; i < QR_NBMAX; ++i) {
-    if (i < b) {
-      const dcplx v = Vm[r + ldv * i], z = __ldg(&Z[i + b * n]);
-      a.x -= v.x * z.x - v.y * z.y;
-      a.y -= v.x * z.y + v.y * z.x;
+    if (FULL || i < b) {
+      const dcplx z = __ldg(&Z[i + b * n]);
+      a.x -= fma(v[i].x, z.x, -(v[i].y * z.y));
+      a.y -= fma(v[i].x, z.y, v[i].y * z.x);
     }
   }
   A2[r + lda * n] = a;
@@ -501,26 +606,20 @@ __global__ void __launch_bounds__(256) k_apply_small(int R, int N, int b, const 
 // Wh = X^H V (and Z = op(T) Wh^H when T is given) by k_xhv_small.
 void xhv_small(Context* ctx, int N, int b, int K, const dcplx* X, const dcplx* Vm, int64_t ld, dcplx* part,
                dcplx* Wh, const dcplx* T, int ldt, bool conjT, dcplx* Z) {
-  IMPS_REQUIRE(N * b <= XS_NT * XS_MAXO && N <= QR_NBO && b <= QR_NBO, IMPS_INVALID_ARG, "xhv_small: shape");
+  IMPS_REQUIRE(N <= QR_NBO && b <= QR_NBMAX, IMPS_INVALID_ARG, "xhv_small: shape");
   DevBuf& cnt = ctx->buf("qr_xhv_count", 256);
-  if (ctx->qr_count_ptr != cnt.ptr) {  // a new counter starts at zero; each launch leaves it at zero
+  if (ctx->qr_count_ptr != cnt.ptr) {  // new counters start at zero; each launch leaves them at zero
     IMPS_CUDA(cudaMemsetAsync(cnt.ptr, 0, 256, ctx->stream));
     ctx->qr_count_ptr = cnt.ptr;
   }
   // one staged chunk of XS_ROWS rows per CTA, at most 64 partials (more rows per CTA past
-  // that): the last CTA sums g N b values
+  // that): the last CTA of a column group sums g values per output
   int g = std::max(1, std::min(64, (K + XS_ROWS - 1) / XS_ROWS));
   const int kc = (K + g - 1) / g;
   g = (K + kc - 1) / kc;
   ScopedTimer tm(ctx, "qr_small", 8.0 * N * b * (double)K);
-  const size_t smem = (size_t)XS_LD * (N + b) * sizeof(dcplx);
-  static DeviceOnce attr;
-  attr.run(ctx->device, [] {
-    IMPS_CUDA(cudaFuncSetAttribute(k_xhv_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)((size_t)XS_LD * 2 * QR_NBO * sizeof(dcplx))));
-  });
-  k_xhv_small<<<g, XS_NT, smem, ctx->stream>>>(K, N, b, kc, X, Vm, ld, part, static_cast<unsigned*>(cnt.ptr), Wh,
-                                               T, ldt, conjT ? 1 : 0, Z);
+  k_xhv_small<<<dim3(g, (N + XS_COLS - 1) / XS_COLS), XS_NT, 0, ctx->stream>>>(
+      K, N, b, kc, X, Vm, ld, part, static_cast<unsigned*>(cnt.ptr), Wh, T, ldt, conjT ? 1 : 0, Z);
   ctx->n_kernels++;
   IMPS_CUDA(cudaPeekAtLastError());
 }
@@ -529,7 +628,9 @@ void apply_small(Context* ctx, int R, int N, int b, const dcplx* Vm, int64_t ldv
                  int64_t lda) {
   IMPS_REQUIRE(b <= QR_NBMAX && N <= QR_NBO, IMPS_INVALID_ARG, "apply_small: shape");
   ScopedTimer tm(ctx, "qr_small", 8.0 * R * N * (double)b);
-  k_apply_small<<<dim3((R + 63) / 64, (N + 3) / 4), 256, 0, ctx->stream>>>(R, N, b, Vm, ldv, Z, A2, lda);
+  const dim3 grid((R + 63) / 64, (N + 3) / 4);
+  if (b == QR_NBMAX) k_apply_small<true><<<grid, 256, 0, ctx->stream>>>(R, N, b, Vm, ldv, Z, A2, lda);
+  else k_apply_small<false><<<grid, 256, 0, ctx->stream>>>(R, N, b, Vm, ldv, Z, A2, lda);
   ctx->n_kernels++;
   IMPS_CUDA(cudaPeekAtLastError());
 }
@@ -545,7 +646,8 @@ void gemm_xhv(Context* ctx, int N, int b, int K, const dcplx* X, const dcplx* Vm
   int kc = (K + nc - 1) / nc;
   kc = (kc + 15) / 16 * 16;
   nc = (K + kc - 1) / kc;
-  if (nc == 1) {
+  // (zgemm_fp64 shares the K stages itself where the order of the sum is free)
+  if (nc == 1 || !ctx->ordered_sums()) {
     zgemm_fp64(ctx, OP_C, OP_N, N, b, K, 1.0, X, ld, 0, Vm, ld, 0, 0.0, Wh, N, 0, 1);
     return;
   }
@@ -615,10 +717,17 @@ void qr_factor(Context* ctx, int m, int n, const dcplx* M, int64_t ldm, dcplx* R
       dcplx* Vp = Vb.z() + p + (int64_t)m * p;
       dcplx* Tp = Tin.z() + (size_t)pl.n * QR_NBMAX * QR_NBMAX;
       switch (panel_width(Rr)) {
-        case 16: launch_panel<16, 1>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX); break;
-        case 8: launch_panel<8, 2>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX); break;
-        case 4: launch_panel<4, 4>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX); break;
-        default: launch_panel<2, 8>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX); break;
+        case 16:
+          if (Rr <= 128) launch_panel<16, 1, 1, 128>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX);
+          else if (Rr <= 256) launch_panel<16, 1, 1, 256>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX);
+          else if (Rr <= 512) launch_panel<16, 1, 8, 64>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX);
+          else if (Rr <= 1024) launch_panel<16, 1, 8, 128>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX);
+          else if (Rr <= 2048) launch_panel<16, 1, 8, 256>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX);
+          else launch_panel<16, 1, 8, 512>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX);
+          break;
+        case 8: launch_panel<8, 2, 8, 512>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX); break;
+        case 4: launch_panel<4, 4, 8, 512>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX); break;
+        default: launch_panel<2, 8, 8, 512>(ctx, Rr, b, p - P, Ap, m, Vp, m, taub.z() + p, Tp, QR_NBMAX); break;
       }
       pl.off[pl.n] = (short)(p - P);
       pl.w[pl.n] = (short)b;
@@ -642,7 +751,7 @@ void qr_factor(Context* ctx, int m, int n, const dcplx* M, int64_t ldm, dcplx* R
     merge_attr.run(ctx->device, [] {
       IMPS_CUDA(cudaFuncSetAttribute(k_merge_t, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QR_MERGE_SMEM));
     });
-    k_merge_t<<<1, 256, QR_MERGE_SMEM, ctx->stream>>>(bo, pl, Tin.z(), Gb.z(), Tb);
+    k_merge_t<<<1, QR_MERGE_NT, QR_MERGE_SMEM, ctx->stream>>>(bo, pl, Tin.z(), Gb.z(), Tb);
     ctx->n_kernels++;
     const int n2 = n - (P + bo);
     if (n2 > 0) {
