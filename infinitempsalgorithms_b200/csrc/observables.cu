@@ -101,6 +101,135 @@ __global__ void __launch_bounds__(kJacThreads) k_jacobi_round(int n, int ncol, i
   if (threadIdx.x == 0) atomicAdd(rot, 1);
 }
 
+// Block form of the round for values only: the columns are taken in blocks of 8, CTA k
+// orthogonalises the 16 columns of blocks (a, b) of the round-robin schedule of blocks in
+// shared memory (round 0 also the pairs inside each block), a warp per pair.  A warp keeps
+// its column of block a in registers while the 8 columns of block b come to it in turn, so a
+// sweep is nblk - 1 launches of 8 steps instead of 8 nblk - 1 launches of one.
+// n <= 32 EPL rows; the columns past the last one are zero (never rotated).  Bound by the
+// latency of a step (two sums over the warp, two square roots, two divisions): 10 us a launch
+// of 16 CTAs at n = 256, against 24 us for 8 rounds of k_jacobi_round.
+constexpr int kJacBlk = 8;
+
+// Orthogonalises x, y (a row i = lane + 32 u of each per register); true when it rotated.
+template <int EPL>
+__device__ __forceinline__ bool jacobi_pair(dcplx (&x)[EPL], dcplx (&y)[EPL], double tol2, int lane) {
+  double v[4] = {0.0, 0.0, 0.0, 0.0};   // ||x||^2, ||y||^2, x^H y
+#pragma unroll
+  for (int u = 0; u < EPL; ++u) {
+    v[0] = fma(x[u].x, x[u].x, fma(x[u].y, x[u].y, v[0]));
+    v[1] = fma(y[u].x, y[u].x, fma(y[u].y, y[u].y, v[1]));
+    v[2] = fma(x[u].x, y[u].x, fma(x[u].y, y[u].y, v[2]));
+    v[3] = fma(x[u].x, y[u].y, fma(-x[u].y, y[u].x, v[3]));
+  }
+  // lanes of the upper half keep v[2..3], then every quarter one sum
+#pragma unroll
+  for (int o = 16, half = 2; half >= 1; o >>= 1, half >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int q = 0; q < half; ++q) {
+      const double send = up ? v[q] : v[q + half], keep = up ? v[q + half] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+#pragma unroll
+  for (int o = 4; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  const double al = __shfl_sync(0xffffffffu, v[0], 0), be = __shfl_sync(0xffffffffu, v[0], 8);
+  const double gr = __shfl_sync(0xffffffffu, v[0], 16), gi = __shfl_sync(0xffffffffu, v[0], 24);
+  const double g2 = gr * gr + gi * gi;
+  if (!(g2 > tol2 * al * be)) return false;
+  // tan of the rotation that annihilates the off-diagonal of [[al, g], [g, be]], g = |x^H y|
+  const double g = sqrt(g2), d = be - al;
+  const double t = copysign(2.0 * g / (fabs(d) + sqrt(fma(d, d, 4.0 * g2))), d);
+  const double c = 1.0 / sqrt(fma(t, t, 1.0)), s = c * t, ig = 1.0 / g;
+  const double er = gr * ig, ei = gi * ig;
+  const double sr = s * er, si = s * ei;
+#pragma unroll
+  for (int u = 0; u < EPL; ++u) {
+    const dcplx a = x[u], b = y[u];
+    // x' = c x - s e^{-i phi} y,  y' = s e^{i phi} x + c y
+    x[u] = make_double2(c * a.x - (sr * b.x + si * b.y), c * a.y - (sr * b.y - si * b.x));
+    y[u] = make_double2((sr * a.x - si * a.y) + c * b.x, (sr * a.y + si * a.x) + c * b.y);
+  }
+  return true;
+}
+
+template <int EPL>
+__global__ void __launch_bounds__(32 * kJacBlk) k_jacobi_block(int n, int nblk, int r, dcplx* __restrict__ U,
+                                                               int64_t ldu, double tol2, int* __restrict__ rot) {
+  extern __shared__ dcplx cols[];   // [16][32 EPL]
+  constexpr int LDC = 32 * EPL;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k = blockIdx.x;
+  const int ba = rr_player(k, r, nblk) * kJacBlk, bb = rr_player(nblk - 1 - k, r, nblk) * kJacBlk;
+  dcplx x[EPL], y[EPL];
+  int cnt = 0;
+  auto global_col = [&](int q) { return U + ldu * (int64_t)((q < kJacBlk ? ba : bb - kJacBlk) + q); };
+  auto get = [&](const dcplx* p, dcplx (&z)[EPL]) {
+#pragma unroll
+    for (int u = 0; u < EPL; ++u) z[u] = p[lane + 32 * u];
+  };
+  auto put = [&](dcplx* p, const dcplx (&z)[EPL]) {
+#pragma unroll
+    for (int u = 0; u < EPL; ++u) p[lane + 32 * u] = z[u];
+  };
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const dcplx* src = global_col(w + kJacBlk * h);
+#pragma unroll
+    for (int u = 0; u < EPL; ++u)
+      cols[(w + kJacBlk * h) * LDC + lane + 32 * u] = lane + 32 * u < n ? src[lane + 32 * u] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  if (r == 0) {
+    const int off = w < 4 ? 0 : kJacBlk, q = w & 3;
+    for (int s = 0; s < kJacBlk - 1; ++s) {
+      dcplx* px = cols + (off + rr_player(q, s, kJacBlk)) * LDC;
+      dcplx* py = cols + (off + rr_player(kJacBlk - 1 - q, s, kJacBlk)) * LDC;
+      get(px, x);
+      get(py, y);
+      if (jacobi_pair<EPL>(x, y, tol2, lane)) {
+        ++cnt;
+        put(px, x);
+        put(py, y);
+      }
+      __syncthreads();
+    }
+  }
+  get(cols + w * LDC, x);
+  for (int s = 0; s < kJacBlk; ++s) {
+    dcplx* py = cols + (kJacBlk + ((w + s) & (kJacBlk - 1))) * LDC;
+    get(py, y);
+    if (jacobi_pair<EPL>(x, y, tol2, lane)) {
+      ++cnt;
+      put(py, y);
+    }
+    __syncthreads();
+  }
+  if (!__syncthreads_or(cnt)) return;
+  if (lane == 0 && cnt) atomicAdd(rot, cnt);
+  dcplx* da = global_col(w);
+  dcplx* db = global_col(w + kJacBlk);
+  get(cols + (w + kJacBlk) * LDC, y);
+#pragma unroll
+  for (int u = 0; u < EPL; ++u) {
+    const int i = lane + 32 * u;
+    if (i < n) {
+      da[i] = x[u];
+      db[i] = y[u];
+    }
+  }
+}
+
+template <int EPL>
+void jacobi_block_round(Context* ctx, int n, int nblk, int r, dcplx* U, double tol, int* rot) {
+  constexpr int SMEM = 2 * kJacBlk * 32 * EPL * (int)sizeof(dcplx);
+  static DeviceOnce attr;
+  attr.run(ctx->device, [] {
+    IMPS_CUDA(cudaFuncSetAttribute(k_jacobi_block<EPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+  });
+  k_jacobi_block<EPL><<<nblk / 2, 32 * kJacBlk, SMEM, ctx->stream>>>(n, nblk, r, U, n, tol * tol, rot);
+}
+
 // out[:, j] = scale_j * in[:, perm[j]] for j < k (column gather with optional scaling)
 __global__ void k_gather_cols(int rows, int k, const dcplx* __restrict__ in, int64_t ldi, const int* __restrict__ perm,
                               const double* __restrict__ scale, dcplx* __restrict__ out, int64_t ldo) {
@@ -134,31 +263,86 @@ void check(Context* ctx) {
 
 }  // namespace
 
-std::vector<double> singular_values_sq(Context* ctx, int m, int n, const dcplx* A, int64_t lda) {
-  IMPS_REQUIRE(m > 0 && n > 0, IMPS_INVALID_ARG, "singular values: empty matrix");
-  const int P = n + (n & 1);
-  DevBuf& U = ctx->buf("jac_u", (size_t)m * P * sizeof(dcplx));
+// Jacobi sweeps over the columns of U (n rows, ncol columns, room for a multiple of 16) until
+// no pair rotates.
+static void jacobi_sweeps(Context* ctx, int n, int ncol, dcplx* U) {
   DevBuf& flag = ctx->buf("jac_flag", 64);
-  DevBuf& nr = ctx->buf("jac_norms", (size_t)P * sizeof(double));
-  zcopy2d(ctx, m, n, A, lda, U.z(), m);
-  ScopedTimer tm(ctx, "jacobi_svd", 0.0);
-  const double tol = 1e-15 * std::sqrt((double)m);
+  int* rot = static_cast<int*>(flag.ptr);
+  const double tol = 1e-15 * std::sqrt((double)n);
+  const int P = ncol + (ncol & 1), nblk = (ncol + 2 * kJacBlk - 1) / (2 * kJacBlk) * 2;
   for (int sweep = 0; sweep < 60; ++sweep) {
-    IMPS_CUDA(cudaMemsetAsync(flag.ptr, 0, sizeof(int), ctx->stream));
-    for (int r = 0; r < P - 1; ++r) {
-      k_jacobi_round<<<P / 2, kJacThreads, 0, ctx->stream>>>(m, n, P, r, U.z(), m, tol, static_cast<int*>(flag.ptr),
-                                                             nullptr, 0, 0);
-      check(ctx);
+    IMPS_CUDA(cudaMemsetAsync(rot, 0, sizeof(int), ctx->stream));
+    if (n <= 512) {
+      for (int r = 0; r < nblk - 1; ++r) {
+        if (n <= 128) jacobi_block_round<4>(ctx, n, nblk, r, U, tol, rot);
+        else if (n <= 256) jacobi_block_round<8>(ctx, n, nblk, r, U, tol, rot);
+        else jacobi_block_round<16>(ctx, n, nblk, r, U, tol, rot);
+        check(ctx);
+      }
+    } else {  // 16 columns do not fit in a CTA's shared memory and registers
+      for (int r = 0; r < P - 1; ++r) {
+        k_jacobi_round<<<P / 2, kJacThreads, 0, ctx->stream>>>(n, ncol, P, r, U, n, tol, rot, nullptr, 0, 0);
+        check(ctx);
+      }
     }
-    int rot = 0;
-    download(ctx, &rot, flag.ptr, sizeof(int));
-    if (rot == 0) break;
+    int done = 0;
+    download(ctx, &done, rot, sizeof(int));
+    if (done == 0) break;
   }
-  k_col_norms2<<<n, kJacThreads, 0, ctx->stream>>>(m, n, U.z(), m, nr.d());
-  check(ctx);
-  std::vector<double> s2(n);
-  download(ctx, s2.data(), nr.ptr, n * sizeof(double));
+}
+
+// The squared singular values of the D x D matrix A, descending.  One-sided Jacobi on A itself
+// takes many sweeps when A's columns are far from orthogonal (34 for a bond matrix in a
+// general basis, D = 256: 34 ms); on the conjugate transpose of the R factor of A with its
+// columns by descending norm, whose columns are graded and nearly orthogonal, it takes 11,
+// in blocks (5.2 ms with the QR).  With a workspace cap A is taken as it is.
+std::vector<double> singular_values_sq(Context* ctx, int D, const dcplx* A, int64_t lda) {
+  IMPS_REQUIRE(D > 0, IMPS_INVALID_ARG, "singular values: empty matrix");
+  const int P = (D + 2 * kJacBlk - 1) / (2 * kJacBlk) * (2 * kJacBlk);
+  DevBuf& U = ctx->buf("jac_u", (size_t)D * P * sizeof(dcplx));
+  DevBuf& nr = ctx->buf("jac_norms", (size_t)P * sizeof(double));
+  ScopedTimer tm(ctx, "jacobi_svd", 0.0);
+  zfill(ctx, (int64_t)D * P, 0.0, U.z());
+  std::vector<double> s2(D);
+  auto norms = [&] {
+    k_col_norms2<<<D, kJacThreads, 0, ctx->stream>>>(D, D, U.z(), D, nr.d());
+    check(ctx);
+    download(ctx, s2.data(), nr.ptr, D * sizeof(double));
+  };
+  zcopy2d(ctx, D, D, A, lda, U.z(), D);
+  norms();
+  const double top = *std::max_element(s2.begin(), s2.end());
+  bool finite = true;
+  for (double v : s2) finite = finite && std::isfinite(v);
+  double unscale = 1.0;
+  if (finite && top > 0.0) {   // an exact scale that keeps the squares' squares in range
+    int e;
+    std::frexp(std::sqrt(top), &e);
+    zscal(ctx, (int64_t)D * D, std::ldexp(1.0, -e), U.z());
+    unscale = std::ldexp(1.0, 2 * e);
+  }
+  if (finite && top > 0.0 && ctx->workspace_limit == 0 && D <= 32768) {
+    try {
+      std::vector<int> perm(D);
+      for (int j = 0; j < D; ++j) perm[j] = j;
+      std::stable_sort(perm.begin(), perm.end(), [&](int a, int b) { return s2[a] > s2[b]; });
+      DevBuf& W = ctx->buf("jac_w", (size_t)D * D * sizeof(dcplx));
+      DevBuf& R = ctx->buf("jac_r", (size_t)D * D * sizeof(dcplx));
+      int* pd = static_cast<int*>(ctx->buf("jac_perm", (size_t)D * sizeof(int)).ptr);
+      upload(ctx, pd, perm.data(), (size_t)D * sizeof(int));
+      k_gather_cols<<<148 * 8, 256, 0, ctx->stream>>>(D, D, U.z(), D, pd, nullptr, W.z(), D);
+      check(ctx);
+      qr_factor(ctx, D, D, W.z(), D, R.z(), "qr");
+      zconj_transpose(ctx, D, D, R.z(), D, U.z(), D);
+    } catch (const Error& err) {
+      if (err.status != IMPS_OOM) throw;
+      cudaGetLastError();   // U still holds A
+    }
+  }
+  jacobi_sweeps(ctx, D, D, U.z());
+  norms();
   std::sort(s2.begin(), s2.end(), [](double x, double y) { return x > y; });
+  for (double& v : s2) v *= unscale;
   return s2;
 }
 
@@ -229,7 +413,7 @@ std::vector<double> entanglement_spectrum(Context* ctx, imps_state* st, int bond
   Fp64Scope fp64(ctx);
   const int b = ((bond % st->N) + st->N) % st->N;
   const int D = st->Dr(b);
-  std::vector<double> p = singular_values_sq(ctx, D, D, st->C[b].z(), D);
+  std::vector<double> p = singular_values_sq(ctx, D, st->C[b].z(), D);
   double tot = 0.0;
   for (double v : p) tot += v;
   IMPS_REQUIRE(tot > 0.0, IMPS_INVALID_ARG, "entanglement spectrum: zero center matrix");

@@ -7,8 +7,8 @@
 
 namespace imps {
 
-// Squared singular values (descending) of the m x n matrix A, by one-sided Jacobi.
-std::vector<double> singular_values_sq(Context* ctx, int m, int n, const dcplx* A, int64_t lda);
+// Squared singular values (descending) of the D x D matrix A, by one-sided Jacobi.
+std::vector<double> singular_values_sq(Context* ctx, int D, const dcplx* A, int64_t lda);
 // Thin SVD A = U diag(s) V^H by one-sided Jacobi (descending s), truncated to at most
 // kmax (> 0) values and to those above `cutoff` (at least one kept); U (m x k), V (n x k)
 // column-major with leading dimensions m and n.  Returns k.
