@@ -123,7 +123,8 @@ int imps_ctx_create(int device, imps_ctx** out) {
     IMPS_CUDA(cudaSetDevice(device));
     IMPS_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
     c.own_stream = true;
-    IMPS_CUDA(cudaMalloc((void**)&c.dev_info, sizeof(int) * 4));
+    IMPS_CUDA(cudaMalloc((void**)&c.counters, sizeof(unsigned) * 16));
+    IMPS_CUDA(cudaMemset(c.counters, 0, sizeof(unsigned) * 16));
     IMPS_CUDA(cudaMalloc((void**)&c.err_dev, sizeof(int) * 4));
     IMPS_CUDA(cudaMemset(c.err_dev, 0, sizeof(int) * 4));
     IMPS_CUDA(cudaMallocHost((void**)&c.err_host, sizeof(int) * 4));
@@ -157,7 +158,7 @@ int imps_ctx_destroy(imps_ctx* h) {
   c.optional.clear();
   c.red.release();
   if (c.host_pinned) cudaFreeHost(c.host_pinned);
-  if (c.dev_info) cudaFree(c.dev_info);
+  if (c.counters) cudaFree(c.counters);
   if (c.err_dev) cudaFree(c.err_dev);
   if (c.err_host) cudaFreeHost(c.err_host);
   if (c.own_stream && c.stream) cudaStreamDestroy(c.stream);

@@ -135,8 +135,7 @@ struct Builder {
 
   // regularize!(X, rho, I): X -= tr(rho X) I
   void regularize(int D, dcplx* X, int64_t ldx, const dcplx* rho) {
-    cplx c = ztrace_prod(ctx, D, rho, D, X, ldx);
-    zadd_diag(ctx, D, X, ldx, -c);
+    zregularize(ctx, D, rho, D, X, ldx);
   }
 
   void run() {

@@ -108,7 +108,7 @@ struct Context {
   DevBuf red;
   double* host_pinned = nullptr;
   size_t host_pinned_bytes = 0;
-  int* dev_info = nullptr;
+  unsigned* counters = nullptr;   // completion counters, zero between launches
   // device error flag of the bounded waits (split GEMM) and its pinned host copy;
   // armed while a kernel that may set it has not been checked at a synchronisation
   int* err_dev = nullptr;
@@ -436,6 +436,8 @@ void zgemv_set(Context* ctx, int64_t n, int nv, const dcplx* V, int64_t ldv, con
 void zconj_transpose(Context* ctx, int m, int n, const dcplx* X, int64_t ldx, dcplx* Y, int64_t ldy);
 // trace(L * V) with L, V  D x D (regularize! coefficient, sum L[a,b] V[b,a])
 cplx ztrace_prod(Context* ctx, int D, const dcplx* L, int64_t ldl, const dcplx* V, int64_t ldv);
+// X -= tr(rho X) I on the device (regularize!)
+void zregularize(Context* ctx, int D, const dcplx* rho, int64_t ldr, dcplx* X, int64_t ldx);
 void zadd_diag(Context* ctx, int D, dcplx* X, int64_t ld, cplx v);
 void zfill2d(Context* ctx, int rows, int cols, cplx v, dcplx* Y, int64_t ldy);
 // X[:, lvl-slice] strided copy helpers

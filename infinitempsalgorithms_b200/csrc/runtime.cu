@@ -382,6 +382,49 @@ __global__ void k_trace_prod_partial(int D, const dcplx* __restrict__ L, int64_t
   }
 }
 
+// X -= tr(rho X) I in one launch: the partial sums of k_trace_prod_partial, added in block
+// order by the last block to finish (so the value does not depend on timing), which then
+// corrects the diagonal; no trip to the host.  The counter is left at zero.
+__global__ void k_regularize(int D, const dcplx* __restrict__ L, int64_t ldl, dcplx* __restrict__ V, int64_t ldv,
+                             double* __restrict__ part, unsigned* __restrict__ counter) {
+  __shared__ double sh[kRedThreads / 32];
+  __shared__ double all[2 * kMaxRedBlocks];
+  __shared__ double tr[2];
+  __shared__ bool last;
+  double sr = 0.0, si = 0.0;
+  const int64_t total = (int64_t)D * D;
+  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
+    const int a = (int)(t % D), b = (int)(t / D);
+    const dcplx p = cmul(L[a + ldl * b], V[b + ldv * a]);
+    sr += p.x;
+    si += p.y;
+  }
+  const double r = block_sum<kRedThreads>(sr, sh), q = block_sum<kRedThreads>(si, sh);
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = r;
+    part[2 * blockIdx.x + 1] = q;
+    __threadfence();
+    last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  for (int i = threadIdx.x; i < 2 * (int)gridDim.x; i += blockDim.x) all[i] = __ldcg(&part[i]);
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    double s = 0.0;
+#pragma unroll 16
+    for (int i = 0; i < (int)gridDim.x; ++i) s += all[2 * i + threadIdx.x];
+    tr[threadIdx.x] = s;
+  }
+  if (threadIdx.x == 0) *counter = 0u;
+  __syncthreads();
+  for (int i = threadIdx.x; i < D; i += blockDim.x) {
+    const dcplx u = V[i + ldv * i];
+    V[i + ldv * i] = make_double2(u.x - tr[0], u.y - tr[1]);
+  }
+}
+
 __global__ void k_copy2d(int rows, int cols, const dcplx* __restrict__ X, int64_t ldx, dcplx* __restrict__ Y,
                          int64_t ldy, int add) {
   int64_t total = (int64_t)rows * cols;
@@ -750,6 +793,13 @@ cplx ztrace_prod(Context* ctx, int D, const dcplx* L, int64_t ldl, const dcplx* 
   double sr = 0.0, si = 0.0;
   for (int i = 0; i < nb; ++i) { sr += p[2 * i]; si += p[2 * i + 1]; }
   return cplx(sr, si);
+}
+
+void zregularize(Context* ctx, int D, const dcplx* rho, int64_t ldr, dcplx* X, int64_t ldx) {
+  const int nb = red_blocks((int64_t)D * D);
+  DevBuf& red = ctx->buf("red_part", (size_t)(2 * nb + 8) * sizeof(double));
+  k_regularize<<<nb, kRedThreads, 0, ctx->stream>>>(D, rho, ldr, X, ldx, red.d(), ctx->counters);
+  check_launch(ctx);
 }
 
 void zcopy2d(Context* ctx, int rows, int cols, const dcplx* X, int64_t ldx, dcplx* Y, int64_t ldy) {

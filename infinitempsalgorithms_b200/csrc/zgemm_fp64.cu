@@ -129,8 +129,9 @@ __global__ void __launch_bounds__(NT, 2)
 
 // ---------------------------------------------------------------------------
 // FP64 tensor-core variant: mma.sync m8n8k4 f64 (DMMA).  64 x 64 complex output tile per
-// CTA of 8 warps (2 x 4 warps of 32 x 16), two CTAs per SM, a K stage of 16 complex, a
-// 3-stage cp.async ring (zero-filled at the matrix edges).  A complex product is four real
+// CTA of 8 warps (2 x 4 warps of 32 x 16), two CTAs per SM, or for small grids 32 x 32 per
+// CTA of 4 warps (2 x 2 of 16 x 16); a K stage of 16 complex, a 3-stage cp.async ring
+// (zero-filled at the matrix edges).  A complex product is four real
 // DMMAs per 8 x 8 block: re += ar br - ai bi, im += ar bi + ai br; the conjugate of an
 // operand only flips the sign of its imaginary fragment.
 // Shared tiles are k-major rows of double2.  A fragment read takes 4 k x 2 m (or n)
@@ -144,11 +145,15 @@ __global__ void __launch_bounds__(NT, 2)
 // 32 us (was 210).
 // ---------------------------------------------------------------------------
 namespace dm {
-constexpr int BM = 64, BN = 64, BK = 16, STAGES = 3, NT = 256;
-constexpr int LD = BM + 2;
-constexpr int TILE = BK * LD;                    // elements of one operand's stage
-constexpr int SMEM = STAGES * 2 * TILE * 16;
-constexpr int SMEM_ALONE = 120 * 1024;           // keeps a second CTA off the SM
+constexpr int BK = 16, STAGES = 3;
+template <int T>
+struct Tile {
+  static constexpr int NT = 4 * T;                // threads: 2 x T / 16 warps of T / 2 x 16
+  static constexpr int MI = T / 16, NJ = 2;       // 8 x 8 blocks of a warp
+  static constexpr int LD = T + 2;
+  static constexpr int TILE = BK * LD;            // elements of one operand's stage
+  static constexpr int SMEM = STAGES * 2 * TILE * 16;
+};
 }  // namespace dm
 
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int bytes) {
@@ -167,31 +172,32 @@ __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b)
 // SPLITK: nsplit CTAs (along x) share one output tile, each summing its part of the K
 // stages; CTA r writes its plain partial sums to part[r] (M x N each), which
 // k_sum_split adds in order (so the result does not depend on timing).
-template <int OPA, int OPB, bool BETA, bool SPLITK>
-__global__ void __launch_bounds__(dm::NT, 2)
+template <int OPA, int OPB, bool BETA, bool SPLITK, int T>
+__global__ void __launch_bounds__(4 * T, T == 64 ? 2 : 4)
     k_zgemm_dmma(int M, int N, int K, double2 alpha, const double2* __restrict__ A, int64_t lda, int64_t sA,
                  const double2* __restrict__ B, int64_t ldb, int64_t sB, double2 beta, double2* __restrict__ C,
                  int64_t ldc, int64_t sC, int nsplit, double2* __restrict__ part) {
+  using D = dm::Tile<T>;
   extern __shared__ __align__(16) double2 smem_dm[];   // [STAGES][A tile, B tile][BK][LD]
   const int bz = blockIdx.z;
   A += sA * bz;
   B += sB * bz;
   C += sC * bz;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = warp & 1, wn = warp >> 1;  // warp tile origin (32 wm, 16 wn)
+  const int wm = warp & 1, wn = warp >> 1;  // warp tile origin (T / 2 wm, 16 wn)
   const int rank = SPLITK ? (int)(blockIdx.x % nsplit) : 0;
-  const int m0 = (int)(SPLITK ? blockIdx.x / nsplit : blockIdx.x) * dm::BM, n0 = blockIdx.y * dm::BN;
+  const int m0 = (int)(SPLITK ? blockIdx.x / nsplit : blockIdx.x) * T, n0 = blockIdx.y * T;
   const uint32_t sbase = static_cast<uint32_t>(__cvta_generic_to_shared(smem_dm));
 
-  // Load coordinates.  An operand whose line index (m or n) is contiguous: line tid % 64,
-  // k = tid / 64 + 4 r; one contiguous in k: k from bits 0, 1, 3, 4 of tid, line from bit 2
-  // and the warp, + 16 r.
+  // Load coordinates.  An operand whose line index (m or n) is contiguous: line tid % T,
+  // k = tid / T + 4 r; one contiguous in k: k from bits 0, 1, 3, 4 of tid, line from bit 2
+  // and the warp, + T / 4 r.
   constexpr bool AK = OPA != OP_N, BKc = OPB == OP_N;   // contiguous along k
   const int kc = (tid & 3) | ((tid >> 1) & 12), lc = ((tid >> 2) & 1) | (warp << 1);
-  const int ll = tid & 63, kl = tid >> 6;
+  const int ll = tid % T, kl = tid / T;
   const int am = AK ? lc : ll, ak = AK ? kc : kl;
   const int bn = BKc ? lc : ll, bk = BKc ? kc : kl;
-  const int64_t a_r = AK ? 16 * lda : 4 * lda, b_r = BKc ? 16 * ldb : 4 * ldb;         // step of r
+  const int64_t a_r = AK ? T / 4 * lda : 4 * lda, b_r = BKc ? T / 4 * ldb : 4 * ldb;   // step of r
   const int64_t a_s = AK ? dm::BK : dm::BK * lda, b_s = BKc ? dm::BK : dm::BK * ldb;   // step of a stage
   // this CTA's K stages
   const int kall = (K + dm::BK - 1) / dm::BK;
@@ -199,29 +205,29 @@ __global__ void __launch_bounds__(dm::NT, 2)
   const int ktiles = (SPLITK ? (int)((int64_t)kall * (rank + 1) / nsplit) : kall) - kt0;
   const double2* pa = A + (AK ? ak + lda * (int64_t)(m0 + am) : (m0 + am) + lda * (int64_t)ak) + a_s * kt0;
   const double2* pb = B + (BKc ? bk + ldb * (int64_t)(n0 + bn) : (n0 + bn) + ldb * (int64_t)bk) + b_s * kt0;
-  const uint32_t da = sbase + 16u * (ak * dm::LD + am), db = sbase + 16u * (dm::TILE + bk * dm::LD + bn);
-  constexpr uint32_t DA_R = 16u * (AK ? 16 : 4 * dm::LD), DB_R = 16u * (BKc ? 16 : 4 * dm::LD);
+  const uint32_t da = sbase + 16u * (ak * D::LD + am), db = sbase + 16u * (D::TILE + bk * D::LD + bn);
+  constexpr uint32_t DA_R = 16u * (AK ? T / 4 : 4 * D::LD), DB_R = 16u * (BKc ? T / 4 : 4 * D::LD);
 
   auto issue = [&](int stage, int kt) {
     const int k0 = (kt0 + kt) * dm::BK;
     const double2* qa = pa + a_s * kt;
     const double2* qb = pb + b_s * kt;
-    const uint32_t so = 16u * (uint32_t)(stage * 2 * dm::TILE);
+    const uint32_t so = 16u * (uint32_t)(stage * 2 * D::TILE);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      const bool ok = AK ? (m0 + am + 16 * r < M && k0 + ak < K) : (m0 + am < M && k0 + ak + 4 * r < K);
+      const bool ok = AK ? (m0 + am + T / 4 * r < M && k0 + ak < K) : (m0 + am < M && k0 + ak + 4 * r < K);
       cp_async16(da + so + DA_R * r, ok ? qa + a_r * r : A, ok ? 16 : 0);
     }
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
-      const bool ok = BKc ? (n0 + bn + 16 * r < N && k0 + bk < K) : (n0 + bn < N && k0 + bk + 4 * r < K);
+      const bool ok = BKc ? (n0 + bn + T / 4 * r < N && k0 + bk < K) : (n0 + bn < N && k0 + bk + 4 * r < K);
       cp_async16(db + so + DB_R * r, ok ? qb + b_r * r : B, ok ? 16 : 0);
     }
   };
 
-  double cre[4][2][2], cim[4][2][2];
+  double cre[D::MI][2][2], cim[D::MI][2][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < D::MI; ++i)
 #pragma unroll
     for (int j = 0; j < 2; ++j) cre[i][j][0] = cre[i][j][1] = cim[i][j][0] = cim[i][j][1] = 0.0;
 
@@ -231,39 +237,39 @@ __global__ void __launch_bounds__(dm::NT, 2)
     cp_async_commit();
   }
   const int fr = lane >> 2, fk = lane & 3;  // fragment row/col (A: row m, col k; B: col n, row k)
-  const int fa = fk * dm::LD + 32 * wm + fr, fb = dm::TILE + fk * dm::LD + 16 * wn + fr;
+  const int fa = fk * D::LD + T / 2 * wm + fr, fb = D::TILE + fk * D::LD + 16 * wn + fr;
   int stage = 0, nstage = dm::STAGES - 1;
   for (int kt = 0; kt < ktiles; ++kt) {
     cp_async_wait<dm::STAGES - 2>();
     __syncthreads();
     if (kt + dm::STAGES - 1 < ktiles) issue(nstage, kt + dm::STAGES - 1);
     cp_async_commit();
-    const double2* ss = smem_dm + stage * 2 * dm::TILE;
+    const double2* ss = smem_dm + stage * 2 * D::TILE;
 #pragma unroll
     for (int kb = 0; kb < dm::BK; kb += 4) {
-      double ar[4], ai[4], br[2], bi[2];
+      double ar[D::MI], ai[D::MI], br[2], bi[2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const double2 v = ss[kb * dm::LD + fa + 8 * i];
+      for (int i = 0; i < D::MI; ++i) {
+        const double2 v = ss[kb * D::LD + fa + 8 * i];
         ar[i] = v.x;
         ai[i] = (OPA == OP_C) ? -v.y : v.y;
       }
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const double2 v = ss[kb * dm::LD + fb + 8 * j];
+        const double2 v = ss[kb * D::LD + fb + 8 * j];
         br[j] = v.x;
         bi[j] = (OPB == OP_C) ? -v.y : v.y;
       }
-      // the two updates of one accumulator are 16 MMAs apart
+      // the two updates of one accumulator are 4 MI MMAs apart
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < D::MI; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           dmma(cre[i][j][0], cre[i][j][1], ar[i], br[j]);
           dmma(cim[i][j][0], cim[i][j][1], ar[i], bi[j]);
         }
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < D::MI; ++i)
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
           dmma(cre[i][j][0], cre[i][j][1], -ai[i], bi[j]);
@@ -277,8 +283,8 @@ __global__ void __launch_bounds__(dm::NT, 2)
   // D fragment: row = lane >> 2, cols 2 (lane & 3) + {0, 1} of each 8 x 8 block
   double2* P = SPLITK ? part + ((int64_t)bz * nsplit + rank) * M * (int64_t)N : nullptr;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int gm = m0 + 32 * wm + 8 * i + fr;
+  for (int i = 0; i < D::MI; ++i) {
+    const int gm = m0 + T / 2 * wm + 8 * i + fr;
     if (gm >= M) continue;
 #pragma unroll
     for (int j = 0; j < 2; ++j)
@@ -340,42 +346,45 @@ __global__ void __launch_bounds__(256) k_sum_split(int M, int N, int nsplit, con
   }
 }
 
-template <int OPA, int OPB, bool BETA, bool SPLITK>
+template <int OPA, int OPB, bool BETA, bool SPLITK, int T>
 void launch_dmma(Context* ctx, int nsplit, double2* part, int M, int N, int K, double2 alpha, const dcplx* A,
                  int64_t lda, int64_t sA, const dcplx* B, int64_t ldb, int64_t sB, double2 beta, dcplx* C, int64_t ldc,
                  int64_t sC, int batch) {
-  auto kern = k_zgemm_dmma<OPA, OPB, BETA, SPLITK>;
+  using D = dm::Tile<T>;
+  auto kern = k_zgemm_dmma<OPA, OPB, BETA, SPLITK, T>;
   static DeviceOnce attr;  // the dynamic shared-memory opt-in
   attr.run(ctx->device, [&] {
-    IMPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dm::SMEM));
+    IMPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, D::SMEM));
   });
-  const dim3 grid((M + dm::BM - 1) / dm::BM * nsplit, (N + dm::BN - 1) / dm::BN, batch);
-  kern<<<grid, dm::NT, dm::SMEM, ctx->stream>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, nsplit, part);
+  const dim3 grid((M + T - 1) / T * nsplit, (N + T - 1) / T, batch);
+  kern<<<grid, D::NT, D::SMEM, ctx->stream>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, nsplit, part);
 }
 
-// CTAs that share one 64 x 64 output tile (1: none): the smallest time of a model of the
-// grid.  Measured on a B200: a K stage of one CTA takes 3.3 us alone on its SM and 2.46 us
-// of the SM when others run beside it; the partial products cost one more launch (4 us) and
-// their bytes at 3 TB/s.
-struct SplitK {
-  int n;       // CTAs per tile
-  double us;   // modelled time of the product
+// Tile size and CTAs that share a tile's K stages (1: none): the smallest time of a model of
+// the grid.  Measured on a B200: a K stage of a 64 x 64 tile takes 3.3 us alone on its SM and
+// 2.46 us of the SM when others run beside it, one of a 32 x 32 tile 0.85 and 0.68 us; partial
+// products cost one more launch (2.2 us and 0.1 us each) and their bytes at 3 TB/s.  Small
+// tiles give 64 x 64 x 64 5.2 us (64 x 64 tiles: 13.2, shared 7.7), 448 x 448 x 64 7.1 us (12.4)
+// and, where the sums are ordered and may not be shared, 384 x 384 x 1536 103 us (300).
+struct DmmaPlan {
+  int tile, nsplit;
+  double us;
 };
-SplitK split_k(const Context* ctx, int M, int N, int K, int batch) {
-  const int64_t tiles = (int64_t)((M + dm::BM - 1) / dm::BM) * ((N + dm::BN - 1) / dm::BN) * batch;
+DmmaPlan dmma_plan(const Context* ctx, int M, int N, int K, int batch, bool share) {
   const int kall = (K + dm::BK - 1) / dm::BK;
-  int best = 1;
-  double tbest = 1e300;
-  for (int s = 1; s <= kall && s <= 64; ++s) {
-    const int64_t per_sm = (tiles * s + ctx->num_sms - 1) / ctx->num_sms;
-    double t = ((kall + s - 1) / s) * (per_sm == 1 ? 3.3 : 2.46 * (double)per_sm);
-    if (s > 1) t += 4.0 + (double)tiles * s * (dm::BM * dm::BN * 16 / 3e6);
-    if (t < tbest) {
-      tbest = t;
-      best = s;
+  DmmaPlan best{64, 1, 1e300};
+  for (int T : {64, 32}) {
+    const int64_t tiles = (int64_t)((M + T - 1) / T) * ((N + T - 1) / T) * batch;
+    if (T == 32 && (N + 31) / 32 > 65535) continue;   // grid limit
+    const double alone = T == 64 ? 3.3 : 0.85, shared = T == 64 ? 2.46 : 0.68;
+    for (int s = 1; s <= kall && s <= (share ? 64 : 1); ++s) {
+      const double per_sm = (double)((tiles * s + ctx->num_sms - 1) / ctx->num_sms);
+      double t = ((kall + s - 1) / s) * std::max(alone, shared * per_sm);
+      if (s > 1) t += 2.2 + 0.1 * s + (double)tiles * s * (T * T * 16 / 3e6);
+      if (t < best.us) best = {T, s, t};
     }
   }
-  return {best, tbest};
+  return best;
 }
 
 template <int OPA, int OPB>
@@ -393,17 +402,28 @@ void launch(Context* ctx, int M, int N, int K, double2 alpha, const dcplx* A, in
   }
   auto go = [&](auto beta_tag) {
     constexpr bool BETA = decltype(beta_tag)::value;
-    // the K stages of a tile are shared by several CTAs where the tiles alone would leave
-    // SMs idle (the long-K products of the pushes and of the QR, every product of a small state)
-    const int s = ctx->ordered_sums() ? 1 : split_k(ctx, M, N, K, batch).n;
+    // small tiles, and the K stages of a tile shared by several CTAs, where 64 x 64 tiles alone
+    // would leave SMs idle (the long-K products of the pushes and of the QR, every product of
+    // a small state)
+    DmmaPlan plan = dmma_plan(ctx, M, N, K, batch, !ctx->ordered_sums());
+    const int s = plan.nsplit;
     const int64_t len = (int64_t)M * N;
     double2* part = nullptr;
     if (s > 1) part = static_cast<double2*>(ctx->optional_buf("gemm_part", (size_t)len * s * batch * sizeof(double2)));
+    if (s > 1 && !part) plan = dmma_plan(ctx, M, N, K, batch, false);
+    auto run = [&](auto split_tag, auto tile_tag) {
+      launch_dmma<OPA, OPB, BETA, decltype(split_tag)::value, decltype(tile_tag)::value>(
+          ctx, part ? s : 1, part, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
+    };
+    using Big = std::integral_constant<int, 64>;
+    using Small = std::integral_constant<int, 32>;
     if (!part) {
-      launch_dmma<OPA, OPB, BETA, false>(ctx, 1, nullptr, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
+      if (plan.tile == 64) run(std::false_type{}, Big{});
+      else run(std::false_type{}, Small{});
       return;
     }
-    launch_dmma<OPA, OPB, BETA, true>(ctx, s, part, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, batch);
+    if (plan.tile == 64) run(std::true_type{}, Big{});
+    else run(std::true_type{}, Small{});
     const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((len + 255) / 256, ctx->num_sms * 8 / batch));
     k_sum_split<BETA><<<dim3(g, batch), 256, 0, ctx->stream>>>(M, N, s, part, alpha, beta, C, ldc, sC);
     ctx->n_kernels++;
@@ -419,7 +439,7 @@ void zgemm_fp64(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha, c
                 int64_t strideC, int batch) {
   if (M <= 0 || N <= 0 || batch <= 0) return;
   IMPS_REQUIRE(batch <= 65535, IMPS_INVALID_ARG, "zgemm: batch too large");
-  IMPS_REQUIRE((N + dm::BN - 1) / dm::BN <= 65535, IMPS_INVALID_ARG, "zgemm: N too large");
+  IMPS_REQUIRE((N + 31) / 32 <= 65535 * 2, IMPS_INVALID_ARG, "zgemm: N too large");
   if (K <= 0) {
     // C = beta C
     for (int b = 0; b < batch; ++b) {
@@ -432,7 +452,7 @@ void zgemm_fp64(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha, c
   }
   // products large enough: residue arithmetic on the int8 tensor cores
   if (batch == 1 && ctx->fp64_engine == 0 && !ctx->ordered_sums() &&
-      zgemm_modular(ctx, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, split_k(ctx, M, N, K, 1).us))
+      zgemm_modular(ctx, opA, opB, M, N, K, alpha, A, lda, B, ldb, beta, C, ldc, dmma_plan(ctx, M, N, K, 1, true).us))
     return;
   double2 a = make_double2(alpha.real(), alpha.imag()), bt = make_double2(beta.real(), beta.imag());
   bool use_beta = beta != cplx(0.0, 0.0);
