@@ -154,6 +154,7 @@ int imps_ctx_destroy(imps_ctx* h) {
     cudaEventDestroy(p.second.second);
   }
   for (auto e : c.event_pool) cudaEventDestroy(e);
+  c.pool->close();
   c.scratch.clear();
   c.optional.clear();
   c.red.release();
@@ -381,6 +382,7 @@ int imps_state_create(imps_ctx* h, int N, const int* d, const int* chi, imps_sta
     st->AR.resize(N);
     st->C.resize(N);
     st->AC.resize(N);
+    for (auto* f : {&st->AL, &st->AR, &st->C, &st->AC}) h->c.pooled(*f);
     for (int l = 0; l < N; ++l) {
       size_t se = st->site_elems(l) * sizeof(imps::dcplx), be = st->bond_elems(l) * sizeof(imps::dcplx);
       st->AL[l].ensure(se);

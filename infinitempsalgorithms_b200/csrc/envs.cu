@@ -326,6 +326,7 @@ void envs_allocate(imps_envs* E, const imps_state* st, const imps_mpo* H) {
   E->init_lefts.resize(N);
   E->init_rights.resize(N);
   E->GLp.resize(N);
+  for (auto* f : {&E->lefts, &E->rights, &E->init_lefts, &E->init_rights, &E->GLp}) E->ctx->pooled(*f);
   E->GLp_valid.assign(N, false);
   E->hest_ac.assign(N, 0.0);
   E->hest_c.assign(N, 0.0);

@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <set>
 #include <tuple>
 #include <stdexcept>
@@ -52,27 +53,69 @@ struct Error : public std::runtime_error {
 // ---------------------------------------------------------------------------
 // Device buffers
 // ---------------------------------------------------------------------------
+// Blocks given up by a context's states and environments, kept for its next ones: a run
+// makes a state and an environment per call, and a cudaMalloc / cudaFree pair costs 0.7 ms
+// (now and then a second, when the driver unmaps) and synchronises the device.  The context's
+// objects use its one stream, so a block may be handed on while earlier work on it is queued.
+// Bounded, exact sizes only; emptied when an allocation fails anywhere and when the context
+// goes; an object that outlives its context frees its blocks itself.
+class BlockPool {
+ public:
+  BlockPool();
+  ~BlockPool();
+  void* take(size_t bytes);               // nullptr: none of this size
+  bool give(void* ptr, size_t bytes);     // false: not kept
+  void trim();                            // frees what is idle
+  void close();                           // trim, and keep nothing from now on
+  static void trim_all();
+
+ private:
+  static constexpr size_t kMost = (size_t)256 << 20;
+  std::mutex mu_;
+  std::multimap<size_t, void*> idle_;
+  size_t held_ = 0;
+  bool open_ = true;
+};
+
 struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;
+  std::shared_ptr<BlockPool> pool;   // where blocks come from and go to, if anywhere
   DevBuf() = default;
   explicit DevBuf(size_t b) { alloc(b); }
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
-  DevBuf(DevBuf&& o) noexcept : ptr(o.ptr), bytes(o.bytes) { o.ptr = nullptr; o.bytes = 0; }
+  DevBuf(DevBuf&& o) noexcept : ptr(o.ptr), bytes(o.bytes), pool(std::move(o.pool)) { o.ptr = nullptr; o.bytes = 0; }
   DevBuf& operator=(DevBuf&& o) noexcept {
-    if (this != &o) { release(); ptr = o.ptr; bytes = o.bytes; o.ptr = nullptr; o.bytes = 0; }
+    if (this != &o) {
+      release();
+      ptr = o.ptr;
+      bytes = o.bytes;
+      pool = std::move(o.pool);
+      o.ptr = nullptr;
+      o.bytes = 0;
+    }
     return *this;
   }
   ~DevBuf() { release(); }
   void alloc(size_t b) {
     release();
-    if (b) IMPS_CUDA(cudaMalloc(&ptr, b));
+    if (b && pool) ptr = pool->take(b);
+    if (b && !ptr && cudaMalloc(&ptr, b) != cudaSuccess) {
+      cudaGetLastError();
+      ptr = nullptr;
+      BlockPool::trim_all();
+      IMPS_CUDA(cudaMalloc(&ptr, b));
+    }
     bytes = b;
   }
   // Grow-only: keeps the allocation when it is already large enough.
   void ensure(size_t b) { if (b > bytes) alloc(b); }
-  void release() { if (ptr) cudaFree(ptr); ptr = nullptr; bytes = 0; }
+  void release() {
+    if (ptr && !(pool && pool->give(ptr, bytes))) cudaFree(ptr);
+    ptr = nullptr;
+    bytes = 0;
+  }
   dcplx* z() const { return static_cast<dcplx*>(ptr); }
   double* d() const { return static_cast<double*>(ptr); }
 };
@@ -102,6 +145,11 @@ struct Context {
   bool adaptive_slices = false;
   int fp64_engine = 0;       // FP64 GEMM kernel: 0 = DMMA tensor cores, 1 = SIMT DFMA (env IMPS_FP64_ENGINE)
   std::string last_error;
+  // blocks of the context's states and environments between objects
+  std::shared_ptr<BlockPool> pool = std::make_shared<BlockPool>();
+  void pooled(std::vector<DevBuf>& v) const {
+    for (DevBuf& b : v) b.pool = pool;
+  }
   // named grow-only scratch buffers
   std::map<std::string, DevBuf> scratch;
   // reduction scratch (per-block partials) and pinned host staging

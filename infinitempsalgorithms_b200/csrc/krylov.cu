@@ -34,6 +34,13 @@ std::vector<cplx> herm_part(const std::vector<cplx>& H, int ldh, int m) {
   return S;
 }
 
+// A Krylov step ends with a small dense problem on the host that decides whether another
+// step follows.  For vectors up to this length (a matvec of some 200 us at most) the next
+// matvec is queued before the host turns to it, so the device works meanwhile; the one of
+// the last step is thrown away.  Longer vectors' matvecs hide the host's time less than the
+// extra one costs.
+constexpr int64_t kAheadMax = (int64_t)1 << 18;
+
 void phase_align(Context* ctx, int64_t n, const dcplx* x0n, dcplx* x) {
   cplx ov = zdotc(ctx, n, x0n, x);
   double a = std::abs(ov);
@@ -61,12 +68,19 @@ KrylovResult lanczos_eigsolve(Context* ctx, int64_t n, const LinOp& A, const dcp
   int nvec = 1;
   std::vector<double> theta;
   std::vector<cplx> U;
+  bool ahead = false;   // the next matvec is already queued
   while (true) {
     const int k = nvec - 1;
     dcplx* w = V + n * (int64_t)nvec;
-    A(V + n * (int64_t)k, w);
+    if (!ahead) A(V + n * (int64_t)k, w);
+    ahead = false;
     res.numops++;
     double beta = cgs2(ctx, n, nvec, V, w, h);
+    if (n <= kAheadMax && k + 1 < kdim && beta > 1e-100) {
+      zscal(ctx, n, 1.0 / beta, w);
+      A(w, w + n);
+      ahead = true;
+    }
     for (int i = 0; i <= k; ++i) H[i + (size_t)ldh * k] = h[i];
     H[k + 1 + (size_t)ldh * k] = beta;
     const int m = k + 1;
@@ -114,7 +128,7 @@ KrylovResult lanczos_eigsolve(Context* ctx, int64_t n, const LinOp& A, const dcp
       nvec = keep + 1;
       res.numiter++;
     } else {
-      zscal(ctx, n, 1.0 / beta, w);
+      if (!ahead) zscal(ctx, n, 1.0 / beta, w);
       nvec++;
     }
   }
@@ -230,12 +244,19 @@ KrylovResult exponentiate(Context* ctx, int64_t n, const LinOp& A, cplx t, const
     cplx tau = remaining;
     int m = 0;
     double err = 0.0;
+    bool ahead = false;   // the next matvec is already queued
     while (true) {
       const int k = m;
       dcplx* w = V + n * (int64_t)(k + 1);
-      A(V + n * (int64_t)k, w);
+      if (!ahead) A(V + n * (int64_t)k, w);
+      ahead = false;
       res.numops++;
       double hn = cgs2(ctx, n, k + 1, V, w, h);
+      if (n <= kAheadMax && k + 1 < kdim && hn > 1e-100) {
+        zscal(ctx, n, 1.0 / hn, w);
+        A(w, w + n);
+        ahead = true;
+      }
       for (int i = 0; i <= k; ++i) H[i + (size_t)ldh * k] = h[i];
       H[k + 1 + (size_t)ldh * k] = hn;
       m = k + 1;
@@ -254,7 +275,7 @@ KrylovResult exponentiate(Context* ctx, int64_t n, const LinOp& A, cplx t, const
         }
         break;
       }
-      zscal(ctx, n, 1.0 / hn, w);
+      if (!ahead) zscal(ctx, n, 1.0 / hn, w);
     }
     std::vector<cplx> coef(m);
     for (int i = 0; i < m; ++i) coef[i] = beta * E[i];
@@ -290,12 +311,19 @@ KrylovResult arnoldi_dominant(Context* ctx, int64_t n, const LinOp& A, const dcp
   std::vector<cplx> H((size_t)ldh * kdim, 0.0), h, lam, Y;
   res.numiter = 1;
   int nvec = 1;
+  bool ahead = false;   // the next matvec is already queued
   while (true) {
     const int k = nvec - 1;
     dcplx* w = V + n * (int64_t)nvec;
-    A(V + n * (int64_t)k, w);
+    if (!ahead) A(V + n * (int64_t)k, w);
+    ahead = false;
     res.numops++;
     double hn = cgs2(ctx, n, nvec, V, w, h);
+    if (n <= kAheadMax && k + 1 < kdim && hn > 1e-100) {
+      zscal(ctx, n, 1.0 / hn, w);
+      A(w, w + n);
+      ahead = true;
+    }
     for (int i = 0; i <= k; ++i) H[i + (size_t)ldh * k] = h[i];
     H[k + 1 + (size_t)ldh * k] = hn;
     const int m = k + 1;
@@ -360,7 +388,7 @@ KrylovResult arnoldi_dominant(Context* ctx, int64_t n, const LinOp& A, const dcp
       nvec = keep + 1;
       res.numiter++;
     } else {
-      zscal(ctx, n, 1.0 / hn, w);
+      if (!ahead) zscal(ctx, n, 1.0 / hn, w);
       nvec++;
     }
   }

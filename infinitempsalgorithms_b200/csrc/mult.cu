@@ -504,6 +504,7 @@ imps_state* mult_guess(Context* ctx, const imps_mpo* W, const imps_state* ket, i
     st->AR.resize(N);
     st->C.resize(N);
     st->AC.resize(N);
+    for (auto* f : {&st->AL, &st->AR, &st->C, &st->AC}) ctx->pooled(*f);
     for (int l = 0; l < N; ++l) {
       st->AL[l].alloc(st->site_elems(l) * sizeof(dcplx));
       st->AR[l].alloc(st->site_elems(l) * sizeof(dcplx));

@@ -7,6 +7,8 @@
 #include <vector>
 #include <cmath>
 #include <cstring>
+#include <system_error>
+#include <thread>
 
 namespace imps {
 
@@ -469,6 +471,63 @@ void check_launch(Context* ctx) {
 
 }  // namespace
 
+namespace {
+// never destroyed: a context may go after the library's statics
+std::mutex& pools_mu() {
+  static auto* m = new std::mutex;
+  return *m;
+}
+std::set<BlockPool*>& pools() {
+  static auto* s = new std::set<BlockPool*>;
+  return *s;
+}
+}  // namespace
+
+BlockPool::BlockPool() {
+  std::lock_guard<std::mutex> lock(pools_mu());
+  pools().insert(this);
+}
+BlockPool::~BlockPool() {
+  {
+    std::lock_guard<std::mutex> lock(pools_mu());
+    pools().erase(this);
+  }
+  trim();
+}
+void* BlockPool::take(size_t bytes) {
+  std::lock_guard<std::mutex> lock(mu_);
+  auto it = idle_.find(bytes);
+  if (it == idle_.end()) return nullptr;
+  void* p = it->second;
+  idle_.erase(it);
+  held_ -= bytes;
+  return p;
+}
+bool BlockPool::give(void* ptr, size_t bytes) {
+  std::lock_guard<std::mutex> lock(mu_);
+  if (!open_ || held_ + bytes > kMost) return false;
+  idle_.emplace(bytes, ptr);
+  held_ += bytes;
+  return true;
+}
+void BlockPool::trim() {
+  std::lock_guard<std::mutex> lock(mu_);
+  for (auto& kv : idle_) cudaFree(kv.second);
+  idle_.clear();
+  held_ = 0;
+}
+void BlockPool::close() {
+  {
+    std::lock_guard<std::mutex> lock(mu_);
+    open_ = false;
+  }
+  trim();
+}
+void BlockPool::trim_all() {
+  std::lock_guard<std::mutex> lock(pools_mu());
+  for (BlockPool* p : pools()) p->trim();
+}
+
 double* Context::pinned(size_t bytes) {
   if (bytes > host_pinned_bytes) {
     if (host_pinned) cudaFreeHost(host_pinned);
@@ -529,18 +588,124 @@ void check_device_errors(Context* ctx) {
   err_after_sync(ctx);
 }
 
+namespace {
+// Large arrays of the caller's pageable memory go through page-locked chunks, moved by a few
+// threads: one thread's copies (and, into a fresh array, its page faults) take longer than
+// the transfer.  Each thread owns a contiguous part and two chunks and overlaps its memory
+// copies with its transfers on the context's stream.  One staging area per process; a second
+// context that finds it taken, small arrays and page-locked ones use the plain copy.
+constexpr int kStageThreads = 4;
+constexpr size_t kStageChunk = (size_t)1 << 20, kStageMin = (size_t)4 << 20;
+
+struct Staging {
+  std::mutex mu;
+  char* mem = nullptr;   // kStageThreads x 2 chunks
+};
+Staging& staging() {
+  static auto* s = new Staging;   // as long as the process, like the driver's own
+  return *s;
+}
+
+bool page_locked(const void* p) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return true;   // leave it to the plain copy
+  }
+  return a.type != cudaMemoryTypeUnregistered;
+}
+
+cudaError_t stage_part(const Context* ctx, char* dev, char* host, size_t bytes, bool to_device, char* buf) {
+  cudaError_t e = cudaSetDevice(ctx->device);
+  cudaEvent_t ev[2] = {nullptr, nullptr};
+  for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
+  const size_t n = (bytes + kStageChunk - 1) / kStageChunk;
+  auto len = [&](size_t i) { return std::min(kStageChunk, bytes - i * kStageChunk); };
+  for (size_t i = 0; i < n + 1 && e == cudaSuccess; ++i) {
+    char* c = buf + (i & 1) * kStageChunk;
+    if (to_device) {
+      if (i == n) break;
+      if (i >= 2) e = cudaEventSynchronize(ev[i & 1]);
+      if (e != cudaSuccess) break;
+      std::memcpy(c, host + i * kStageChunk, len(i));
+      e = cudaMemcpyAsync(dev + i * kStageChunk, c, len(i), cudaMemcpyHostToDevice, ctx->stream);
+      if (e == cudaSuccess) e = cudaEventRecord(ev[i & 1], ctx->stream);
+    } else {
+      // chunk i is on its way while chunk i - 1 is copied out
+      if (i < n) {
+        e = cudaMemcpyAsync(c, dev + i * kStageChunk, len(i), cudaMemcpyDeviceToHost, ctx->stream);
+        if (e == cudaSuccess) e = cudaEventRecord(ev[i & 1], ctx->stream);
+      }
+      if (i > 0 && e == cudaSuccess) {
+        e = cudaEventSynchronize(ev[(i - 1) & 1]);
+        if (e == cudaSuccess) std::memcpy(host + (i - 1) * kStageChunk, buf + ((i - 1) & 1) * kStageChunk, len(i - 1));
+      }
+    }
+  }
+  for (auto v : ev)
+    if (v) {
+      const cudaError_t w = cudaEventSynchronize(v);   // this part's chunks are free again
+      if (e == cudaSuccess) e = w;
+      cudaEventDestroy(v);
+    }
+  return e;
+}
+
+// false: not staged, nothing done
+bool staged_copy(Context* ctx, void* dev, void* host, size_t bytes, bool to_device) {
+  if (bytes < kStageMin || std::thread::hardware_concurrency() < 2 * kStageThreads || page_locked(host)) return false;
+  Staging& s = staging();
+  std::unique_lock<std::mutex> lock(s.mu, std::try_to_lock);
+  if (!lock.owns_lock()) return false;
+  if (!s.mem &&
+      cudaHostAlloc((void**)&s.mem, 2 * kStageThreads * kStageChunk, cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    s.mem = nullptr;
+    return false;
+  }
+  const size_t part = ((bytes + kStageThreads - 1) / kStageThreads + 4095) / 4096 * 4096;
+  cudaError_t err[kStageThreads] = {};
+  auto work = [&](int t) {
+    const size_t o = std::min(bytes, part * t), b = std::min(part, bytes - o);
+    if (b)
+      err[t] = stage_part(ctx, static_cast<char*>(dev) + o, static_cast<char*>(host) + o, b, to_device,
+                          s.mem + 2 * kStageChunk * t);
+  };
+  std::thread th[kStageThreads];
+  bool here[kStageThreads] = {true};
+  for (int t = 1; t < kStageThreads; ++t) {
+    try {
+      th[t] = std::thread(work, t);
+    } catch (const std::system_error&) {
+      here[t] = true;   // no thread to be had
+    }
+  }
+  for (int t = 0; t < kStageThreads; ++t)
+    if (here[t]) work(t);
+  for (auto& t : th)
+    if (t.joinable()) t.join();
+  for (cudaError_t e : err) IMPS_CUDA(e);
+  return true;
+}
+}  // namespace
+
 void upload(Context* ctx, void* dst, const void* src, size_t bytes) {
   if (!bytes) return;
-  IMPS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
+  if (!staged_copy(ctx, dst, const_cast<void*>(src), bytes, true))
+    IMPS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
   err_copy(ctx);
   IMPS_CUDA(cudaStreamSynchronize(ctx->stream));
   err_after_sync(ctx);
 }
 void download(Context* ctx, void* dst, const void* src, size_t bytes) {
   if (!bytes) return;
-  IMPS_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+  // a solver's scalars through page-locked memory: half the latency of a pageable copy
+  void* to = bytes <= 65536 ? (void*)ctx->pinned(bytes) : dst;
+  if (!staged_copy(ctx, const_cast<void*>(src), dst, bytes, false))
+    IMPS_CUDA(cudaMemcpyAsync(to, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
   err_copy(ctx);
   IMPS_CUDA(cudaStreamSynchronize(ctx->stream));
+  if (to != dst) std::memcpy(dst, to, bytes);
   err_after_sync(ctx);
 }
 
