@@ -20,9 +20,9 @@
 // NaN or an Inf are recognised and their elements computed by a plain FP64 loop.
 //
 // The four kernels: partial row norms, residue planes, the int8 GEMMs, the reconstruction.
-// Measured (B200): 6144 x 4096 x 1024 1.21 ms = 33 + 141 + 651 + 375 us (6.50 ms on the FP64
-// tensor cores), 4096 x 1024 x 6144 1.09 ms = 90 + 405 + 524 + 69 us (6.57 ms), i.e. 171 and
-// 188 TFLOP/s of FP64 products; error against 80-bit sums 1e-16 .. 3e-16 of the result's norm
+// Measured (B200): 6144 x 4096 x 1024 1.15 ms = 35 + 139 + 650 + 326 us (6.50 ms on the FP64
+// tensor cores), 4096 x 1024 x 6144 1.08 ms = 90 + 399 + 522 + 64 us (6.57 ms), i.e. 179 and
+// 191 TFLOP/s of FP64 products; error against 80-bit sums 1e-16 .. 3e-16 of the result's norm
 // for K = 256 .. 8192 (FP64 tensor cores 8e-16 .. 6e-15).
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -30,6 +30,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <utility>
 
 #include "gemm_modular.h"
 #include "split_gemm.h"
@@ -128,6 +129,10 @@ constexpr ModTables make_tables() {
   }
   return t;
 }
+// In unrolled code the constants of modulus I are immediates (a cold constant cache costs a
+// short kernel microseconds); the GEMM's epilogue, which meets one modulus per tile, reads
+// them from constant memory.
+constexpr ModTables kT = make_tables();
 __constant__ ModTables kTab = make_tables();
 
 // ---------------------------------------------------------------------------
@@ -240,19 +245,48 @@ __device__ __forceinline__ unsigned pack4(int r0, int r1, int r2, int r3) {
   return __byte_perm(__byte_perm(r0, r1, 0x0040), __byte_perm(r2, r3, 0x0040), 0x5410);
 }
 
-// Residue planes.  A block covers 32 lines x 64 k of the padded extent, transposed through
-// shared memory; a thread turns 8 consecutive k of a line into 8 bytes of each plane.
-// Bound by its integer instructions (about 300 a complex element) and the 32 plane bytes.
-__global__ void __launch_bounds__(256, 4) k_mod_split(const ModOperand a, const ModOperand b) {
-  __shared__ double2 tile[32][65];
-  __shared__ int ex[32];
+// The u and v bytes of 8 integers modulo modulus I into its two planes.
+template <int I>
+__device__ __forceinline__ void split_modulus(const unsigned (&xlo)[8], const unsigned (&xhi)[8],
+                                              const unsigned (&ylo)[8], const unsigned (&yhi)[8], int8_t* out,
+                                              int64_t plane) {
+  constexpr int wal = kT.wa_lo[I], wah = kT.wa_hi[I], wbl = kT.wb_lo[I], wbh = kT.wb_hi[I];
+  constexpr int offu = kT.off_u[I], offv = kT.off_v[I], p = kT.p[I];
+  constexpr float inv = kT.inv[I];
+  int u[8], v[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const int sx = dp4a_us(xhi[c], wah, dp4a_us(xlo[c], wal, offu));
+    const int sy = dp4a_us(yhi[c], wbh, dp4a_us(ylo[c], wbl, 0));
+    u[c] = mod_byte(sx + sy, p, inv);
+    v[c] = mod_byte(sx - sy + offv, p, inv);
+  }
+  *reinterpret_cast<uint2*>(out + plane * I) = make_uint2(pack4(u[0], u[1], u[2], u[3]), pack4(u[4], u[5], u[6], u[7]));
+  *reinterpret_cast<uint2*>(out + plane * (NMOD + I)) =
+      make_uint2(pack4(v[0], v[1], v[2], v[3]), pack4(v[4], v[5], v[6], v[7]));
+}
+template <int... I>
+__device__ __forceinline__ void split_moduli(const unsigned (&xlo)[8], const unsigned (&xhi)[8],
+                                             const unsigned (&ylo)[8], const unsigned (&yhi)[8], int8_t* out,
+                                             int64_t plane, std::integer_sequence<int, I...>) {
+  (split_modulus<I>(xlo, xhi, ylo, yhi, out, plane), ...);
+}
+
+// Residue planes.  A block covers SPL_LINES lines x 64 k of the padded extent, transposed
+// through shared memory; a thread turns 8 consecutive k of a line into 8 bytes of each plane.
+// Bound by its integer instructions (about 250 a complex element) and the 32 plane bytes;
+// small blocks let one's loads run beside another's arithmetic.
+constexpr int SPL_LINES = 16, SPL_NT = SPL_LINES * 8;
+__global__ void __launch_bounds__(SPL_NT, 1024 / SPL_NT) k_mod_split(const ModOperand a, const ModOperand b) {
+  __shared__ double2 tile[SPL_LINES][65];
+  __shared__ int ex[SPL_LINES];
   const bool first = (int)blockIdx.x < a.nblocks_split;
   const ModOperand& o = first ? a : b;
   const int blk = first ? blockIdx.x : blockIdx.x - a.nblocks_split;
   const int nk = (int)(o.Kp / 64);
-  const int k0 = (blk % nk) * 64, l0 = (blk / nk) * 32;
+  const int k0 = (blk % nk) * 64, l0 = (blk / nk) * SPL_LINES;
   const int tid = threadIdx.x;
-  if (tid < 32) {
+  if (tid < SPL_LINES) {
     const int e = l0 + tid < o.lines ? line_exponent(o, l0 + tid) : 0;
     ex[tid] = e == EXP_NONFINITE ? 0 : e;
     if (k0 == 0 && l0 + tid < o.lines) o.expo[l0 + tid] = e;
@@ -260,12 +294,12 @@ __global__ void __launch_bounds__(256, 4) k_mod_split(const ModOperand a, const 
   if (o.kcontig) {
     const int kx = tid & 63, ly = tid >> 6;
 #pragma unroll
-    for (int r = 0; r < 32; r += 4) {
+    for (int r = 0; r < SPL_LINES; r += SPL_NT / 64) {
       const int l = l0 + r + ly, k = k0 + kx;
       tile[r + ly][kx] = (l < o.lines && k < o.K) ? o.X[k + o.ld * l] : make_double2(0.0, 0.0);
     }
   } else {
-    const int lx = tid & 31, ky = tid >> 5;
+    const int lx = tid % SPL_LINES, ky = tid / SPL_LINES;
 #pragma unroll
     for (int r = 0; r < 64; r += 8) {
       const int l = l0 + lx, k = k0 + r + ky;
@@ -290,21 +324,7 @@ __global__ void __launch_bounds__(256, 4) k_mod_split(const ModOperand a, const 
   }
   int8_t* out = o.planes + (int64_t)(l0 + ll) * o.Kp + k0 + 8 * kq;
   const int64_t plane = (int64_t)o.lines * o.Kp;
-#pragma unroll
-  for (int i = 0; i < NMOD; ++i) {
-    int u[8], v[8];
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const int sx = dp4a_us(xhi[c], kTab.wa_hi[i], dp4a_us(xlo[c], kTab.wa_lo[i], kTab.off_u[i]));
-      const int sy = dp4a_us(yhi[c], kTab.wb_hi[i], dp4a_us(ylo[c], kTab.wb_lo[i], 0));
-      u[c] = mod_byte(sx + sy, kTab.p[i], kTab.inv[i]);
-      v[c] = mod_byte(sx - sy + kTab.off_v[i], kTab.p[i], kTab.inv[i]);
-    }
-    *reinterpret_cast<uint2*>(out + plane * i) =
-        make_uint2(pack4(u[0], u[1], u[2], u[3]), pack4(u[4], u[5], u[6], u[7]));
-    *reinterpret_cast<uint2*>(out + plane * (NMOD + i)) =
-        make_uint2(pack4(v[0], v[1], v[2], v[3]), pack4(v[4], v[5], v[6], v[7]));
-  }
+  split_moduli(xlo, xhi, ylo, yhi, out, plane, std::make_integer_sequence<int, NMOD>{});
 }
 
 // ---------------------------------------------------------------------------
@@ -596,6 +616,28 @@ struct ModJoinArgs {
   int64_t ldc;
 };
 
+template <int I>
+__device__ __forceinline__ void join_modulus(unsigned wu, unsigned wv, unsigned (&x1)[4], unsigned (&y1)[4],
+                                             double (&x2)[4], double (&y2)[4]) {
+  constexpr unsigned re1 = kT.re1[I], im1 = kT.im1[I];
+  constexpr double re2 = kT.re2[I], im2 = kT.im2[I];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const unsigned u = __byte_perm(wu, 0, 0x4440 + e), v = __byte_perm(wv, 0, 0x4440 + e);
+    const unsigned sp = u + v, sm = u - v + 256u;
+    x1[e] += sp * re1;
+    y1[e] += sm * im1;
+    x2[e] = fma(__hiloint2double(0x43300000, (int)sp) - 4503599627370496.0, re2, x2[e]);
+    y2[e] = fma(__hiloint2double(0x43300000, (int)sm) - 4503599627370496.0, im2, y2[e]);
+  }
+}
+template <int... I>
+__device__ __forceinline__ void join_moduli(const unsigned (&wu)[NMOD], const unsigned (&wv)[NMOD], unsigned (&x1)[4],
+                                            unsigned (&y1)[4], double (&x2)[4], double (&y2)[4],
+                                            std::integer_sequence<int, I...>) {
+  (join_modulus<I>(wu[I], wv[I], x1, y1, x2, y2), ...);
+}
+
 // A block joins a 64 x 16 tile of C: a thread reads 4 columns of a row from the 32 planes
 // and sums the CRT fractions of its 4 elements, modulo 1 in 32-bit integers for their
 // leading bits, in FP64 below; the tile goes through shared memory so that C is written
@@ -613,14 +655,16 @@ __global__ void __launch_bounds__(256, 3) k_mod_join(const ModJoinArgs g, const 
   if (row < g.M) {
     const uint8_t* src = g.res + (int64_t)n0 * g.M + (int64_t)row * 16 + c4;
     const int64_t plane = (int64_t)g.M * g.ldo;
+    constexpr unsigned re1_0 = kT.re1_0, im1_0 = kT.im1_0;
+    constexpr double re2_0 = kT.re2_0, im2_0 = kT.im2_0, P = kT.P;
     unsigned x1[4], y1[4];
     double x2[4], y2[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      x1[e] = kTab.re1_0;
-      y1[e] = kTab.im1_0;
-      x2[e] = kTab.re2_0;
-      y2[e] = kTab.im2_0;
+      x1[e] = re1_0;
+      y1[e] = im1_0;
+      x2[e] = re2_0;
+      y2[e] = im2_0;
     }
     // all 32 loads in flight before the first use
     unsigned wu[NMOD], wv[NMOD];
@@ -629,18 +673,7 @@ __global__ void __launch_bounds__(256, 3) k_mod_join(const ModJoinArgs g, const 
       wu[i] = __ldcs(reinterpret_cast<const unsigned*>(src + plane * i));
       wv[i] = __ldcs(reinterpret_cast<const unsigned*>(src + plane * (NMOD + i)));
     }
-#pragma unroll
-    for (int i = 0; i < NMOD; ++i) {
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const unsigned u = __byte_perm(wu[i], 0, 0x4440 + e), v = __byte_perm(wv[i], 0, 0x4440 + e);
-        const unsigned sp = u + v, sm = u - v + 256u;
-        x1[e] += sp * kTab.re1[i];
-        y1[e] += sm * kTab.im1[i];
-        x2[e] = fma(__hiloint2double(0x43300000, (int)sp) - 4503599627370496.0, kTab.re2[i], x2[e]);
-        y2[e] = fma(__hiloint2double(0x43300000, (int)sm) - 4503599627370496.0, kTab.im2[i], y2[e]);
-      }
-    }
+    join_moduli(wu, wv, x1, y1, x2, y2, std::make_integer_sequence<int, NMOD>{});
     const int ea = g.ea[row];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
@@ -658,8 +691,8 @@ __global__ void __launch_bounds__(256, 3) k_mod_join(const ModJoinArgs g, const 
       } else {
         const int t = max(-(ea + eb), -2000), th = t / 2;
         const double s1 = pow2(th), s2 = pow2(t - th);
-        v.x = fma((double)(int)x1[e], 0x1p-32, x2[e]) * kTab.P * s1 * s2;
-        v.y = fma((double)(int)y1[e], 0x1p-32, y2[e]) * kTab.P * s1 * s2;
+        v.x = fma((double)(int)x1[e], 0x1p-32, x2[e]) * P * s1 * s2;
+        v.y = fma((double)(int)y1[e], 0x1p-32, y2[e]) * P * s1 * s2;
       }
       tile[c4 + e][r] = v;
     }
@@ -744,11 +777,11 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
     o->nchunk = nchunk;
     o->kchunk = (K + nchunk - 1) / nchunk;
     o->nblocks_norm = (o->lines + (o->kcontig ? 31 : 63)) / (o->kcontig ? 32 : 64) * nchunk;
-    o->nblocks_split = (int)(Kp / 64) * ((o->lines + 31) / 32);
+    o->nblocks_split = (int)(Kp / 64) * ((o->lines + SPL_LINES - 1) / SPL_LINES);
   }
   ScopedTimer tm(ctx, "zgemm_modular", 8.0 * M * (double)N * K);
   k_mod_norms<<<a.nblocks_norm + b.nblocks_norm, 256, 0, ctx->stream>>>(a, b);
-  k_mod_split<<<a.nblocks_split + b.nblocks_split, 256, 0, ctx->stream>>>(a, b);
+  k_mod_split<<<a.nblocks_split + b.nblocks_split, SPL_NT, 0, ctx->stream>>>(a, b);
   static DeviceOnce attr;
   attr.run(ctx->device, [] {
     IMPS_CUDA(cudaFuncSetAttribute(k_mod_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, GSMEM));
