@@ -60,6 +60,128 @@ __global__ void __launch_bounds__(128) k_level_mix(const MixArgs a, const double
   }
 }
 
+// The whole AC application of a small state in one launch (GEMM, level mix, GEMM as above), a
+// cluster of 8 CTAs: CTA r takes columns [Dr r / 8, Dr (r + 1) / 8) of x through both steps,
+//   T1 = GL x,  T2 = W T1,  y_r = T2 GR  (its share of the sum over c),
+// and then adds element block r of the eight partial results in rank order.  All operands
+// and intermediates in shared memory; a thread forms 4 columns of a row of a product.  Bound by
+// launch and shared-memory latency: TFIM D = 16 8.2 us a call, 16.4 us in three
+// launches; the two meet near 7e5 complex multiply-adds (XXZ D = 32 18.5 and 20 us, TFIM
+// D = 40 22.5 and 19 us).
+constexpr int kSmallCl = 8, kSmallNt = 256;
+
+struct SmallShape {
+  int Dl, Dr, m, d;
+  int64_t gr_ld;
+  int wsz;       // elements of the MPO tensor
+};
+struct SmallLayout {   // offsets into shared memory, in elements
+  int gl, x, gr, w, t1, t2, y, total;
+};
+__host__ __device__ inline SmallLayout small_layout(const SmallShape& h, int nq) {
+  const int nc = (h.Dr + kSmallCl - 1) / kSmallCl;
+  SmallLayout o;
+  o.gl = 0;
+  o.x = o.gl + h.Dl * h.m * h.Dl;
+  o.gr = o.x + h.Dl * h.d * nc;
+  o.w = o.gr + nc * nq * h.Dr;
+  o.t1 = o.w + h.wsz;
+  o.t2 = o.t1 + h.Dl * h.m * h.d * nc;
+  o.y = o.t2 + h.Dl * h.d * nc * nq;
+  o.total = o.y + h.Dl * h.d * h.Dr;
+  return o;
+}
+
+// out[r + rows c] = sum_k A[r + rows k] B[c, k], 4 columns c a thread; B(c, k) = b[c cs + k ks]
+__device__ __forceinline__ void small_gemm(int rows, int cols, int K, const double2* a, const double2* b, int cs, int ks,
+                                           double2* out) {
+  const int groups = (cols + 3) / 4;
+  for (int t = threadIdx.x; t < rows * groups; t += kSmallNt) {
+    const int r = t % rows, c0 = t / rows * 4;
+    double2 acc[4];
+    const double2* bp[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc[j] = make_double2(0.0, 0.0);
+      bp[j] = b + min(c0 + j, cols - 1) * cs;
+    }
+#pragma unroll 4
+    for (int k = 0; k < K; ++k) {
+      const double2 v = a[r + rows * k];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const double2 w = bp[j][k * ks];
+        acc[j].x = fma(v.x, w.x, fma(-v.y, w.y, acc[j].x));
+        acc[j].y = fma(v.x, w.y, fma(v.y, w.x, acc[j].y));
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (c0 + j < cols) out[r + rows * (c0 + j)] = acc[j];
+  }
+}
+
+__global__ void __cluster_dims__(kSmallCl, 1, 1) __launch_bounds__(kSmallNt)
+    k_ac_small(const SmallShape h, const MixArgs mx, const double2* __restrict__ GL, const double2* __restrict__ GR,
+               const double2* __restrict__ W, const double2* __restrict__ x, double2* __restrict__ y) {
+  extern __shared__ __align__(16) double2 sm[];
+  const SmallLayout o = small_layout(h, mx.nq);
+  const int tid = threadIdx.x;
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int c0 = h.Dr * (int)rank / kSmallCl, nc = h.Dr * ((int)rank + 1) / kSmallCl - c0;
+  const int rows1 = h.Dl * h.m, rowsY = h.Dl * h.d, nk = nc * mx.nq;
+  for (int e = tid; e < rows1 * h.Dl; e += kSmallNt) sm[o.gl + e] = GL[e];
+  for (int e = tid; e < rowsY * nc; e += kSmallNt) sm[o.x + e] = x[(int64_t)rowsY * c0 + e];
+  for (int e = tid; e < nk * h.Dr; e += kSmallNt) {
+    const int k = e % nk, c = e / nk;   // k = cl + nc iq
+    sm[o.gr + e] = GR[c0 + k % nc + h.Dr * mx.qval[k / nc] + h.gr_ld * c];
+  }
+  for (int e = tid; e < h.wsz; e += kSmallNt) sm[o.w + e] = W[e];
+  __syncthreads();
+  // T1[(b, i), (s, c)]
+  if (nc > 0) small_gemm(rows1, h.d * nc, h.Dl, sm + o.gl, sm + o.x, h.Dl, 1, sm + o.t1);
+  __syncthreads();
+  // T2[(b, u), (c, iq)]
+  for (int t = tid; t < rowsY * nk; t += kSmallNt) {
+    const int b = t % h.Dl, u = t / h.Dl % h.d, k = t / rowsY, cl = k % nc, iq = k / nc;
+    double2 acc = make_double2(0.0, 0.0);
+    for (int e = mx.qstart[iq]; e < mx.qstart[iq + 1]; ++e) {
+      const int r = mx.rval[e];
+      for (int s = 0; s < h.d; ++s) {
+        const double2 v = sm[o.t1 + b + h.Dl * r + rows1 * (s + h.d * cl)];
+        const double2 w = sm[o.w + r + mx.R * (u + h.d * (mx.qval[iq] + mx.Q * s))];
+        acc.x = fma(w.x, v.x, fma(-w.y, v.y, acc.x));
+        acc.y = fma(w.x, v.y, fma(w.y, v.x, acc.y));
+      }
+    }
+    sm[o.t2 + t] = acc;
+  }
+  __syncthreads();
+  small_gemm(rowsY, h.Dr, nk, sm + o.t2, sm + o.gr, nk, 1, sm + o.y);
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const int ny = rowsY * h.Dr, e0 = (int)((int64_t)ny * rank / kSmallCl), e1 = (int)((int64_t)ny * (rank + 1) / kSmallCl);
+  for (int e = e0 + tid; e < e1; e += kSmallNt) {
+    const uint32_t local = static_cast<uint32_t>(__cvta_generic_to_shared(sm + o.y + e));
+    double2 v[kSmallCl];
+#pragma unroll
+    for (uint32_t q = 0; q < kSmallCl; ++q) {
+      uint32_t a;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local), "r"(q));
+      asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v[q].x), "=d"(v[q].y) : "r"(a) : "memory");
+    }
+    double2 acc = v[0];
+#pragma unroll
+    for (int q = 1; q < kSmallCl; ++q) {
+      acc.x += v[q].x;
+      acc.y += v[q].y;
+    }
+    y[e] = acc;
+  }
+  // no CTA leaves while a peer can still read its shared memory
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 __global__ void k_scale_cols_rows(int m, int n, int k, dcplx* Q, int64_t ldq, dcplx* R, int64_t ldr,
                                   const dcplx* __restrict__ ph) {
   // Q[:, i] *= ph[i] (m x k), R[i, :] *= conj(ph[i]) (k x n)
@@ -79,9 +201,7 @@ __global__ void k_scale_cols_rows(int m, int n, int k, dcplx* Q, int64_t ldq, dc
 
 }  // namespace
 
-void level_mix_nz(Context* ctx, const MixPlan& plan, const std::pair<int, int>* nz_in, int nnz, const dcplx* in,
-                  dcplx* out) {
-  MixArgs a;
+static void mix_args(const MixPlan& plan, const std::pair<int, int>* nz_in, int nnz, MixArgs& a) {
   a.Db = plan.Db; a.R = plan.R; a.P = plan.P; a.Q = plan.Q; a.S = plan.S; a.Cn = plan.C;
   a.in_r = plan.in_r; a.in_s = plan.in_s; a.in_c = plan.in_c;
   a.out_p = plan.out_p; a.out_q = plan.out_q; a.out_c = plan.out_c;
@@ -109,6 +229,12 @@ void level_mix_nz(Context* ctx, const MixPlan& plan, const std::pair<int, int>* 
     a.rval[t] = (short)nz[t].first;
   }
   a.qstart[a.nq] = (short)nnz;
+}
+
+void level_mix_nz(Context* ctx, const MixPlan& plan, const std::pair<int, int>* nz_in, int nnz, const dcplx* in,
+                  dcplx* out) {
+  MixArgs a;
+  mix_args(plan, nz_in, nnz, a);
   if (a.nq == 0 || plan.Db <= 0 || plan.C <= 0) return;
   dim3 block(128);
   dim3 grid((plan.Db + 127) / 128, std::min(plan.C, 65535));
@@ -154,15 +280,39 @@ void ac_apply(Context* ctx, const imps_envs* envs, const imps_mpo* mpo, int site
   const int64_t gr_ld = GRover ? GRover_ld : (int64_t)Dr * n;
   ctx->n_ac_apply++;
   const int64_t t1n = (int64_t)Dl * m * d * Dr, t2n = (int64_t)Dl * d * Dr * n;
-  DevBuf& T1 = ctx->buf("ac_t1", t1n * sizeof(dcplx));
-  DevBuf& T2 = ctx->buf("ac_t2", t2n * sizeof(dcplx));
-  zgemm(ctx, OP_N, OP_N, Dl * m, d * Dr, Dl, 1.0, GL, (int64_t)Dl * m, 0, x, Dl, 0, 0.0, T1.z(), (int64_t)Dl * m, 0, 1);
   MixPlan pl;
   pl.Db = Dl; pl.R = m; pl.P = d; pl.Q = n; pl.S = d; pl.C = Dr;
   pl.in_r = Dl; pl.in_s = (int64_t)Dl * m; pl.in_c = (int64_t)Dl * m * d;
   pl.out_p = Dl; pl.out_q = (int64_t)Dl * d * Dr; pl.out_c = (int64_t)Dl * d;
   pl.M = W.Wdev.z();
   pl.nz = W.nz;
+  // Small states in one launch while its 1/8 of the products per SM (16 complex multiply-adds
+  // a clock) stays below the three launches' time, everything fits in shared memory and every
+  // level is written (a level without blocks is multiplied as a zero by the general path).
+  // The split engine never takes products this small.
+  const double macs = (double)Dl * m * d * Dr * Dl + (double)Dl * d * Dr * Dr * n;
+  if (macs <= 7e5 && !ctx->ordered_sums() && ctx->fp64_engine == 0 && (int)W.nz.size() <= kMaxNz && n <= kMaxQ) {
+    MixArgs a;
+    mix_args(pl, pl.nz.data(), (int)pl.nz.size(), a);
+    const SmallShape h{Dl, Dr, m, d, gr_ld, m * d * n * d};
+    const size_t bytes = (size_t)small_layout(h, a.nq).total * sizeof(dcplx);
+    if (a.nq == n && bytes <= 220 * 1024) {
+      static DeviceOnce attr;
+      attr.run(ctx->device, [] {
+        IMPS_CUDA(cudaFuncSetAttribute(k_ac_small, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+      });
+      ScopedTimer t(ctx, "ac_small", 8.0 * macs);
+      ctx->gemm_flops += 8.0 * macs;
+      k_ac_small<<<kSmallCl, kSmallNt, bytes, ctx->stream>>>(h, a, GL, GR, W.Wdev.z(), x, y);
+      ctx->n_kernels++;
+      cudaError_t e = cudaPeekAtLastError();
+      if (e != cudaSuccess) throw Error(IMPS_CUDA_ERROR, std::string("ac_small launch: ") + cudaGetErrorString(e));
+      return;
+    }
+  }
+  DevBuf& T1 = ctx->buf("ac_t1", t1n * sizeof(dcplx));
+  DevBuf& T2 = ctx->buf("ac_t2", t2n * sizeof(dcplx));
+  zgemm(ctx, OP_N, OP_N, Dl * m, d * Dr, Dl, 1.0, GL, (int64_t)Dl * m, 0, x, Dl, 0, 0.0, T1.z(), (int64_t)Dl * m, 0, 1);
   // levels q without any nonzero block must read as zero in the second GEMM
   {
     std::vector<bool> hit(n, false);
