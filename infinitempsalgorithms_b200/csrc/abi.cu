@@ -193,7 +193,7 @@ int imps_ctx_set_precision(imps_ctx* h, int mode, int nslices) {
 int imps_ctx_synchronize(imps_ctx* h) {
   if (!h) return IMPS_INVALID_ARG;
   return guard(&h->c, [&] {
-    IMPS_CUDA(cudaStreamSynchronize(h->c.stream));
+    imps::synchronize(&h->c);
     return IMPS_OK;
   });
 }
@@ -705,7 +705,7 @@ int imps_zgemm(imps_ctx* h, int opA, int opB, int M, int N, int K, double alpha_
     imps::zgemm(&h->c, (imps::Op)opA, (imps::Op)opB, M, N, K, imps::cplx(alpha_re, alpha_im),
                 static_cast<const imps::dcplx*>(A), lda, 0, static_cast<const imps::dcplx*>(B), ldb, 0,
                 imps::cplx(beta_re, beta_im), static_cast<imps::dcplx*>(Cp), ldc, 0, 1, true);
-    IMPS_CUDA(cudaStreamSynchronize(h->c.stream));
+    imps::synchronize(&h->c);
     return IMPS_OK;
   });
 }

@@ -366,7 +366,7 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
       : "=r"(ok)
       : "r"(smem_u32(bar)), "r"(parity)
       : "memory");
@@ -574,8 +574,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GTHREADS, 1)
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
           if (lane == 0)
-            asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(leader_addr(&tempty[buf]))
-                         : "memory");
+            // (not .release.cluster, which would wait for this warp's stores of the last chunk;
+            // the fence above orders the reads of TMEM)
+            asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(leader_addr(&tempty[buf])) : "memory");
         }
         const int col = nb * GT + h * ECOLS + ch * 32;
         if (row < g.M && col < g.ldo) {
@@ -823,7 +824,7 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
   }
   IMPS_CUDA(cudaPeekAtLastError());
   ctx->n_gemm++;
-  ctx->err_armed = true;   // the bounded waits' flag is read at the next synchronisation
+  ctx->err_later = true;   // the bounded waits' flag is read at the next synchronisation
   return true;
 }
 

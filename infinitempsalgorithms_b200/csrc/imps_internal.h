@@ -162,6 +162,9 @@ struct Context {
   int* err_dev = nullptr;
   int* err_host = nullptr;
   bool err_armed = false;
+  // armed by the FP64 products: asynchronous entry points stay asynchronous, and the flag is
+  // read at the context's next synchronisation, whichever call makes it
+  bool err_later = false;
   void* qr_count_ptr = nullptr;       // completion counter of the QR small products, zeroed at this address
   long long wait_cycles = 2000000000LL;  // bound of each pipeline wait (~1 s at 1.9 GHz)
   // profiling
@@ -506,6 +509,8 @@ void lq_form_q(Context* ctx, int m, int n, dcplx* Q, const char* slot);
 // Reads the device error flag if a kernel that may set it ran since the last check
 // (synchronises the stream); a set flag is cleared and raised as IMPS_TIMEOUT.
 void check_device_errors(Context* ctx);
+// Waits for the context's stream and reads the flag if any kernel may have set it.
+void synchronize(Context* ctx);
 
 // Host <-> device
 void upload(Context* ctx, void* dst, const void* src, size_t bytes);

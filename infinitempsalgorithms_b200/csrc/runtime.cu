@@ -569,12 +569,12 @@ ScopedTimer::~ScopedTimer() {
 
 // The error flag rides along with a synchronisation that happens anyway.
 static void err_copy(Context* ctx) {
-  if (ctx->err_armed)
+  if (ctx->err_armed || ctx->err_later)
     IMPS_CUDA(cudaMemcpyAsync(ctx->err_host, ctx->err_dev, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
 }
 static void err_after_sync(Context* ctx) {
-  if (!ctx->err_armed) return;
-  ctx->err_armed = false;
+  if (!ctx->err_armed && !ctx->err_later) return;
+  ctx->err_armed = ctx->err_later = false;
   if (ctx->err_host[0] != 0) {
     ctx->err_host[0] = 0;
     IMPS_CUDA(cudaMemsetAsync(ctx->err_dev, 0, sizeof(int), ctx->stream));
@@ -582,7 +582,9 @@ static void err_after_sync(Context* ctx) {
   }
 }
 void check_device_errors(Context* ctx) {
-  if (!ctx->err_armed) return;
+  if (ctx->err_armed) synchronize(ctx);
+}
+void synchronize(Context* ctx) {
   err_copy(ctx);
   IMPS_CUDA(cudaStreamSynchronize(ctx->stream));
   err_after_sync(ctx);
