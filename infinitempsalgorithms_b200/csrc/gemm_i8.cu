@@ -39,6 +39,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <type_traits>
 
 #include "imps_internal.h"
 #include "split_gemm.h"
@@ -497,7 +498,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned long long)__double_as_longlong(x); }
 
-// per complex row i of op(A) (opA N: A[i + lda k]) -> atomicMax of max(|re|,|im|) bits
+// per strided line i (A[i + lda k]) -> atomicMax of max(|re|,|im|) bits
 __global__ void k_rowmax_colmajor(int M, int K, const double2* __restrict__ A, int64_t lda, int kchunk,
                                   unsigned long long* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -524,154 +525,152 @@ __global__ void k_linemax_contig(int L, int K, const double2* __restrict__ A, in
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
   if (lane == 0) out[l] = dbits(m);
 }
-// column max of a row-major-strided view: out[j] = max_k |B[j + ld k]|  (thread per j, chunked k)
-__global__ void k_colmax_strided(int Ncol, int K, const double2* __restrict__ B, int64_t ld, int kchunk,
-                                 unsigned long long* __restrict__ out) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= Ncol) return;
-  const int k0 = blockIdx.y * kchunk, k1 = min(K, k0 + kchunk);
-  double m = 0.0;
-  for (int k = k0; k < k1; ++k) {
-    double2 v = B[j + ld * k];
-    m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
-  }
-  atomicMax(&out[j], dbits(m));
-}
-
-// max bits -> scale 2^e > max, and its inverse (exact powers of two)
-__global__ void k_scales(int n, const unsigned long long* __restrict__ mx, double* __restrict__ scale,
-                         double* __restrict__ inv) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double m = __longlong_as_double((long long)mx[i]);
-  if (!(m > 0.0) || !isfinite(m)) {
-    scale[i] = 0.0;
-    inv[i] = 0.0;
-    return;
-  }
+// The scale 2^e > max of a line (0 for a line of zeros or one that holds a non-finite value)
+// and its inverse, exact powers of two.
+__device__ __forceinline__ void line_scale(double m, double& scale, double& inv) {
+  scale = inv = 0.0;
+  if (!(m > 0.0) || !isfinite(m)) return;
   int e;
   frexp(m, &e);  // m = f 2^e, f in [0.5, 1)  =>  m < 2^e
-  scale[i] = ldexp(1.0, e);
-  inv[i] = ldexp(1.0, -e);
+  scale = ldexp(1.0, e);
+  inv = ldexp(1.0, -e);
 }
 
-__device__ __forceinline__ void slice_value(double x, int s, int8_t* out) {
-  // x in (-1, 1): the s leading base-128 digits of x, truncated toward zero, each with
-  // the sign of x (x = sum_t out[t] 128^-(t+1) + r, |r| < 128^-s).  x 2^(7s) is exact
-  // (a power-of-two scaling below 2^56), so its integer part carries all s digits.
-  const double y = ldexp(x, 7 * s);
+// x inv in (-1, 1): the S leading base-128 digits, truncated toward zero, each with the sign of
+// x (x inv = sum_t digit_t 128^-(t+1) + r, |r| < 128^-S), four digits a word, digit t in byte
+// t % 4 of word t / 4.  x inv 2^(7S) is exact (powers of two, below 2^56), so its integer part
+// carries all digits; seven-bit fields spread to bytes by shifts and masks, and a word's bytes
+// change sign together: (128 - d) ^ 128 = -d as a signed byte, without borrows for d <= 127.
+struct Digits {
+  uint32_t pos[2], neg[2];   // the digits of |x|, and their negatives
+  bool minus;
+};
+template <int S>
+__device__ __forceinline__ Digits digits_of(double x, double inv) {
+  Digits g;
+  const double y = x * inv * (double)(1ull << (7 * S));
   const long long n = (fabs(y) < 9.0e18) ? (long long)y : 0;  // non-finite input: zero slices
-  const long long a = n < 0 ? -n : n;
-  for (int t = 0; t < s; ++t) {
-    const int dg = (int)((a >> (7 * (s - 1 - t))) & 127);
-    out[t] = (int8_t)(n < 0 ? -dg : dg);
+  g.minus = n < 0;
+  const unsigned long long a = (unsigned long long)(n < 0 ? -n : n);
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    uint32_t p = 0;
+    if (4 * w < S) {
+      const int left = S - 4 * w - 4;   // digits below this word's
+      const uint32_t c = left >= 0 ? (uint32_t)(a >> (7 * (left > 0 ? left : 0))) & 0xFFFFFFFu
+                                   : ((uint32_t)a << (7 * (left < 0 ? -left : 0))) & 0xFFFFFFFu;
+      p = (c >> 21) | ((c >> 6) & 0x7F00u) | ((c << 9) & 0x7F0000u) | ((c & 0x7Fu) << 24);
+    }
+    g.pos[w] = p;
+    g.neg[w] = (0x80808080u - p) ^ 0x80808080u;
+  }
+  return g;
+}
+// byte t of a, b, c, d as one word
+__device__ __forceinline__ uint32_t gather_byte(uint32_t a, uint32_t b, uint32_t c, uint32_t d, int t) {
+  const uint32_t sel = (uint32_t)t | (uint32_t)(4 + t) << 4;
+  return __byte_perm(__byte_perm(a, b, sel), __byte_perm(c, d, sel), 0x5410);
+}
+
+// 4 consecutive complex k of a line into its planes: SIDE 0 (rows of op(A), expanded) rows 2i:
+// (Re, -Im) pairs and 2i + 1: (Im, Re); SIDE 1 (columns of op(B)): (Re, Im).  8-byte stores.
+template <int SIDE, int S>
+__device__ __forceinline__ void slice4(const double2* v, double inv, int8_t* p0, int64_t Kp, int64_t plane) {
+  uint32_t re[4][2], im[4][2], ni[4][2];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const Digits x = digits_of<S>(v[c].x, inv), y = digits_of<S>(v[c].y, inv);
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      re[c][w] = x.minus ? x.neg[w] : x.pos[w];
+      im[c][w] = y.minus ? y.neg[w] : y.pos[w];
+      ni[c][w] = y.minus ? y.pos[w] : y.neg[w];
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < S; ++t) {
+    const int w = t / 4, j = t % 4;
+    if (SIDE == 0) {
+      *reinterpret_cast<uint2*>(p0 + plane * t) = make_uint2(gather_byte(re[0][w], ni[0][w], re[1][w], ni[1][w], j),
+                                                             gather_byte(re[2][w], ni[2][w], re[3][w], ni[3][w], j));
+      *reinterpret_cast<uint2*>(p0 + plane * t + Kp) = make_uint2(
+          gather_byte(im[0][w], re[0][w], im[1][w], re[1][w], j), gather_byte(im[2][w], re[2][w], im[3][w], re[3][w], j));
+    } else {
+      *reinterpret_cast<uint2*>(p0 + plane * t) = make_uint2(gather_byte(re[0][w], im[0][w], re[1][w], im[1][w], j),
+                                                             gather_byte(re[2][w], im[2][w], re[3][w], im[3][w], j));
+    }
   }
 }
 
-// Split op(A) into expanded K-major planes.  A block covers 32 complex rows x 64
-// complex k of the *padded* extent (so no separate zero fill is needed); each
-// thread slices 4 consecutive complex k and stores 8 bytes into each of the two
-// expanded rows per plane.
-// opA == 0: A[i + lda k] (transposed through shared memory), opA == 2: conj(A[k + lda i]).
-template <int OPA>
-__global__ void __launch_bounds__(256) k_split_a(int M, int K, const double2* __restrict__ A, int64_t lda,
-                                                 const double* __restrict__ inv, int s, int8_t* __restrict__ out,
-                                                 int64_t Kp, int64_t plane) {
+// Slices of an operand given its lines' maxima (lines: rows of op(A), columns of op(B)),
+// element (l, k) at X[l + ld k], or X[k + ld l] (KC).  A block covers 32 lines x 64 complex k
+// of the padded extent (no separate zero fill), transposed through shared memory; blocks at
+// k = 0 write the lines' scales.  Memory bound (16 bytes read, 4 S or 2 S written an
+// element): 99 us for 6144 x 1024 and 4096 x 6144 complex at 5 slices, on average (148 us with
+// a loop over the digits' bytes).
+template <int SIDE, int S, bool KC>
+__global__ void __launch_bounds__(256) k_split_tile(int L, int K, const double2* __restrict__ X, int64_t ld, int conj,
+                                                       const unsigned long long* __restrict__ mx,
+                                                       double* __restrict__ scale, int8_t* __restrict__ out, int64_t Kp,
+                                                       int64_t plane) {
   __shared__ double2 tile[32][65];
-  const int i0 = blockIdx.y * 32, k0 = blockIdx.x * 64;
+  __shared__ double inv[32];
+  const int l0 = blockIdx.y * 32, k0 = blockIdx.x * 64;
   const int tid = threadIdx.x;
-  if (OPA == 0) {
-    const int tx = tid & 31, ty = tid >> 5;
-    for (int r = ty; r < 64; r += 8) {
-      const int i = i0 + tx, k = k0 + r;
-      tile[tx][r] = (i < M && k < K) ? A[i + lda * k] : make_double2(0.0, 0.0);
+  if (tid < 32) {
+    double sc = 0.0, iv = 0.0;
+    if (l0 + tid < L) {
+      line_scale(__longlong_as_double((long long)mx[l0 + tid]), sc, iv);
+      if (k0 == 0) scale[l0 + tid] = sc;
     }
-  } else {
-    const int kx = tid & 63, iy = tid >> 6;
-    for (int r = iy; r < 32; r += 4) {
-      const int i = i0 + r, k = k0 + kx;
-      double2 v = (i < M && k < K) ? A[k + lda * i] : make_double2(0.0, 0.0);
-      v.y = -v.y;
-      tile[r][kx] = v;
-    }
+    inv[tid] = iv;
+  }
+  const int tl = KC ? tid >> 6 : tid & 31, tk = KC ? tid & 63 : tid >> 5;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) {
+    const int ll = tl + (KC ? 4 * r : 0), kk = tk + (KC ? 0 : 8 * r);
+    const int l = l0 + ll, k = k0 + kk;
+    double2 v = make_double2(0.0, 0.0);
+    if (l < L && k < K) v = KC ? X[k + ld * l] : X[l + ld * k];
+    if (conj) v.y = -v.y;
+    tile[ll][kk] = v;
   }
   __syncthreads();
+#pragma unroll 1
   for (int item = tid; item < 32 * 16; item += 256) {
     const int il = item >> 4, kq = item & 15;
-    const int i = i0 + il;
-    const double sc = (i < M) ? inv[i] : 0.0;
-    int8_t re[4][8], im[4][8];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const double2 v = tile[il][4 * kq + c];
-      slice_value(v.x * sc, s, re[c]);
-      slice_value(v.y * sc, s, im[c]);
-    }
-    int8_t* p0 = out + (int64_t)(2 * i) * Kp + 2 * (k0 + 4 * kq);
-    for (int t = 0; t < s; ++t) {
-      // row 2i: (Re, -Im) pairs; row 2i+1: (Im, Re) pairs
-      uint32_t lo0 = 0, hi0 = 0, lo1 = 0, hi1 = 0;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        lo0 |= ((uint32_t)(uint8_t)re[c][t] | ((uint32_t)(uint8_t)(int8_t)(-im[c][t]) << 8)) << (16 * c);
-        hi0 |= ((uint32_t)(uint8_t)re[c + 2][t] | ((uint32_t)(uint8_t)(int8_t)(-im[c + 2][t]) << 8)) << (16 * c);
-        lo1 |= ((uint32_t)(uint8_t)im[c][t] | ((uint32_t)(uint8_t)re[c][t] << 8)) << (16 * c);
-        hi1 |= ((uint32_t)(uint8_t)im[c + 2][t] | ((uint32_t)(uint8_t)re[c + 2][t] << 8)) << (16 * c);
-      }
-      *reinterpret_cast<uint2*>(p0 + plane * t) = make_uint2(lo0, hi0);
-      *reinterpret_cast<uint2*>(p0 + plane * t + Kp) = make_uint2(lo1, hi1);
-    }
+    const int64_t row = (SIDE == 0 ? 2 : 1) * (int64_t)(l0 + il);
+    slice4<SIDE, S>(&tile[il][4 * kq], inv[il], out + row * Kp + 2 * (k0 + 4 * kq), Kp, plane);
   }
 }
 
-// Split op(B) (K x N complex) into K-major planes Bt[j][2k + p], same tiling over
-// the padded extent; 8-byte stores of 4 consecutive complex k.
-// opB == 0: B[k + ldb j] (contiguous in k); opB == 2: conj(B[j + ldb k]) (tile transpose).
-template <int OPB>
-__global__ void __launch_bounds__(256) k_split_b(int K, int N, const double2* __restrict__ B, int64_t ldb,
-                                                 const double* __restrict__ inv, int s, int8_t* __restrict__ out,
-                                                 int64_t Kp, int64_t plane) {
-  __shared__ double2 tile[32][65];
-  const int j0 = blockIdx.y * 32, k0 = blockIdx.x * 64;
-  const int tid = threadIdx.x;
-  if (OPB == 0) {
-    const int kx = tid & 63, jy = tid >> 6;
-    for (int r = jy; r < 32; r += 4) {
-      const int j = j0 + r, k = k0 + kx;
-      tile[r][kx] = (k < K && j < N) ? B[k + ldb * j] : make_double2(0.0, 0.0);
-    }
-  } else {
-    const int tx = tid & 31, ty = tid >> 5;
-    for (int r = ty; r < 64; r += 8) {
-      const int j = j0 + tx, k = k0 + r;
-      double2 v = (k < K && j < N) ? B[j + ldb * k] : make_double2(0.0, 0.0);
-      v.y = -v.y;
-      tile[tx][r] = v;
-    }
+// The same for lines that are contiguous in k, element (l, k) at X[k + ld l]: a block takes LB
+// whole lines into shared memory, so their maxima, scales and slices need one launch and one
+// read (a clearing, a maximum, a scale and a slicing launch otherwise).
+constexpr int LB = 4;
+template <int SIDE, int S>
+__global__ void __launch_bounds__(32 * LB) k_split_lines(int L, int K, const double2* __restrict__ X, int64_t ld, int conj,
+                                                         double* __restrict__ scale, int8_t* __restrict__ out,
+                                                         int64_t Kp, int64_t plane) {
+  extern __shared__ __align__(16) double2 lines[];   // [LB][Kp / 2], one warp a line
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = blockIdx.x * LB + w;
+  const int Kc = (int)(Kp / 2);
+  double2* row = lines + (int64_t)w * Kc;
+  double m = 0.0;
+  for (int k = lane; k < Kc; k += 32) {
+    double2 v = (l < L && k < K) ? X[k + ld * l] : make_double2(0.0, 0.0);
+    m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
+    if (conj) v.y = -v.y;
+    row[k] = v;
   }
-  __syncthreads();
-  for (int item = tid; item < 32 * 16; item += 256) {
-    const int jl = item >> 4, kq = item & 15;
-    const int j = j0 + jl;
-    const double sc = (j < N) ? inv[j] : 0.0;
-    int8_t re[4][8], im[4][8];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const double2 v = tile[jl][4 * kq + c];
-      slice_value(v.x * sc, s, re[c]);
-      slice_value(v.y * sc, s, im[c]);
-    }
-    int8_t* p0 = out + (int64_t)j * Kp + 2 * (k0 + 4 * kq);
-    for (int t = 0; t < s; ++t) {
-      uint32_t lo = 0, hi = 0;
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        lo |= ((uint32_t)(uint8_t)re[c][t] | ((uint32_t)(uint8_t)im[c][t] << 8)) << (16 * c);
-        hi |= ((uint32_t)(uint8_t)re[c + 2][t] | ((uint32_t)(uint8_t)im[c + 2][t] << 8)) << (16 * c);
-      }
-      *reinterpret_cast<uint2*>(p0 + plane * t) = make_uint2(lo, hi);
-    }
-  }
+  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  double sc, iv;
+  line_scale(m, sc, iv);
+  if (lane == 0 && l < L) scale[l] = sc;
+  __syncwarp();
+  const int64_t r0 = (SIDE == 0 ? 2 : 1) * (int64_t)l;
+  for (int k = 4 * lane; k < Kc; k += 128) slice4<SIDE, S>(row + k, iv, out + r0 * Kp + 2 * k, Kp, plane);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
@@ -710,71 +709,88 @@ CUtensorMap plane_map(const int8_t* base, int64_t Kp, int64_t rows, int planes, 
 }
 
 // ---------------------------------------------------------------------------
-void split_operand_a(Context* ctx, SplitOperand& S, Op op, int M, int K, const dcplx* A, int64_t lda, int s) {
-  IMPS_REQUIRE(op == OP_N || op == OP_C, IMPS_INVALID_ARG, "split: op T is not supported");
-  IMPS_REQUIRE(s >= 1 && s <= 8, IMPS_INVALID_ARG, "split: 1..8 slices");
-  S.rows = M;
-  S.K = K;
-  S.s = s;
-  S.Rp = round_up(2 * (int64_t)M, BM);
-  S.Kp = round_up(2 * (int64_t)K, KPAD);
-  const size_t plane = (size_t)S.Rp * S.Kp;
-  S.data.ensure(plane * s);
-  S.scale.ensure((size_t)M * sizeof(double));
-  S.inv.ensure((size_t)M * sizeof(double));
-  S.mx.ensure((size_t)M * sizeof(unsigned long long));
-  ScopedTimer tm(ctx, "split_slice", 16.0 * M * K + (double)plane * s);
-  IMPS_CUDA(cudaMemsetAsync(S.mx.ptr, 0, (size_t)M * 8, ctx->stream));
-  auto* mx = static_cast<unsigned long long*>(S.mx.ptr);
-  if (op == OP_N) {
-    const int kchunk = 64;
-    dim3 g((M + 127) / 128, (K + kchunk - 1) / kchunk);
-    k_rowmax_colmajor<<<g, 128, 0, ctx->stream>>>(M, K, A, lda, kchunk, mx);
-  } else {
-    k_linemax_contig<<<(M + 7) / 8, 256, 0, ctx->stream>>>(M, K, A, lda, mx);
+namespace {
+template <int SIDE, int S>
+void slice_launch(Context* ctx, SplitOperand& O, bool kcontig, int conj, int L, int K, const dcplx* X, int64_t ld,
+                  bool have_max) {
+  const int64_t plane = O.Rp * O.Kp;
+  int8_t* out = static_cast<int8_t*>(O.data.ptr);
+  const int padded = (int)(SIDE == 0 ? O.Rp / 2 : O.Rp);   // lines with planes, a multiple of LB and 32
+  const size_t smem = (size_t)LB * (O.Kp / 2) * sizeof(double2);
+  if (kcontig && smem <= 200 * 1024) {
+    static DeviceOnce attr;
+    attr.run(ctx->device, [] {
+      IMPS_CUDA(cudaFuncSetAttribute(k_split_lines<SIDE, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    });
+    k_split_lines<SIDE, S><<<padded / LB, 32 * LB, smem, ctx->stream>>>(L, K, X, ld, conj, O.scale.d(), out, O.Kp, plane);
+    ctx->n_kernels++;
+    return;
   }
-  k_scales<<<(M + 255) / 256, 256, 0, ctx->stream>>>(M, mx, S.scale.d(), S.inv.d());
-  // grid over the padded extent: Kp / 2 complex columns, Rp / 2 complex rows
-  dim3 g2((unsigned)(S.Kp / 2 / 64), (unsigned)(S.Rp / 2 / 32));
-  if (op == OP_N)
-    k_split_a<0><<<g2, 256, 0, ctx->stream>>>(M, K, A, lda, S.inv.d(), s, static_cast<int8_t*>(S.data.ptr), S.Kp, plane);
-  else
-    k_split_a<2><<<g2, 256, 0, ctx->stream>>>(M, K, A, lda, S.inv.d(), s, static_cast<int8_t*>(S.data.ptr), S.Kp, plane);
-  ctx->n_kernels += 5;
+  auto* mx = static_cast<unsigned long long*>(O.mx.ptr);
+  const dim3 grid((unsigned)(O.Kp / 128), (unsigned)(padded / 32));
+  if (kcontig) {   // lines too long for a block
+    k_linemax_contig<<<(L + 7) / 8, 256, 0, ctx->stream>>>(L, K, X, ld, mx);
+    k_split_tile<SIDE, S, true><<<grid, 256, 0, ctx->stream>>>(L, K, X, ld, conj, mx, O.scale.d(), out, O.Kp, plane);
+    ctx->n_kernels += 2;
+    return;
+  }
+  if (!have_max) {
+    IMPS_CUDA(cudaMemsetAsync(mx, 0, (size_t)L * 8, ctx->stream));
+    const int kchunk = 64;
+    k_rowmax_colmajor<<<dim3((L + 127) / 128, (K + kchunk - 1) / kchunk), 128, 0, ctx->stream>>>(L, K, X, ld, kchunk, mx);
+    ctx->n_kernels += 2;
+  }
+  k_split_tile<SIDE, S, false><<<grid, 256, 0, ctx->stream>>>(L, K, X, ld, conj, mx, O.scale.d(), out, O.Kp, plane);
+  ctx->n_kernels++;
+}
+
+template <int SIDE>
+void slice_operand(Context* ctx, SplitOperand& O, bool kcontig, bool conj, int L, int K, const dcplx* X, int64_t ld,
+                   int s, bool have_max) {
+  IMPS_REQUIRE(s >= 1 && s <= 8, IMPS_INVALID_ARG, "split: 1..8 slices");
+  O.rows = L;
+  O.K = K;
+  O.s = s;
+  // whole tiles of rows: every B box (64 or 128 rows) lies inside the planes
+  O.Rp = SIDE == 0 ? round_up(2 * (int64_t)L, BM) : round_up(L, BN_MAX);
+  O.Kp = round_up(2 * (int64_t)K, KPAD);
+  const size_t plane = (size_t)O.Rp * O.Kp;
+  O.data.ensure(plane * s);
+  O.scale.ensure((size_t)L * sizeof(double));
+  O.mx.ensure((size_t)L * sizeof(unsigned long long));
+  ScopedTimer tm(ctx, "split_slice", 16.0 * L * K + (double)plane * s);
+  auto run = [&](auto s_tag) {
+    slice_launch<SIDE, decltype(s_tag)::value>(ctx, O, kcontig, conj ? 1 : 0, L, K, X, ld, have_max);
+  };
+  switch (s) {
+    case 1: run(std::integral_constant<int, 1>{}); break;
+    case 2: run(std::integral_constant<int, 2>{}); break;
+    case 3: run(std::integral_constant<int, 3>{}); break;
+    case 4: run(std::integral_constant<int, 4>{}); break;
+    case 5: run(std::integral_constant<int, 5>{}); break;
+    case 6: run(std::integral_constant<int, 6>{}); break;
+    case 7: run(std::integral_constant<int, 7>{}); break;
+    default: run(std::integral_constant<int, 8>{}); break;
+  }
   IMPS_CUDA(cudaPeekAtLastError());
+}
+}  // namespace
+
+unsigned long long* split_line_max(Context* ctx, SplitOperand& S, int lines) {
+  S.mx.ensure((size_t)lines * sizeof(unsigned long long));
+  IMPS_CUDA(cudaMemsetAsync(S.mx.ptr, 0, (size_t)lines * 8, ctx->stream));
+  return static_cast<unsigned long long*>(S.mx.ptr);
+}
+
+void split_operand_a(Context* ctx, SplitOperand& S, Op op, int M, int K, const dcplx* A, int64_t lda, int s,
+                     bool have_max) {
+  IMPS_REQUIRE(op == OP_N || op == OP_C, IMPS_INVALID_ARG, "split: op T is not supported");
+  slice_operand<0>(ctx, S, op == OP_C, op == OP_C, M, K, A, lda, s, have_max && op == OP_N);
 }
 
 void split_operand_b(Context* ctx, SplitOperand& S, Op op, int K, int N, const dcplx* B, int64_t ldb, int s) {
   IMPS_REQUIRE(op == OP_N || op == OP_C, IMPS_INVALID_ARG, "split: op T is not supported");
-  IMPS_REQUIRE(s >= 1 && s <= 8, IMPS_INVALID_ARG, "split: 1..8 slices");
-  S.rows = N;
-  S.K = K;
-  S.s = s;
-  S.Rp = round_up(N, BN_MAX);  // every B box (64 or 128 rows) lies inside the planes
-  S.Kp = round_up(2 * (int64_t)K, KPAD);
-  const size_t plane = (size_t)S.Rp * S.Kp;
-  S.data.ensure(plane * s);
-  S.scale.ensure((size_t)N * sizeof(double));
-  S.inv.ensure((size_t)N * sizeof(double));
-  S.mx.ensure((size_t)N * sizeof(unsigned long long));
-  ScopedTimer tm(ctx, "split_slice", 16.0 * K * N + (double)plane * s);
-  IMPS_CUDA(cudaMemsetAsync(S.mx.ptr, 0, (size_t)N * 8, ctx->stream));
-  auto* mx = static_cast<unsigned long long*>(S.mx.ptr);
-  if (op == OP_N) {
-    k_linemax_contig<<<(N + 7) / 8, 256, 0, ctx->stream>>>(N, K, B, ldb, mx);
-  } else {
-    const int kchunk = 64;
-    dim3 g((N + 127) / 128, (K + kchunk - 1) / kchunk);
-    k_colmax_strided<<<g, 128, 0, ctx->stream>>>(N, K, B, ldb, kchunk, mx);
-  }
-  k_scales<<<(N + 255) / 256, 256, 0, ctx->stream>>>(N, mx, S.scale.d(), S.inv.d());
-  dim3 g2((unsigned)(S.Kp / 2 / 64), (unsigned)(S.Rp / 32));
-  if (op == OP_N)
-    k_split_b<0><<<g2, 256, 0, ctx->stream>>>(K, N, B, ldb, S.inv.d(), s, static_cast<int8_t*>(S.data.ptr), S.Kp, plane);
-  else
-    k_split_b<2><<<g2, 256, 0, ctx->stream>>>(K, N, B, ldb, S.inv.d(), s, static_cast<int8_t*>(S.data.ptr), S.Kp, plane);
-  ctx->n_kernels += 5;
-  IMPS_CUDA(cudaPeekAtLastError());
+  slice_operand<1>(ctx, S, op == OP_N, op == OP_C, N, K, B, ldb, s, false);
 }
 
 void split_gemm(Context* ctx, const SplitOperand& A, const SplitOperand& B, int s, double alpha, bool accumulate,

@@ -23,17 +23,29 @@ struct MixArgs {
   short qval[kMaxQ];
   short qstart[kMaxQ + 1];
   short rval[kMaxNz];
+  unsigned long long* row_max;
 };
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(fma(a.x, b.x, -a.y * b.y), fma(a.x, b.y, a.y * b.x));
 }
 
-template <int P>
+// MAX: also the rows' maxima for the split engine that takes `out` next (it would read all of
+// `out` again for them).  Only their exponents count there, so the upper words are compared
+// as integers (FP64 maxima made the kernel slower than the extra read); a NaN is ignored, as
+// a maximum of doubles would.
+__device__ __forceinline__ uint32_t upper_word(double x) {
+  const uint32_t h = (uint32_t)__double2hiint(x) & 0x7fffffffu;
+  return h > 0x7ff00000u ? 0u : h;
+}
+template <int P, bool MAX>
 __global__ void __launch_bounds__(128) k_level_mix(const MixArgs a, const double2* __restrict__ M,
                                                    const double2* __restrict__ in, double2* __restrict__ out) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= a.Db) return;
+  uint32_t top[MAX ? P : 1];
+#pragma unroll
+  for (int p = 0; p < (MAX ? P : 1); ++p) top[p] = 0u;
   for (int c = blockIdx.y; c < a.Cn; c += gridDim.y) {
     const double2* inb = in + b + a.in_c * c;
     double2* outb = out + b + a.out_c * c;
@@ -55,7 +67,19 @@ __global__ void __launch_bounds__(128) k_level_mix(const MixArgs a, const double
         }
       }
 #pragma unroll
-      for (int p = 0; p < P; ++p) outb[a.out_p * p + a.out_q * q] = cmul(a.scale, acc[p]);
+      for (int p = 0; p < P; ++p) {
+        const double2 v = cmul(a.scale, acc[p]);
+        outb[a.out_p * p + a.out_q * q] = v;
+        if (MAX) top[p] = max(top[p], max(upper_word(v.x), upper_word(v.y)));
+      }
+    }
+  }
+  if (MAX) {
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      const unsigned long long bits = (unsigned long long)top[p] << 32;
+      unsigned long long* slot = &a.row_max[b + a.Db * p];
+      if (bits > *(volatile unsigned long long*)slot) atomicMax(slot, bits);
     }
   }
 }
@@ -206,6 +230,7 @@ static void mix_args(const MixPlan& plan, const std::pair<int, int>* nz_in, int 
   a.in_r = plan.in_r; a.in_s = plan.in_s; a.in_c = plan.in_c;
   a.out_p = plan.out_p; a.out_q = plan.out_q; a.out_c = plan.out_c;
   a.scale = make_double2(plan.scale.real(), plan.scale.imag());
+  a.row_max = plan.row_max;
   IMPS_REQUIRE(nnz <= kMaxNz, IMPS_INVALID_ARG, "level_mix: too many MPO blocks");
   // group the nonzero (r, q) blocks by q (insertion sort into a fixed array: no heap use)
   std::pair<int, int> nz[kMaxNz];
@@ -238,11 +263,16 @@ void level_mix_nz(Context* ctx, const MixPlan& plan, const std::pair<int, int>* 
   if (a.nq == 0 || plan.Db <= 0 || plan.C <= 0) return;
   dim3 block(128);
   dim3 grid((plan.Db + 127) / 128, std::min(plan.C, 65535));
+  if (plan.row_max)   // several columns a block: fewer meetings at the maxima
+    grid.y = std::min<unsigned>(grid.y, std::max(1u, (unsigned)(ctx->num_sms * 16) / grid.x));
   double bytes = 16.0 * plan.Db * (double)plan.C * (plan.R * plan.S + plan.P * a.nq);
   ScopedTimer t(ctx, "level_mix", bytes);
   switch (plan.P) {
 #define IMPS_MIX_CASE(PP) \
-  case PP: k_level_mix<PP><<<grid, block, 0, ctx->stream>>>(a, plan.M, in, out); break;
+  case PP:                                                                                  \
+    if (plan.row_max) k_level_mix<PP, true><<<grid, block, 0, ctx->stream>>>(a, plan.M, in, out); \
+    else k_level_mix<PP, false><<<grid, block, 0, ctx->stream>>>(a, plan.M, in, out);             \
+    break;
     IMPS_MIX_CASE(1) IMPS_MIX_CASE(2) IMPS_MIX_CASE(3) IMPS_MIX_CASE(4)
     IMPS_MIX_CASE(5) IMPS_MIX_CASE(6) IMPS_MIX_CASE(7) IMPS_MIX_CASE(8)
 #undef IMPS_MIX_CASE
@@ -320,6 +350,11 @@ void ac_apply(Context* ctx, const imps_envs* envs, const imps_mpo* mpo, int site
     for (int q = 0; q < n; ++q)
       if (!hit[q]) zfill(ctx, (int64_t)Dl * d * Dr, 0.0, T2.z() + (int64_t)Dl * d * Dr * q);
   }
+  struct Forget {   // the maxima are for this product only, whatever becomes of it
+    Context* ctx;
+    ~Forget() { ctx->max_ready = nullptr; }
+  } forget{ctx};
+  pl.row_max = split_collect_max(ctx, T2.z(), Dl * d, Dr, Dr * n);
   level_mix(ctx, pl, T1.z(), T2.z());
   zgemm(ctx, OP_N, OP_N, Dl * d, Dr, Dr * n, 1.0, T2.z(), (int64_t)Dl * d, 0, GR, gr_ld, 0, 0.0, y,
         (int64_t)Dl * d, 0, 1);

@@ -187,6 +187,9 @@ struct Context {
   std::multiset<const void*> const_ptrs;
   std::map<SplitKey, std::shared_ptr<SplitOperand>> split_cache;
   std::shared_ptr<SplitOperand> split_scratch[2];
+  // the operand whose row maxima a kernel has just collected into split_scratch[0], for the
+  // next split product only
+  const void* max_ready = nullptr;
   // split operands released by a ConstScope, kept (with their device buffers) for the
   // next constant operands: no cudaMalloc / cudaFree, and so no implicit device
   // synchronisation, per solve
@@ -438,6 +441,12 @@ enum Op { OP_N = 0, OP_T = 1, OP_C = 2 };
 void zgemm(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha, const dcplx* A, int64_t lda,
            int64_t strideA, const dcplx* B, int64_t ldb, int64_t strideB, cplx beta, dcplx* C, int64_t ldc,
            int64_t strideC, int batch, bool allow_split = true);
+// Whether zgemm would take this product (real alpha, beta 0 or 1) to the split engine now.
+bool zgemm_splits(const Context* ctx, Op opA, Op opB, int M, int N, int K);
+// When the M x K operand A about to be written will go to the split engine as op(A) = A of an
+// M x N x K product: where the kernel that writes it is to collect its rows' maxima (the bits
+// of max(|re|, |im|), by atomicMax); nullptr otherwise.  The product must be the next one.
+unsigned long long* split_collect_max(Context* ctx, const dcplx* A, int M, int N, int K);
 // Always the FP64 engine.
 void zgemm_fp64(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha, const dcplx* A, int64_t lda,
                 int64_t strideA, const dcplx* B, int64_t ldb, int64_t strideB, cplx beta, dcplx* C,
@@ -453,6 +462,8 @@ struct MixPlan {
   const dcplx* M;             // dense (R, P, Q, S) column-major
   std::vector<std::pair<int, int>> nz;  // (r, q) nonzero blocks
   cplx scale = cplx(1.0, 0.0);
+  // when set: maxima of |re|, |im| of the output's rows b + Db p over q and c (split_collect_max)
+  unsigned long long* row_max = nullptr;
 };
 void level_mix(Context* ctx, const MixPlan& plan, const dcplx* in, dcplx* out);
 // same with the block list given as a pointer (uses no heap memory; plan.nz is ignored)

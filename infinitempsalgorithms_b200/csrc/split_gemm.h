@@ -10,16 +10,19 @@ namespace imps {
 struct SplitOperand {
   DevBuf data;    // s planes of Rp x Kp bytes
   DevBuf scale;   // per complex row (A side) / column (B side): power of two > max |re|,|im|
-  DevBuf inv;     // 1 / scale
-  DevBuf mx;      // scratch for the max reduction
+  DevBuf mx;      // per line: bits of the largest |re|, |im|
   int rows = 0;   // complex rows (A: M, B: N)
   int K = 0;      // complex inner dimension
   int s = 0;      // slices stored
   int64_t Rp = 0, Kp = 0;
 };
 
-// op(A) (M x K), op in {N, C}: expanded real rows (2M) x (2K) int8 planes
-void split_operand_a(Context* ctx, SplitOperand& S, Op op, int M, int K, const dcplx* A, int64_t lda, int s);
+// op(A) (M x K), op in {N, C}: expanded real rows (2M) x (2K) int8 planes; have_max: S.mx
+// already holds the rows' maxima (op N)
+void split_operand_a(Context* ctx, SplitOperand& S, Op op, int M, int K, const dcplx* A, int64_t lda, int s,
+                     bool have_max = false);
+// S.mx for this many lines, cleared, for a kernel that collects them while it writes the operand
+unsigned long long* split_line_max(Context* ctx, SplitOperand& S, int lines);
 // op(B) (K x N), op in {N, C}: N rows x (2K) int8 planes
 void split_operand_b(Context* ctx, SplitOperand& S, Op op, int K, int N, const dcplx* B, int64_t ldb, int s);
 // C (complex, ldc) = alpha * op(A) op(B) (+ C when accumulate) using `s` slice diagonals

@@ -533,10 +533,24 @@ static std::shared_ptr<SplitOperand> get_split(Context* ctx, int side, Op op, in
     if (!ctx->split_scratch[side]) ctx->split_scratch[side] = std::make_shared<SplitOperand>();
     S = ctx->split_scratch[side];
   }
-  if (side == 0) split_operand_a(ctx, *S, op, rows, K, X, ld, s);
+  const bool have_max = side == 0 && !constant && ctx->max_ready == X;   // (in the scratch operand)
+  ctx->max_ready = nullptr;
+  if (side == 0) split_operand_a(ctx, *S, op, rows, K, X, ld, s, have_max);
   else split_operand_b(ctx, *S, op, K, rows, X, ld, s);
   if (constant) ctx->split_cache[key] = S;
   return S;
+}
+
+bool zgemm_splits(const Context* ctx, Op opA, Op opB, int M, int N, int K) {
+  return active_slices(ctx) > 0 && opA != OP_T && opB != OP_T && M >= 64 && N >= 64 && K >= 32 &&
+         (double)M * N * K >= 33554432.0;
+}
+
+unsigned long long* split_collect_max(Context* ctx, const dcplx* A, int M, int N, int K) {
+  if (!zgemm_splits(ctx, OP_N, OP_N, M, N, K) || ctx->const_ptrs.count(A) > 0) return nullptr;
+  if (!ctx->split_scratch[0]) ctx->split_scratch[0] = std::make_shared<SplitOperand>();
+  ctx->max_ready = A;
+  return split_line_max(ctx, *ctx->split_scratch[0], M);
 }
 
 void zgemm(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha, const dcplx* A, int64_t lda,
@@ -544,9 +558,8 @@ void zgemm(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha, const 
            int64_t strideC, int batch, bool allow_split) {
   ctx->gemm_flops += 8.0 * (double)M * (double)N * (double)K * (double)batch;
   const int s = active_slices(ctx);
-  const bool split = s > 0 && allow_split && opA != OP_T && opB != OP_T && alpha.imag() == 0.0 &&
-                     (beta == cplx(0.0, 0.0) || beta == cplx(1.0, 0.0)) && M >= 64 && N >= 64 && K >= 32 &&
-                     (double)M * N * K >= 33554432.0;
+  const bool split = allow_split && alpha.imag() == 0.0 && (beta == cplx(0.0, 0.0) || beta == cplx(1.0, 0.0)) &&
+                     zgemm_splits(ctx, opA, opB, M, N, K);
   if (!split) {
     zgemm_fp64(ctx, opA, opB, M, N, K, alpha, A, lda, strideA, B, ldb, strideB, beta, C, ldc, strideC, batch);
     return;
