@@ -27,10 +27,13 @@
 //   warp 0: TMA producer (cp.async.bulk.tensor, 64B swizzle, 2-8 stages by s)
 //   warp 1: TMEM allocator + single-thread tcgen05.mma issuer (M=128, N=BN, K=32)
 //   warps 2-9: epilogue, tcgen05.ld 32x32b, two warps per TMEM lane quarter, each
-//           owning BN/2 columns in chunks of 32, 16 or 8; a thread sums its row's chunk over
-//           all diagonals in FP64 registers and writes it (adds it, for the later
-//           K groups of a tile).  When two tiles' accumulators fit in TMEM the
-//           epilogue of one tile overlaps the MMAs of the next.
+//           owning BN/2 columns; a thread sums its row's columns over all diagonals (and
+//           K groups) in FP64 registers, hands the buffer back and writes them once.  With
+//           2 slices two tiles' accumulators fit in TMEM and the epilogue of one tile
+//           overlaps the MMAs of the next.
+// Pairs of CTAs (cta_group::2) gain nothing here: 5 slices 1080 us against 1108 for 6144 x
+// 4096 x 1024, the same at 2 to 4, 8 % less at 96 rows: each SM's share of an MMA still
+// reads its A rows and all of B, and what a tile lacks is columns, which TMEM bounds.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -186,7 +189,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, int32_t* r) {
         "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
         "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, int32_t* r) {
@@ -196,20 +198,26 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, int32_t* r) {
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
         "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, int32_t* r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
                : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void tmem_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 // CW columns of this warp's 32 TMEM lanes, one register per column
 template <int CW>
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, int32_t* r) {
-  if constexpr (CW == 32) tmem_ld32(taddr, r);
-  else if constexpr (CW == 16) tmem_ld16(taddr, r);
+  if constexpr (CW >= 32) tmem_ld32(taddr, r);
+  else if constexpr (CW >= 16) tmem_ld16(taddr, r);
   else tmem_ld8(taddr, r);
+  constexpr int DONE = CW >= 32 ? 32 : (CW >= 16 ? 16 : 8);
+  if constexpr (CW > DONE) tmem_ld<CW - DONE>(taddr + DONE, r + DONE);
+}
+// exact int -> double: the integer as the low word of 2^52 + 2^31 + r, less that offset (the
+// conversion instruction runs at a quarter of the rate of the addition)
+__device__ __forceinline__ double int_to_double(int32_t r) {
+  return __hiloint2double(0x43300000, r ^ (int)0x80000000) - 4503601774854144.0;
 }
 
 struct GemmArgs {
@@ -381,105 +389,61 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       }
     }
   } else {
-    // epilogue warps 2..9: TMEM lane quarter q = warp % 4, column half h
-    constexpr int HC = BN / 2;   // columns per epilogue thread
-    constexpr int CW = (HC % 32 == 0) ? 32 : ((HC % 16 == 0) ? 16 : 8);  // columns per tcgen05.ld
-    constexpr int NCH = HC / CW; // chunks (one tcgen05.ld each per diagonal)
-    static_assert(HC % CW == 0, "half tile is a whole number of chunks");
+    // epilogue warps 2..9: TMEM lane quarter q = warp % 4, column half h.  A thread sums its
+    // row's columns over all diagonals and K groups of the tile in FP64 registers, so that the
+    // buffer goes back to the MMA thread before anything is scaled and written: from 3 slices
+    // on a tile has the only buffer, and the tensor cores idle while it is read.  (6144 x 4096
+    // x 1024: 1167 -> 1108 us at 5 slices, 1797 -> 1665 at 6, 505 -> 472 at 3, against chunks
+    // of columns converted by I2F and written before the next was read.  Diagonals handed over
+    // one by one gained nothing: 1125 us.)
+    constexpr int HC = BN / 2;              // columns per epilogue thread
+    constexpr int LD = HC <= 48 ? HC : 16;  // columns read between two waits
     const int q = warp & 3;
     const int h = (warp - 2) / 4;
     const int row = q * 32 + lane;  // tile row == TMEM lane
     double* Cd = reinterpret_cast<double*>(g.C);
-    if constexpr (NCH == 1) {
-      // one chunk per thread: the row's FP64 sums are kept over all K groups of the
-      // tile and written once
-      int grp = 0;
-      for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-        int mb, nb;
-        tile_coords(g, t, mb, nb);
-        double part[32];
+    int grp = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
+      int mb, nb;
+      tile_coords(g, t, mb, nb);
+      double part[HC];
 #pragma unroll
-        for (int j = 0; j < 32; ++j) part[j] = 0.0;
-        bool ok = true;
-        for (GroupIter gi(&g); gi.valid(); gi.next(), ++grp) {
-          const int buf = grp % NBUF;
-          if (!mbar_wait(&tfull[buf], (grp / NBUF) & 1, err, g.wait_cycles)) { ok = false; break; }
-          tc_fence_after();
-          for (int d = 0; d < S; ++d) {
-            const double w = ldexp(1.0, -7 * (d + 2));
-            int32_t r[32];
-            tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)((buf * S + d) * BN + h * HC), r);
+      for (int j = 0; j < HC; ++j) part[j] = 0.0;
+      for (GroupIter gi(&g); gi.valid(); gi.next(), ++grp) {
+        const int buf = grp % NBUF;
+        if (!mbar_wait(&tfull[buf], (grp / NBUF) & 1, err, g.wait_cycles)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t src = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * S * BN + h * HC);
+#pragma unroll 1
+        for (int d = 0; d < S; ++d) {
+          const double w = __hiloint2double((1023 - 7 * (d + 2)) << 20, 0);  // 2^-7(d + 2)
 #pragma unroll
-            for (int j = 0; j < 32; ++j) part[j] = fma((double)r[j], w, part[j]);
-          }
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&tempty[buf]);
-        }
-        if (!ok) break;
-        const int rr = mb * BM + row;              // real row of At
-        const int ci = rr >> 1, part_im = rr & 1;  // complex row, re/im
-        if (ci < g.Mc) {
-          const double rs = g.row_scale[ci] * g.alpha;
+          for (int c = 0; c < HC; c += LD) {
+            int32_t r[LD];
+            tmem_ld<LD>(src + (uint32_t)(d * BN + c), r);
+            tmem_wait();
 #pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            const int cj = nb * BN + h * HC + j;
-            if (cj < g.Nc) {
-              const double v = part[j] * rs * __ldg(&g.col_scale[cj]);
-              double* p = Cd + 2 * ((int64_t)ci + g.ldc * cj) + part_im;
-              *p = g.accumulate ? (*p + v) : v;
-            }
+            for (int j = 0; j < LD; ++j) part[c + j] = fma(int_to_double(r[j]), w, part[c + j]);
           }
         }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&tempty[buf]);
       }
-    } else {
-      int grp = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
-        int mb, nb;
-        tile_coords(g, t, mb, nb);
-        const int rr = mb * BM + row;              // real row of At
-        const int ci = rr >> 1, part_im = rr & 1;  // complex row, re/im
-        const double rs = (ci < g.Mc) ? g.row_scale[ci] * g.alpha : 0.0;
-        bool first = true;  // first K group of the tile writes (or adds, when accumulating)
-        for (GroupIter gi(&g); gi.valid(); gi.next(), ++grp) {
-          const int buf = grp % NBUF;
-          if (!mbar_wait(&tfull[buf], (grp / NBUF) & 1, err, g.wait_cycles)) { ok = false; break; }
-          tc_fence_after();
-#pragma unroll 1
-          for (int ch = 0; ch < NCH; ++ch) {
-            // FP64 sum of this thread's CW columns over all slice diagonals of the group
-            double part[CW];
+      if (!ok) break;
+      const int rr = mb * BM + row;              // real row of At
+      const int ci = rr >> 1, part_im = rr & 1;  // complex row, re/im
+      if (ci < g.Mc) {
+        const double rs = g.row_scale[ci] * g.alpha;
 #pragma unroll
-            for (int j = 0; j < CW; ++j) part[j] = 0.0;
-#pragma unroll 1
-            for (int d = 0; d < S; ++d) {
-              const double w = ldexp(1.0, -7 * (d + 2));
-              int32_t r[CW];
-              tmem_ld<CW>(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)((buf * S + d) * BN + h * HC + ch * CW), r);
-#pragma unroll
-              for (int j = 0; j < CW; ++j) part[j] = fma((double)r[j], w, part[j]);
-            }
-            if (ch == NCH - 1) {
-              // every column of this buffer has been read: hand it back to the MMA thread
-              tc_fence_before();
-              __syncwarp();
-              if (lane == 0) mbar_arrive(&tempty[buf]);
-            }
-            if (ci < g.Mc) {
-              const bool add = g.accumulate || !first;
-#pragma unroll
-              for (int j = 0; j < CW; ++j) {
-                const int cj = nb * BN + h * HC + ch * CW + j;
-                if (cj < g.Nc) {
-                  const double v = part[j] * rs * __ldg(&g.col_scale[cj]);
-                  double* p = Cd + 2 * ((int64_t)ci + g.ldc * cj) + part_im;
-                  *p = add ? (*p + v) : v;
-                }
-              }
-            }
+        for (int j = 0; j < HC; ++j) {
+          const int cj = nb * BN + h * HC + j;
+          if (cj < g.Nc) {
+            const double v = part[j] * rs * __ldg(&g.col_scale[cj]);
+            double* p = Cd + 2 * ((int64_t)ci + g.ldc * cj) + part_im;
+            *p = g.accumulate ? (*p + v) : v;
           }
-          first = false;
         }
       }
     }
