@@ -393,6 +393,9 @@ __device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
   while (!mbar_try(bar, parity) && clock64() - t0 < GDRAIN) {
   }
 }
+__device__ __forceinline__ void mbar_expect(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
 // the leader's copy of a barrier, as a shared::cluster address
 __device__ __forceinline__ uint32_t leader_addr(const void* p) {
   uint32_t a;
@@ -436,6 +439,40 @@ __device__ __forceinline__ void commit_pair(uint64_t* bar) {
 __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// What each role of a pair got done, told to both CTAs: the stages that the two producers
+// filled and that the MMA thread has read
+enum : uint32_t { DONE_FILL0, DONE_FILL1, DONE_MMA, DONE_SLOTS };
+__device__ __forceinline__ void publish(uint32_t* slot, uint32_t n) {
+#pragma unroll
+  for (uint32_t r = 0; r < 2; ++r) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(slot)), "r"(r));
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(n) : "memory");
+  }
+}
+// The end of both CTAs, by all their threads.  With every stage read nothing is in flight.
+// After a wait that gave up, the leader completes each outstanding phase of the `full`
+// barriers (an arrival for a stage that only its peer filled, the peer's bytes for one that
+// only it filled) and waits for the copies; the peer stays until then.
+__device__ __forceinline__ void leave_pair(uint64_t* full, uint32_t nst, uint32_t bytes, const uint32_t* done,
+                                           uint32_t rank, uint32_t total) {
+  __syncthreads();
+  cluster_sync();
+  if (done[DONE_MMA] == total) return;
+  const uint32_t n0 = done[DONE_FILL0], n1 = done[DONE_FILL1];
+  if (rank == 0 && threadIdx.x == 0) {
+    const uint32_t end = max(n0, n1);
+    for (uint32_t i = end > nst ? end - nst : 0; i < end; ++i) {
+      uint64_t* bar = &full[i % nst];
+      if (i >= n0) mbar_expect(bar, bytes);
+      if (i >= n1)
+        asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
+                     : "memory");
+      mbar_drain(bar, (i / nst) & 1);
+    }
+  }
+  cluster_sync();
+}
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -459,6 +496,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GTHREADS, 1)
   uint64_t* tempty = bars + 2 * GSTAGES + GBUF;        // leader: both CTAs have read them
   uint64_t* drain = bars + 2 * GSTAGES + 2 * GBUF;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * GSTAGES + 2 * GBUF + 1);
+  uint32_t* done = tmem_slot + 1;                      // [DONE_SLOTS]
   volatile int* err = g.err;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint32_t rank;
@@ -492,38 +530,30 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GTHREADS, 1)
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      int issued[GSTAGES];
-      for (int s = 0; s < GSTAGES; ++s) issued[s] = -1;
+      uint32_t nfilled = 0;
       for (int t = pair; t < ntiles && ok; t += npairs) {
         const int pl = t / per, mb = (t % per) % g.num_m, nb = (t % per) / g.num_m;
         for (int kb = 0; kb < g.kblocks && ok; ++kb) {
           ok = mbar_wait(&empty[stage], phase ^ 1, err, g.wait_cycles);
           if (!ok) break;
           uint8_t* base = smem + stage * GSTAGE_BYTES;
-          if (rank == 0)
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&full[stage])),
-                         "r"((uint32_t)(2 * GSTAGE_BYTES))
-                         : "memory");
+          if (rank == 0) mbar_expect(&full[stage], 2 * GSTAGE_BYTES);
           const uint32_t bar = leader_addr(&full[stage]);
           tma_load_pair(base, &mapA, bar, kb * GKB, mb * GT + (int)rank * HALF, pl);
           tma_load_pair(base + HALF * GKB, &mapB, bar, kb * GKB, nb * GT + (int)rank * HALF, pl);
-          issued[stage] = (int)phase;
+          ++nfilled;
           if (++stage == GSTAGES) {
             stage = 0;
             phase ^= 1;
           }
         }
       }
-      // both CTAs' copies must land before either leaves (the leader's barriers count both;
-      // the cluster barrier at the end holds the other CTA until then)
-      if (rank == 0)
-        for (int s = 0; s < GSTAGES; ++s)
-          if (issued[s] >= 0) mbar_drain(&full[s], (uint32_t)issued[s]);
+      publish(&done[DONE_FILL0 + rank], nfilled);
     }
   } else if (warp == 1) {
     if (rank == 0 && lane == 0) {
       int stage = 0, n = 0;
-      uint32_t phase = 0;
+      uint32_t phase = 0, nread = 0;
       bool ok = true;
       for (int t = pair; t < ntiles && ok; t += npairs, ++n) {
         const int buf = n % GBUF;
@@ -541,6 +571,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GTHREADS, 1)
             mma_pair(tmem + (uint32_t)(buf * GT), da + (uint64_t)(kk * 2), db + (uint64_t)(kk * 2),
                      (kb == 0 && kk == 0) ? 0u : 1u);
           commit_pair(&empty[stage]);
+          ++nread;
           if (++stage == GSTAGES) {
             stage = 0;
             phase ^= 1;
@@ -551,6 +582,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GTHREADS, 1)
       }
       commit_pair(drain);
       mbar_drain(drain, 0);
+      publish(&done[DONE_MMA], nread);
     }
   } else {
     constexpr int ECOLS = GT / (GEPI / 4);   // columns of a warp
@@ -594,9 +626,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GTHREADS, 1)
       }
     }
   }
-  __syncthreads();
   // no CTA leaves, and no TMEM is released, while the pair's MMAs or copies are in flight
-  cluster_sync();
+  const uint32_t mine = pair < ntiles ? (uint32_t)((ntiles - pair + npairs - 1) / npairs) : 0u;
+  leave_pair(full, GSTAGES, (uint32_t)GSTAGE_BYTES, done, rank, mine * (uint32_t)g.kblocks);
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem));

@@ -107,3 +107,21 @@ def test_without_scratch_the_fp64_tensor_cores_answer(ctx):
     got = _gemm(ctx, X, Y, 0, 0, kernels=1)
     L.check(ctx.lib.imps_ctx_set_workspace_limit(ctx.h, 0), ctx.h)
     assert np.array_equal(got, X @ Y)
+
+
+def test_bounded_wait_runs_out_and_context_recovers():
+    """A one-cycle bound: a wait of a CTA pair gives up, both CTAs' copies land before either
+    leaves, the status comes with the synchronisation, and the context goes on."""
+    c = imps.Context(0)
+    rng = np.random.default_rng(5)
+    A = rng.integers(-9, 10, (1100, 900)) + 1j * rng.integers(-9, 10, (1100, 900))
+    B = rng.integers(-9, 10, (900, 700)) + 1j * rng.integers(-9, 10, (900, 700))
+    L.check(c.lib.imps_ctx_set_wait_limit(c.h, 1), c.h)
+    for _ in range(3):
+        with pytest.raises(L.ImpsError) as e:
+            _gemm(c, A, B, 0, 0)
+            c.synchronize()
+        assert e.value.status == L.IMPS_TIMEOUT
+    L.check(c.lib.imps_ctx_set_wait_limit(c.h, 0), c.h)
+    assert np.linalg.norm(_gemm(c, A, B, 0, 0) - A @ B) <= 1e-14 * np.linalg.norm(A) * np.linalg.norm(B)
+    c.close()
