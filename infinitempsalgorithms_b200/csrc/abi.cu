@@ -824,6 +824,7 @@ int imps_exponentiate_c(imps_envs* E, int site, double dt_re, double dt_im, cons
 namespace {
 __global__ void k_diag_apply(int64_t n, const double2* __restrict__ dv, const double2* __restrict__ x,
                              double2* __restrict__ y) {
+  imps::grid_enter();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double2 a = dv[i], b = x[i];
     y[i] = make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -832,7 +833,7 @@ __global__ void k_diag_apply(int64_t n, const double2* __restrict__ dv, const do
 imps::LinOp diag_op(imps::Context* ctx, int64_t n, const imps::dcplx* dv) {
   return [ctx, n, dv](const imps::dcplx* x, imps::dcplx* y) {
     int g = (int)std::min<int64_t>((n + 255) / 256, 148 * 16);
-    k_diag_apply<<<std::max(g, 1), 256, 0, ctx->stream>>>(n, dv, x, y);
+    imps::launch_kernel(ctx, k_diag_apply, std::max(g, 1), 256, 0, n, dv, x, y);
     ctx->n_kernels++;
   };
 }

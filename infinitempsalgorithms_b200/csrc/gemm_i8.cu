@@ -319,6 +319,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  grid_enter();
   const uint32_t tmem_base = *tmem_slot;
   const int ntiles = g.num_m * g.num_n;
 
@@ -465,6 +466,7 @@ __device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned
 // per strided line i (A[i + lda k]) -> atomicMax of max(|re|,|im|) bits
 __global__ void k_rowmax_colmajor(int M, int K, const double2* __restrict__ A, int64_t lda, int kchunk,
                                   unsigned long long* __restrict__ out) {
+  grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= M) return;
   const int k0 = blockIdx.y * kchunk, k1 = min(K, k0 + kchunk);
@@ -478,6 +480,7 @@ __global__ void k_rowmax_colmajor(int M, int K, const double2* __restrict__ A, i
 // per "contiguous line" l (A[k + ld l], k < K): max over k (warp per line)
 __global__ void k_linemax_contig(int L, int K, const double2* __restrict__ A, int64_t ld,
                                  unsigned long long* __restrict__ out) {
+  grid_enter();
   const int l = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (l >= L) return;
@@ -577,6 +580,7 @@ __global__ void __launch_bounds__(256) k_split_tile(int L, int K, const double2*
                                                        const unsigned long long* __restrict__ mx,
                                                        double* __restrict__ scale, int8_t* __restrict__ out, int64_t Kp,
                                                        int64_t plane) {
+  grid_enter();
   __shared__ double2 tile[32][65];
   __shared__ double inv[32];
   const int l0 = blockIdx.y * 32, k0 = blockIdx.x * 64;
@@ -616,6 +620,7 @@ template <int SIDE, int S>
 __global__ void __launch_bounds__(32 * LB) k_split_lines(int L, int K, const double2* __restrict__ X, int64_t ld, int conj,
                                                          double* __restrict__ scale, int8_t* __restrict__ out,
                                                          int64_t Kp, int64_t plane) {
+  grid_enter();
   extern __shared__ __align__(16) double2 lines[];   // [LB][Kp / 2], one warp a line
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = blockIdx.x * LB + w;
   const int Kc = (int)(Kp / 2);
@@ -686,25 +691,25 @@ void slice_launch(Context* ctx, SplitOperand& O, bool kcontig, int conj, int L, 
     attr.run(ctx->device, [] {
       IMPS_CUDA(cudaFuncSetAttribute(k_split_lines<SIDE, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     });
-    k_split_lines<SIDE, S><<<padded / LB, 32 * LB, smem, ctx->stream>>>(L, K, X, ld, conj, O.scale.d(), out, O.Kp, plane);
+    launch_kernel(ctx, k_split_lines<SIDE, S>, padded / LB, 32 * LB, smem, L, K, X, ld, conj, O.scale.d(), out, O.Kp, plane);
     ctx->n_kernels++;
     return;
   }
   auto* mx = static_cast<unsigned long long*>(O.mx.ptr);
   const dim3 grid((unsigned)(O.Kp / 128), (unsigned)(padded / 32));
   if (kcontig) {   // lines too long for a block
-    k_linemax_contig<<<(L + 7) / 8, 256, 0, ctx->stream>>>(L, K, X, ld, mx);
-    k_split_tile<SIDE, S, true><<<grid, 256, 0, ctx->stream>>>(L, K, X, ld, conj, mx, O.scale.d(), out, O.Kp, plane);
+    launch_kernel(ctx, k_linemax_contig, (L + 7) / 8, 256, 0, L, K, X, ld, mx);
+    launch_kernel(ctx, k_split_tile<SIDE, S, true>, grid, 256, 0, L, K, X, ld, conj, mx, O.scale.d(), out, O.Kp, plane);
     ctx->n_kernels += 2;
     return;
   }
   if (!have_max) {
     IMPS_CUDA(cudaMemsetAsync(mx, 0, (size_t)L * 8, ctx->stream));
     const int kchunk = 64;
-    k_rowmax_colmajor<<<dim3((L + 127) / 128, (K + kchunk - 1) / kchunk), 128, 0, ctx->stream>>>(L, K, X, ld, kchunk, mx);
+    launch_kernel(ctx, k_rowmax_colmajor, dim3((L + 127) / 128, (K + kchunk - 1) / kchunk), 128, 0, L, K, X, ld, kchunk, mx);
     ctx->n_kernels += 2;
   }
-  k_split_tile<SIDE, S, false><<<grid, 256, 0, ctx->stream>>>(L, K, X, ld, conj, mx, O.scale.d(), out, O.Kp, plane);
+  launch_kernel(ctx, k_split_tile<SIDE, S, false>, grid, 256, 0, L, K, X, ld, conj, mx, O.scale.d(), out, O.Kp, plane);
   ctx->n_kernels++;
 }
 
@@ -802,12 +807,12 @@ void split_gemm(Context* ctx, const SplitOperand& A, const SplitOperand& B, int 
     ScopedTimer tm(ctx, "gemm_split",
                    2.0 * (double)A.Rp * (double)g.num_n * bn * (double)A.Kp * (double)(s * (s + 1) / 2));
     switch (s) {
-      case 2: k_gemm_i8<2, 128><<<grid, NTHREADS, smem, ctx->stream>>>(mapA, mapB, g); break;
-      case 3: k_gemm_i8<3, 128><<<grid, NTHREADS, smem, ctx->stream>>>(mapA, mapB, g); break;
-      case 4: k_gemm_i8<4, 128><<<grid, NTHREADS, smem, ctx->stream>>>(mapA, mapB, g); break;
-      case 5: k_gemm_i8<5, 96><<<grid, NTHREADS, smem, ctx->stream>>>(mapA, mapB, g); break;
-      case 6: k_gemm_i8<6, 80><<<grid, NTHREADS, smem, ctx->stream>>>(mapA, mapB, g); break;
-      default: k_gemm_i8<0, 64><<<grid, NTHREADS, smem, ctx->stream>>>(mapA, mapB, g); break;
+      case 2: launch_kernel(ctx, k_gemm_i8<2, 128>, grid, NTHREADS, smem, mapA, mapB, g); break;
+      case 3: launch_kernel(ctx, k_gemm_i8<3, 128>, grid, NTHREADS, smem, mapA, mapB, g); break;
+      case 4: launch_kernel(ctx, k_gemm_i8<4, 128>, grid, NTHREADS, smem, mapA, mapB, g); break;
+      case 5: launch_kernel(ctx, k_gemm_i8<5, 96>, grid, NTHREADS, smem, mapA, mapB, g); break;
+      case 6: launch_kernel(ctx, k_gemm_i8<6, 80>, grid, NTHREADS, smem, mapA, mapB, g); break;
+      default: launch_kernel(ctx, k_gemm_i8<0, 64>, grid, NTHREADS, smem, mapA, mapB, g); break;
     }
     ctx->n_kernels++;
     ctx->n_gemm++;

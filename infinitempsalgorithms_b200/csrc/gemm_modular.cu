@@ -162,6 +162,7 @@ __device__ __forceinline__ double2 load_elem(const ModOperand& o, int l, int k) 
 // Partial sums of squares and maxima of every line over the K chunks (a fixed order, so
 // that the scales do not depend on timing).  Blocks [0, a.nblocks_norm) serve a.
 __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const ModOperand b) {
+  grid_enter();
   __shared__ double ss[4][64], sm[4][64];
   const bool first = (int)blockIdx.x < a.nblocks_norm;
   const ModOperand& o = first ? a : b;
@@ -278,6 +279,7 @@ __device__ __forceinline__ void split_moduli(const unsigned (&xlo)[8], const uns
 // small blocks let one's loads run beside another's arithmetic.
 constexpr int SPL_LINES = 16, SPL_NT = SPL_LINES * 8;
 __global__ void __launch_bounds__(SPL_NT, 1024 / SPL_NT) k_mod_split(const ModOperand a, const ModOperand b) {
+  grid_enter();
   __shared__ double2 tile[SPL_LINES][65];
   __shared__ int ex[SPL_LINES];
   const bool first = (int)blockIdx.x < a.nblocks_split;
@@ -521,6 +523,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GTHREADS, 1)
   __syncthreads();
   cluster_sync();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  grid_enter();
   const uint32_t tmem = *tmem_slot;
   const int per = g.num_m * g.num_n, ntiles = per * NPL;
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
@@ -680,6 +683,7 @@ __device__ __forceinline__ void join_moduli(const unsigned (&wu)[NMOD], const un
 // 48 bytes of memory traffic.
 template <bool BETA>
 __global__ void __launch_bounds__(256, 3) k_mod_join(const ModJoinArgs g, const ModOperand a, const ModOperand b) {
+  grid_enter();
   __shared__ double2 tile[16][65];
   const int tid = threadIdx.x;
   const int r = tid >> 2, c4 = (tid & 3) * 4;
@@ -813,8 +817,8 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
     o->nblocks_split = (int)(Kp / 64) * ((o->lines + SPL_LINES - 1) / SPL_LINES);
   }
   ScopedTimer tm(ctx, "zgemm_modular", 8.0 * M * (double)N * K);
-  k_mod_norms<<<a.nblocks_norm + b.nblocks_norm, 256, 0, ctx->stream>>>(a, b);
-  k_mod_split<<<a.nblocks_split + b.nblocks_split, SPL_NT, 0, ctx->stream>>>(a, b);
+  launch_kernel(ctx, k_mod_norms, a.nblocks_norm + b.nblocks_norm, 256, 0, a, b);
+  launch_kernel(ctx, k_mod_split, a.nblocks_split + b.nblocks_split, SPL_NT, 0, a, b);
   static DeviceOnce attr;
   attr.run(ctx->device, [] {
     IMPS_CUDA(cudaFuncSetAttribute(k_mod_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, GSMEM));
@@ -834,7 +838,7 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
     g.err = ctx->err_dev;
     g.wait_cycles = ctx->wait_cycles;
     const int pairs = std::min(g.num_m * g.num_n * NPL, ctx->num_sms / 2);
-    k_mod_gemm<<<2 * pairs, GTHREADS, GSMEM, ctx->stream>>>(mapA, mapB, g);
+    launch_kernel(ctx, k_mod_gemm, 2 * pairs, GTHREADS, GSMEM, mapA, mapB, g);
     ModJoinArgs j;
     j.M = M;
     j.N = nn;
@@ -850,8 +854,8 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
     ModOperand bj = b;
     bj.X = b.kcontig ? B + ldb * n0 : B + n0;
     const dim3 grid((M + 63) / 64, (nn + 15) / 16);
-    if (beta != cplx(0.0, 0.0)) k_mod_join<true><<<grid, 256, 0, ctx->stream>>>(j, a, bj);
-    else k_mod_join<false><<<grid, 256, 0, ctx->stream>>>(j, a, bj);
+    if (beta != cplx(0.0, 0.0)) launch_kernel(ctx, k_mod_join<true>, grid, 256, 0, j, a, bj);
+    else launch_kernel(ctx, k_mod_join<false>, grid, 256, 0, j, a, bj);
     ctx->n_kernels += 2;
   }
   IMPS_CUDA(cudaPeekAtLastError());

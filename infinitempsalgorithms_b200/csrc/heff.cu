@@ -41,6 +41,7 @@ __device__ __forceinline__ uint32_t upper_word(double x) {
 template <int P, bool MAX>
 __global__ void __launch_bounds__(128) k_level_mix(const MixArgs a, const double2* __restrict__ M,
                                                    const double2* __restrict__ in, double2* __restrict__ out) {
+  grid_enter();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= a.Db) return;
   uint32_t top[MAX ? P : 1];
@@ -148,6 +149,7 @@ __device__ __forceinline__ void small_gemm(int rows, int cols, int K, const doub
 __global__ void __cluster_dims__(kSmallCl, 1, 1) __launch_bounds__(kSmallNt)
     k_ac_small(const SmallShape h, const MixArgs mx, const double2* __restrict__ GL, const double2* __restrict__ GR,
                const double2* __restrict__ W, const double2* __restrict__ x, double2* __restrict__ y) {
+  grid_enter();
   extern __shared__ __align__(16) double2 sm[];
   const SmallLayout o = small_layout(h, mx.nq);
   const int tid = threadIdx.x;
@@ -208,6 +210,7 @@ __global__ void __cluster_dims__(kSmallCl, 1, 1) __launch_bounds__(kSmallNt)
 
 __global__ void k_scale_cols_rows(int m, int n, int k, dcplx* Q, int64_t ldq, dcplx* R, int64_t ldr,
                                   const dcplx* __restrict__ ph) {
+  grid_enter();
   // Q[:, i] *= ph[i] (m x k), R[i, :] *= conj(ph[i]) (k x n)
   int64_t tq = (int64_t)m * k, tr = (int64_t)k * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tq + tr; t += (int64_t)gridDim.x * blockDim.x) {
@@ -270,8 +273,8 @@ void level_mix_nz(Context* ctx, const MixPlan& plan, const std::pair<int, int>* 
   switch (plan.P) {
 #define IMPS_MIX_CASE(PP) \
   case PP:                                                                                  \
-    if (plan.row_max) k_level_mix<PP, true><<<grid, block, 0, ctx->stream>>>(a, plan.M, in, out); \
-    else k_level_mix<PP, false><<<grid, block, 0, ctx->stream>>>(a, plan.M, in, out);             \
+    if (plan.row_max) launch_kernel(ctx, k_level_mix<PP, true>, grid, block, 0, a, plan.M, in, out); \
+    else launch_kernel(ctx, k_level_mix<PP, false>, grid, block, 0, a, plan.M, in, out);             \
     break;
     IMPS_MIX_CASE(1) IMPS_MIX_CASE(2) IMPS_MIX_CASE(3) IMPS_MIX_CASE(4)
     IMPS_MIX_CASE(5) IMPS_MIX_CASE(6) IMPS_MIX_CASE(7) IMPS_MIX_CASE(8)
@@ -291,7 +294,7 @@ void level_mix(Context* ctx, const MixPlan& plan, const dcplx* in, dcplx* out) {
 void scale_q_r(Context* ctx, int m, int n, int k, dcplx* Q, int64_t ldq, dcplx* R, int64_t ldr, const dcplx* ph) {
   int64_t tot = (int64_t)m * k + (int64_t)k * n;
   int g = (int)std::min<int64_t>((tot + 255) / 256, 148 * 16);
-  k_scale_cols_rows<<<std::max(g, 1), 256, 0, ctx->stream>>>(m, n, k, Q, ldq, R, ldr, ph);
+  launch_kernel(ctx, k_scale_cols_rows, std::max(g, 1), 256, 0, m, n, k, Q, ldq, R, ldr, ph);
   ctx->n_kernels++;
 }
 
@@ -333,7 +336,7 @@ void ac_apply(Context* ctx, const imps_envs* envs, const imps_mpo* mpo, int site
       });
       ScopedTimer t(ctx, "ac_small", 8.0 * macs);
       ctx->gemm_flops += 8.0 * macs;
-      k_ac_small<<<kSmallCl, kSmallNt, bytes, ctx->stream>>>(h, a, GL, GR, W.Wdev.z(), x, y);
+      launch_kernel(ctx, k_ac_small, kSmallCl, kSmallNt, bytes, h, a, GL, GR, W.Wdev.z(), x, y);
       ctx->n_kernels++;
       cudaError_t e = cudaPeekAtLastError();
       if (e != cudaSuccess) throw Error(IMPS_CUDA_ERROR, std::string("ac_small launch: ") + cudaGetErrorString(e));

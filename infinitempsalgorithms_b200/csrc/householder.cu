@@ -120,6 +120,7 @@ template <int NB, int RPT, int CL, int NT>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT, 1)
     k_qr_panel(int R, int b, int zabove, dcplx* __restrict__ A, int64_t lda, dcplx* __restrict__ V, int64_t ldv,
                dcplx* __restrict__ tau, dcplx* __restrict__ T, int ldt) {
+  grid_enter();
   constexpr int NV = 2 * NB;             // reduction slots: [0] ||x||^2, [2q - 1, 2q] position q
   constexpr int NW = NT / 32;
   constexpr bool WARPS = CL > 1 && NT < QR_NT;   // the warps' sums travel, not the CTAs'
@@ -381,6 +382,7 @@ constexpr int QR_MERGE_NT = 1024;   // one thread per output of a panel's step: 
 
 __global__ void __launch_bounds__(QR_MERGE_NT) k_merge_t(int bo, PanelList pl, const dcplx* __restrict__ Tin,
                                                  const dcplx* __restrict__ G, dcplx* __restrict__ Tb) {
+  grid_enter();
   extern __shared__ __align__(16) dcplx msm[];
   const int ld = bo + 1;
   dcplx* Ts = msm;                            // Ts[r + ld c]
@@ -428,6 +430,7 @@ __global__ void __launch_bounds__(QR_MERGE_NT) k_merge_t(int bo, PanelList pl, c
 
 __global__ void k_extract_r(int k, int n, const dcplx* __restrict__ A, int64_t lda, dcplx* __restrict__ R,
                             int64_t ldr, dcplx* __restrict__ ph) {
+  grid_enter();
   int64_t tot = (int64_t)k * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
     int r = (int)(t % k), c = (int)(t / k);
@@ -443,6 +446,7 @@ __global__ void k_extract_r(int k, int n, const dcplx* __restrict__ A, int64_t l
 // out[i] = sum_c part[i + stride c] over nc partials, in a fixed order
 __global__ void k_sum_partials(int64_t len, int nc, const dcplx* __restrict__ part, int64_t stride,
                                dcplx* __restrict__ out) {
+  grid_enter();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < len; i += (int64_t)gridDim.x * blockDim.x) {
     dcplx s = make_double2(0.0, 0.0);
     for (int c = 0; c < nc; ++c) {
@@ -458,7 +462,7 @@ template <int NB, int RPT, int CL, int NT>
 void launch_panel(Context* ctx, int R, int b, int zabove, dcplx* A, int64_t lda, dcplx* V, int64_t ldv, dcplx* tau,
                   dcplx* T, int ldt) {
   static_assert(NB * RPT == QR_NBMAX, "a thread holds 16 complex numbers");
-  k_qr_panel<NB, RPT, CL, NT><<<CL, NT, 0, ctx->stream>>>(R, b, zabove, A, lda, V, ldv, tau, T, ldt);
+  launch_kernel(ctx, k_qr_panel<NB, RPT, CL, NT>, CL, NT, 0, R, b, zabove, A, lda, V, ldv, tau, T, ldt);
   ctx->n_kernels++;
   cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess) throw Error(IMPS_CUDA_ERROR, std::string("qr panel launch: ") + cudaGetErrorString(e));
@@ -492,6 +496,7 @@ __global__ void __launch_bounds__(XS_NT) k_xhv_small(int K, int N, int b, int kc
                                                       dcplx* __restrict__ part, unsigned* __restrict__ counter,
                                                       dcplx* __restrict__ Wh, const dcplx* __restrict__ T, int ldt,
                                                       int conjT, dcplx* __restrict__ Z) {
+  grid_enter();
   __shared__ dcplx sh[(XS_COLS + QR_NBMAX) * XS_LD];  // [16 columns of X, b of V][XS_LD rows], later the summed Wh
   __shared__ dcplx Ts[QR_NBMAX][QR_NBMAX + 1];
   __shared__ bool last;
@@ -584,6 +589,7 @@ template <bool FULL>
 __global__ void __launch_bounds__(256) k_apply_small(int R, int N, int b, const dcplx* __restrict__ Vm, int64_t ldv,
                                                      const dcplx* __restrict__ Z, dcplx* __restrict__ A2,
                                                      int64_t lda) {
+  grid_enter();
   const int r = blockIdx.x * 64 + (threadIdx.x & 63);
   const int n = blockIdx.y * 4 + (threadIdx.x >> 6);
   if (r >= R || n >= N) return;
@@ -618,8 +624,8 @@ void xhv_small(Context* ctx, int N, int b, int K, const dcplx* X, const dcplx* V
   const int kc = (K + g - 1) / g;
   g = (K + kc - 1) / kc;
   ScopedTimer tm(ctx, "qr_small", 8.0 * N * b * (double)K);
-  k_xhv_small<<<dim3(g, (N + XS_COLS - 1) / XS_COLS), XS_NT, 0, ctx->stream>>>(
-      K, N, b, kc, X, Vm, ld, part, static_cast<unsigned*>(cnt.ptr), Wh, T, ldt, conjT ? 1 : 0, Z);
+  launch_kernel(ctx, k_xhv_small, dim3(g, (N + XS_COLS - 1) / XS_COLS), XS_NT, 0, K, N, b, kc, X, Vm, ld, part,
+                static_cast<unsigned*>(cnt.ptr), Wh, T, ldt, conjT ? 1 : 0, Z);
   ctx->n_kernels++;
   IMPS_CUDA(cudaPeekAtLastError());
 }
@@ -629,8 +635,8 @@ void apply_small(Context* ctx, int R, int N, int b, const dcplx* Vm, int64_t ldv
   IMPS_REQUIRE(b <= QR_NBMAX && N <= QR_NBO, IMPS_INVALID_ARG, "apply_small: shape");
   ScopedTimer tm(ctx, "qr_small", 8.0 * R * N * (double)b);
   const dim3 grid((R + 63) / 64, (N + 3) / 4);
-  if (b == QR_NBMAX) k_apply_small<true><<<grid, 256, 0, ctx->stream>>>(R, N, b, Vm, ldv, Z, A2, lda);
-  else k_apply_small<false><<<grid, 256, 0, ctx->stream>>>(R, N, b, Vm, ldv, Z, A2, lda);
+  if (b == QR_NBMAX) launch_kernel(ctx, k_apply_small<true>, grid, 256, 0, R, N, b, Vm, ldv, Z, A2, lda);
+  else launch_kernel(ctx, k_apply_small<false>, grid, 256, 0, R, N, b, Vm, ldv, Z, A2, lda);
   ctx->n_kernels++;
   IMPS_CUDA(cudaPeekAtLastError());
 }
@@ -659,7 +665,7 @@ void gemm_xhv(Context* ctx, int N, int b, int K, const dcplx* X, const dcplx* Vm
     zgemm_fp64(ctx, OP_C, OP_N, N, b, rem, 1.0, X + (int64_t)nfull * kc, ld, 0, Vm + (int64_t)nfull * kc, ld, 0,
                0.0, part + pstride * nfull, N, 0, 1);
   const int g = (int)std::min<int64_t>((pstride + 255) / 256, 148 * 8);
-  k_sum_partials<<<std::max(g, 1), 256, 0, ctx->stream>>>(pstride, nc, part, pstride, Wh);
+  launch_kernel(ctx, k_sum_partials, std::max(g, 1), 256, 0, pstride, nc, part, pstride, Wh);
   ctx->n_kernels++;
 }
 
@@ -751,7 +757,7 @@ void qr_factor(Context* ctx, int m, int n, const dcplx* M, int64_t ldm, dcplx* R
     merge_attr.run(ctx->device, [] {
       IMPS_CUDA(cudaFuncSetAttribute(k_merge_t, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)QR_MERGE_SMEM));
     });
-    k_merge_t<<<1, QR_MERGE_NT, QR_MERGE_SMEM, ctx->stream>>>(bo, pl, Tin.z(), Gb.z(), Tb);
+    launch_kernel(ctx, k_merge_t, 1, QR_MERGE_NT, QR_MERGE_SMEM, bo, pl, Tin.z(), Gb.z(), Tb);
     ctx->n_kernels++;
     const int n2 = n - (P + bo);
     if (n2 > 0) {
@@ -765,7 +771,7 @@ void qr_factor(Context* ctx, int m, int n, const dcplx* M, int64_t ldm, dcplx* R
   {
     int64_t tot = (int64_t)k * n;
     int g = (int)std::min<int64_t>((tot + 255) / 256, 148 * 16);
-    k_extract_r<<<std::max(g, 1), 256, 0, ctx->stream>>>(k, n, A, m, R, k, ph.z());
+    launch_kernel(ctx, k_extract_r, std::max(g, 1), 256, 0, k, n, A, m, R, k, ph.z());
     ctx->n_kernels++;
   }
   scale_q_r(ctx, 0, n, k, nullptr, 1, R, k, ph.z());  // R rows by conj(phase)

@@ -23,6 +23,7 @@ namespace {
 // Y = diag(s) X (rows) or X diag(s) (cols), rows x cols column-major, in place allowed
 __global__ void k_scale_diag(int rows, int cols, const dcplx* __restrict__ X, int64_t ldx, dcplx* Y, int64_t ldy,
                              const dcplx* __restrict__ s, int by_row) {
+  grid_enter();
   const int64_t tot = (int64_t)rows * cols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(t % rows), c = (int)(t / rows);
@@ -33,6 +34,7 @@ __global__ void k_scale_diag(int rows, int cols, const dcplx* __restrict__ X, in
 }
 
 __global__ void k_set_diag(int k, const dcplx* __restrict__ s, dcplx* C) {
+  grid_enter();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) C[i + (int64_t)k * i] = s[i];
 }
 
@@ -69,7 +71,7 @@ struct Sweep2 {
     upload(ctx, sd.ptr, s.data(), s.size() * sizeof(dcplx));
     const int64_t tot = (int64_t)rows * cols;
     if (tot == 0) return;
-    k_scale_diag<<<grid_for(tot), 256, 0, ctx->stream>>>(rows, cols, X, rows, Y, rows, sd.z(), by_row ? 1 : 0);
+    launch_kernel(ctx, k_scale_diag, grid_for(tot), 256, 0, rows, cols, X, rows, Y, rows, sd.z(), by_row ? 1 : 0);
     launched(ctx);
   }
 
@@ -183,7 +185,7 @@ struct Sweep2 {
     zfill(ctx, (int64_t)k * k, 0.0, st->C[p].z());
     DevBuf& sd = ctx->buf("idmrg2_sdiag", (size_t)k * sizeof(dcplx));
     upload(ctx, sd.ptr, sc.data(), (size_t)k * sizeof(dcplx));
-    k_set_diag<<<grid_for(k), 256, 0, ctx->stream>>>(k, sd.z(), st->C[p].z());
+    launch_kernel(ctx, k_set_diag, grid_for(k), 256, 0, k, sd.z(), st->C[p].z());
     launched(ctx);
     reshape(st->AR[q], (int64_t)k * n);
     zconj_transpose(ctx, n, k, V.z(), n, st->AR[q].z(), k);

@@ -31,6 +31,7 @@ int grid_for(int64_t t) { return (int)std::max<int64_t>(1, std::min<int64_t>((t 
 // v[k] = exp(2 pi i frac(k phi)), phi the golden-ratio conjugate: the deterministic start of
 // the environment eigensolves (the reference draws randn)
 __global__ void k_env_start(int64_t n, dcplx* v) {
+  grid_enter();
   for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
     const double f = fmod((double)k * 0.6180339887498949, 1.0);
     double s, c;
@@ -42,6 +43,7 @@ __global__ void k_env_start(int64_t n, dcplx* v) {
 // B[(wl + Wl bl), u, (wr + Wr br)] = sum_d W[wl,u,wr,d] A[bl,d,br]   (operators/linalg.jl:15-20)
 __global__ void k_mult_site(int wl, int d, int wr, int bl, int br, const dcplx* __restrict__ W,
                             const dcplx* __restrict__ A, dcplx* __restrict__ B) {
+  grid_enter();
   const int64_t rows = (int64_t)wl * bl, cols = (int64_t)wr * br, tot = rows * d * cols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = t % rows, rest = t / rows;
@@ -62,6 +64,7 @@ __global__ void k_mult_site(int wl, int d, int wr, int bl, int br, const dcplx* 
 // B[(wl + Wl bl), u, f] = sum_{wr, s} W[wl,u,wr,s] Tb[bl,s,wr,f]
 __global__ void k_mult_carry(int wl, int d, int wr, int bl, int f, const dcplx* __restrict__ W,
                              const dcplx* __restrict__ Tb, dcplx* __restrict__ B) {
+  grid_enter();
   const int64_t rows = (int64_t)wl * bl, tot = rows * d * f;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
     const int64_t r = t % rows, rest = t / rows;
@@ -81,6 +84,7 @@ __global__ void k_mult_carry(int wl, int d, int wr, int bl, int f, const dcplx* 
 
 // Y[br, wr, f] = X[wr, br, f] (swap of the two leading dims)
 __global__ void k_swap01(int a, int b, int64_t c, const dcplx* __restrict__ X, dcplx* __restrict__ Y) {
+  grid_enter();
   const int64_t tot = (int64_t)a * b * c;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
     const int i = (int)(t % a);
@@ -93,6 +97,7 @@ __global__ void k_swap01(int a, int b, int64_t c, const dcplx* __restrict__ X, d
 
 // X[r, c] *= s[c] (real), rows x cols column-major
 __global__ void k_scale_cols_real(int rows, int cols, dcplx* X, const double* __restrict__ s) {
+  grid_enter();
   const int64_t tot = (int64_t)rows * cols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
     const double a = s[t / rows];
@@ -104,7 +109,7 @@ __global__ void k_scale_cols_real(int rows, int cols, dcplx* X, const double* __
 void scale_cols(Context* ctx, int rows, int cols, dcplx* X, const std::vector<double>& s) {
   DevBuf& sd = ctx->buf("mult_scale", s.size() * sizeof(double));
   upload(ctx, sd.ptr, s.data(), s.size() * sizeof(double));
-  k_scale_cols_real<<<grid_for((int64_t)rows * cols), 256, 0, ctx->stream>>>(rows, cols, X, sd.d());
+  launch_kernel(ctx, k_scale_cols_real, grid_for((int64_t)rows * cols), 256, 0, rows, cols, X, sd.d());
   launched(ctx, "mult scale");
 }
 
@@ -239,7 +244,7 @@ KrylovResult mult_fixedpoints(Context* ctx, imps_mult_envs* E, double tol, int m
     DevBuf& v0 = ctx->buf("mult_v0", n * sizeof(dcplx));
     if (warm) zcopy(ctx, n, E->lefts[0].z(), v0.z());
     else {
-      k_env_start<<<grid_for(n), 256, 0, ctx->stream>>>(n, v0.z());
+      launch_kernel(ctx, k_env_start, grid_for(n), 256, 0, n, v0.z());
       launched(ctx, "mult env start");
     }
     size_t mx = 0;
@@ -270,7 +275,7 @@ KrylovResult mult_fixedpoints(Context* ctx, imps_mult_envs* E, double tol, int m
     DevBuf& v0 = ctx->buf("mult_v0", n * sizeof(dcplx));
     if (warm) zcopy(ctx, n, E->rights[N - 1].z(), v0.z());
     else {
-      k_env_start<<<grid_for(n), 256, 0, ctx->stream>>>(n, v0.z());
+      launch_kernel(ctx, k_env_start, grid_for(n), 256, 0, n, v0.z());
       launched(ctx, "mult env start");
     }
     size_t mx = 0;
@@ -409,7 +414,7 @@ imps_state* mult_guess(Context* ctx, const imps_mpo* W, const imps_state* ket, i
     if (!carry) {
       Bcols = wr * br;
       Bb.ensure((size_t)Brows * d * Bcols * sizeof(dcplx));
-      k_mult_site<<<grid_for((int64_t)Brows * d * Bcols), 256, 0, ctx->stream>>>(wl, d, wr, bl, br, Wi.Wdev.z(),
+      launch_kernel(ctx, k_mult_site, grid_for((int64_t)Brows * d * Bcols), 256, 0, wl, d, wr, bl, br, Wi.Wdev.z(),
                                                                                  ket->AL[i].z(), Bb.z());
       launched(ctx, "mult site");
       return;
@@ -417,13 +422,13 @@ imps_state* mult_guess(Context* ctx, const imps_mpo* W, const imps_state* ket, i
     Bcols = f;
     // l4[wr, br, f] -> l4p[br, wr, f]; Tb = AL (bl d x br) l4p (br x wr f) = Tb[bl, d, wr, f]
     DevBuf& l4p = ctx->buf("guess_l4p", (size_t)wr * br * f * sizeof(dcplx));
-    k_swap01<<<grid_for((int64_t)wr * br * f), 256, 0, ctx->stream>>>(wr, br, f, carry, l4p.z());
+    launch_kernel(ctx, k_swap01, grid_for((int64_t)wr * br * f), 256, 0, wr, br, f, carry, l4p.z());
     launched(ctx, "mult swap");
     DevBuf& Tb = ctx->buf("guess_tb", (size_t)bl * d * wr * f * sizeof(dcplx));
     zgemm(ctx, OP_N, OP_N, bl * d, wr * f, br, 1.0, ket->AL[i].z(), (int64_t)bl * d, 0, l4p.z(), br, 0, 0.0, Tb.z(),
           (int64_t)bl * d, 0, 1);
     Bb.ensure((size_t)Brows * d * f * sizeof(dcplx));
-    k_mult_carry<<<grid_for((int64_t)Brows * d * f), 256, 0, ctx->stream>>>(wl, d, wr, bl, f, Wi.Wdev.z(), Tb.z(),
+    launch_kernel(ctx, k_mult_carry, grid_for((int64_t)Brows * d * f), 256, 0, wl, d, wr, bl, f, Wi.Wdev.z(), Tb.z(),
                                                                             Bb.z());
     launched(ctx, "mult carry");
   };

@@ -46,6 +46,7 @@ __device__ __forceinline__ int rr_player(int pos, int r, int P) {
 __global__ void __launch_bounds__(kJacThreads) k_jacobi_round(int n, int ncol, int P, int r, dcplx* __restrict__ U,
                                                           int64_t ldu, double tol, int* __restrict__ rot,
                                                           dcplx* __restrict__ V, int nv, int64_t ldv) {
+  grid_enter();
   __shared__ double sh[kJacThreads / 32];
   const int k = blockIdx.x;
   int a = rr_player(k, r, P), b = rr_player(P - 1 - k, r, P);
@@ -157,6 +158,7 @@ __device__ __forceinline__ bool jacobi_pair(dcplx (&x)[EPL], dcplx (&y)[EPL], do
 template <int EPL>
 __global__ void __launch_bounds__(32 * kJacBlk) k_jacobi_block(int n, int nblk, int r, dcplx* __restrict__ U,
                                                                int64_t ldu, double tol2, int* __restrict__ rot) {
+  grid_enter();
   extern __shared__ dcplx cols[];   // [16][32 EPL]
   constexpr int LDC = 32 * EPL;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k = blockIdx.x;
@@ -227,12 +229,13 @@ void jacobi_block_round(Context* ctx, int n, int nblk, int r, dcplx* U, double t
   attr.run(ctx->device, [] {
     IMPS_CUDA(cudaFuncSetAttribute(k_jacobi_block<EPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
   });
-  k_jacobi_block<EPL><<<nblk / 2, 32 * kJacBlk, SMEM, ctx->stream>>>(n, nblk, r, U, n, tol * tol, rot);
+  launch_kernel(ctx, k_jacobi_block<EPL>, nblk / 2, 32 * kJacBlk, SMEM, n, nblk, r, U, n, tol * tol, rot);
 }
 
 // out[:, j] = scale_j * in[:, perm[j]] for j < k (column gather with optional scaling)
 __global__ void k_gather_cols(int rows, int k, const dcplx* __restrict__ in, int64_t ldi, const int* __restrict__ perm,
                               const double* __restrict__ scale, dcplx* __restrict__ out, int64_t ldo) {
+  grid_enter();
   const int64_t tot = (int64_t)rows * k;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
     const int i = (int)(t % rows), j = (int)(t / rows);
@@ -243,6 +246,7 @@ __global__ void k_gather_cols(int rows, int k, const dcplx* __restrict__ in, int
 }
 
 __global__ void k_col_norms2(int n, int ncol, const dcplx* __restrict__ U, int64_t ldu, double* __restrict__ out) {
+  grid_enter();
   __shared__ double sh[kJacThreads / 32];
   const int j = blockIdx.x;
   if (j >= ncol) return;
@@ -281,7 +285,7 @@ static void jacobi_sweeps(Context* ctx, int n, int ncol, dcplx* U) {
       }
     } else {  // 16 columns do not fit in a CTA's shared memory and registers
       for (int r = 0; r < P - 1; ++r) {
-        k_jacobi_round<<<P / 2, kJacThreads, 0, ctx->stream>>>(n, ncol, P, r, U, n, tol, rot, nullptr, 0, 0);
+        launch_kernel(ctx, k_jacobi_round, P / 2, kJacThreads, 0, n, ncol, P, r, U, n, tol, rot, nullptr, 0, 0);
         check(ctx);
       }
     }
@@ -305,7 +309,7 @@ std::vector<double> singular_values_sq(Context* ctx, int D, const dcplx* A, int6
   zfill(ctx, (int64_t)D * P, 0.0, U.z());
   std::vector<double> s2(D);
   auto norms = [&] {
-    k_col_norms2<<<D, kJacThreads, 0, ctx->stream>>>(D, D, U.z(), D, nr.d());
+    launch_kernel(ctx, k_col_norms2, D, kJacThreads, 0, D, D, U.z(), D, nr.d());
     check(ctx);
     download(ctx, s2.data(), nr.ptr, D * sizeof(double));
   };
@@ -330,7 +334,7 @@ std::vector<double> singular_values_sq(Context* ctx, int D, const dcplx* A, int6
       DevBuf& R = ctx->buf("jac_r", (size_t)D * D * sizeof(dcplx));
       int* pd = static_cast<int*>(ctx->buf("jac_perm", (size_t)D * sizeof(int)).ptr);
       upload(ctx, pd, perm.data(), (size_t)D * sizeof(int));
-      k_gather_cols<<<148 * 8, 256, 0, ctx->stream>>>(D, D, U.z(), D, pd, nullptr, W.z(), D);
+      launch_kernel(ctx, k_gather_cols, 148 * 8, 256, 0, D, D, U.z(), D, pd, nullptr, W.z(), D);
       check(ctx);
       qr_factor(ctx, D, D, W.z(), D, R.z(), "qr");
       zconj_transpose(ctx, D, D, R.z(), D, U.z(), D);
@@ -371,7 +375,7 @@ int svd_thin(Context* ctx, int m, int n, const dcplx* A, int64_t lda, int kmax, 
   for (int sweep = 0; sweep < 60; ++sweep) {
     IMPS_CUDA(cudaMemsetAsync(flag.ptr, 0, sizeof(int), ctx->stream));
     for (int r = 0; r < P - 1; ++r) {
-      k_jacobi_round<<<P / 2, kJacThreads, 0, ctx->stream>>>(m, n, P, r, W.z(), m, tol, static_cast<int*>(flag.ptr),
+      launch_kernel(ctx, k_jacobi_round, P / 2, kJacThreads, 0, m, n, P, r, W.z(), m, tol, static_cast<int*>(flag.ptr),
                                                              Vw.z(), n, n);
       check(ctx);
     }
@@ -379,7 +383,7 @@ int svd_thin(Context* ctx, int m, int n, const dcplx* A, int64_t lda, int kmax, 
     download(ctx, &rot, flag.ptr, sizeof(int));
     if (rot == 0) break;
   }
-  k_col_norms2<<<n, kJacThreads, 0, ctx->stream>>>(m, n, W.z(), m, nr.d());
+  launch_kernel(ctx, k_col_norms2, n, kJacThreads, 0, m, n, W.z(), m, nr.d());
   check(ctx);
   std::vector<double> n2(n);
   download(ctx, n2.data(), nr.ptr, n * sizeof(double));
@@ -402,9 +406,9 @@ int svd_thin(Context* ctx, int m, int n, const dcplx* A, int64_t lda, int kmax, 
   upload(ctx, sd, inv.data(), (size_t)k * sizeof(double));
   auto grid = [](int64_t t) { return (int)std::max<int64_t>(1, std::min<int64_t>((t + 255) / 256, 148 * 8)); };
   // U = W[:, perm] / s (columns of exactly zero singular value stay zero), V = Vw[:, perm]
-  k_gather_cols<<<grid((int64_t)m * k), 256, 0, ctx->stream>>>(m, k, W.z(), m, pd, sd, U, m);
+  launch_kernel(ctx, k_gather_cols, grid((int64_t)m * k), 256, 0, m, k, W.z(), m, pd, sd, U, m);
   check(ctx);
-  k_gather_cols<<<grid((int64_t)n * k), 256, 0, ctx->stream>>>(n, k, Vw.z(), n, pd, nullptr, V, n);
+  launch_kernel(ctx, k_gather_cols, grid((int64_t)n * k), 256, 0, n, k, Vw.z(), n, pd, nullptr, V, n);
   check(ctx);
   return k;
 }

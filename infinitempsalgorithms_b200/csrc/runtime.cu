@@ -43,6 +43,7 @@ __device__ __forceinline__ double block_sum(double v, double* sh) {
 }
 
 __global__ void k_nrm2_partial(int64_t n, const dcplx* __restrict__ x, double* __restrict__ part) {
+  grid_enter();
   __shared__ double sh[kRedThreads / 32];
   double s = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -55,6 +56,7 @@ __global__ void k_nrm2_partial(int64_t n, const dcplx* __restrict__ x, double* _
 
 __global__ void k_dotc_partial(int64_t n, const dcplx* __restrict__ x, const dcplx* __restrict__ y,
                                double* __restrict__ part) {
+  grid_enter();
   __shared__ double sh[kRedThreads / 32];
   double sr = 0.0, si = 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -72,6 +74,7 @@ __global__ void k_dotc_partial(int64_t n, const dcplx* __restrict__ x, const dcp
 
 // Sum `ncol` columns of partials (each `nb` long, stride ld) in a fixed order.
 __global__ void k_final_sum(int nb, int ncol, const double* __restrict__ part, int64_t ld, double* __restrict__ out) {
+  grid_enter();
   __shared__ double sh[kRedThreads / 32];
   for (int c = 0; c < ncol; ++c) {
     double s = 0.0;
@@ -83,6 +86,7 @@ __global__ void k_final_sum(int nb, int ncol, const double* __restrict__ part, i
 
 // One block per column: out[c] = sum_i part[i + ld c] (same order as k_final_sum).
 __global__ void k_final_sum_cols(int nb, const double* __restrict__ part, int64_t ld, double* __restrict__ out) {
+  grid_enter();
   __shared__ double sh[kRedThreads / 32];
   const int c = blockIdx.x;
   double s = 0.0;
@@ -96,6 +100,7 @@ __global__ void k_final_sum_cols(int nb, const double* __restrict__ part, int64_
 template <int CH>
 __global__ void k_proj_dots(int64_t n, int nv, const dcplx* __restrict__ V, int64_t ldv, const dcplx* __restrict__ w,
                             double* __restrict__ part, int64_t ldp, int col0, int norm_col) {
+  grid_enter();
   __shared__ double sh[kRedThreads / 32];
   double ar[CH], ai[CH], nn = 0.0;
 #pragma unroll
@@ -134,6 +139,7 @@ __global__ void k_proj_dots(int64_t n, int nv, const dcplx* __restrict__ V, int6
 // of the new ||w||^2 (one per block) go to `npart`.
 __global__ void k_proj_update(int64_t n, int nv, const dcplx* __restrict__ V, int64_t ldv,
                               const double* __restrict__ hdev, dcplx* __restrict__ w, double* __restrict__ npart) {
+  grid_enter();
   __shared__ double2 c[32];
   __shared__ double sh[kRedThreads / 32];
   if (threadIdx.x < nv) c[threadIdx.x] = make_double2(-hdev[2 * threadIdx.x], -hdev[2 * threadIdx.x + 1]);
@@ -182,6 +188,7 @@ template <int NV, bool UPDATE>
 __global__ void __launch_bounds__(GS_THREADS) k_gs_pass(int64_t n, int nv, const dcplx* __restrict__ V, int64_t ldv,
                                                        const double* __restrict__ hdev, dcplx* __restrict__ w,
                                                        double* __restrict__ part, int64_t ldp) {
+  grid_enter();
   constexpr int TPC = GS_THREADS / NV;   // threads per column in the dot phase
   constexpr int RPD = GS_ROWS / TPC;     // rows per thread in the dot phase
   constexpr int STAGE = (NV + 1) * GS_ROWS;
@@ -299,6 +306,7 @@ struct CoefPack {
 
 __global__ void k_gemv_acc(int64_t n, int nv, const dcplx* __restrict__ V, int64_t ldv, CoefPack coef,
                            dcplx* __restrict__ w, int set) {
+  grid_enter();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     dcplx acc = set ? make_double2(0.0, 0.0) : w[i];
     for (int j = 0; j < nv; ++j) {
@@ -311,11 +319,13 @@ __global__ void k_gemv_acc(int64_t n, int nv, const dcplx* __restrict__ V, int64
 }
 
 __global__ void k_scal(int64_t n, double2 a, dcplx* x) {
+  grid_enter();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     x[i] = cmul(a, x[i]);
 }
 __global__ void k_axpby(int64_t n, double2 a, const dcplx* __restrict__ x, double2 b, dcplx* __restrict__ y,
                         int use_b) {
+  grid_enter();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     dcplx v = cmul(a, x[i]);
     if (use_b) {
@@ -327,6 +337,7 @@ __global__ void k_axpby(int64_t n, double2 a, const dcplx* __restrict__ x, doubl
   }
 }
 __global__ void k_axpy(int64_t n, double2 a, const dcplx* __restrict__ x, dcplx* __restrict__ y) {
+  grid_enter();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     dcplx v = cmul(a, x[i]);
     dcplx u = y[i];
@@ -334,10 +345,12 @@ __global__ void k_axpy(int64_t n, double2 a, const dcplx* __restrict__ x, dcplx*
   }
 }
 __global__ void k_fill(int64_t n, double2 v, dcplx* x) {
+  grid_enter();
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     x[i] = v;
 }
 __global__ void k_set_identity(int D, dcplx* X, int64_t ld, double2 diag) {
+  grid_enter();
   int64_t total = (int64_t)D * D;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     int a = (int)(t % D), b = (int)(t / D);
@@ -348,6 +361,7 @@ __global__ void k_set_identity(int D, dcplx* X, int64_t ld, double2 diag) {
 // 32 x 32 tiled conjugate transpose: Y[j + ldy i] = conj(X[i + ldx j]).
 __global__ void k_conj_transpose(int m, int n, const dcplx* __restrict__ X, int64_t ldx, dcplx* __restrict__ Y,
                                  int64_t ldy) {
+  grid_enter();
   __shared__ dcplx tile[32][33];
   int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32;
   for (int r = threadIdx.y; r < 32; r += blockDim.y) {
@@ -367,6 +381,7 @@ __global__ void k_conj_transpose(int m, int n, const dcplx* __restrict__ X, int6
 // partials of sum_{a,b} L[a,b] V[b,a]
 __global__ void k_trace_prod_partial(int D, const dcplx* __restrict__ L, int64_t ldl, const dcplx* __restrict__ V,
                                      int64_t ldv, double* __restrict__ part) {
+  grid_enter();
   __shared__ double sh[kRedThreads / 32];
   double sr = 0.0, si = 0.0;
   int64_t total = (int64_t)D * D;
@@ -389,6 +404,7 @@ __global__ void k_trace_prod_partial(int D, const dcplx* __restrict__ L, int64_t
 // corrects the diagonal; no trip to the host.  The counter is left at zero.
 __global__ void k_regularize(int D, const dcplx* __restrict__ L, int64_t ldl, dcplx* __restrict__ V, int64_t ldv,
                              double* __restrict__ part, unsigned* __restrict__ counter) {
+  grid_enter();
   __shared__ double sh[kRedThreads / 32];
   __shared__ double all[2 * kMaxRedBlocks];
   __shared__ double tr[2];
@@ -429,6 +445,7 @@ __global__ void k_regularize(int D, const dcplx* __restrict__ L, int64_t ldl, dc
 
 __global__ void k_copy2d(int rows, int cols, const dcplx* __restrict__ X, int64_t ldx, dcplx* __restrict__ Y,
                          int64_t ldy, int add) {
+  grid_enter();
   int64_t total = (int64_t)rows * cols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     int r = (int)(t % rows), c = (int)(t / rows);
@@ -443,12 +460,14 @@ __global__ void k_copy2d(int rows, int cols, const dcplx* __restrict__ X, int64_
 }
 
 __global__ void k_add_diag(int D, dcplx* X, int64_t ld, double2 v) {
+  grid_enter();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < D; i += gridDim.x * blockDim.x) {
     dcplx u = X[i + ld * i];
     X[i + ld * i] = make_double2(u.x + v.x, u.y + v.y);
   }
 }
 __global__ void k_fill2d(int rows, int cols, dcplx* Y, int64_t ldy, double2 v) {
+  grid_enter();
   int64_t total = (int64_t)rows * cols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     int r = (int)(t % rows), c = (int)(t / rows);
@@ -717,27 +736,27 @@ void zcopy(Context* ctx, int64_t n, const dcplx* x, dcplx* y) {
 }
 void zscal(Context* ctx, int64_t n, cplx a, dcplx* x) {
   if (n <= 0) return;
-  k_scal<<<grid_for(n), 256, 0, ctx->stream>>>(n, d2(a), x);
+  launch_kernel(ctx, k_scal, grid_for(n), 256, 0, n, d2(a), x);
   check_launch(ctx);
 }
 void zaxpy(Context* ctx, int64_t n, cplx a, const dcplx* x, dcplx* y) {
   if (n <= 0) return;
-  k_axpy<<<grid_for(n), 256, 0, ctx->stream>>>(n, d2(a), x, y);
+  launch_kernel(ctx, k_axpy, grid_for(n), 256, 0, n, d2(a), x, y);
   check_launch(ctx);
 }
 void zaxpby(Context* ctx, int64_t n, cplx a, const dcplx* x, cplx b, dcplx* y) {
   if (n <= 0) return;
-  k_axpby<<<grid_for(n), 256, 0, ctx->stream>>>(n, d2(a), x, d2(b), y, b != cplx(0.0, 0.0));
+  launch_kernel(ctx, k_axpby, grid_for(n), 256, 0, n, d2(a), x, d2(b), y, b != cplx(0.0, 0.0));
   check_launch(ctx);
 }
 void zfill(Context* ctx, int64_t n, cplx v, dcplx* x) {
   if (n <= 0) return;
-  k_fill<<<grid_for(n), 256, 0, ctx->stream>>>(n, d2(v), x);
+  launch_kernel(ctx, k_fill, grid_for(n), 256, 0, n, d2(v), x);
   check_launch(ctx);
 }
 void zset_identity(Context* ctx, int D, dcplx* X, int64_t ld, cplx diag) {
   if (D <= 0) return;
-  k_set_identity<<<grid_for((int64_t)D * D), 256, 0, ctx->stream>>>(D, X, ld, d2(diag));
+  launch_kernel(ctx, k_set_identity, grid_for((int64_t)D * D), 256, 0, D, X, ld, d2(diag));
   check_launch(ctx);
 }
 
@@ -747,9 +766,9 @@ double dznrm2(Context* ctx, int64_t n, const dcplx* x) {
   DevBuf& red = ctx->buf("red_part", (size_t)(nb + 8) * sizeof(double));
   DevBuf& out = ctx->buf("red_out", 64 * sizeof(double));
   ScopedTimer t(ctx, "blas1", (double)n * 16);
-  k_nrm2_partial<<<nb, kRedThreads, 0, ctx->stream>>>(n, x, red.d());
+  launch_kernel(ctx, k_nrm2_partial, nb, kRedThreads, 0, n, x, red.d());
   check_launch(ctx);
-  k_final_sum<<<1, kRedThreads, 0, ctx->stream>>>(nb, 1, red.d(), nb, out.d());
+  launch_kernel(ctx, k_final_sum, 1, kRedThreads, 0, nb, 1, red.d(), nb, out.d());
   check_launch(ctx);
   double h;
   download(ctx, &h, out.d(), sizeof(double));
@@ -763,7 +782,7 @@ cplx zdotc(Context* ctx, int64_t n, const dcplx* x, const dcplx* y) {
   DevBuf& out = ctx->buf("red_out", 64 * sizeof(double));
   ScopedTimer t(ctx, "blas1", (double)n * 32);
   (void)out;
-  k_dotc_partial<<<nb, kRedThreads, 0, ctx->stream>>>(n, x, y, red.d());
+  launch_kernel(ctx, k_dotc_partial, nb, kRedThreads, 0, n, x, y, red.d());
   check_launch(ctx);
   double h[2];
   {
@@ -787,7 +806,7 @@ static void gemv_common(Context* ctx, int64_t n, int nv, const dcplx* V, int64_t
     int cnt = std::min(32, nv - done);
     CoefPack p;
     for (int j = 0; j < cnt; ++j) p.c[j] = d2(coef[done + j]);
-    k_gemv_acc<<<grid_for(n), 256, 0, ctx->stream>>>(n, cnt, V + ldv * (int64_t)done, ldv, p, w,
+    launch_kernel(ctx, k_gemv_acc, grid_for(n), 256, 0, n, cnt, V + ldv * (int64_t)done, ldv, p, w,
                                                       (first && set) ? 1 : 0);
     check_launch(ctx);
     done += cnt;
@@ -815,29 +834,29 @@ double proj_pass(Context* ctx, int64_t n, int nv, const dcplx* V, int64_t ldv, d
   ScopedTimer t(ctx, "orth", (double)n * 16 * (2 * nv + 3));
   const int norm_col = nw_old2 ? 2 * nv : -1;
   if (nv == 0 && nw_old2) {
-    k_proj_dots<CH><<<nb, kRedThreads, 0, ctx->stream>>>(n, 0, V, ldv, w, red.d(), nb, 0, norm_col);
+    launch_kernel(ctx, k_proj_dots<CH>, nb, kRedThreads, 0, n, 0, V, ldv, w, red.d(), nb, 0, norm_col);
     check_launch(ctx);
   }
   for (int c0 = 0; c0 < nv; c0 += CH) {
     const int nvc = std::min(CH, nv - c0);
-    k_proj_dots<CH><<<nb, kRedThreads, 0, ctx->stream>>>(n, nvc, V + ldv * (int64_t)c0, ldv, w, red.d(), nb, 2 * c0,
+    launch_kernel(ctx, k_proj_dots<CH>, nb, kRedThreads, 0, n, nvc, V + ldv * (int64_t)c0, ldv, w, red.d(), nb, 2 * c0,
                                                          c0 == 0 ? norm_col : -1);
     check_launch(ctx);
   }
   const int ndots = 2 * nv + (nw_old2 ? 1 : 0);
   if (ndots > 0) {
-    k_final_sum_cols<<<ndots, kRedThreads, 0, ctx->stream>>>(nb, red.d(), nb, out.d());
+    launch_kernel(ctx, k_final_sum_cols, ndots, kRedThreads, 0, nb, red.d(), nb, out.d());
     check_launch(ctx);
   }
   for (int c0 = 0; c0 < nv || (nv == 0 && c0 == 0); c0 += 32) {
     const int cnt = std::min(32, nv - c0);
     const bool last = c0 + 32 >= nv;
-    k_proj_update<<<nb, kRedThreads, 0, ctx->stream>>>(n, cnt, V + ldv * (int64_t)c0, ldv, out.d() + 2 * c0, w,
+    launch_kernel(ctx, k_proj_update, nb, kRedThreads, 0, n, cnt, V + ldv * (int64_t)c0, ldv, out.d() + 2 * c0, w,
                                                        last ? red.d() + (size_t)nb * (2 * nv + 1) : nullptr);
     check_launch(ctx);
     if (nv == 0) break;
   }
-  k_final_sum_cols<<<1, kRedThreads, 0, ctx->stream>>>(nb, red.d() + (size_t)nb * (2 * nv + 1), nb,
+  launch_kernel(ctx, k_final_sum_cols, 1, kRedThreads, 0, nb, red.d() + (size_t)nb * (2 * nv + 1), nb,
                                                        out.d() + 2 * nv + 1);
   check_launch(ctx);
   std::vector<double> hv(ncol);
@@ -862,7 +881,7 @@ void launch_gs_kernel(Context* ctx, int nb, int64_t n, int nv, const dcplx* V, i
     IMPS_CUDA(cudaFuncSetAttribute(k_gs_pass<NV, UPDATE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)gs_smem_bytes<NV>()));
   });
-  k_gs_pass<NV, UPDATE><<<nb, GS_THREADS, gs_smem_bytes<NV>(), ctx->stream>>>(n, nv, V, ldv, hdev, w, part, ldp);
+  launch_kernel(ctx, k_gs_pass<NV, UPDATE>, nb, GS_THREADS, gs_smem_bytes<NV>(), n, nv, V, ldv, hdev, w, part, ldp);
 }
 int gs_pass_blocks(int64_t n, int nv) {
   return nv <= 8 ? gs_blocks_for<8>(n) : nv <= 16 ? gs_blocks_for<16>(n) : gs_blocks_for<32>(n);
@@ -881,7 +900,7 @@ void gs_pass(Context* ctx, bool update, int64_t n, int nv, const dcplx* V, int64
     else launch_gs_kernel<32, false>(ctx, nb, n, nv, V, ldv, hdev, w, part, ldp);
   }
   check_launch(ctx);
-  k_final_sum_cols<<<2 * nv + 1, kRedThreads, 0, ctx->stream>>>(nb, part, ldp, out);
+  launch_kernel(ctx, k_final_sum_cols, 2 * nv + 1, kRedThreads, 0, nb, part, ldp, out);
   check_launch(ctx);
 }
 const char* kNonFinite =
@@ -945,7 +964,7 @@ void zconj_transpose(Context* ctx, int m, int n, const dcplx* X, int64_t ldx, dc
   if (m <= 0 || n <= 0) return;
   dim3 grid((m + 31) / 32, (n + 31) / 32), block(32, 8);
   ScopedTimer t(ctx, "permute", (double)m * n * 32);
-  k_conj_transpose<<<grid, block, 0, ctx->stream>>>(m, n, X, ldx, Y, ldy);
+  launch_kernel(ctx, k_conj_transpose, grid, block, 0, m, n, X, ldx, Y, ldy);
   check_launch(ctx);
 }
 
@@ -953,7 +972,7 @@ cplx ztrace_prod(Context* ctx, int D, const dcplx* L, int64_t ldl, const dcplx* 
   int64_t n = (int64_t)D * D;
   int nb = red_blocks(n);
   DevBuf& red = ctx->buf("red_part", (size_t)(2 * nb + 8) * sizeof(double));
-  k_trace_prod_partial<<<nb, kRedThreads, 0, ctx->stream>>>(D, L, ldl, V, ldv, red.d());
+  launch_kernel(ctx, k_trace_prod_partial, nb, kRedThreads, 0, D, L, ldl, V, ldv, red.d());
   check_launch(ctx);
   std::vector<double> p(2 * nb);
   download(ctx, p.data(), red.d(), p.size() * sizeof(double));
@@ -965,24 +984,24 @@ cplx ztrace_prod(Context* ctx, int D, const dcplx* L, int64_t ldl, const dcplx* 
 void zregularize(Context* ctx, int D, const dcplx* rho, int64_t ldr, dcplx* X, int64_t ldx) {
   const int nb = red_blocks((int64_t)D * D);
   DevBuf& red = ctx->buf("red_part", (size_t)(2 * nb + 8) * sizeof(double));
-  k_regularize<<<nb, kRedThreads, 0, ctx->stream>>>(D, rho, ldr, X, ldx, red.d(), ctx->counters);
+  launch_kernel(ctx, k_regularize, nb, kRedThreads, 0, D, rho, ldr, X, ldx, red.d(), ctx->counters);
   check_launch(ctx);
 }
 
 void zcopy2d(Context* ctx, int rows, int cols, const dcplx* X, int64_t ldx, dcplx* Y, int64_t ldy) {
   if (rows <= 0 || cols <= 0) return;
-  k_copy2d<<<grid_for((int64_t)rows * cols), 256, 0, ctx->stream>>>(rows, cols, X, ldx, Y, ldy, 0);
+  launch_kernel(ctx, k_copy2d, grid_for((int64_t)rows * cols), 256, 0, rows, cols, X, ldx, Y, ldy, 0);
   check_launch(ctx);
 }
 
 void zadd_diag(Context* ctx, int D, dcplx* X, int64_t ld, cplx v) {
   if (D <= 0) return;
-  k_add_diag<<<grid_for(D), 256, 0, ctx->stream>>>(D, X, ld, d2(v));
+  launch_kernel(ctx, k_add_diag, grid_for(D), 256, 0, D, X, ld, d2(v));
   check_launch(ctx);
 }
 void zfill2d(Context* ctx, int rows, int cols, cplx v, dcplx* Y, int64_t ldy) {
   if (rows <= 0 || cols <= 0) return;
-  k_fill2d<<<grid_for((int64_t)rows * cols), 256, 0, ctx->stream>>>(rows, cols, Y, ldy, d2(v));
+  launch_kernel(ctx, k_fill2d, grid_for((int64_t)rows * cols), 256, 0, rows, cols, Y, ldy, d2(v));
   check_launch(ctx);
 }
 

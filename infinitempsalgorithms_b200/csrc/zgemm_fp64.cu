@@ -25,6 +25,7 @@ __global__ void __launch_bounds__(NT, 2)
     k_zgemm(int M, int N, int K, double2 alpha, const double2* __restrict__ A, int64_t lda, int64_t sA,
             const double2* __restrict__ B, int64_t ldb, int64_t sB, double2 beta, double2* __restrict__ C,
             int64_t ldc, int64_t sC) {
+  grid_enter();
   __shared__ double2 As[2][BK][BM + 1];
   __shared__ double2 Bs[2][BK][BN + 1];
   const int bz = blockIdx.z;
@@ -177,6 +178,7 @@ __global__ void __launch_bounds__(4 * T, T == 64 ? 2 : 4)
     k_zgemm_dmma(int M, int N, int K, double2 alpha, const double2* __restrict__ A, int64_t lda, int64_t sA,
                  const double2* __restrict__ B, int64_t ldb, int64_t sB, double2 beta, double2* __restrict__ C,
                  int64_t ldc, int64_t sC, int nsplit, double2* __restrict__ part) {
+  grid_enter();
   using D = dm::Tile<T>;
   extern __shared__ __align__(16) double2 smem_dm[];   // [STAGES][A tile, B tile][BK][LD]
   const int bz = blockIdx.z;
@@ -314,6 +316,7 @@ template <bool BETA>
 __global__ void __launch_bounds__(256) k_sum_split(int M, int N, int nsplit, const double2* __restrict__ part,
                                                    double2 alpha, double2 beta, double2* __restrict__ C, int64_t ldc,
                                                    int64_t sC) {
+  grid_enter();
   const int64_t len = (int64_t)M * N;
   part += (int64_t)blockIdx.y * nsplit * len;
   C += sC * blockIdx.y;
@@ -357,7 +360,7 @@ void launch_dmma(Context* ctx, int nsplit, double2* part, int M, int N, int K, d
     IMPS_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, D::SMEM));
   });
   const dim3 grid((M + T - 1) / T * nsplit, (N + T - 1) / T, batch);
-  kern<<<grid, D::NT, D::SMEM, ctx->stream>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, nsplit, part);
+  launch_kernel(ctx, kern, grid, D::NT, D::SMEM, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC, nsplit, part);
 }
 
 // Tile size and CTAs that share a tile's K stages (1: none): the smallest time of a model of
@@ -394,9 +397,9 @@ void launch(Context* ctx, int M, int N, int K, double2 alpha, const dcplx* A, in
   if (ctx->fp64_engine == 1) {
     dim3 grid((M + BM - 1) / BM, (N + BN - 1) / BN, batch);
     if (use_beta)
-      k_zgemm<OPA, OPB, true><<<grid, NT, 0, ctx->stream>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC);
+      launch_kernel(ctx, k_zgemm<OPA, OPB, true>, grid, NT, 0, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc, sC);
     else
-      k_zgemm<OPA, OPB, false><<<grid, NT, 0, ctx->stream>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc,
+      launch_kernel(ctx, k_zgemm<OPA, OPB, false>, grid, NT, 0, M, N, K, alpha, A, lda, sA, B, ldb, sB, beta, C, ldc,
                                                               sC);
     return;
   }
@@ -425,7 +428,7 @@ void launch(Context* ctx, int M, int N, int K, double2 alpha, const dcplx* A, in
     if (plan.tile == 64) run(std::true_type{}, Big{});
     else run(std::true_type{}, Small{});
     const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((len + 255) / 256, ctx->num_sms * 8 / batch));
-    k_sum_split<BETA><<<dim3(g, batch), 256, 0, ctx->stream>>>(M, N, s, part, alpha, beta, C, ldc, sC);
+    launch_kernel(ctx, k_sum_split<BETA>, dim3(g, batch), 256, 0, M, N, s, part, alpha, beta, C, ldc, sC);
     ctx->n_kernels++;
   };
   if (use_beta) go(std::true_type{});
