@@ -463,34 +463,50 @@ __global__ void __launch_bounds__(NTHREADS, 1)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long dbits(double x) { return (unsigned long long)__double_as_longlong(x); }
 
-// per strided line i (A[i + lda k]) -> atomicMax of max(|re|,|im|) bits
-__global__ void k_rowmax_colmajor(int M, int K, const double2* __restrict__ A, int64_t lda, int kchunk,
-                                  unsigned long long* __restrict__ out) {
+// per strided line i (A[i + lda k]) -> atomicMax of max(|re|,|im|) bits; RM_K values of k at
+// a time, all loads in flight (2304 x 384: 11 us; 20 us in chunks of 64, a few loads at a time,
+// whose blocks did not fill the chip)
+constexpr int RM_K = 16;
+__global__ void __launch_bounds__(128) k_rowmax_colmajor(int M, int K, const double2* __restrict__ A, int64_t lda,
+                                                         unsigned long long* __restrict__ out) {
   grid_enter();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= M) return;
-  const int k0 = blockIdx.y * kchunk, k1 = min(K, k0 + kchunk);
   double m = 0.0;
-  for (int k = k0; k < k1; ++k) {
-    double2 v = A[i + lda * k];
-    m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
+  for (int64_t k0 = (int64_t)blockIdx.y * RM_K; k0 < K; k0 += (int64_t)gridDim.y * RM_K) {
+    const double2* a = A + i + lda * k0;
+    double2 v[RM_K];
+#pragma unroll
+    for (int j = 0; j < RM_K; ++j) v[j] = k0 + j < K ? a[lda * j] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int j = 0; j < RM_K; ++j) m = fmax(m, fmax(fabs(v[j].x), fabs(v[j].y)));
   }
   atomicMax(&out[i], dbits(m));
 }
-// per "contiguous line" l (A[k + ld l], k < K): max over k (warp per line)
-__global__ void k_linemax_contig(int L, int K, const double2* __restrict__ A, int64_t ld,
-                                 unsigned long long* __restrict__ out) {
+// per "contiguous line" l (A[k + ld l], k < K): max over k, a block a line (1024 lines of
+// 6144: 28 us; 45 us with a warp a line, which left the chip nearly empty)
+constexpr int LM_NT = 256;
+__global__ void __launch_bounds__(LM_NT) k_linemax_contig(int K, const double2* __restrict__ A, int64_t ld,
+                                                          unsigned long long* __restrict__ out) {
   grid_enter();
-  const int l = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (l >= L) return;
+  __shared__ double wm[LM_NT / 32];
+  const double2* a = A + ld * blockIdx.x;
   double m = 0.0;
-  for (int k = lane; k < K; k += 32) {
-    double2 v = A[k + ld * l];
-    m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
+  for (int k = threadIdx.x; k < K; k += 8 * LM_NT) {
+    double2 v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = k + j * LM_NT < K ? a[k + j * LM_NT] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) m = fmax(m, fmax(fabs(v[j].x), fabs(v[j].y)));
   }
+#pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) out[l] = dbits(m);
+  if ((threadIdx.x & 31) == 0) wm[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < LM_NT / 32; ++w) m = fmax(m, wm[w]);
+    out[blockIdx.x] = dbits(m);
+  }
 }
 // The scale 2^e > max of a line (0 for a line of zeros or one that holds a non-finite value)
 // and its inverse, exact powers of two.
@@ -625,12 +641,21 @@ __global__ void __launch_bounds__(32 * LB) k_split_lines(int L, int K, const dou
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, l = blockIdx.x * LB + w;
   const int Kc = (int)(Kp / 2);
   double2* row = lines + (int64_t)w * Kc;
-  double m = 0.0;
+  // the whole line in flight at once (4096 lines of 1024 at 5 slices, 109 MB: 31 us; 50 us by
+  // loads through registers, a few at a time)
   for (int k = lane; k < Kc; k += 32) {
-    double2 v = (l < L && k < K) ? X[k + ld * l] : make_double2(0.0, 0.0);
+    const bool live = l < L && k < K;
+    const uint32_t size = live ? 16u : 0u;   // 0: zeros
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(row + k)),
+                 "l"(live ? X + k + ld * l : X), "r"(size)
+                 : "memory");
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  double m = 0.0;
+  for (int k = lane; k < Kc; k += 32) {   // what this lane copied
+    const double2 v = row[k];
     m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
-    if (conj) v.y = -v.y;
-    row[k] = v;
+    if (conj) row[k].y = -v.y;
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -698,15 +723,15 @@ void slice_launch(Context* ctx, SplitOperand& O, bool kcontig, int conj, int L, 
   auto* mx = static_cast<unsigned long long*>(O.mx.ptr);
   const dim3 grid((unsigned)(O.Kp / 128), (unsigned)(padded / 32));
   if (kcontig) {   // lines too long for a block
-    launch_kernel(ctx, k_linemax_contig, (L + 7) / 8, 256, 0, L, K, X, ld, mx);
+    launch_kernel(ctx, k_linemax_contig, L, LM_NT, 0, K, X, ld, mx);
     launch_kernel(ctx, k_split_tile<SIDE, S, true>, grid, 256, 0, L, K, X, ld, conj, mx, O.scale.d(), out, O.Kp, plane);
     ctx->n_kernels += 2;
     return;
   }
   if (!have_max) {
     IMPS_CUDA(cudaMemsetAsync(mx, 0, (size_t)L * 8, ctx->stream));
-    const int kchunk = 64;
-    launch_kernel(ctx, k_rowmax_colmajor, dim3((L + 127) / 128, (K + kchunk - 1) / kchunk), 128, 0, L, K, X, ld, kchunk, mx);
+    const int gx = (L + 127) / 128, gy = std::min((K + RM_K - 1) / RM_K, std::max(1, ctx->num_sms * 32 / gx));
+    launch_kernel(ctx, k_rowmax_colmajor, dim3(gx, gy), 128, 0, L, K, X, ld, mx);
     ctx->n_kernels += 2;
   }
   launch_kernel(ctx, k_split_tile<SIDE, S, false>, grid, 256, 0, L, K, X, ld, conj, mx, O.scale.d(), out, O.Kp, plane);
