@@ -43,7 +43,9 @@ enum {
 /* Precision modes of the Heff / transfer contractions. */
 enum {
   IMPS_PREC_FP64 = 0,       /* plain method: FP64 results; large products through
-                               exact residue arithmetic, no less accurate          */
+                               residue arithmetic, where an element of a product
+                               over K is off by at most 2^-57 sqrt(2 K) of its row's
+                               and column's 2-norms, and its own rounding           */
   IMPS_PREC_SPLIT_I8 = 1    /* int8 split products on tcgen05, exact int32 sums    */
 };
 

@@ -28,6 +28,7 @@ thread_local std::string g_last_error;
 template <class F>
 int guard(imps::Context* ctx, F&& f) {
   try {
+    imps::RunningCall running(ctx);
     if (ctx) cudaSetDevice(ctx->device);
     int r = f();
     // a bounded wait that ran out inside this call surfaces here at the latest

@@ -77,6 +77,10 @@ class BlockPool {
   bool open_ = true;
 };
 
+// The device is out of memory: frees the idle blocks of all pools and the scratch that the
+// running call's context can do without.
+void give_back_idle();
+
 struct DevBuf {
   void* ptr = nullptr;
   size_t bytes = 0;
@@ -104,7 +108,7 @@ struct DevBuf {
     if (b && !ptr && cudaMalloc(&ptr, b) != cudaSuccess) {
       cudaGetLastError();
       ptr = nullptr;
-      BlockPool::trim_all();
+      give_back_idle();
       IMPS_CUDA(cudaMalloc(&ptr, b));
     }
     bytes = b;
@@ -211,14 +215,7 @@ struct Context {
         throw Error(IMPS_OOM, "workspace limit of " + std::to_string(workspace_limit) + " bytes reached (buffer '" +
                                   name + "' needs " + std::to_string(bytes) + " bytes)");
     }
-    try {
-      b.ensure(bytes);
-    } catch (const Error& e) {
-      if (e.status != IMPS_OOM || optional.empty()) throw;
-      cudaGetLastError();
-      release_optional();
-      b.ensure(bytes);
-    }
+    b.ensure(bytes);
     return b;
   }
   // Whether FP64 sums keep one order (k ascending) whatever the grid.  The split engine
@@ -230,14 +227,20 @@ struct Context {
   // Scratch that only makes a call faster (partial tiles, residue planes): nullptr when it
   // is not to be had -- a workspace cap is set, the call may not allocate, or the device is
   // out of memory -- and the caller then takes its path without it.  Kept between calls;
-  // given back when a cap is set or a required buffer does not fit.
+  // given back when a cap is set or when any other allocation of the context does not fit.
   std::map<std::string, DevBuf> optional;
-  int no_scratch = 0;   // > 0: a call that must not allocate is running
+  int no_scratch = 0;   // > 0: a call that must not allocate is running, or the map is in use
+  struct Count {
+    int& n;
+    explicit Count(int& x) : n(x) { ++n; }
+    ~Count() { --n; }
+  };
   void* optional_buf(const char* name, size_t bytes) {
     if (no_scratch > 0 || workspace_limit > 0) return nullptr;
     DevBuf& b = optional[name];
     if (bytes > b.bytes && capturing()) return nullptr;   // no allocation inside a graph capture
     try {
+      Count growing(no_scratch);   // (give_back_idle leaves the map alone)
       b.ensure(bytes);
     } catch (const Error& e) {
       if (e.status != IMPS_OOM) throw;
@@ -258,6 +261,14 @@ struct Context {
     optional.clear();
   }
   double* pinned(size_t bytes);
+};
+
+// The context whose entry point runs on this thread, while alive: only its own thread may
+// take its scratch from it.
+struct RunningCall {
+  Context* old;
+  explicit RunningCall(Context* ctx);
+  ~RunningCall();
 };
 
 // Every kernel begins with this: the grid before it in the stream has finished and its writes

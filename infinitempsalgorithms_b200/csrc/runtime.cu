@@ -547,6 +547,16 @@ void BlockPool::trim_all() {
   for (BlockPool* p : pools()) p->trim();
 }
 
+static thread_local Context* g_running = nullptr;
+RunningCall::RunningCall(Context* ctx) : old(g_running) { g_running = ctx; }
+RunningCall::~RunningCall() { g_running = old; }
+
+void give_back_idle() {
+  BlockPool::trim_all();
+  Context* c = g_running;
+  if (c && c->no_scratch == 0 && !c->optional.empty() && !c->capturing()) c->release_optional();
+}
+
 double* Context::pinned(size_t bytes) {
   if (bytes > host_pinned_bytes) {
     if (host_pinned) cudaFreeHost(host_pinned);
