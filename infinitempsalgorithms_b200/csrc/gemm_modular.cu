@@ -176,20 +176,11 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
     s = fma(v.x, v.x, fma(v.y, v.y, s));
     m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
   };
-  // elements k, k + step, ... of a line, eight loads in flight (zeros past the end add nothing)
-  auto walk = [&](const double2* x, int64_t stride, int k, int step) {
-    for (; k < k1; k += 8 * step) {
-      double2 v[8];
-#pragma unroll
-      for (int j = 0; j < 8; ++j) v[j] = k + j * step < k1 ? x[stride * (k + j * step)] : make_double2(0.0, 0.0);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) add(v[j]);
-    }
-  };
   if (o.kcontig) {
     // eight lanes a line, 32 lines a block
     const int l = grp * 32 + (threadIdx.x >> 3);
-    if (l < o.lines) walk(o.X + o.ld * l, 1, k0 + (threadIdx.x & 7), 8);
+    if (l < o.lines)
+      for (int k = k0 + (threadIdx.x & 7); k < k1; k += 8) add(o.X[k + o.ld * l]);
 #pragma unroll
     for (int d = 4; d >= 1; d >>= 1) {
       s += __shfl_xor_sync(0xffffffffu, s, d);
@@ -201,7 +192,8 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
     }
   } else {
     const int tl = threadIdx.x & 63, tk = threadIdx.x >> 6, l = grp * 64 + tl;
-    if (l < o.lines) walk(o.X + l, o.ld, k0 + tk, 4);
+    if (l < o.lines)
+      for (int k = k0 + tk; k < k1; k += 4) add(o.X[l + o.ld * k]);
     ss[tk][tl] = s;
     sm[tk][tl] = m;
     __syncthreads();
@@ -219,7 +211,6 @@ __device__ __forceinline__ double pow2(int e) { return __longlong_as_double((lon
 // adds at most sqrt(K / 2), far below the 2^0.6 that 2^116 leaves under P / 2).
 __device__ int line_exponent(const ModOperand& o, int l) {
   double s = 0.0, m = 0.0;
-#pragma unroll 8
   for (int c = 0; c < o.nchunk; ++c) {
     s += o.part[(int64_t)c * o.lines + l];
     m = fmax(m, o.part[(int64_t)(o.nchunk + c) * o.lines + l]);
@@ -297,24 +288,26 @@ __global__ void __launch_bounds__(SPL_NT, 1024 / SPL_NT) k_mod_split(const ModOp
   const int nk = (int)(o.Kp / 64);
   const int k0 = (blk % nk) * 64, l0 = (blk / nk) * SPL_LINES;
   const int tid = threadIdx.x;
-  // the tile's loads are on their way while the first threads find the scales
-  constexpr int NLD = SPL_LINES * 64 / SPL_NT;
-  const int tl = o.kcontig ? tid >> 6 : tid % SPL_LINES, tk = o.kcontig ? tid & 63 : tid / SPL_LINES;
-  const int dl = o.kcontig ? SPL_NT / 64 : 0, dk = o.kcontig ? 0 : SPL_NT / SPL_LINES;
-  const int64_t sl = o.kcontig ? o.ld : 1, sk = o.kcontig ? 1 : o.ld;
-  double2 in[NLD];
-#pragma unroll
-  for (int r = 0; r < NLD; ++r) {
-    const int l = l0 + tl + dl * r, k = k0 + tk + dk * r;
-    in[r] = (l < o.lines && k < o.K) ? o.X[sl * l + sk * k] : make_double2(0.0, 0.0);
-  }
   if (tid < SPL_LINES) {
     const int e = l0 + tid < o.lines ? line_exponent(o, l0 + tid) : 0;
     ex[tid] = e == EXP_NONFINITE ? 0 : e;
     if (k0 == 0 && l0 + tid < o.lines) o.expo[l0 + tid] = e;
   }
+  if (o.kcontig) {
+    const int kx = tid & 63, ly = tid >> 6;
 #pragma unroll
-  for (int r = 0; r < NLD; ++r) tile[tl + dl * r][tk + dk * r] = in[r];
+    for (int r = 0; r < SPL_LINES; r += SPL_NT / 64) {
+      const int l = l0 + r + ly, k = k0 + kx;
+      tile[r + ly][kx] = (l < o.lines && k < o.K) ? o.X[k + o.ld * l] : make_double2(0.0, 0.0);
+    }
+  } else {
+    const int lx = tid % SPL_LINES, ky = tid / SPL_LINES;
+#pragma unroll
+    for (int r = 0; r < 64; r += 8) {
+      const int l = l0 + lx, k = k0 + r + ky;
+      tile[lx][r + ky] = (l < o.lines && k < o.K) ? o.X[l + o.ld * k] : make_double2(0.0, 0.0);
+    }
+  }
   __syncthreads();
   const int ll = tid >> 3, kq = tid & 7;
   if (l0 + ll >= o.lines) return;
@@ -717,16 +710,13 @@ __global__ void __launch_bounds__(256, 3) k_mod_join(const ModJoinArgs g, const 
       wu[i] = __ldcs(reinterpret_cast<const unsigned*>(src + plane * i));
       wv[i] = __ldcs(reinterpret_cast<const unsigned*>(src + plane * (NMOD + i)));
     }
-    const int ea = g.ea[row];
-    int ebs[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) ebs[e] = n0 + c4 + e < g.N ? g.eb[n0 + c4 + e] : 0;
     join_moduli(wu, wv, x1, y1, x2, y2, std::make_integer_sequence<int, NMOD>{});
+    const int ea = g.ea[row];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int col = n0 + c4 + e;
       if (col >= g.N) continue;
-      const int eb = ebs[e];
+      const int eb = g.eb[col];
       double2 v;
       if (ea == EXP_NONFINITE || eb == EXP_NONFINITE) {
         v = make_double2(0.0, 0.0);
