@@ -50,11 +50,15 @@ __device__ __forceinline__ uint32_t cluster_rank() {
 }
 // all threads of every CTA of the cluster; release / acquire order the shared
 // (and global) writes before the barrier with the reads after it
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  cluster_arrive();
+  cluster_wait();
 }
 // store v into the same shared variable of CTA `rank` of the cluster (made visible to
-// that CTA by the next cluster barrier's release / acquire)
+// that CTA by the next cluster barrier's release / acquire).  Defined only once that CTA
+// runs: a cluster barrier has to lie between the kernel's start and the first one.
 __device__ __forceinline__ void st_peer(double* local, uint32_t rank, double v) {
   uint32_t a;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(local)), "r"(rank));
@@ -120,6 +124,9 @@ template <int NB, int RPT, int CL, int NT>
 __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT, 1)
     k_qr_panel(int R, int b, int zabove, dcplx* __restrict__ A, int64_t lda, dcplx* __restrict__ V, int64_t ldv,
                dcplx* __restrict__ tau, dcplx* __restrict__ T, int ldt) {
+  // every CTA of the cluster runs before the first store into a peer's shared memory (a CTA
+  // without rows gets there at once); the wait comes behind the panel's loads
+  if constexpr (CL > 1) cluster_arrive();
   grid_enter();
   constexpr int NV = 2 * NB;             // reduction slots: [0] ||x||^2, [2q - 1, 2q] position q
   constexpr int NW = NT / 32;
@@ -150,6 +157,7 @@ __global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(NT, 1)
   }
   if (rank == 0)
     for (int e = tid; e < NB * (NB + 1); e += NT) Tsh[e / (NB + 1)][e % (NB + 1)] = make_double2(0.0, 0.0);
+  if constexpr (CL > 1) cluster_wait();
 
 #pragma unroll 1
   for (int c = 0; c < b; ++c) {
