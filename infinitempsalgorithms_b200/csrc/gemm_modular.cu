@@ -452,14 +452,27 @@ __device__ __forceinline__ void publish(uint32_t* slot, uint32_t n) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(n) : "memory");
   }
 }
-// The end of both CTAs, by all their threads.  With every stage read nothing is in flight.
+// The end of both CTAs, by all their threads.  Every commit of the leader arrives at the
+// barriers of both, so each CTA stays until its own copies have completed: the `empty` phases
+// of the last stages read, the `tfull` phases of the last tiles (kblocks stages each) and
+// `drain`.  With every stage read nothing is in flight then.
 // After a wait that gave up, the leader completes each outstanding phase of the `full`
 // barriers (an arrival for a stage that only its peer filled, the peer's bytes for one that
 // only it filled) and waits for the copies; the peer stays until then.
-__device__ __forceinline__ void leave_pair(uint64_t* full, uint32_t nst, uint32_t bytes, const uint32_t* done,
-                                           uint32_t rank, uint32_t total) {
+struct PairBars {
+  uint64_t *full, *empty, *tfull, *drain;
+};
+__device__ __forceinline__ void leave_pair(const PairBars& b, uint32_t nst, uint32_t nbuf, uint32_t bytes,
+                                           const uint32_t* done, uint32_t rank, uint32_t total, uint32_t kblocks) {
+  uint64_t* full = b.full;
   __syncthreads();
-  cluster_sync();
+  cluster_sync();   // the leader has committed for the last time and its MMAs have retired
+  if (threadIdx.x == 0) {
+    const uint32_t nread = done[DONE_MMA], tiles = nread / kblocks;
+    for (uint32_t i = nread > nst ? nread - nst : 0; i < nread; ++i) mbar_drain(&b.empty[i % nst], (i / nst) & 1);
+    for (uint32_t i = tiles > nbuf ? tiles - nbuf : 0; i < tiles; ++i) mbar_drain(&b.tfull[i % nbuf], (i / nbuf) & 1);
+    mbar_drain(b.drain, 0);
+  }
   if (done[DONE_MMA] == total) return;
   const uint32_t n0 = done[DONE_FILL0], n1 = done[DONE_FILL1];
   if (rank == 0 && threadIdx.x == 0) {
@@ -473,6 +486,7 @@ __device__ __forceinline__ void leave_pair(uint64_t* full, uint32_t nst, uint32_
       mbar_drain(bar, (i / nst) & 1);
     }
   }
+  __syncwarp();
   cluster_sync();
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
@@ -631,7 +645,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GTHREADS, 1)
   }
   // no CTA leaves, and no TMEM is released, while the pair's MMAs or copies are in flight
   const uint32_t mine = pair < ntiles ? (uint32_t)((ntiles - pair + npairs - 1) / npairs) : 0u;
-  leave_pair(full, GSTAGES, (uint32_t)GSTAGE_BYTES, done, rank, mine * (uint32_t)g.kblocks);
+  leave_pair(PairBars{full, empty, tfull, drain}, GSTAGES, GBUF, (uint32_t)GSTAGE_BYTES, done, rank,
+             mine * (uint32_t)g.kblocks, (uint32_t)g.kblocks);
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem));
