@@ -225,9 +225,10 @@ struct Context {
   // trajectory keeps the plain order, so that it does not depend on how a product was cut up.
   bool ordered_sums() const { return precision == PREC_SPLIT_I8; }
   // Scratch that only makes a call faster (partial tiles, residue planes): nullptr when it
-  // is not to be had -- a workspace cap is set, the call may not allocate, or the device is
-  // out of memory -- and the caller then takes its path without it.  Kept between calls;
-  // given back when a cap is set or when any other allocation of the context does not fit.
+  // is not to be had -- a workspace cap is set, the call may not allocate, the stream is being
+  // captured, or the device is out of memory -- and the caller then takes its path without
+  // it.  Kept between calls; given back when a cap is set or when any other allocation of the
+  // context does not fit, and replaced when a call needs more, so no graph may hold it.
   std::map<std::string, DevBuf> optional;
   int no_scratch = 0;   // > 0: a call that must not allocate is running, or the map is in use
   struct Count {
@@ -236,9 +237,8 @@ struct Context {
     ~Count() { --n; }
   };
   void* optional_buf(const char* name, size_t bytes) {
-    if (no_scratch > 0 || workspace_limit > 0) return nullptr;
+    if (no_scratch > 0 || workspace_limit > 0 || capturing()) return nullptr;
     DevBuf& b = optional[name];
-    if (bytes > b.bytes && capturing()) return nullptr;   // no allocation inside a graph capture
     try {
       Count growing(no_scratch);   // (give_back_idle leaves the map alone)
       b.ensure(bytes);
