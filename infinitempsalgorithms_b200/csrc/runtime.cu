@@ -7,6 +7,7 @@
 #include <vector>
 #include <cmath>
 #include <cstring>
+#include <atomic>
 #include <system_error>
 #include <thread>
 
@@ -620,17 +621,19 @@ void synchronize(Context* ctx) {
 }
 
 namespace {
-// Large arrays of the caller's pageable memory go through page-locked chunks, moved by a few
-// threads: one thread's copies (and, into a fresh array, its page faults) take longer than
-// the transfer.  Each thread owns a contiguous part and two chunks and overlaps its memory
-// copies with its transfers on the context's stream.  One staging area per process; a second
-// context that finds it taken, small arrays and page-locked ones use the plain copy.
+// Large arrays of the caller's pageable memory go through page-locked chunks, filled or emptied
+// by a few threads: one thread's copies (and, into a fresh array, its page faults) take longer
+// than the transfer.  The threads only move memory: the calling thread issues every transfer and
+// event on the context's stream, whose handle may name another stream in another thread
+// (cudaStreamPerThread).  One staging area per process; a second context that finds it taken,
+// small arrays and page-locked ones use the plain copy.
 constexpr int kStageThreads = 4;
+constexpr int kStageSlots = 2 * kStageThreads;
 constexpr size_t kStageChunk = (size_t)1 << 20, kStageMin = (size_t)4 << 20;
 
 struct Staging {
   std::mutex mu;
-  char* mem = nullptr;   // kStageThreads x 2 chunks
+  char* mem = nullptr;   // kStageSlots chunks
 };
 Staging& staging() {
   static auto* s = new Staging;   // as long as the process, like the driver's own
@@ -646,41 +649,69 @@ bool page_locked(const void* p) {
   return a.type != cudaMemoryTypeUnregistered;
 }
 
-cudaError_t stage_part(const Context* ctx, char* dev, char* host, size_t bytes, bool to_device, char* buf) {
-  cudaError_t e = cudaSetDevice(ctx->device);
-  cudaEvent_t ev[2] = {nullptr, nullptr};
-  for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming);
-  const size_t n = (bytes + kStageChunk - 1) / kStageChunk;
-  auto len = [&](size_t i) { return std::min(kStageChunk, bytes - i * kStageChunk); };
-  for (size_t i = 0; i < n + 1 && e == cudaSuccess; ++i) {
-    char* c = buf + (i & 1) * kStageChunk;
-    if (to_device) {
-      if (i == n) break;
-      if (i >= 2) e = cudaEventSynchronize(ev[i & 1]);
-      if (e != cudaSuccess) break;
-      std::memcpy(c, host + i * kStageChunk, len(i));
-      e = cudaMemcpyAsync(dev + i * kStageChunk, c, len(i), cudaMemcpyHostToDevice, ctx->stream);
-      if (e == cudaSuccess) e = cudaEventRecord(ev[i & 1], ctx->stream);
-    } else {
-      // chunk i is on its way while chunk i - 1 is copied out
-      if (i < n) {
-        e = cudaMemcpyAsync(c, dev + i * kStageChunk, len(i), cudaMemcpyDeviceToHost, ctx->stream);
-        if (e == cudaSuccess) e = cudaEventRecord(ev[i & 1], ctx->stream);
-      }
-      if (i > 0 && e == cudaSuccess) {
-        e = cudaEventSynchronize(ev[(i - 1) & 1]);
-        if (e == cudaSuccess) std::memcpy(host + (i - 1) * kStageChunk, buf + ((i - 1) & 1) * kStageChunk, len(i - 1));
-      }
+// One array's way through the slots: chunk i uses slot i % kStageSlots and is moved in host
+// memory by thread i % kStageThreads, in ascending order each.
+struct StagedCopy {
+  char *dev, *host, *slots;
+  size_t bytes, n;
+  bool to_device;
+  int device;
+  cudaStream_t stream;
+  cudaEvent_t ev[kStageSlots] = {};
+  std::atomic<size_t> issued{0};                 // chunks whose transfer and event are queued
+  std::atomic<size_t> moved[kStageSlots] = {};   // 1 + the last chunk of the slot moved in host memory
+  std::atomic<int> failed{0};
+
+  char* slot(size_t i) const { return slots + i % kStageSlots * kStageChunk; }
+  size_t len(size_t i) const { return std::min(kStageChunk, bytes - i * kStageChunk); }
+  cudaError_t fail(cudaError_t e) {
+    if (e != cudaSuccess) {
+      int none = 0;
+      failed.compare_exchange_strong(none, (int)e);
     }
+    return e;
   }
-  for (auto v : ev)
-    if (v) {
-      const cudaError_t w = cudaEventSynchronize(v);   // this part's chunks are free again
-      if (e == cudaSuccess) e = w;
-      cudaEventDestroy(v);
+  template <class F>
+  bool wait(F&& ready) const {   // false: another thread failed
+    while (!ready()) {
+      if (failed.load()) return false;
+      std::this_thread::yield();
     }
-  return e;
-}
+    return failed.load() == 0;
+  }
+  // the host memory's side
+  void move(size_t i) {
+    const size_t s = i % kStageSlots;
+    if (to_device) {
+      if (i >= kStageSlots) {   // the slot's last transfer has left it
+        if (!wait([&] { return issued.load() > i - kStageSlots; })) return;
+        if (fail(cudaEventSynchronize(ev[s])) != cudaSuccess) return;
+      }
+      std::memcpy(slot(i), host + i * kStageChunk, len(i));
+    } else {
+      if (!wait([&] { return issued.load() > i; })) return;
+      if (fail(cudaEventSynchronize(ev[s])) != cudaSuccess) return;
+      std::memcpy(host + i * kStageChunk, slot(i), len(i));
+    }
+    moved[s].store(i + 1);
+  }
+  void work(size_t t) {
+    if (fail(cudaSetDevice(device)) != cudaSuccess) return;
+    for (size_t i = t; i < n && !failed.load(); i += kStageThreads) move(i);
+  }
+  // the stream's side, by the calling thread
+  void issue(size_t i) {
+    const size_t s = i % kStageSlots;
+    const size_t need = to_device ? i + 1 : (i >= kStageSlots ? i - kStageSlots + 1 : 0);
+    if (!wait([&] { return moved[s].load() >= need; })) return;
+    char* d = dev + i * kStageChunk;
+    if (fail(to_device ? cudaMemcpyAsync(d, slot(i), len(i), cudaMemcpyHostToDevice, stream)
+                       : cudaMemcpyAsync(slot(i), d, len(i), cudaMemcpyDeviceToHost, stream)) != cudaSuccess)
+      return;
+    if (fail(cudaEventRecord(ev[s], stream)) != cudaSuccess) return;
+    issued.store(i + 1);
+  }
+};
 
 // false: not staged, nothing done
 bool staged_copy(Context* ctx, void* dev, void* host, size_t bytes, bool to_device) {
@@ -688,34 +719,44 @@ bool staged_copy(Context* ctx, void* dev, void* host, size_t bytes, bool to_devi
   Staging& s = staging();
   std::unique_lock<std::mutex> lock(s.mu, std::try_to_lock);
   if (!lock.owns_lock()) return false;
-  if (!s.mem &&
-      cudaHostAlloc((void**)&s.mem, 2 * kStageThreads * kStageChunk, cudaHostAllocPortable) != cudaSuccess) {
+  if (!s.mem && cudaHostAlloc((void**)&s.mem, kStageSlots * kStageChunk, cudaHostAllocPortable) != cudaSuccess) {
     cudaGetLastError();
     s.mem = nullptr;
     return false;
   }
-  const size_t part = ((bytes + kStageThreads - 1) / kStageThreads + 4095) / 4096 * 4096;
-  cudaError_t err[kStageThreads] = {};
-  auto work = [&](int t) {
-    const size_t o = std::min(bytes, part * t), b = std::min(part, bytes - o);
-    if (b)
-      err[t] = stage_part(ctx, static_cast<char*>(dev) + o, static_cast<char*>(host) + o, b, to_device,
-                          s.mem + 2 * kStageChunk * t);
-  };
+  StagedCopy c;
+  c.dev = static_cast<char*>(dev);
+  c.host = static_cast<char*>(host);
+  c.slots = s.mem;
+  c.bytes = bytes;
+  c.n = (bytes + kStageChunk - 1) / kStageChunk;
+  c.to_device = to_device;
+  c.device = ctx->device;
+  c.stream = ctx->stream;
+  for (auto& e : c.ev) c.fail(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   std::thread th[kStageThreads];
-  bool here[kStageThreads] = {true};
-  for (int t = 1; t < kStageThreads; ++t) {
+  for (int t = 0; t < kStageThreads; ++t) {
     try {
-      th[t] = std::thread(work, t);
+      th[t] = std::thread(&StagedCopy::work, &c, (size_t)t);
     } catch (const std::system_error&) {
-      here[t] = true;   // no thread to be had
+      break;   // no thread to be had
     }
   }
-  for (int t = 0; t < kStageThreads; ++t)
-    if (here[t]) work(t);
+  // the chunks of threads that did not start are the calling thread's
+  for (size_t i = 0; i < c.n && !c.failed.load(); ++i) {
+    const bool mine = !th[i % kStageThreads].joinable();
+    if (mine && to_device) c.move(i);
+    c.issue(i);
+    if (mine && !to_device) c.move(i);
+  }
   for (auto& t : th)
     if (t.joinable()) t.join();
-  for (cudaError_t e : err) IMPS_CUDA(e);
+  // every transfer has left the slots before the next array uses them
+  const cudaError_t w = cudaStreamSynchronize(ctx->stream);
+  for (auto e : c.ev)
+    if (e) cudaEventDestroy(e);
+  IMPS_CUDA((cudaError_t)c.failed.load());
+  IMPS_CUDA(w);
   return true;
 }
 }  // namespace
