@@ -116,8 +116,8 @@ int imps_ctx_synchronize(imps_ctx* ctx);
  * (0 restores the default 2e9, about 1 s).  A wait that runs out sets a device
  * error flag and the kernel returns early; the flag is read at the context's next
  * host synchronisation (at the latest when the entry point returns) and the call
- * returns IMPS_TIMEOUT; the context stays usable.  An asynchronous call's FP64 products
- * (imps_ac_apply_dev, imps_c_apply_dev) report at the next call that synchronises,
+ * returns IMPS_TIMEOUT; the context stays usable.  The FP64 products of the asynchronous
+ * calls (imps_ac_apply_dev, imps_c_apply_dev) report at the next other call,
  * imps_ctx_synchronize among them.  No reference counterpart (the
  * reference has no device code): the bounded-wait failure detection of this
  * library. */

@@ -25,14 +25,18 @@ struct imps_ctx {
 namespace {
 thread_local std::string g_last_error;
 
-template <class F>
+// An entry point that returns with its work queued checks the split products' flag alone;
+// every other one has read the flag of all its products when it returns.
+enum class Returns { kDone, kQueued };
+
+template <Returns R = Returns::kDone, class F>
 int guard(imps::Context* ctx, F&& f) {
   try {
     imps::RunningCall running(ctx);
     if (ctx) cudaSetDevice(ctx->device);
     int r = f();
     // a bounded wait that ran out inside this call surfaces here at the latest
-    if (ctx) imps::check_device_errors(ctx);
+    if (ctx) imps::check_device_errors(ctx, R == Returns::kDone);
     return r;
   } catch (const imps::Error& e) {
     g_last_error = e.what();
@@ -576,7 +580,7 @@ int imps_envs_set(imps_envs* E, int side, int site, const double* host) {
 // ------------------------------------------------------------------ Heff
 int imps_ac_apply_dev(imps_envs* E, const imps_mpo* mpo, int site, const void* x, void* y) {
   if (!E || !mpo || !x || !y) return IMPS_INVALID_ARG;
-  return guard(E->ctx, [&] {
+  return guard<Returns::kQueued>(E->ctx, [&] {
     check_site(E, site);
     imps::ac_apply(E->ctx, E, mpo, site, static_cast<const imps::dcplx*>(x), static_cast<imps::dcplx*>(y));
     return IMPS_OK;
@@ -601,7 +605,7 @@ int imps_ac_apply(imps_envs* E, const imps_mpo* mpo, int site, const double* x, 
 int imps_ac_apply_noalloc(imps_ctx* h, int Dl, int d, int Dr, int m, int n, const double* W_host, const void* GL,
                           const void* GR, const void* x, void* y) {
   if (!h || !W_host || !GL || !GR || !x || !y) return IMPS_INVALID_ARG;
-  return guard(&h->c, [&] {
+  return guard<Returns::kQueued>(&h->c, [&] {
     imps::ac_apply_noalloc(&h->c, Dl, d, Dr, m, n, hc(W_host), static_cast<const imps::dcplx*>(GL),
                            static_cast<const imps::dcplx*>(GR), static_cast<const imps::dcplx*>(x),
                            static_cast<imps::dcplx*>(y));
@@ -611,7 +615,7 @@ int imps_ac_apply_noalloc(imps_ctx* h, int Dl, int d, int Dr, int m, int n, cons
 
 int imps_c_apply_dev(imps_envs* E, int site, const void* x, void* y) {
   if (!E || !x || !y) return IMPS_INVALID_ARG;
-  return guard(E->ctx, [&] {
+  return guard<Returns::kQueued>(E->ctx, [&] {
     check_site(E, site);
     imps::c_apply(E->ctx, E, site, static_cast<const imps::dcplx*>(x), static_cast<imps::dcplx*>(y));
     return IMPS_OK;

@@ -167,7 +167,8 @@ struct Context {
   int* err_host = nullptr;
   bool err_armed = false;
   // armed by the FP64 products: asynchronous entry points stay asynchronous, and the flag is
-  // read at the context's next synchronisation, whichever call makes it
+  // read at the context's next synchronisation, whichever call makes it; every other entry
+  // point reads it before it returns
   bool err_later = false;
   void* qr_count_ptr = nullptr;       // completion counter of the QR small products, zeroed at this address
   long long wait_cycles = 2000000000LL;  // bound of each pipeline wait (~1 s at 1.9 GHz)
@@ -557,8 +558,9 @@ void lq_factor(Context* ctx, int m, int n, const dcplx* M, int64_t ldm, dcplx* L
 void lq_form_q(Context* ctx, int m, int n, dcplx* Q, const char* slot);
 
 // Reads the device error flag if a kernel that may set it ran since the last check
-// (synchronises the stream); a set flag is cleared and raised as IMPS_TIMEOUT.
-void check_device_errors(Context* ctx);
+// (synchronises the stream); a set flag is cleared and raised as IMPS_TIMEOUT.  all: also for
+// the FP64 products, which an asynchronous entry point leaves to a later call.
+void check_device_errors(Context* ctx, bool all);
 // Waits for the context's stream and reads the flag if any kernel may have set it.
 void synchronize(Context* ctx);
 

@@ -611,8 +611,8 @@ static void err_after_sync(Context* ctx) {
     throw Error(IMPS_TIMEOUT, "a bounded device wait of a GEMM pipeline ran out");
   }
 }
-void check_device_errors(Context* ctx) {
-  if (ctx->err_armed) synchronize(ctx);
+void check_device_errors(Context* ctx, bool all) {
+  if (ctx->err_armed || (all && ctx->err_later)) synchronize(ctx);
 }
 void synchronize(Context* ctx) {
   err_copy(ctx);
