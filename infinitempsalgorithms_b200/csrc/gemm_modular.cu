@@ -159,8 +159,19 @@ __device__ __forceinline__ double2 load_elem(const ModOperand& o, int l, int k) 
   return v;
 }
 
+// 2^e in the double range, and x 2^e for any |e| <= 1100
+__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+__device__ __forceinline__ double scale2(double x, int e) { return x * pow2(e / 2) * pow2(e - e / 2); }
+
+// Whether a sum of squares has left (or may have left) the double range; m is the largest element
+__device__ __forceinline__ bool squares_lost(double s, double m) {
+  return m > 0.0 && !isinf(m) && !isnan(s) && !(s > 1e-280 && s < 1e280);
+}
+
 // Partial sums of squares and maxima of every line over the K chunks (a fixed order, so
-// that the scales do not depend on timing).  Blocks [0, a.nblocks_norm) serve a.
+// that the scales do not depend on timing).  Blocks [0, a.nblocks_norm) serve a.  A chunk
+// whose squares leave the double range is summed again in units of 2^e > its largest element
+// (frexp), and the sum stored with a minus sign.
 __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const ModOperand b) {
   grid_enter();
   __shared__ double ss[4][64], sm[4][64];
@@ -176,15 +187,30 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
     s = fma(v.x, v.x, fma(v.y, v.y, s));
     m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
   };
+  auto add_scaled = [&](double2 v, int e) {
+    v.x = scale2(v.x, -e);
+    v.y = scale2(v.y, -e);
+    s = fma(v.x, v.x, fma(v.y, v.y, s));
+  };
   if (o.kcontig) {
     // eight lanes a line, 32 lines a block
     const int l = grp * 32 + (threadIdx.x >> 3);
     if (l < o.lines)
       for (int k = k0 + (threadIdx.x & 7); k < k1; k += 8) add(o.X[k + o.ld * l]);
+    const unsigned mine = 0xffu << (threadIdx.x & 24);
 #pragma unroll
     for (int d = 4; d >= 1; d >>= 1) {
       s += __shfl_xor_sync(0xffffffffu, s, d);
       m = fmax(m, __shfl_xor_sync(0xffffffffu, m, d));
+    }
+    if (squares_lost(s, m)) {   // the same for the line's eight lanes
+      int e;
+      frexp(m, &e);
+      s = 0.0;
+      for (int k = k0 + (threadIdx.x & 7); k < k1; k += 8) add_scaled(o.X[k + o.ld * l], e);
+#pragma unroll
+      for (int d = 4; d >= 1; d >>= 1) s += __shfl_xor_sync(mine, s, d);
+      s = -s;
     }
     if (l < o.lines && (threadIdx.x & 7) == 0) {
       psum[l] = s;
@@ -197,37 +223,57 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
     ss[tk][tl] = s;
     sm[tk][tl] = m;
     __syncthreads();
+    double t = (ss[0][tl] + ss[1][tl]) + (ss[2][tl] + ss[3][tl]);
+    m = fmax(fmax(sm[0][tl], sm[1][tl]), fmax(sm[2][tl], sm[3][tl]));
+    const bool lost = squares_lost(t, m);
+    if (__syncthreads_or(lost)) {
+      if (lost) {
+        int e;
+        frexp(m, &e);
+        s = 0.0;
+        for (int k = k0 + tk; k < k1; k += 4) add_scaled(o.X[l + o.ld * k], e);
+        ss[tk][tl] = s;
+      }
+      __syncthreads();
+      if (lost) t = -((ss[0][tl] + ss[1][tl]) + (ss[2][tl] + ss[3][tl]));
+    }
     if (tk == 0 && l < o.lines) {
-      psum[l] = (ss[0][tl] + ss[1][tl]) + (ss[2][tl] + ss[3][tl]);
-      pmax[l] = fmax(fmax(sm[0][tl], sm[1][tl]), fmax(sm[2][tl], sm[3][tl]));
+      psum[l] = t;
+      pmax[l] = m;
     }
   }
 }
 
-// 2^e in the double range
-__device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
-
-// The scale exponent of a line: x 2^e rounds to integers of 2-norm <= 2^58 (the rounding
-// adds at most sqrt(K / 2), far below the 2^0.6 that 2^116 leaves under P / 2).
+// The scale exponent of a line: x 2^e rounds to integers of 2-norm in [2^57, 2^58] (the
+// rounding adds at most sqrt(K / 2), far below the 2^0.6 that 2^116 leaves under P / 2).
 __device__ int line_exponent(const ModOperand& o, int l) {
   double s = 0.0, m = 0.0;
+  bool lost = false;
   for (int c = 0; c < o.nchunk; ++c) {
-    s += o.part[(int64_t)c * o.lines + l];
+    const double t = o.part[(int64_t)c * o.lines + l];
+    lost = lost || t < 0.0;
+    s += t;
     m = fmax(m, o.part[(int64_t)(o.nchunk + c) * o.lines + l]);
   }
   // a NaN does not pass fmax but does reach the sum of squares
   if (isnan(s) || isinf(m)) return EXP_NONFINITE;
   if (m == 0.0) return 0;
-  int e;
-  if (s > 1e-280 && s < 1e280) {
-    frexp(sqrt(s) * (1.0 + 1e-12), &e);
-  } else {  // squares that left the range: bound the norm by the largest element
-    int e2;
-    frexp(m, &e);
-    frexp(sqrt(2.0 * o.K), &e2);
-    e += e2;
+  int e, unit = 0;
+  if (lost) {   // all chunks in units of 2^unit > m
+    frexp(m, &unit);
+    s = 0.0;
+    for (int c = 0; c < o.nchunk; ++c) {
+      const double t = o.part[(int64_t)c * o.lines + l], mc = o.part[(int64_t)(o.nchunk + c) * o.lines + l];
+      int ec = 0;
+      if (t < 0.0) frexp(mc, &ec);
+      // (a plain sum beside one that left the range is no larger than 2^930; what underflows
+      // here is nothing to the result)
+      const double u = scale2(fabs(t), max(ec - unit, -1100));
+      s += scale2(u, max(ec - unit, -1100));
+    }
   }
-  return BETA_BITS - e;
+  frexp(sqrt(s) * (1.0 + 1e-12), &e);
+  return BETA_BITS - (e + unit);
 }
 
 __device__ __forceinline__ int dp4a_us(unsigned a, int b, int c) {
