@@ -17,7 +17,7 @@
 // 2-norm per element, and those of the final conversion (2^-52 relative).  An element of
 // C is off by about 3e-18 ||a_i|| ||b_j||; an FP64 sum over K random terms is off by
 // 0.3 sqrt(K) 2^-53 of its result, i.e. by more for every K here.  Rows or columns with a
-// NaN or an Inf are recognised and their elements computed by a plain FP64 loop.
+// NaN or an Inf are recognised and their elements computed as plain FP64 sums.
 //
 // The four kernels: partial row norms, residue planes, the int8 GEMMs, the reconstruction.
 // Measured (B200): 6144 x 4096 x 1024 1.15 ms = 35 + 139 + 650 + 326 us (6.50 ms on the FP64
@@ -735,6 +735,77 @@ __device__ __forceinline__ void join_moduli(const unsigned (&wu)[NMOD], const un
   (join_modulus<I>(wu[I], wv[I], x1, y1, x2, y2), ...);
 }
 
+// Elements of a 64 x 16 tile that residues do not give, as plain FP64 sums: `bad` marks those
+// of this thread's four columns c4 .. c4 + 3 of row r.  All threads of the block call it.  A few
+// elements take a warp each; from 64 on the block sums the whole tile, K stages of 16 through
+// shared memory (an all-NaN 6144 x 4096 x 1024 product in the time of the FP64 pipe, where a
+// serial sum per element took thousands of times as long).  An element's sum is the same
+// whatever the timing.
+constexpr int RD_K = 16, RD_FEW = 64;
+__device__ __noinline__ void fp64_elements(const ModOperand& a, const ModOperand& b, int M, int N, int K, int m0, int n0,
+                                           unsigned bad, double2 (*tile)[65]) {
+  __shared__ double2 as[RD_K][65], bs[RD_K][17];
+  __shared__ unsigned short list[RD_FEW];
+  __shared__ int count;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int r = tid >> 2, c4 = (tid & 3) * 4;
+  auto mac = [](double2& s, double2 x, double2 y) {
+    s.x = fma(-x.y, y.y, fma(x.x, y.x, s.x));
+    s.y = fma(x.y, y.x, fma(x.x, y.y, s.y));
+  };
+  if (tid == 0) count = 0;
+  __syncthreads();
+  if (bad) {
+    int at = atomicAdd(&count, __popc(bad));
+    for (int e = 0; e < 4; ++e)
+      if (bad >> e & 1) {
+        if (at < RD_FEW) list[at] = (unsigned short)(r << 4 | (c4 + e));
+        ++at;
+      }
+  }
+  __syncthreads();
+  const int n = count;
+  if (n <= RD_FEW) {
+    for (int i = tid >> 5; i < n; i += 8) {
+      const int er = list[i] >> 4, ec = list[i] & 15;
+      double2 s = make_double2(0.0, 0.0);
+#pragma unroll 4
+      for (int k = lane; k < K; k += 32) mac(s, load_elem(a, m0 + er, k), load_elem(b, n0 + ec, k));
+#pragma unroll
+      for (int d = 16; d >= 1; d >>= 1) {
+        s.x += __shfl_xor_sync(0xffffffffu, s.x, d);
+        s.y += __shfl_xor_sync(0xffffffffu, s.y, d);
+      }
+      if (lane == 0) tile[ec][er] = s;
+    }
+  } else {
+    double2 s[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) s[e] = make_double2(0.0, 0.0);
+    for (int k0 = 0; k0 < K; k0 += RD_K) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int k = a.kcontig ? tid & 15 : (tid >> 6) + 4 * q, l = a.kcontig ? (tid >> 4) + 16 * q : tid & 63;
+        as[k][l] = k0 + k < K && m0 + l < M ? load_elem(a, m0 + l, k0 + k) : make_double2(0.0, 0.0);
+      }
+      const int k = b.kcontig ? tid & 15 : tid >> 4, l = b.kcontig ? tid >> 4 : tid & 15;
+      bs[k][l] = k0 + k < K && n0 + l < N ? load_elem(b, n0 + l, k0 + k) : make_double2(0.0, 0.0);
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < RD_K; ++q) {
+        const double2 x = as[q][r];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) mac(s[e], x, bs[q][c4 + e]);
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (bad >> e & 1) tile[c4 + e][r] = s[e];
+  }
+  __syncthreads();
+}
+
 // A block joins a 64 x 16 tile of C: a thread reads 4 columns of a row from the 32 planes
 // and sums the CRT fractions of its 4 elements, modulo 1 in 32-bit integers for their
 // leading bits, in FP64 below; the tile goes through shared memory so that C is written
@@ -743,13 +814,15 @@ __device__ __forceinline__ void join_moduli(const unsigned (&wu)[NMOD], const un
 // element: 32 integer and 32 double multiply-adds, 32 conversions by exponent trick and
 // 48 bytes of memory traffic.
 template <bool BETA>
-__global__ void __launch_bounds__(256, 3) k_mod_join(const ModJoinArgs g, const ModOperand a, const ModOperand b) {
+__global__ void __launch_bounds__(256, 3)
+    k_mod_join(const ModJoinArgs g, const __grid_constant__ ModOperand a, const __grid_constant__ ModOperand b) {
   grid_enter();
   __shared__ double2 tile[16][65];
   const int tid = threadIdx.x;
   const int r = tid >> 2, c4 = (tid & 3) * 4;
   const int m0 = blockIdx.x * 64, n0 = blockIdx.y * 16;
   const int row = m0 + r;
+  unsigned bad = 0;   // columns whose sum an infinity or a NaN takes part in
   if (row < g.M) {
     const uint8_t* src = g.res + (int64_t)n0 * g.M + (int64_t)row * 16 + c4;
     const int64_t plane = (int64_t)g.M * g.ldo;
@@ -778,24 +851,17 @@ __global__ void __launch_bounds__(256, 3) k_mod_join(const ModJoinArgs g, const 
       const int col = n0 + c4 + e;
       if (col >= g.N) continue;
       const int eb = g.eb[col];
-      double2 v;
       if (ea == EXP_NONFINITE || eb == EXP_NONFINITE) {
-        v = make_double2(0.0, 0.0);
-        for (int k = 0; k < g.K; ++k) {
-          const double2 x = load_elem(a, row, k), y = load_elem(b, col, k);
-          v.x = fma(-x.y, y.y, fma(x.x, y.x, v.x));
-          v.y = fma(x.y, y.x, fma(x.x, y.y, v.y));
-        }
-      } else {
-        const int t = max(-(ea + eb), -2000), th = t / 2;
-        const double s1 = pow2(th), s2 = pow2(t - th);
-        v.x = fma((double)(int)x1[e], 0x1p-32, x2[e]) * P * s1 * s2;
-        v.y = fma((double)(int)y1[e], 0x1p-32, y2[e]) * P * s1 * s2;
+        bad |= 1u << e;
+        continue;
       }
-      tile[c4 + e][r] = v;
+      const int t = max(-(ea + eb), -2000), th = t / 2;
+      const double s1 = pow2(th), s2 = pow2(t - th);
+      tile[c4 + e][r] = make_double2(fma((double)(int)x1[e], 0x1p-32, x2[e]) * P * s1 * s2,
+                                     fma((double)(int)y1[e], 0x1p-32, y2[e]) * P * s1 * s2);
     }
   }
-  __syncthreads();
+  if (__syncthreads_or(bad)) fp64_elements(a, b, g.M, g.N, g.K, m0, n0, bad, tile);
   const int tr = tid & 63;
   if (m0 + tr >= g.M) return;
 #pragma unroll
