@@ -42,10 +42,15 @@ enum {
 
 /* Precision modes of the Heff / transfer contractions. */
 enum {
-  IMPS_PREC_FP64 = 0,       /* plain method: FP64 results; large products through
-                               residue arithmetic, where an element of a product
-                               over K is off by at most 2^-57 sqrt(2 K) of its row's
-                               and column's 2-norms, and its own rounding           */
+  IMPS_PREC_FP64 = 0,       /* plain method: every element of a product is as
+                               accurate as an FP64 sum of its n nonzero terms, i.e.
+                               off by at most (n + 1) 2^-53 sum_k |a_ik| |b_kj| and
+                               its own rounding.  Large products go through residue
+                               arithmetic where that holds of it (checked for every
+                               element), and through FP64 sums otherwise.  Which
+                               engine forms a product, and so its last bits, depends
+                               on its sizes and on whether scratch is to be had
+                               (none under a workspace cap or a graph capture)     */
   IMPS_PREC_SPLIT_I8 = 1    /* int8 split products on tcgen05, exact int32 sums    */
 };
 

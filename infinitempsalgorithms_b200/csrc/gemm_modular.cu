@@ -13,17 +13,28 @@
 //  3. The 32 residues of an output give Re c' / P and Im c' / P as fractions modulo 1
 //     (Chinese remainder theorem), then the product with P and the power-of-two scales.
 //
-// Accuracy: the only errors are the roundings of step 1, below 2^-58 of the row's (column's)
-// 2-norm per element, and those of the final conversion (2^-52 relative).  An element of
-// C is off by about 3e-18 ||a_i|| ||b_j||; an FP64 sum over K random terms is off by
-// 0.3 sqrt(K) 2^-53 of its result, i.e. by more for every K here.  Rows or columns with a
-// NaN or an Inf are recognised and their elements computed as plain FP64 sums.
+// Accuracy: the roundings of step 1 are below 2^-58 of the row's (column's) 2-norm per
+// component, so an element of C is off by about 0.58 2^-57 ||a_i|| ||b_j||, and by its own
+// rounding.  An FP64 sum is off by up to (n + 1) 2^-53 S for its n nonzero terms, S =
+// sum_k |a_ik| |b_kj|, which is less where the large elements of one line meet the small
+// ones of the other.  So S is bounded from below for every element by one more int8 product,
+// of the magnitudes (plane NPL - 1 below), and an element of which it does not follow that
+// the FP64 bound holds is summed in FP64 in the reconstruction:
+//   by Cauchy-Schwarz over the n terms, with lines of norm >= 2^57 and elements off by
+//   2^-1/2, the error is at most sqrt(n / 2) 2^-56 ||a_i|| ||b_j||; it meets the FP64 bound
+//   when S >= ||a_i|| ||b_j|| 2^-3.5 / sqrt(n).  n is at least nnz(a_i) + nnz(b_j) - K.
+// Unstructured lines have S = 0.8 ||a_i|| ||b_j||, a flat line times one that a single element
+// dominates still ||a_i|| ||b_j|| / sqrt(K).  A line with one nonzero element (the identity
+// level of an environment) gives plain FP64 products, as exact as on the FP64 tensor cores.
+// Rows or columns with a NaN or an Inf are recognised and their elements computed as plain
+// FP64 sums.
 //
-// The four kernels: partial row norms, residue planes, the int8 GEMMs, the reconstruction.
-// Measured (B200): 6144 x 4096 x 1024 1.15 ms = 35 + 139 + 650 + 326 us (6.50 ms on the FP64
-// tensor cores), 4096 x 1024 x 6144 1.08 ms = 90 + 399 + 522 + 64 us (6.57 ms), i.e. 179 and
-// 191 TFLOP/s of FP64 products; error against 80-bit sums 1e-16 .. 3e-16 of the result's norm
-// for K = 256 .. 8192 (FP64 tensor cores 8e-16 .. 6e-15).
+// The four kernels: partial row norms, residue and magnitude planes, the int8 GEMMs, the
+// reconstruction.  Measured (B200): 6144 x 4096 x 1024 1.14 ms = 30 + 154 + 644 + 313 us
+// (6.50 ms on the FP64 tensor cores), 4096 x 1024 x 6144 1.10 ms = 78 + 435 + 534 + 55 us
+// (6.57 ms); the magnitudes and the checks cost 5 % of that.  With operands graded so that
+// every element is summed in FP64, 6144 x 4096 x 1024 takes 12.4 ms; with an identity and
+// noise of 1e-17 as one operand 2.9 ms.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -39,7 +50,8 @@ namespace imps {
 namespace {
 
 constexpr int NMOD = 16;
-constexpr int NPL = 2 * NMOD;    // residue planes: u of every modulus, then v
+constexpr int NRES = 2 * NMOD;   // residue planes: u of every modulus, then v
+constexpr int NPL = NRES + 1;    // and the magnitudes
 constexpr int BETA_BITS = 58;    // the integer operands' lines have 2-norm <= 2^58
 constexpr int EXP_NONFINITE = 1 << 20;
 
@@ -149,7 +161,8 @@ struct ModOperand {
   int64_t Kp;
   double* part;       // per K chunk and line: sum of squares, then max |re|, |im|
   int nchunk, kchunk;
-  int* expo;          // per line: the scale's exponent
+  int* count;         // per K chunk and line: nonzero elements, then the largest k of one
+  int4* info;         // per line: the scale's exponent, nonzero elements, the last one's k
   int nblocks_norm, nblocks_split;
 };
 
@@ -175,6 +188,7 @@ __device__ __forceinline__ bool squares_lost(double s, double m) {
 __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const ModOperand b) {
   grid_enter();
   __shared__ double ss[4][64], sm[4][64];
+  __shared__ int sn[4][64], sk[4][64];
   const bool first = (int)blockIdx.x < a.nblocks_norm;
   const ModOperand& o = first ? a : b;
   const int blk = first ? blockIdx.x : blockIdx.x - a.nblocks_norm;
@@ -182,10 +196,18 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
   const int k0 = chunk * o.kchunk, k1 = min(o.K, k0 + o.kchunk);
   double* psum = o.part + (int64_t)chunk * o.lines;
   double* pmax = o.part + (int64_t)(o.nchunk + chunk) * o.lines;
+  int* pnnz = o.count + (int64_t)chunk * o.lines;
+  int* plast = o.count + (int64_t)(o.nchunk + chunk) * o.lines;
   double s = 0.0, m = 0.0;
-  auto add = [&](double2 v) {
+  int nz = 0, last = 0;
+  auto add = [&](double2 v, int k) {
     s = fma(v.x, v.x, fma(v.y, v.y, s));
     m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
+    // nonzero (a NaN too), by integer instructions beside the FP64 ones
+    if (((unsigned)(__double2hiint(v.x) | __double2hiint(v.y)) << 1 | __double2loint(v.x) | __double2loint(v.y)) != 0u) {
+      ++nz;
+      last = k;
+    }
   };
   auto add_scaled = [&](double2 v, int e) {
     v.x = scale2(v.x, -e);
@@ -196,12 +218,14 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
     // eight lanes a line, 32 lines a block
     const int l = grp * 32 + (threadIdx.x >> 3);
     if (l < o.lines)
-      for (int k = k0 + (threadIdx.x & 7); k < k1; k += 8) add(o.X[k + o.ld * l]);
+      for (int k = k0 + (threadIdx.x & 7); k < k1; k += 8) add(o.X[k + o.ld * l], k);
     const unsigned mine = 0xffu << (threadIdx.x & 24);
 #pragma unroll
     for (int d = 4; d >= 1; d >>= 1) {
       s += __shfl_xor_sync(0xffffffffu, s, d);
       m = fmax(m, __shfl_xor_sync(0xffffffffu, m, d));
+      nz += __shfl_xor_sync(0xffffffffu, nz, d);
+      last = max(last, __shfl_xor_sync(0xffffffffu, last, d));
     }
     if (squares_lost(s, m)) {   // the same for the line's eight lanes
       int e;
@@ -215,13 +239,17 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
     if (l < o.lines && (threadIdx.x & 7) == 0) {
       psum[l] = s;
       pmax[l] = m;
+      pnnz[l] = nz;
+      plast[l] = last;
     }
   } else {
     const int tl = threadIdx.x & 63, tk = threadIdx.x >> 6, l = grp * 64 + tl;
     if (l < o.lines)
-      for (int k = k0 + tk; k < k1; k += 4) add(o.X[l + o.ld * k]);
+      for (int k = k0 + tk; k < k1; k += 4) add(o.X[l + o.ld * k], k);
     ss[tk][tl] = s;
     sm[tk][tl] = m;
+    sn[tk][tl] = nz;
+    sk[tk][tl] = last;
     __syncthreads();
     double t = (ss[0][tl] + ss[1][tl]) + (ss[2][tl] + ss[3][tl]);
     m = fmax(fmax(sm[0][tl], sm[1][tl]), fmax(sm[2][tl], sm[3][tl]));
@@ -240,13 +268,17 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
     if (tk == 0 && l < o.lines) {
       psum[l] = t;
       pmax[l] = m;
+      pnnz[l] = (sn[0][tl] + sn[1][tl]) + (sn[2][tl] + sn[3][tl]);
+      plast[l] = max(max(sk[0][tl], sk[1][tl]), max(sk[2][tl], sk[3][tl]));
     }
   }
 }
 
 // The scale exponent of a line: x 2^e rounds to integers of 2-norm in [2^57, 2^58] (the
 // rounding adds at most sqrt(K / 2), far below the 2^0.6 that 2^116 leaves under P / 2).
-__device__ int line_exponent(const ModOperand& o, int l) {
+// frac: that norm as a fraction of 2^58.
+__device__ int line_exponent(const ModOperand& o, int l, double& frac) {
+  frac = 1.0;
   double s = 0.0, m = 0.0;
   bool lost = false;
   for (int c = 0; c < o.nchunk; ++c) {
@@ -272,7 +304,7 @@ __device__ int line_exponent(const ModOperand& o, int l) {
       s += scale2(u, max(ec - unit, -1100));
     }
   }
-  frexp(sqrt(s) * (1.0 + 1e-12), &e);
+  frac = frexp(sqrt(s) * (1.0 + 1e-12), &e);
   return BETA_BITS - (e + unit);
 }
 
@@ -290,6 +322,31 @@ __device__ __forceinline__ int mod_byte(int sb, int p, float inv) {
 // low bytes of four words
 __device__ __forceinline__ unsigned pack4(int r0, int r1, int r2, int r3) {
   return __byte_perm(__byte_perm(r0, r1, 0x0040), __byte_perm(r2, r3, 0x0040), 0x5410);
+}
+
+// Magnitudes: element k of a line as q = floor(mag_units max(|re|, |im|)) <= 127, in units of
+// 16 / 127 of the line's root mean square, so that sum_k q_ik q_kj is at most
+// 127^2 K / 256 S / (||a_i|| ||b_j||), with S as above.  (Larger elements are cut off, which
+// keeps it a lower bound; the usual ones have eight levels.)  The GEMM's epilogue keeps the
+// sum's exponent and three bits of its mantissa in a byte.
+constexpr float MAG_TOP = 127.0f, MAG_RMS = 16.0f;
+__device__ __forceinline__ uint32_t mag_byte(int sum) {
+  const int bits = __float_as_int(__int2float_rz(sum));   // sum >= 0
+  return (uint32_t)max(0, (bits >> 20) - (127 << 3));
+}
+__device__ __forceinline__ float mag_sum(uint32_t byte) { return byte ? __int_as_float((int)(byte + (127 << 3)) << 20) : 0.0f; }
+// Whether a sum (its byte) shows the FP64 bound for n terms: sum >= 127^2 K / 256 2^-3.5 / sqrt(n)
+// (and the roundings of the magnitudes, below 2^-10 in all); limit = mag_limit(K)
+__device__ __forceinline__ float mag_limit(int K) {
+  const float t = MAG_TOP * MAG_TOP / (MAG_RMS * MAG_RMS) * 0.0885f * (float)K;
+  return t * t;
+}
+__device__ __forceinline__ bool mag_shows(uint32_t byte, int n, float limit) {
+  const float t = mag_sum(byte);
+  return t * t * (float)max(n, 1) >= limit;
+}
+__device__ __forceinline__ float mag_units(int K, double frac) {   // for max(|re|, |im|) / 2^32
+  return MAG_TOP / MAG_RMS * sqrtf((float)K) / (float)frac * 0x1p-26f;
 }
 
 // The u and v bytes of 8 integers modulo modulus I into its two planes.
@@ -328,6 +385,7 @@ __global__ void __launch_bounds__(SPL_NT, 1024 / SPL_NT) k_mod_split(const ModOp
   grid_enter();
   __shared__ double2 tile[SPL_LINES][65];
   __shared__ int ex[SPL_LINES];
+  __shared__ float mu[SPL_LINES];
   const bool first = (int)blockIdx.x < a.nblocks_split;
   const ModOperand& o = first ? a : b;
   const int blk = first ? blockIdx.x : blockIdx.x - a.nblocks_split;
@@ -335,9 +393,19 @@ __global__ void __launch_bounds__(SPL_NT, 1024 / SPL_NT) k_mod_split(const ModOp
   const int k0 = (blk % nk) * 64, l0 = (blk / nk) * SPL_LINES;
   const int tid = threadIdx.x;
   if (tid < SPL_LINES) {
-    const int e = l0 + tid < o.lines ? line_exponent(o, l0 + tid) : 0;
+    const int l = l0 + tid;
+    double frac = 1.0;
+    const int e = l < o.lines ? line_exponent(o, l, frac) : 0;
     ex[tid] = e == EXP_NONFINITE ? 0 : e;
-    if (k0 == 0 && l0 + tid < o.lines) o.expo[l0 + tid] = e;
+    mu[tid] = mag_units(o.K, frac);
+    if (k0 == 0 && l < o.lines) {
+      int nz = 0, last = 0;
+      for (int c = 0; c < o.nchunk; ++c) {
+        nz += o.count[(int64_t)c * o.lines + l];
+        last = max(last, o.count[(int64_t)(o.nchunk + c) * o.lines + l]);
+      }
+      o.info[l] = make_int4(e, nz, last, 0);
+    }
   }
   if (o.kcontig) {
     const int kx = tid & 63, ly = tid >> 6;
@@ -359,7 +427,8 @@ __global__ void __launch_bounds__(SPL_NT, 1024 / SPL_NT) k_mod_split(const ModOp
   if (l0 + ll >= o.lines) return;
   const int e = ex[ll], eh = e / 2;
   const double s1 = pow2(eh), s2 = pow2(e - eh);
-  unsigned xlo[8], xhi[8], ylo[8], yhi[8];
+  const float unit = mu[ll];
+  unsigned xlo[8], xhi[8], ylo[8], yhi[8], q[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
     const double2 v = tile[ll][8 * kq + c];
@@ -369,9 +438,15 @@ __global__ void __launch_bounds__(SPL_NT, 1024 / SPL_NT) k_mod_split(const ModOp
     xhi[c] = (unsigned)(nx >> 32);
     ylo[c] = (unsigned)ny;
     yhi[c] = (unsigned)(ny >> 32);
+    // (the floors of both components, one less in magnitude where negative: a lower bound)
+    const int hx = (int)xhi[c] - (1 << 30), hy = (int)yhi[c] - (1 << 30);
+    const int h = max(max(hx, -1 - hx), max(hy, -1 - hy));
+    q[c] = (unsigned)__float_as_int(__fadd_rz(fminf((float)h * unit, MAG_TOP), 8388608.0f));
   }
   int8_t* out = o.planes + (int64_t)(l0 + ll) * o.Kp + k0 + 8 * kq;
   const int64_t plane = (int64_t)o.lines * o.Kp;
+  *reinterpret_cast<uint2*>(out + plane * NRES) =
+      make_uint2(pack4((int)q[0], (int)q[1], (int)q[2], (int)q[3]), pack4((int)q[4], (int)q[5], (int)q[6], (int)q[7]));
   split_moduli(xlo, xhi, ylo, yhi, out, plane, std::make_integer_sequence<int, NMOD>{});
 }
 
@@ -656,6 +731,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GTHREADS, 1)
       const int mi = pl % NMOD;
       const int p = kTab.p[mi], wgt = kTab.wa_lo[mi], off = kTab.off_s[mi];
       const float inv = kTab.inv[mi];
+      const uint32_t flip = pl < NRES ? 0x80808080u : 0u;   // residues are stored with an offset of 128
       const int buf = n % GBUF;
       if (!mbar_wait(&tfull[buf], (n / GBUF) & 1, err, g.wait_cycles)) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -676,12 +752,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GTHREADS, 1)
         const int col = nb * GT + h * ECOLS + ch * 32;
         if (row < g.M && col < g.ldo) {
           uint32_t w[8];
+          if (pl < NRES) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            r[j] = (uint32_t)mod_byte(dp4a_us(r[j] ^ 0x80000000u, wgt, off), p, inv);
+            for (int j = 0; j < 32; ++j)
+              r[j] = (uint32_t)mod_byte(dp4a_us(r[j] ^ 0x80000000u, wgt, off), p, inv);
+          } else {
 #pragma unroll
-          for (int j = 0; j < 8; ++j)   // stored with an offset of 128
-            w[j] = pack4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]) ^ 0x80808080u;
+            for (int j = 0; j < 32; ++j) r[j] = mag_byte((int)r[j]);
+          }
+#pragma unroll
+          for (int j = 0; j < 8; ++j) w[j] = pack4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]) ^ flip;
           uint8_t* o = orow + (int64_t)col * g.M;   // column block col / 16
           *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
           *reinterpret_cast<uint4*>(o + (int64_t)16 * g.M) = make_uint4(w[4], w[5], w[6], w[7]);
@@ -706,8 +786,7 @@ struct ModJoinArgs {
   int M, N, K;
   int64_t ldo;
   const uint8_t* res;
-  const int* ea;
-  const int* eb;
+  const int4 *ia, *ib;
   double2 alpha, beta;
   double2* C;
   int64_t ldc;
@@ -735,27 +814,30 @@ __device__ __forceinline__ void join_moduli(const unsigned (&wu)[NMOD], const un
   (join_modulus<I>(wu[I], wv[I], x1, y1, x2, y2), ...);
 }
 
-// Elements of a 64 x 16 tile that residues do not give, as plain FP64 sums: `bad` marks those
-// of this thread's four columns c4 .. c4 + 3 of row r.  All threads of the block call it.  A few
-// elements take a warp each; from 64 on the block sums the whole tile, K stages of 16 through
-// shared memory (an all-NaN 6144 x 4096 x 1024 product in the time of the FP64 pipe, where a
-// serial sum per element took thousands of times as long).  An element's sum is the same
-// whatever the timing.
-constexpr int RD_K = 16, RD_FEW = 64;
+// Elements of a 64 x 16 tile that residues do not give to the accuracy of FP64, as plain FP64
+// sums: `bad` marks those of this thread's four columns c4 .. c4 + 3 of row r.  All threads of
+// the block call it.  A few elements take a warp each; from 32 on the block forms the whole
+// tile on the FP64 tensor cores, K stages of 16 through shared memory.  An element's sum does
+// not depend on timing.
+constexpr int RD_K = 16, RD_FEW = 32;
+__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
 __device__ __noinline__ void fp64_elements(const ModOperand& a, const ModOperand& b, int M, int N, int K, int m0, int n0,
                                            unsigned bad, double2 (*tile)[65]) {
-  __shared__ double2 as[RD_K][65], bs[RD_K][17];
+  __shared__ double2 as[RD_K][66], bs[RD_K][18];   // strides of 2 mod 8: fragment reads without bank conflicts
+  __shared__ unsigned mask[64];                    // bits: columns of a row to be replaced
   __shared__ unsigned short list[RD_FEW];
   __shared__ int count;
-  const int tid = threadIdx.x, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int r = tid >> 2, c4 = (tid & 3) * 4;
-  auto mac = [](double2& s, double2 x, double2 y) {
-    s.x = fma(-x.y, y.y, fma(x.x, y.x, s.x));
-    s.y = fma(x.y, y.x, fma(x.x, y.y, s.y));
-  };
   if (tid == 0) count = 0;
+  if (tid < 64) mask[tid] = 0u;
   __syncthreads();
   if (bad) {
+    atomicOr(&mask[r], bad << c4);
     int at = atomicAdd(&count, __popc(bad));
     for (int e = 0; e < 4; ++e)
       if (bad >> e & 1) {
@@ -766,11 +848,15 @@ __device__ __noinline__ void fp64_elements(const ModOperand& a, const ModOperand
   __syncthreads();
   const int n = count;
   if (n <= RD_FEW) {
-    for (int i = tid >> 5; i < n; i += 8) {
+    for (int i = warp; i < n; i += 8) {
       const int er = list[i] >> 4, ec = list[i] & 15;
       double2 s = make_double2(0.0, 0.0);
 #pragma unroll 4
-      for (int k = lane; k < K; k += 32) mac(s, load_elem(a, m0 + er, k), load_elem(b, n0 + ec, k));
+      for (int k = lane; k < K; k += 32) {
+        const double2 x = load_elem(a, m0 + er, k), y = load_elem(b, n0 + ec, k);
+        s.x = fma(-x.y, y.y, fma(x.x, y.x, s.x));
+        s.y = fma(x.y, y.x, fma(x.x, y.y, s.y));
+      }
 #pragma unroll
       for (int d = 16; d >= 1; d >>= 1) {
         s.x += __shfl_xor_sync(0xffffffffu, s.x, d);
@@ -778,41 +864,65 @@ __device__ __noinline__ void fp64_elements(const ModOperand& a, const ModOperand
       }
       if (lane == 0) tile[ec][er] = s;
     }
-  } else {
-    double2 s[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) s[e] = make_double2(0.0, 0.0);
-    for (int k0 = 0; k0 < K; k0 += RD_K) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int k = a.kcontig ? tid & 15 : (tid >> 6) + 4 * q, l = a.kcontig ? (tid >> 4) + 16 * q : tid & 63;
-        as[k][l] = k0 + k < K && m0 + l < M ? load_elem(a, m0 + l, k0 + k) : make_double2(0.0, 0.0);
-      }
-      const int k = b.kcontig ? tid & 15 : tid >> 4, l = b.kcontig ? tid >> 4 : tid & 15;
-      bs[k][l] = k0 + k < K && n0 + l < N ? load_elem(b, n0 + l, k0 + k) : make_double2(0.0, 0.0);
-      __syncthreads();
-#pragma unroll
-      for (int q = 0; q < RD_K; ++q) {
-        const double2 x = as[q][r];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) mac(s[e], x, bs[q][c4 + e]);
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      if (bad >> e & 1) tile[c4 + e][r] = s[e];
+    __syncthreads();
+    return;
   }
+  // a warp's 8 rows x 16 columns, in the order of sums of the FP64 tensor-core kernel
+  const int ak = a.kcontig ? tid & 15 : tid >> 6, al = a.kcontig ? tid >> 4 : tid & 63;
+  const int bk = b.kcontig ? tid & 15 : tid >> 4, bl = b.kcontig ? tid >> 4 : tid & 15;
+  const int dk = a.kcontig ? 0 : 4, dl = a.kcontig ? 16 : 0;
+  double2 pa[4], pb;
+  auto fetch = [&](int k0) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int k = k0 + ak + dk * q, l = m0 + al + dl * q;
+      pa[q] = k < K && l < M ? load_elem(a, l, k) : make_double2(0.0, 0.0);
+    }
+    pb = k0 + bk < K && n0 + bl < N ? load_elem(b, n0 + bl, k0 + bk) : make_double2(0.0, 0.0);
+  };
+  double re[2][2] = {}, im[2][2] = {};
+  const int fr = lane >> 2, fk = lane & 3;
+  fetch(0);
+  for (int k0 = 0; k0 < K; k0 += RD_K) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) as[ak + dk * q][al + dl * q] = pa[q];
+    bs[bk][bl] = pb;
+    __syncthreads();
+    if (k0 + RD_K < K) fetch(k0 + RD_K);
+#pragma unroll
+    for (int kb = 0; kb < RD_K; kb += 4) {
+      const double2 x = as[kb + fk][8 * warp + fr];
+      const double2 y[2] = {bs[kb + fk][fr], bs[kb + fk][8 + fr]};
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        dmma_8x8x4(re[j], x.x, y[j].x);
+        dmma_8x8x4(im[j], x.x, y[j].y);
+      }
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        dmma_8x8x4(re[j], -x.y, y[j].y);
+        dmma_8x8x4(im[j], x.y, y[j].x);
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int row = 8 * warp + fr, col = 8 * j + 2 * fk + e;
+      if (mask[row] >> col & 1) tile[col][row] = make_double2(re[j][e], im[j][e]);
+    }
   __syncthreads();
 }
 
-// A block joins a 64 x 16 tile of C: a thread reads 4 columns of a row from the 32 planes
+// A block joins a 64 x 16 tile of C: a thread reads 4 columns of a row from the planes
 // and sums the CRT fractions of its 4 elements, modulo 1 in 32-bit integers for their
 // leading bits, in FP64 below; the tile goes through shared memory so that C is written
 // along its columns.  The stored bytes are residues + 128, so u + v and u - v + 256 exceed
 // the sums meant by 256 each, which the accumulators' starting values take out.  Per
 // element: 32 integer and 32 double multiply-adds, 32 conversions by exponent trick and
-// 48 bytes of memory traffic.
+// 49 bytes of memory traffic.
 template <bool BETA>
 __global__ void __launch_bounds__(256, 3)
     k_mod_join(const ModJoinArgs g, const __grid_constant__ ModOperand a, const __grid_constant__ ModOperand b) {
@@ -822,7 +932,7 @@ __global__ void __launch_bounds__(256, 3)
   const int r = tid >> 2, c4 = (tid & 3) * 4;
   const int m0 = blockIdx.x * 64, n0 = blockIdx.y * 16;
   const int row = m0 + r;
-  unsigned bad = 0;   // columns whose sum an infinity or a NaN takes part in
+  unsigned bad = 0;   // columns to be summed in FP64
   if (row < g.M) {
     const uint8_t* src = g.res + (int64_t)n0 * g.M + (int64_t)row * 16 + c4;
     const int64_t plane = (int64_t)g.M * g.ldo;
@@ -844,21 +954,41 @@ __global__ void __launch_bounds__(256, 3)
       wu[i] = __ldcs(reinterpret_cast<const unsigned*>(src + plane * i));
       wv[i] = __ldcs(reinterpret_cast<const unsigned*>(src + plane * (NMOD + i)));
     }
+    const unsigned wm = __ldcs(reinterpret_cast<const unsigned*>(src + plane * NRES));
     join_moduli(wu, wv, x1, y1, x2, y2, std::make_integer_sequence<int, NMOD>{});
-    const int ea = g.ea[row];
+    const int4 ia = g.ia[row];
+    const int ea = ia.x, na = ia.y;
+    const float limit = mag_limit(g.K);
+    unsigned one = 0;   // columns whose sum has one term
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const int col = n0 + c4 + e;
-      if (col >= g.N) continue;
-      const int eb = g.eb[col];
-      if (ea == EXP_NONFINITE || eb == EXP_NONFINITE) {
+      const int4 ib = g.ib[min(n0 + c4 + e, g.N - 1)];
+      const int eb = ib.x, nb = ib.y;
+      const bool finite = ea != EXP_NONFINITE && eb != EXP_NONFINITE, single = na == 1 || nb == 1;
+      if (!finite || (na > 0 && nb > 0 && !single && !mag_shows(__byte_perm(wm, 0, 0x4440 + e), na + nb - g.K, limit)))
         bad |= 1u << e;
-        continue;
-      }
-      const int t = max(-(ea + eb), -2000), th = t / 2;
+      else if (single) one |= 1u << e;
+      const int t = finite ? max(-(ea + eb), -2000) : 0, th = t / 2;
       const double s1 = pow2(th), s2 = pow2(t - th);
       tile[c4 + e][r] = make_double2(fma((double)(int)x1[e], 0x1p-32, x2[e]) * P * s1 * s2,
                                      fma((double)(int)y1[e], 0x1p-32, y2[e]) * P * s1 * s2);
+    }
+    const int live = min(4, g.N - n0 - c4);   // (columns past the last one were read in its place)
+    const unsigned in = live > 0 ? (1u << live) - 1u : 0u;
+    bad &= in;
+    one &= in;
+    if (one) {
+      double2 x[4], y[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int col = min(n0 + c4 + e, g.N - 1), k = na == 1 ? ia.z : g.ib[col].z;
+        x[e] = load_elem(a, row, k);
+        y[e] = load_elem(b, col, k);
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (one >> e & 1)
+          tile[c4 + e][r] = make_double2(fma(-x[e].y, y[e].y, x[e].x * y[e].x), fma(x[e].y, y[e].x, x[e].x * y[e].y));
     }
   }
   if (__syncthreads_or(bad)) fp64_elements(a, b, g.M, g.N, g.K, m0, n0, bad, tile);
@@ -908,15 +1038,16 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
   const int64_t ldo = up(np, 32);
   const size_t pc = (size_t)NPL * M * ldo;
   const int nchunk = std::max(1, std::min(16, K / 64));
-  const size_t tail = (size_t)(M + N) * (2 * nchunk * sizeof(double) + sizeof(int));
+  const size_t tail = (size_t)(M + N) * (2 * nchunk * (sizeof(double) + sizeof(int)) + sizeof(int4));
   auto at = [](size_t x) { return (x + 1023) / 1024 * 1024; };
   uint8_t* base = static_cast<uint8_t*>(ctx->optional_buf("gemm_modular", at(pa) + at(pb) + at(pc) + tail + 4096));
   if (!base) return false;
   int8_t* planesA = reinterpret_cast<int8_t*>(base);
   int8_t* planesB = reinterpret_cast<int8_t*>(base + at(pa));
   uint8_t* res = base + at(pa) + at(pb);
-  double* part = reinterpret_cast<double*>(res + at(pc));
-  int* expo = reinterpret_cast<int*>(part + (size_t)(M + N) * 2 * nchunk);
+  int4* info = reinterpret_cast<int4*>(res + at(pc));
+  double* part = reinterpret_cast<double*>(info + M + N);
+  int* count = reinterpret_cast<int*>(part + (size_t)(M + N) * 2 * nchunk);
 
   ModOperand a{}, b{};
   a.X = A;
@@ -926,7 +1057,8 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
   a.conj = opA == OP_C;
   a.planes = planesA;
   a.part = part;
-  a.expo = expo;
+  a.count = count;
+  a.info = info;
   b.X = B;
   b.ld = ldb;
   b.lines = N;
@@ -934,7 +1066,8 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
   b.conj = opB == OP_C;
   b.planes = planesB;
   b.part = part + (size_t)M * 2 * nchunk;
-  b.expo = expo + M;
+  b.count = count + (size_t)M * 2 * nchunk;
+  b.info = info + M;
   for (ModOperand* o : {&a, &b}) {
     o->K = K;
     o->Kp = Kp;
@@ -972,8 +1105,8 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
     j.K = K;
     j.ldo = ldo;
     j.res = res;
-    j.ea = a.expo;
-    j.eb = b.expo + n0;
+    j.ia = a.info;
+    j.ib = b.info + n0;
     j.alpha = make_double2(alpha.real(), alpha.imag());
     j.beta = make_double2(beta.real(), beta.imag());
     j.C = C + ldc * n0;
