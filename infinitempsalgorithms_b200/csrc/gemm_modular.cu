@@ -11,7 +11,8 @@
 //     complex product is two real ones (not four).  All residues are int8, the sums over K
 //     exact in int32: 32 real int8 GEMMs of M x N x K.
 //  3. The 32 residues of an output give Re c' / P and Im c' / P as fractions modulo 1
-//     (Chinese remainder theorem), then the product with P and the power-of-two scales.
+//     (Chinese remainder theorem), then the product with P and the power-of-two scales; or,
+//     where both lines were integers up to a power of two, the exact integers c', rounded once.
 //
 // Accuracy: the roundings of step 1 are below 2^-58 of the row's (column's) 2-norm per
 // component, so an element of C is off by about 0.58 2^-57 ||a_i|| ||b_j||, and by its own
@@ -25,15 +26,16 @@
 //   when S >= ||a_i|| ||b_j|| 2^-3.5 / sqrt(n).  n is at least nnz(a_i) + nnz(b_j) - K.
 // Unstructured lines have S = 0.8 ||a_i|| ||b_j||, a flat line times one that a single element
 // dominates still ||a_i|| ||b_j|| / sqrt(K).  A line with one nonzero element (the identity
-// level of an environment) gives plain FP64 products, as exact as on the FP64 tensor cores.
+// level of an environment) gives plain FP64 products, as exact as on the FP64 tensor cores,
+// and lines that lose nothing in step 1 (integers, permutations) a correctly rounded result.
 // Rows or columns with a NaN or an Inf are recognised and their elements computed as plain
 // FP64 sums.
 //
 // The four kernels: partial row norms, residue and magnitude planes, the int8 GEMMs, the
-// reconstruction.  Measured (B200): 6144 x 4096 x 1024 1.14 ms = 30 + 154 + 644 + 313 us
-// (6.50 ms on the FP64 tensor cores), 4096 x 1024 x 6144 1.10 ms = 78 + 435 + 534 + 55 us
-// (6.57 ms); the magnitudes and the checks cost 5 % of that.  With operands graded so that
-// every element is summed in FP64, 6144 x 4096 x 1024 takes 12.4 ms; with an identity and
+// reconstruction.  Measured (B200): 6144 x 4096 x 1024 1.15 ms = 31 + 155 + 636 + 332 us
+// (6.50 ms on the FP64 tensor cores), 4096 x 1024 x 6144 1.10 ms = 80 + 433 + 528 + 58 us
+// (6.57 ms); the magnitudes and the checks cost 6 and 4 % of that.  With operands graded so
+// that every element is summed in FP64, 6144 x 4096 x 1024 takes 12.4 ms; with an identity and
 // noise of 1e-17 as one operand 2.9 ms.
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -73,6 +75,9 @@ struct ModTables {
   unsigned re1_0, im1_0;           // -256 times the sums of the weights (see k_mod_join)
   double re2_0, im2_0;
   double P;
+  // the weights as integers in [0, P), in three pieces w0 + 2^39 w1 + 2^78 w2, -256 times their
+  // sums, P in the same pieces and 2^78 / P
+  double re3[NMOD][3], im3[NMOD][3], re3_0[3], im3_0[3], p3[3], inv_p2;
 };
 
 constexpr int mod_pow(int b, int e, int p) {
@@ -101,11 +106,21 @@ constexpr double low_weight(int g, int p) {
   return (double)((((rem << 41) / (unsigned)p) + 1) >> 1) / 4722366482869645213696.0;   // 2^72
 }
 
+// 39 bits each of an integer below 2^118.  Sums of 16 of them times integers below 2^9 stay
+// below 2^53, so three such sums are exact in doubles.
+constexpr void pieces(unsigned __int128 x, double (&w)[3]) {
+  w[0] = (double)(unsigned long long)(x & (((unsigned __int128)1 << 39) - 1));
+  w[1] = (double)(unsigned long long)((x >> 39) & (((unsigned __int128)1 << 39) - 1));
+  w[2] = (double)(unsigned long long)(x >> 78);
+}
+
 constexpr ModTables make_tables() {
   ModTables t{};
   unsigned __int128 P = 1;
   for (int i = 0; i < NMOD; ++i) P *= (unsigned)kMod[i];
   t.P = (double)(P >> 32) * 4294967296.0;   // the dropped 32 of 118 bits are below 2^-85 of it
+  pieces(P, t.p3);
+  t.inv_p2 = 302231454903657293676544.0 / t.P;   // 2^78 / P
   for (int i = 0; i < NMOD; ++i) {
     const int p = kMod[i], io = mod_iota(p);
     unsigned w[4] = {0, 0, 0, 0};
@@ -138,6 +153,12 @@ constexpr ModTables make_tables() {
     t.im1_0 -= 256u * t.im1[i];
     t.re2_0 -= 256.0 * t.re2[i];
     t.im2_0 -= 256.0 * t.im2[i];
+    pieces(P / (unsigned)p * (unsigned)g, t.re3[i]);
+    pieces(P / (unsigned)p * (unsigned)h, t.im3[i]);
+    for (int k = 0; k < 3; ++k) {
+      t.re3_0[k] -= 256.0 * t.re3[i][k];
+      t.im3_0[k] -= 256.0 * t.im3[i][k];
+    }
   }
   return t;
 }
@@ -161,8 +182,9 @@ struct ModOperand {
   int64_t Kp;
   double* part;       // per K chunk and line: sum of squares, then max |re|, |im|
   int nchunk, kchunk;
-  int* count;         // per K chunk and line: nonzero elements, then the largest k of one
-  int4* info;         // per line: the scale's exponent, nonzero elements, the last one's k
+  int* count;         // per K chunk and line: nonzero elements, the largest k of one, lowest bit
+  int4* info;         // per line: the scale's exponent, nonzero elements, the last one's k,
+                      // whether all elements are integers in the scale
   int nblocks_norm, nblocks_split;
 };
 
@@ -172,6 +194,22 @@ __device__ __forceinline__ double2 load_elem(const ModOperand& o, int l, int k) 
   return v;
 }
 
+// A bound from below for the exponents of all set bits of a set of doubles: from the least
+// exponent of a nonzero one and the zeros below all their mantissas.  (Whole numbers below 2^b
+// come out no lower than 2^-b, which is low enough for the scale of a line up to b = 26, i.e.
+// wherever a sum of such products is itself a double.)
+struct LowBits {
+  unsigned any = 0u, least = 0xffffffffu;
+  __device__ __forceinline__ void add(double x) {
+    const unsigned lo = (unsigned)__double2loint(x), hi = (unsigned)__double2hiint(x) & 0x7fffffffu;
+    any |= lo;
+    least = min(least, hi - (lo == 0u ? 1u : 0u));   // zero: the largest
+  }
+  __device__ __forceinline__ int bound() const {
+    if (least == 0xffffffffu) return 4096;
+    return (int)(least >> 20) - 1075 + (any ? __ffs((int)any) - 1 : 32);
+  }
+};
 // 2^e in the double range, and x 2^e for any |e| <= 1100
 __device__ __forceinline__ double pow2(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
 __device__ __forceinline__ double scale2(double x, int e) { return x * pow2(e / 2) * pow2(e - e / 2); }
@@ -188,7 +226,7 @@ __device__ __forceinline__ bool squares_lost(double s, double m) {
 __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const ModOperand b) {
   grid_enter();
   __shared__ double ss[4][64], sm[4][64];
-  __shared__ int sn[4][64], sk[4][64];
+  __shared__ int sn[4][64], sk[4][64], sb[4][64];
   const bool first = (int)blockIdx.x < a.nblocks_norm;
   const ModOperand& o = first ? a : b;
   const int blk = first ? blockIdx.x : blockIdx.x - a.nblocks_norm;
@@ -198,8 +236,10 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
   double* pmax = o.part + (int64_t)(o.nchunk + chunk) * o.lines;
   int* pnnz = o.count + (int64_t)chunk * o.lines;
   int* plast = o.count + (int64_t)(o.nchunk + chunk) * o.lines;
+  int* plow = o.count + (int64_t)(2 * o.nchunk + chunk) * o.lines;
   double s = 0.0, m = 0.0;
   int nz = 0, last = 0;
+  LowBits bits;
   auto add = [&](double2 v, int k) {
     s = fma(v.x, v.x, fma(v.y, v.y, s));
     m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
@@ -208,6 +248,8 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
       ++nz;
       last = k;
     }
+    bits.add(v.x);
+    bits.add(v.y);
   };
   auto add_scaled = [&](double2 v, int e) {
     v.x = scale2(v.x, -e);
@@ -219,6 +261,7 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
     const int l = grp * 32 + (threadIdx.x >> 3);
     if (l < o.lines)
       for (int k = k0 + (threadIdx.x & 7); k < k1; k += 8) add(o.X[k + o.ld * l], k);
+    int low = bits.bound();
     const unsigned mine = 0xffu << (threadIdx.x & 24);
 #pragma unroll
     for (int d = 4; d >= 1; d >>= 1) {
@@ -226,6 +269,7 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
       m = fmax(m, __shfl_xor_sync(0xffffffffu, m, d));
       nz += __shfl_xor_sync(0xffffffffu, nz, d);
       last = max(last, __shfl_xor_sync(0xffffffffu, last, d));
+      low = min(low, __shfl_xor_sync(0xffffffffu, low, d));
     }
     if (squares_lost(s, m)) {   // the same for the line's eight lanes
       int e;
@@ -241,6 +285,7 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
       pmax[l] = m;
       pnnz[l] = nz;
       plast[l] = last;
+      plow[l] = low;
     }
   } else {
     const int tl = threadIdx.x & 63, tk = threadIdx.x >> 6, l = grp * 64 + tl;
@@ -250,6 +295,7 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
     sm[tk][tl] = m;
     sn[tk][tl] = nz;
     sk[tk][tl] = last;
+    sb[tk][tl] = bits.bound();
     __syncthreads();
     double t = (ss[0][tl] + ss[1][tl]) + (ss[2][tl] + ss[3][tl]);
     m = fmax(fmax(sm[0][tl], sm[1][tl]), fmax(sm[2][tl], sm[3][tl]));
@@ -270,6 +316,7 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
       pmax[l] = m;
       pnnz[l] = (sn[0][tl] + sn[1][tl]) + (sn[2][tl] + sn[3][tl]);
       plast[l] = max(max(sk[0][tl], sk[1][tl]), max(sk[2][tl], sk[3][tl]));
+      plow[l] = min(min(sb[0][tl], sb[1][tl]), min(sb[2][tl], sb[3][tl]));
     }
   }
 }
@@ -399,12 +446,13 @@ __global__ void __launch_bounds__(SPL_NT, 1024 / SPL_NT) k_mod_split(const ModOp
     ex[tid] = e == EXP_NONFINITE ? 0 : e;
     mu[tid] = mag_units(o.K, frac);
     if (k0 == 0 && l < o.lines) {
-      int nz = 0, last = 0;
+      int nz = 0, last = 0, low = 4096;
       for (int c = 0; c < o.nchunk; ++c) {
         nz += o.count[(int64_t)c * o.lines + l];
         last = max(last, o.count[(int64_t)(o.nchunk + c) * o.lines + l]);
+        low = min(low, o.count[(int64_t)(2 * o.nchunk + c) * o.lines + l]);
       }
-      o.info[l] = make_int4(e, nz, last, 0);
+      o.info[l] = make_int4(e, nz, last, low + e >= 0);
     }
   }
   if (o.kcontig) {
@@ -814,6 +862,50 @@ __device__ __forceinline__ void join_moduli(const unsigned (&wu)[NMOD], const un
   (join_modulus<I>(wu[I], wv[I], x1, y1, x2, y2), ...);
 }
 
+// The integer nearest zero that is w0 + 2^39 w1 + 2^78 w2 modulo P (|w| < 2^53), rounded once.
+// It is below 2^116.1 by the operands' scales, so taking the multiple of P from w2 alone is
+// safe.  The leading two pieces are added with their exact remainder; when the result is a
+// double it comes out exactly.
+__device__ __forceinline__ double crt_value(const double (&w)[3]) {
+  const double q = rint(w[2] * kTab.inv_p2);
+  const double h = fma(-q, kTab.p3[2], w[2]) * 0x1p39, m = fma(-q, kTab.p3[1], w[1]), l = fma(-q, kTab.p3[0], w[0]);
+  const double s = h + m, b = s - h;
+  const double r = (h - (s - b)) + (m - b);
+  return fma(s, 0x1p39, fma(r, 0x1p39, l));
+}
+// The columns `which` of a thread's four (its bytes at src) from exact sums.  Products of whole
+// numbers come here; three double multiply-adds per modulus and component where the fractions
+// need one (146 us more for 6144 x 4096, were it done for all).
+__device__ __noinline__ void exact_elements(const ModJoinArgs& g, int m0, int n0, unsigned which, double2 (*tile)[65]) {
+  const int r = threadIdx.x >> 2, c4 = (threadIdx.x & 3) * 4;
+  const uint8_t* src = g.res + (int64_t)n0 * g.M + (int64_t)(m0 + r) * 16 + c4;
+  const int64_t plane = (int64_t)g.M * g.ldo;
+  const int ea = g.ia[m0 + r].x;
+#pragma unroll 1
+  for (int e = 0; e < 4; ++e) {
+    if (!(which >> e & 1)) continue;
+    double x[3], y[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      x[k] = kTab.re3_0[k];
+      y[k] = kTab.im3_0[k];
+    }
+#pragma unroll 4
+    for (int i = 0; i < NMOD; ++i) {
+      const int u = src[plane * i + e], v = src[plane * (NMOD + i) + e];
+      const double sp = (double)(u + v), sm = (double)(u - v + 256);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        x[k] = fma(sp, kTab.re3[i][k], x[k]);
+        y[k] = fma(sm, kTab.im3[i][k], y[k]);
+      }
+    }
+    const int t = max(-(ea + g.ib[n0 + c4 + e].x), -2000), th = t / 2;
+    const double s1 = pow2(th), s2 = pow2(t - th);
+    tile[c4 + e][r] = make_double2(crt_value(x) * s1 * s2, crt_value(y) * s1 * s2);
+  }
+}
+
 // Elements of a 64 x 16 tile that residues do not give to the accuracy of FP64, as plain FP64
 // sums: `bad` marks those of this thread's four columns c4 .. c4 + 3 of row r.  All threads of
 // the block call it.  A few elements take a warp each; from 32 on the block forms the whole
@@ -925,14 +1017,15 @@ __device__ __noinline__ void fp64_elements(const ModOperand& a, const ModOperand
 // 49 bytes of memory traffic.
 template <bool BETA>
 __global__ void __launch_bounds__(256, 3)
-    k_mod_join(const ModJoinArgs g, const __grid_constant__ ModOperand a, const __grid_constant__ ModOperand b) {
+    k_mod_join(const __grid_constant__ ModJoinArgs g, const __grid_constant__ ModOperand a,
+               const __grid_constant__ ModOperand b) {
   grid_enter();
   __shared__ double2 tile[16][65];
   const int tid = threadIdx.x;
   const int r = tid >> 2, c4 = (tid & 3) * 4;
   const int m0 = blockIdx.x * 64, n0 = blockIdx.y * 16;
   const int row = m0 + r;
-  unsigned bad = 0;   // columns to be summed in FP64
+  unsigned bad = 0, whole = 0;   // columns to be summed in FP64, columns of whole numbers
   if (row < g.M) {
     const uint8_t* src = g.res + (int64_t)n0 * g.M + (int64_t)row * 16 + c4;
     const int64_t plane = (int64_t)g.M * g.ldo;
@@ -965,7 +1058,8 @@ __global__ void __launch_bounds__(256, 3)
       const int4 ib = g.ib[min(n0 + c4 + e, g.N - 1)];
       const int eb = ib.x, nb = ib.y;
       const bool finite = ea != EXP_NONFINITE && eb != EXP_NONFINITE, single = na == 1 || nb == 1;
-      if (!finite || (na > 0 && nb > 0 && !single && !mag_shows(__byte_perm(wm, 0, 0x4440 + e), na + nb - g.K, limit)))
+      if (finite && !single && ia.w && ib.w) whole |= 1u << e;
+      else if (!finite || (na > 0 && nb > 0 && !single && !mag_shows(__byte_perm(wm, 0, 0x4440 + e), na + nb - g.K, limit)))
         bad |= 1u << e;
       else if (single) one |= 1u << e;
       const int t = finite ? max(-(ea + eb), -2000) : 0, th = t / 2;
@@ -977,6 +1071,7 @@ __global__ void __launch_bounds__(256, 3)
     const unsigned in = live > 0 ? (1u << live) - 1u : 0u;
     bad &= in;
     one &= in;
+    whole &= in;
     if (one) {
       double2 x[4], y[4];
 #pragma unroll
@@ -991,6 +1086,7 @@ __global__ void __launch_bounds__(256, 3)
           tile[c4 + e][r] = make_double2(fma(-x[e].y, y[e].y, x[e].x * y[e].x), fma(x[e].y, y[e].x, x[e].x * y[e].y));
     }
   }
+  if (whole) exact_elements(g, m0, n0, whole, tile);
   if (__syncthreads_or(bad)) fp64_elements(a, b, g.M, g.N, g.K, m0, n0, bad, tile);
   const int tr = tid & 63;
   if (m0 + tr >= g.M) return;
@@ -1038,7 +1134,7 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
   const int64_t ldo = up(np, 32);
   const size_t pc = (size_t)NPL * M * ldo;
   const int nchunk = std::max(1, std::min(16, K / 64));
-  const size_t tail = (size_t)(M + N) * (2 * nchunk * (sizeof(double) + sizeof(int)) + sizeof(int4));
+  const size_t tail = (size_t)(M + N) * (nchunk * (2 * sizeof(double) + 3 * sizeof(int)) + sizeof(int4));
   auto at = [](size_t x) { return (x + 1023) / 1024 * 1024; };
   uint8_t* base = static_cast<uint8_t*>(ctx->optional_buf("gemm_modular", at(pa) + at(pb) + at(pc) + tail + 4096));
   if (!base) return false;
@@ -1066,7 +1162,7 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
   b.conj = opB == OP_C;
   b.planes = planesB;
   b.part = part + (size_t)M * 2 * nchunk;
-  b.count = count + (size_t)M * 2 * nchunk;
+  b.count = count + (size_t)M * 3 * nchunk;
   b.info = info + M;
   for (ModOperand* o : {&a, &b}) {
     o->K = K;
