@@ -131,11 +131,15 @@ int imps_ctx_set_wait_limit(imps_ctx* ctx, int64_t cycles);
  * buffers the solvers and contractions keep between calls (Krylov bases, Heff
  * intermediates, gauge work arrays).  A call that would grow it past the cap
  * returns IMPS_OOM and leaves the context usable; imps_ctx_workspace_bytes reports
- * the current size.  Object storage (states, environments, MPOs) and the cached
- * int8 operand splits are not counted.  No reference counterpart (Julia's GC owns
- * the reference's arrays). */
+ * the current size, with the scratch that only makes products faster (partial sums
+ * and residue planes, 5 GiB at most) and the blocks of destroyed states and
+ * environments kept for the next ones (256 MiB at most).  A cap gives both back and
+ * keeps neither until it is lifted; imps_ctx_trim gives them back once.  Object
+ * storage (states, environments, MPOs) and the cached int8 operand splits are not
+ * counted.  No reference counterpart (Julia's GC owns the reference's arrays). */
 int imps_ctx_set_workspace_limit(imps_ctx* ctx, int64_t bytes);
 int imps_ctx_workspace_bytes(imps_ctx* ctx, int64_t* bytes);
+int imps_ctx_trim(imps_ctx* ctx);
 const char* imps_ctx_last_error(const imps_ctx* ctx);
 const char* imps_status_string(int status);
 /* Kernel timing with CUDA events on the context stream, per kernel class. */

@@ -89,6 +89,7 @@ _SIGS = {
     "imps_svd": (I32, [P, I32, I32, DP, I32, D, DP, DP, DP, C.POINTER(I32)]),
     "imps_ctx_set_workspace_limit": (I32, [P, I64]),
     "imps_ctx_workspace_bytes": (I32, [P, C.POINTER(I64)]),
+    "imps_ctx_trim": (I32, [P]),
     "imps_ctx_counters_ext": (I32, [P, C.POINTER(I64), I32]),
     "imps_ctx_last_error": (C.c_char_p, [P]),
     "imps_ctx_profile": (I32, [P, I32]),

@@ -129,6 +129,10 @@ class Context:
     def synchronize(self):
         check(self.lib.imps_ctx_synchronize(self.h), self.h)
 
+    def trim(self):
+        """Give back the device memory that the context keeps only to make later calls faster."""
+        check(self.lib.imps_ctx_trim(self.h), self.h)
+
     def profile(self, enable: bool = True):
         check(self.lib.imps_ctx_profile(self.h, int(enable)), self.h)
 

@@ -159,7 +159,7 @@ int imps_ctx_destroy(imps_ctx* h) {
     cudaEventDestroy(p.second.second);
   }
   for (auto e : c.event_pool) cudaEventDestroy(e);
-  c.pool->close();
+  c.pool->keep(false);
   c.scratch.clear();
   c.optional.clear();
   c.red.release();
@@ -212,11 +212,18 @@ int imps_ctx_set_wait_limit(imps_ctx* h, int64_t cycles) {
 int imps_ctx_set_workspace_limit(imps_ctx* h, int64_t bytes) {
   if (!h || bytes < 0) return IMPS_INVALID_ARG;
   h->c.workspace_limit = (size_t)bytes;
-  if (bytes > 0) {
-    cudaSetDevice(h->c.device);
-    h->c.release_optional();
-  }
+  cudaSetDevice(h->c.device);
+  if (bytes > 0) h->c.trim();
+  h->c.pool->keep(bytes == 0);
   return IMPS_OK;
+}
+
+int imps_ctx_trim(imps_ctx* h) {
+  if (!h) return IMPS_INVALID_ARG;
+  return guard(&h->c, [&] {
+    h->c.trim();
+    return IMPS_OK;
+  });
 }
 
 int imps_ctx_workspace_bytes(imps_ctx* h, int64_t* bytes) {
@@ -224,6 +231,7 @@ int imps_ctx_workspace_bytes(imps_ctx* h, int64_t* bytes) {
   size_t total = 0;
   for (const auto& kv : h->c.scratch) total += kv.second.bytes;
   for (const auto& kv : h->c.optional) total += kv.second.bytes;
+  total += h->c.pool->held();
   *bytes = (int64_t)total;
   return IMPS_OK;
 }

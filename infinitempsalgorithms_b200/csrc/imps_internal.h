@@ -57,7 +57,8 @@ struct Error : public std::runtime_error {
 // makes a state and an environment per call, and a cudaMalloc / cudaFree pair costs 0.7 ms
 // (now and then a second, when the driver unmaps) and synchronises the device.  The context's
 // objects use its one stream, so a block may be handed on while earlier work on it is queued.
-// Bounded, exact sizes only; emptied when an allocation fails anywhere and when the context
+// Bounded, exact sizes only; emptied when an allocation fails anywhere, when the caller asks for
+// it or caps the workspace (then nothing is kept until the cap is lifted), and when the context
 // goes; an object that outlives its context frees its blocks itself.
 class BlockPool {
  public:
@@ -66,7 +67,8 @@ class BlockPool {
   void* take(size_t bytes);               // nullptr: none of this size
   bool give(void* ptr, size_t bytes);     // false: not kept
   void trim();                            // frees what is idle
-  void close();                           // trim, and keep nothing from now on
+  void keep(bool on);                     // false: trim, and keep nothing until it is on again
+  size_t held();                          // bytes kept
   static void trim_all();
 
  private:
@@ -260,6 +262,12 @@ struct Context {
   void release_optional() {
     cudaStreamSynchronize(stream);
     optional.clear();
+  }
+  // gives back what only makes later calls faster (not inside a graph capture, which it would end)
+  void trim() {
+    if (capturing()) return;
+    release_optional();
+    pool->trim();
   }
   double* pinned(size_t bytes);
 };

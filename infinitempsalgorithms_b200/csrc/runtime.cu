@@ -536,12 +536,16 @@ void BlockPool::trim() {
   idle_.clear();
   held_ = 0;
 }
-void BlockPool::close() {
+void BlockPool::keep(bool on) {
   {
     std::lock_guard<std::mutex> lock(mu_);
-    open_ = false;
+    open_ = on;
   }
-  trim();
+  if (!on) trim();
+}
+size_t BlockPool::held() {
+  std::lock_guard<std::mutex> lock(mu_);
+  return held_;
 }
 void BlockPool::trim_all() {
   std::lock_guard<std::mutex> lock(pools_mu());
