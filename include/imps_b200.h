@@ -123,7 +123,7 @@ int imps_ctx_synchronize(imps_ctx* ctx);
  * host synchronisation (at the latest when the entry point returns) and the call
  * returns IMPS_TIMEOUT; the context stays usable.  The FP64 products of the asynchronous
  * calls (imps_ac_apply_dev, imps_c_apply_dev) report at the next other call,
- * imps_ctx_synchronize among them.  No reference counterpart (the
+ * imps_ctx_synchronize among them; their results are NaN.  No reference counterpart (the
  * reference has no device code): the bounded-wait failure detection of this
  * library. */
 int imps_ctx_set_wait_limit(imps_ctx* ctx, int64_t cycles);

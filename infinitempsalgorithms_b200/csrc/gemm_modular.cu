@@ -835,6 +835,7 @@ struct ModJoinArgs {
   int64_t ldo;
   const uint8_t* res;
   const int4 *ia, *ib;
+  const int* err;       // set when a wait of the GEMMs (or of a product before) gave up
   double2 alpha, beta;
   double2* C;
   int64_t ldc;
@@ -1025,6 +1026,8 @@ __global__ void __launch_bounds__(256, 3)
   const int r = tid >> 2, c4 = (tid & 3) * 4;
   const int m0 = blockIdx.x * 64, n0 = blockIdx.y * 16;
   const int row = m0 + r;
+  // a product that gave up leaves NaNs, for callers that wait without asking for the status
+  const bool gave_up = *(const volatile int*)g.err != 0;
   unsigned bad = 0, whole = 0;   // columns to be summed in FP64, columns of whole numbers
   if (row < g.M) {
     const uint8_t* src = g.res + (int64_t)n0 * g.M + (int64_t)row * 16 + c4;
@@ -1069,7 +1072,7 @@ __global__ void __launch_bounds__(256, 3)
     }
     const int live = min(4, g.N - n0 - c4);   // (columns past the last one were read in its place)
     const unsigned in = live > 0 ? (1u << live) - 1u : 0u;
-    bad &= in;
+    bad &= gave_up ? 0u : in;
     one &= in;
     whole &= in;
     if (one) {
@@ -1095,6 +1098,7 @@ __global__ void __launch_bounds__(256, 3)
     if (n0 + c >= g.N) break;
     const double2 v = tile[c][tr];
     double2 o = make_double2(g.alpha.x * v.x - g.alpha.y * v.y, g.alpha.x * v.y + g.alpha.y * v.x);
+    if (gave_up) o.x = o.y = __longlong_as_double(0x7ff8000000000000ll);
     double2* p = g.C + (m0 + tr) + g.ldc * (int64_t)(n0 + c);
     if (BETA) {
       const double2 z = *p;
@@ -1203,6 +1207,7 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
     j.res = res;
     j.ia = a.info;
     j.ib = b.info + n0;
+    j.err = ctx->err_dev;
     j.alpha = make_double2(alpha.real(), alpha.imag());
     j.beta = make_double2(beta.real(), beta.imag());
     j.C = C + ldc * n0;

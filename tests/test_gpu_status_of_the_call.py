@@ -60,3 +60,22 @@ def test_the_call_itself_reports(setup, call):
     assert e.value.status == L.IMPS_TIMEOUT
     _limit(ctx, 0)
     assert ctx.lib.imps_ctx_synchronize(ctx.h) == L.IMPS_OK   # nothing left behind
+
+
+def test_a_result_that_gave_up_is_nan(setup):
+    """For a caller that waits on its own stream and does not ask for the status."""
+    ctx, H, psi, envs = setup
+    x = torch.from_numpy(np.ascontiguousarray(psi.AC[0].transpose(2, 1, 0))).cuda()
+    y, z = torch.empty_like(x), torch.empty_like(x)
+    torch.cuda.synchronize()
+
+    def apply(out):
+        return ctx.lib.imps_ac_apply_dev(envs.h, H.handle(ctx), 0, C.c_void_p(x.data_ptr()), C.c_void_p(out.data_ptr()))
+    _limit(ctx, 1)
+    assert apply(y) == L.IMPS_OK
+    torch.cuda.synchronize()
+    assert torch.isnan(y.real).all() and torch.isnan(y.imag).all()
+    _limit(ctx, 0)
+    assert ctx.lib.imps_ctx_synchronize(ctx.h) == L.IMPS_TIMEOUT
+    assert apply(z) == L.IMPS_OK and ctx.lib.imps_ctx_synchronize(ctx.h) == L.IMPS_OK
+    assert torch.isfinite(torch.view_as_real(z)).all()
