@@ -41,6 +41,45 @@ std::vector<cplx> herm_part(const std::vector<cplx>& H, int ldh, int m) {
 // extra one costs.
 constexpr int64_t kAheadMax = (int64_t)1 << 18;
 
+class Ahead {
+ public:
+  Ahead(Context* ctx, int64_t n) : ctx_(ctx), n_(n) {}
+  ~Ahead() {
+    if (!queued_) return;   // thrown away: not one of the solve's applications
+    ctx_->n_ac_apply -= after_counts_.ac - before_counts_.ac;
+    ctx_->n_c_apply -= after_counts_.c - before_counts_.c;
+    ctx_->n_push -= after_counts_.push - before_counts_.push;
+    ctx_->gemm_flops -= after_counts_.flops - before_counts_.flops;
+  }
+  // w is the unnormalised next basis vector
+  void queue(const LinOp& A, dcplx* w, double norm) {
+    if (n_ > kAheadMax || !(norm > 1e-100)) return;
+    zscal(ctx_, n_, 1.0 / norm, w);
+    before_counts_ = counts();
+    A(w, w + n_);
+    queued_ = true;
+    after_counts_ = counts();
+  }
+  // whether w is normalised and its image queued
+  bool queued() const { return queued_; }
+  bool take() {
+    const bool q = queued_;
+    queued_ = false;
+    return q;
+  }
+
+ private:
+  struct Counts {
+    int64_t ac, c, push;
+    double flops;
+  };
+  Counts counts() const { return {ctx_->n_ac_apply, ctx_->n_c_apply, ctx_->n_push, ctx_->gemm_flops}; }
+  Context* ctx_;
+  int64_t n_;
+  Counts before_counts_{}, after_counts_{};
+  bool queued_ = false;
+};
+
 void phase_align(Context* ctx, int64_t n, const dcplx* x0n, dcplx* x) {
   cplx ov = zdotc(ctx, n, x0n, x);
   double a = std::abs(ov);
@@ -68,19 +107,14 @@ KrylovResult lanczos_eigsolve(Context* ctx, int64_t n, const LinOp& A, const dcp
   int nvec = 1;
   std::vector<double> theta;
   std::vector<cplx> U;
-  bool ahead = false;   // the next matvec is already queued
+  Ahead ahead(ctx, n);
   while (true) {
     const int k = nvec - 1;
     dcplx* w = V + n * (int64_t)nvec;
-    if (!ahead) A(V + n * (int64_t)k, w);
-    ahead = false;
+    if (!ahead.take()) A(V + n * (int64_t)k, w);
     res.numops++;
     double beta = cgs2(ctx, n, nvec, V, w, h);
-    if (n <= kAheadMax && k + 1 < kdim && beta > 1e-100) {
-      zscal(ctx, n, 1.0 / beta, w);
-      A(w, w + n);
-      ahead = true;
-    }
+    if (k + 1 < kdim) ahead.queue(A, w, beta);
     for (int i = 0; i <= k; ++i) H[i + (size_t)ldh * k] = h[i];
     H[k + 1 + (size_t)ldh * k] = beta;
     const int m = k + 1;
@@ -128,7 +162,7 @@ KrylovResult lanczos_eigsolve(Context* ctx, int64_t n, const LinOp& A, const dcp
       nvec = keep + 1;
       res.numiter++;
     } else {
-      if (!ahead) zscal(ctx, n, 1.0 / beta, w);
+      if (!ahead.queued()) zscal(ctx, n, 1.0 / beta, w);
       nvec++;
     }
   }
@@ -244,19 +278,14 @@ KrylovResult exponentiate(Context* ctx, int64_t n, const LinOp& A, cplx t, const
     cplx tau = remaining;
     int m = 0;
     double err = 0.0;
-    bool ahead = false;   // the next matvec is already queued
+    Ahead ahead(ctx, n);
     while (true) {
       const int k = m;
       dcplx* w = V + n * (int64_t)(k + 1);
-      if (!ahead) A(V + n * (int64_t)k, w);
-      ahead = false;
+      if (!ahead.take()) A(V + n * (int64_t)k, w);
       res.numops++;
       double hn = cgs2(ctx, n, k + 1, V, w, h);
-      if (n <= kAheadMax && k + 1 < kdim && hn > 1e-100) {
-        zscal(ctx, n, 1.0 / hn, w);
-        A(w, w + n);
-        ahead = true;
-      }
+      if (k + 1 < kdim) ahead.queue(A, w, hn);
       for (int i = 0; i <= k; ++i) H[i + (size_t)ldh * k] = h[i];
       H[k + 1 + (size_t)ldh * k] = hn;
       m = k + 1;
@@ -275,7 +304,7 @@ KrylovResult exponentiate(Context* ctx, int64_t n, const LinOp& A, cplx t, const
         }
         break;
       }
-      if (!ahead) zscal(ctx, n, 1.0 / hn, w);
+      if (!ahead.queued()) zscal(ctx, n, 1.0 / hn, w);
     }
     std::vector<cplx> coef(m);
     for (int i = 0; i < m; ++i) coef[i] = beta * E[i];
@@ -311,19 +340,14 @@ KrylovResult arnoldi_dominant(Context* ctx, int64_t n, const LinOp& A, const dcp
   std::vector<cplx> H((size_t)ldh * kdim, 0.0), h, lam, Y;
   res.numiter = 1;
   int nvec = 1;
-  bool ahead = false;   // the next matvec is already queued
+  Ahead ahead(ctx, n);
   while (true) {
     const int k = nvec - 1;
     dcplx* w = V + n * (int64_t)nvec;
-    if (!ahead) A(V + n * (int64_t)k, w);
-    ahead = false;
+    if (!ahead.take()) A(V + n * (int64_t)k, w);
     res.numops++;
     double hn = cgs2(ctx, n, nvec, V, w, h);
-    if (n <= kAheadMax && k + 1 < kdim && hn > 1e-100) {
-      zscal(ctx, n, 1.0 / hn, w);
-      A(w, w + n);
-      ahead = true;
-    }
+    if (k + 1 < kdim) ahead.queue(A, w, hn);
     for (int i = 0; i <= k; ++i) H[i + (size_t)ldh * k] = h[i];
     H[k + 1 + (size_t)ldh * k] = hn;
     const int m = k + 1;
@@ -388,7 +412,7 @@ KrylovResult arnoldi_dominant(Context* ctx, int64_t n, const LinOp& A, const dcp
       nvec = keep + 1;
       res.numiter++;
     } else {
-      if (!ahead) zscal(ctx, n, 1.0 / hn, w);
+      if (!ahead.queued()) zscal(ctx, n, 1.0 / hn, w);
       nvec++;
     }
   }
