@@ -60,3 +60,16 @@ def test_exponentiate(problem, dt):
     y = np.zeros_like(x0)
     ctx.lib.imps_ac_apply(envs.h, H.handle(ctx), 0, L.dptr(x0), L.dptr(y))
     assert f1 - f0 == n * (ctx.counters()["gemm_flops"] - f1)
+
+
+def test_a_solve_of_one_step_runs_no_second_matvec(problem):
+    """A basis of one vector cannot have one queued ahead: the same launches."""
+    ctx, H, envs, x0, _ = problem
+    out, info, used = np.zeros_like(x0), L.KrylovInfo(), []
+    for krylovdim in (1, 20):
+        for _ in range(2):   # the second without first-use work
+            k0 = ctx.counters()["kernels"]
+            ctx.lib.imps_eigsolve_ac(envs.h, H.handle(ctx), 0, L.dptr(x0), L.dptr(out), 1e6, krylovdim, 3, 1, C.byref(info))
+            assert info.numops == 1
+        used.append(ctx.counters()["kernels"] - k0)
+    assert used[0] == used[1]
