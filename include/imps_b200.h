@@ -132,7 +132,7 @@ int imps_ctx_set_wait_limit(imps_ctx* ctx, int64_t cycles);
  * intermediates, gauge work arrays).  A call that would grow it past the cap
  * returns IMPS_OOM and leaves the context usable; imps_ctx_workspace_bytes reports
  * the current size, with the scratch that only makes products faster (partial sums
- * and residue planes, 5 GiB at most) and the blocks of destroyed states and
+ * and residue planes, 5.2 GiB at most) and the blocks of destroyed states and
  * environments kept for the next ones (256 MiB at most).  A cap gives both back and
  * keeps neither until it is lifted; imps_ctx_trim gives them back once.  Object
  * storage (states, environments, MPOs) and the cached int8 operand splits are not

@@ -1115,7 +1115,7 @@ int64_t up(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 
 bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha, const dcplx* A, int64_t lda,
                    const dcplx* B, int64_t ldb, cplx beta, dcplx* C, int64_t ldc, double t_fp64) {
-  // int32 sums of K products of residues <= 122 stay below 2^31; the planes within 2 GiB a side
+  // int32 sums of K products of residues <= 122 stay below 2^31; planes of 64 MiB at most
   if (M < 64 || N < 64 || K < 64 || K > 131072) return false;
   // Modelled times in us, fitted to both engines on a B200: 16 for the four launches, the
   // operands' and outputs' elements, and the waves of tiles (2.7 of epilogue at least).  The
@@ -1129,10 +1129,10 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
   if (ctx->capturing()) return false;   // its error flag needs a synchronisation
   const int64_t Kp = up(K, GKB);
   const size_t pa = (size_t)NPL * M * Kp, pb = (size_t)NPL * N * Kp;
-  if (pa > ((size_t)2 << 30) || pb > ((size_t)2 << 30)) return false;
-  // the output's residues of one column panel within 1 GiB (panels that stay in L2 were no
+  if (pa > ((size_t)NPL << 26) || pb > ((size_t)NPL << 26)) return false;
+  // the output's planes of one column panel within 32 MiB each (panels that stay in L2 were no
   // faster: 1.47 ms against 1.21 ms for 6144 x 4096 x 1024, the GEMMs' last waves)
-  int64_t np = ((int64_t)1 << 30) / ((int64_t)NPL * M) / GT * GT;
+  int64_t np = ((int64_t)1 << 25) / M / GT * GT;
   if (np < GT) return false;
   np = std::min<int64_t>(np, N);
   const int64_t ldo = up(np, 32);
