@@ -50,7 +50,10 @@ enum {
                                element), and through FP64 sums otherwise.  Which
                                engine forms a product, and so its last bits, depends
                                on its sizes and on whether scratch is to be had
-                               (none under a workspace cap or a graph capture)     */
+                               (none under a workspace cap or a graph capture).  With
+                               IMPS_FP64_ENGINE=2 in the environment when the context
+                               is created every product is an FP64 sum on the FP64
+                               tensor cores (1: without tensor cores)              */
   IMPS_PREC_SPLIT_I8 = 1    /* int8 split products on tcgen05, exact int32 sums    */
 };
 

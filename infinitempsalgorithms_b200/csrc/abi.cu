@@ -135,7 +135,7 @@ int imps_ctx_create(int device, imps_ctx** out) {
     IMPS_CUDA(cudaMallocHost((void**)&c.err_host, sizeof(int) * 4));
     c.err_host[0] = 0;
     cudaDeviceGetAttribute(&c.num_sms, cudaDevAttrMultiProcessorCount, device);
-    if (const char* e = std::getenv("IMPS_FP64_ENGINE")) c.fp64_engine = std::atoi(e) == 1 ? 1 : 0;
+    if (const char* e = std::getenv("IMPS_FP64_ENGINE")) c.fp64_engine = std::max(0, std::min(2, std::atoi(e)));
     // the allocation-free entry point's fixed array is created with the context,
     // before the caller's allocator takes the rest of the device memory
     imps::noalloc_prepare(device);

@@ -324,7 +324,7 @@ void ac_apply(Context* ctx, const imps_envs* envs, const imps_mpo* mpo, int site
   // level is written (a level without blocks is multiplied as a zero by the general path).
   // The split engine never takes products this small.
   const double macs = (double)Dl * m * d * Dr * Dl + (double)Dl * d * Dr * Dr * n;
-  if (macs <= 7e5 && !ctx->ordered_sums() && ctx->fp64_engine == 0 && (int)W.nz.size() <= kMaxNz && n <= kMaxQ) {
+  if (macs <= 7e5 && !ctx->ordered_sums() && ctx->fp64_engine != 1 && (int)W.nz.size() <= kMaxNz && n <= kMaxQ) {
     MixArgs a;
     mix_args(pl, pl.nz.data(), (int)pl.nz.size(), a);
     const SmallShape h{Dl, Dr, m, d, gr_ld, m * d * n * d};

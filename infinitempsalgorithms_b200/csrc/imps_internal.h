@@ -149,7 +149,9 @@ struct Context {
   int nslices = 5;           // int8 slices per operand in split mode
   int max_adaptive_slices = 6;  // adaptive mode: a tolerance needing more slices runs in FP64
   bool adaptive_slices = false;
-  int fp64_engine = 0;       // FP64 GEMM kernel: 0 = DMMA tensor cores, 1 = SIMT DFMA (env IMPS_FP64_ENGINE)
+  // FP64 GEMM kernels (env IMPS_FP64_ENGINE): 0 = large products by residues, the others on the
+  // DMMA tensor cores, 1 = SIMT DFMA, 2 = DMMA tensor cores only
+  int fp64_engine = 0;
   std::string last_error;
   // blocks of the context's states and environments between objects
   std::shared_ptr<BlockPool> pool = std::make_shared<BlockPool>();
