@@ -267,23 +267,23 @@ void check(Context* ctx) {
 
 }  // namespace
 
-// Jacobi sweeps over the columns of U (n rows, ncol columns, room for a multiple of 16) until
-// no pair rotates.
-static void jacobi_sweeps(Context* ctx, int n, int ncol, dcplx* U) {
+// Jacobi sweeps over the columns of U (n rows, ncol columns, room for an even number of them, or
+// with `blocks` for a multiple of 16) until no pair rotates.
+static void jacobi_sweeps(Context* ctx, int n, int ncol, dcplx* U, bool blocks) {
   DevBuf& flag = ctx->buf("jac_flag", 64);
   int* rot = static_cast<int*>(flag.ptr);
   const double tol = 1e-15 * std::sqrt((double)n);
   const int P = ncol + (ncol & 1), nblk = (ncol + 2 * kJacBlk - 1) / (2 * kJacBlk) * 2;
   for (int sweep = 0; sweep < 60; ++sweep) {
     IMPS_CUDA(cudaMemsetAsync(rot, 0, sizeof(int), ctx->stream));
-    if (n <= 512) {
+    if (blocks) {
       for (int r = 0; r < nblk - 1; ++r) {
         if (n <= 128) jacobi_block_round<4>(ctx, n, nblk, r, U, tol, rot);
         else if (n <= 256) jacobi_block_round<8>(ctx, n, nblk, r, U, tol, rot);
         else jacobi_block_round<16>(ctx, n, nblk, r, U, tol, rot);
         check(ctx);
       }
-    } else {  // 16 columns do not fit in a CTA's shared memory and registers
+    } else {
       for (int r = 0; r < P - 1; ++r) {
         launch_kernel(ctx, k_jacobi_round, P / 2, kJacThreads, 0, n, ncol, P, r, U, n, tol, rot, nullptr, 0, 0);
         check(ctx);
@@ -299,10 +299,27 @@ static void jacobi_sweeps(Context* ctx, int n, int ncol, dcplx* U) {
 // takes many sweeps when A's columns are far from orthogonal (34 for a bond matrix in a
 // general basis, D = 256: 34 ms); on the conjugate transpose of the R factor of A with its
 // columns by descending norm, whose columns are graded and nearly orthogonal, it takes 11,
-// in blocks (5.2 ms with the QR).  With a workspace cap A is taken as it is.
+// in blocks (5.2 ms with the QR).  With a workspace cap A is taken as it is, and in blocks only
+// where the padding to whole blocks fits as well.
 std::vector<double> singular_values_sq(Context* ctx, int D, const dcplx* A, int64_t lda) {
   IMPS_REQUIRE(D > 0, IMPS_INVALID_ARG, "singular values: empty matrix");
-  const int P = (D + 2 * kJacBlk - 1) / (2 * kJacBlk) * (2 * kJacBlk);
+  // blocks: 16 columns fit in a CTA's shared memory and registers
+  bool blocks = D <= 512;
+  int P = D + (D & 1);
+  if (blocks) {
+    try {
+      const int padded = (D + 2 * kJacBlk - 1) / (2 * kJacBlk) * (2 * kJacBlk);
+      ctx->buf("jac_norms", (size_t)padded * sizeof(double));
+      ctx->buf("jac_flag", 64);
+      ctx->buf("jac_u", (size_t)D * padded * sizeof(dcplx));
+      P = padded;
+    } catch (const Error& err) {
+      if (err.status != IMPS_OOM) throw;
+      cudaGetLastError();
+      blocks = false;
+      ctx->scratch.erase("jac_norms");   // (its padding may be what is missing)
+    }
+  }
   DevBuf& U = ctx->buf("jac_u", (size_t)D * P * sizeof(dcplx));
   DevBuf& nr = ctx->buf("jac_norms", (size_t)P * sizeof(double));
   ScopedTimer tm(ctx, "jacobi_svd", 0.0);
@@ -343,7 +360,7 @@ std::vector<double> singular_values_sq(Context* ctx, int D, const dcplx* A, int6
       cudaGetLastError();   // U still holds A
     }
   }
-  jacobi_sweeps(ctx, D, D, U.z());
+  jacobi_sweeps(ctx, D, D, U.z(), blocks);
   norms();
   std::sort(s2.begin(), s2.end(), [](double x, double y) { return x > y; });
   for (double& v : s2) v *= unscale;
