@@ -295,7 +295,9 @@ static void jacobi_sweeps(Context* ctx, int n, int ncol, dcplx* U, bool blocks) 
   }
 }
 
-// The squared singular values of the D x D matrix A, descending.  One-sided Jacobi on A itself
+// The squared singular values of the D x D matrix A, descending, divided by a power of four so
+// that the largest is of order one (their own squares, up to 4^1024, need not be doubles).
+// One-sided Jacobi on A itself
 // takes many sweeps when A's columns are far from orthogonal (34 for a bond matrix in a
 // general basis, D = 256: 34 ms); on the conjugate transpose of the R factor of A with its
 // columns by descending norm, whose columns are graded and nearly orthogonal, it takes 11,
@@ -335,12 +337,10 @@ std::vector<double> singular_values_sq(Context* ctx, int D, const dcplx* A, int6
   const double top = *std::max_element(s2.begin(), s2.end());
   bool finite = true;
   for (double v : s2) finite = finite && std::isfinite(v);
-  double unscale = 1.0;
   if (finite && top > 0.0) {   // an exact scale that keeps the squares' squares in range
     int e;
     std::frexp(std::sqrt(top), &e);
     zscal(ctx, (int64_t)D * D, std::ldexp(1.0, -e), U.z());
-    unscale = std::ldexp(1.0, 2 * e);
   }
   if (finite && top > 0.0 && ctx->workspace_limit == 0 && D <= 32768) {
     try {
@@ -363,7 +363,6 @@ std::vector<double> singular_values_sq(Context* ctx, int D, const dcplx* A, int6
   jacobi_sweeps(ctx, D, D, U.z(), blocks);
   norms();
   std::sort(s2.begin(), s2.end(), [](double x, double y) { return x > y; });
-  for (double& v : s2) v *= unscale;
   return s2;
 }
 

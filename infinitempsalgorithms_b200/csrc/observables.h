@@ -7,7 +7,8 @@
 
 namespace imps {
 
-// Squared singular values (descending) of the D x D matrix A, by one-sided Jacobi.
+// Squared singular values (descending) of the D x D matrix A up to a common power of four, by
+// one-sided Jacobi.
 std::vector<double> singular_values_sq(Context* ctx, int D, const dcplx* A, int64_t lda);
 // Thin SVD A = U diag(s) V^H by one-sided Jacobi (descending s), truncated to at most
 // kmax (> 0) values and to those above `cutoff` (at least one kept); U (m x k), V (n x k)

@@ -40,3 +40,18 @@ def test_smallest_cap(D):
             assert np.all(np.abs(got - want) <= 50 * np.sqrt(D) * np.finfo(float).eps * want[0])
         del psi
         ctx.close()
+
+
+@pytest.mark.parametrize("exponent", [-530, -300, 0, 300, 510, 511])
+def test_squares_near_the_ends_of_the_range(exponent):
+    """A matrix of rank two whose leading squared singular value is 1.7 4^exponent."""
+    D = 20
+    Cm = np.zeros((D, D), complex)
+    Cm[3, 5] = np.sqrt(1.7) * 2.0**exponent
+    Cm[4, 6] = 0.5j * np.sqrt(1.7) * 2.0**exponent
+    ctx = imps.Context(0)
+    psi = _state(ctx, Cm)
+    got = imps.entanglement_spectrum(psi, 1)
+    assert np.all(np.abs(got - np.r_[0.8, 0.2, np.zeros(D - 2)]) <= 8 * np.finfo(float).eps)
+    del psi
+    ctx.close()
