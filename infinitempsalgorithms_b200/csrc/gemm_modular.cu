@@ -32,9 +32,9 @@
 // FP64 sums.
 //
 // The four kernels: partial row norms, residue and magnitude planes, the int8 GEMMs, the
-// reconstruction.  Measured (B200): 6144 x 4096 x 1024 1.15 ms = 31 + 155 + 636 + 332 us
-// (6.50 ms on the FP64 tensor cores), 4096 x 1024 x 6144 1.10 ms = 80 + 433 + 528 + 58 us
-// (6.57 ms); the magnitudes and the checks cost 6 and 4 % of that.  With operands graded so
+// reconstruction.  Measured (B200): 6144 x 4096 x 1024 1.15 ms = 31 + 149 + 635 + 332 us
+// (6.50 ms on the FP64 tensor cores), 4096 x 1024 x 6144 1.09 ms = 79 + 425 + 528 + 58 us
+// (6.57 ms); the magnitudes and the checks cost 6 and 3 % of that.  With operands graded so
 // that every element is summed in FP64, 6144 x 4096 x 1024 takes 12.4 ms; with an identity and
 // noise of 1e-17 as one operand 2.9 ms.
 #include <cuda.h>
@@ -321,38 +321,61 @@ __global__ void __launch_bounds__(256) k_mod_norms(const ModOperand a, const Mod
   }
 }
 
-// The scale exponent of a line: x 2^e rounds to integers of 2-norm in [2^57, 2^58] (the
-// rounding adds at most sqrt(K / 2), far below the 2^0.6 that 2^116 leaves under P / 2).
-// frac: that norm as a fraction of 2^58.
-__device__ int line_exponent(const ModOperand& o, int l, double& frac) {
-  frac = 1.0;
+// The scale of a line from its chunks' partial results, by eight lanes together (q of them): x 2^e
+// rounds to integers of 2-norm in [2^57, 2^58] (the rounding adds at most sqrt(K / 2), far
+// below the 2^0.6 that 2^116 leaves under P / 2).  frac: that norm as a fraction of 2^58.
+__device__ __forceinline__ int4 line_info(const ModOperand& o, int l, int q, double& frac) {
   double s = 0.0, m = 0.0;
+  int nz = 0, last = 0, low = 4096;
   bool lost = false;
-  for (int c = 0; c < o.nchunk; ++c) {
-    const double t = o.part[(int64_t)c * o.lines + l];
-    lost = lost || t < 0.0;
-    s += t;
-    m = fmax(m, o.part[(int64_t)(o.nchunk + c) * o.lines + l]);
+  if (l < o.lines)
+    for (int c = q; c < o.nchunk; c += 8) {
+      const double t = o.part[(int64_t)c * o.lines + l];
+      lost = lost || t < 0.0;
+      s += t;
+      m = fmax(m, o.part[(int64_t)(o.nchunk + c) * o.lines + l]);
+      nz += o.count[(int64_t)c * o.lines + l];
+      last = max(last, o.count[(int64_t)(o.nchunk + c) * o.lines + l]);
+      low = min(low, o.count[(int64_t)(2 * o.nchunk + c) * o.lines + l]);
+    }
+#pragma unroll
+  for (int d = 4; d >= 1; d >>= 1) {
+    s += __shfl_xor_sync(0xffffffffu, s, d);
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, d));
+    nz += __shfl_xor_sync(0xffffffffu, nz, d);
+    last = max(last, __shfl_xor_sync(0xffffffffu, last, d));
+    low = min(low, __shfl_xor_sync(0xffffffffu, low, d));
   }
+  frac = 1.0;
   // a NaN does not pass fmax but does reach the sum of squares
-  if (isnan(s) || isinf(m)) return EXP_NONFINITE;
-  if (m == 0.0) return 0;
-  int e, unit = 0;
-  if (lost) {   // all chunks in units of 2^unit > m
-    frexp(m, &unit);
-    s = 0.0;
-    for (int c = 0; c < o.nchunk; ++c) {
-      const double t = o.part[(int64_t)c * o.lines + l], mc = o.part[(int64_t)(o.nchunk + c) * o.lines + l];
-      int ec = 0;
-      if (t < 0.0) frexp(mc, &ec);
-      // (a plain sum beside one that left the range is no larger than 2^930; what underflows
-      // here is nothing to the result)
-      const double u = scale2(fabs(t), max(ec - unit, -1100));
-      s += scale2(u, max(ec - unit, -1100));
+  const bool nonfinite = isnan(s) || isinf(m);
+  int unit = 0;
+  if (__any_sync(0xffffffffu, lost)) {   // all chunks of such a line in units of 2^unit > m
+    const unsigned mine = 0xffu << (threadIdx.x & 24);
+    lost = (__ballot_sync(0xffffffffu, lost) & mine) != 0u && !nonfinite;
+    if (lost) {
+      frexp(m, &unit);
+      s = 0.0;
+      for (int c = q; c < o.nchunk; c += 8) {
+        const double t = o.part[(int64_t)c * o.lines + l], mc = o.part[(int64_t)(o.nchunk + c) * o.lines + l];
+        int ec = 0;
+        if (t < 0.0) frexp(mc, &ec);
+        // (a plain sum beside one that left the range is no larger than 2^930; what underflows
+        // here is nothing to the result)
+        s += scale2(scale2(fabs(t), max(ec - unit, -1100)), max(ec - unit, -1100));
+      }
+#pragma unroll
+      for (int d = 4; d >= 1; d >>= 1) s += __shfl_xor_sync(mine, s, d);
     }
   }
-  frac = frexp(sqrt(s) * (1.0 + 1e-12), &e);
-  return BETA_BITS - (e + unit);
+  int e = 0;
+  if (nonfinite) {
+    e = EXP_NONFINITE;
+  } else if (m > 0.0) {
+    frac = frexp(sqrt(s) * (1.0 + 1e-12), &e);
+    e = BETA_BITS - (e + unit);
+  }
+  return make_int4(e, nz, last, low + e >= 0);
 }
 
 __device__ __forceinline__ int dp4a_us(unsigned a, int b, int c) {
@@ -431,30 +454,13 @@ constexpr int SPL_LINES = 16, SPL_NT = SPL_LINES * 8;
 __global__ void __launch_bounds__(SPL_NT, 1024 / SPL_NT) k_mod_split(const ModOperand a, const ModOperand b) {
   grid_enter();
   __shared__ double2 tile[SPL_LINES][65];
-  __shared__ int ex[SPL_LINES];
-  __shared__ float mu[SPL_LINES];
   const bool first = (int)blockIdx.x < a.nblocks_split;
   const ModOperand& o = first ? a : b;
   const int blk = first ? blockIdx.x : blockIdx.x - a.nblocks_split;
   const int nk = (int)(o.Kp / 64);
   const int k0 = (blk % nk) * 64, l0 = (blk / nk) * SPL_LINES;
   const int tid = threadIdx.x;
-  if (tid < SPL_LINES) {
-    const int l = l0 + tid;
-    double frac = 1.0;
-    const int e = l < o.lines ? line_exponent(o, l, frac) : 0;
-    ex[tid] = e == EXP_NONFINITE ? 0 : e;
-    mu[tid] = mag_units(o.K, frac);
-    if (k0 == 0 && l < o.lines) {
-      int nz = 0, last = 0, low = 4096;
-      for (int c = 0; c < o.nchunk; ++c) {
-        nz += o.count[(int64_t)c * o.lines + l];
-        last = max(last, o.count[(int64_t)(o.nchunk + c) * o.lines + l]);
-        low = min(low, o.count[(int64_t)(2 * o.nchunk + c) * o.lines + l]);
-      }
-      o.info[l] = make_int4(e, nz, last, low + e >= 0);
-    }
-  }
+  const int ll = tid >> 3, kq = tid & 7;
   if (o.kcontig) {
     const int kx = tid & 63, ly = tid >> 6;
 #pragma unroll
@@ -470,12 +476,14 @@ __global__ void __launch_bounds__(SPL_NT, 1024 / SPL_NT) k_mod_split(const ModOp
       tile[lx][r + ky] = (l < o.lines && k < o.K) ? o.X[l + o.ld * k] : make_double2(0.0, 0.0);
     }
   }
+  double frac;
+  const int4 info = line_info(o, l0 + ll, kq, frac);
+  if (k0 == 0 && kq == 0 && l0 + ll < o.lines) o.info[l0 + ll] = info;
   __syncthreads();
-  const int ll = tid >> 3, kq = tid & 7;
   if (l0 + ll >= o.lines) return;
-  const int e = ex[ll], eh = e / 2;
+  const int e = info.x == EXP_NONFINITE ? 0 : info.x, eh = e / 2;
   const double s1 = pow2(eh), s2 = pow2(e - eh);
-  const float unit = mu[ll];
+  const float unit = mag_units(o.K, frac);
   unsigned xlo[8], xhi[8], ylo[8], yhi[8], q[8];
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
