@@ -1127,9 +1127,11 @@ bool zgemm_modular(Context* ctx, Op opA, Op opB, int M, int N, int K, cplx alpha
   if (M < 64 || N < 64 || K < 64 || K > 131072) return false;
   // Modelled times in us, fitted to both engines on a B200: 16 for the four launches, the
   // operands' and outputs' elements, and the waves of tiles (2.7 of epilogue at least).  The
-  // lines cross near 0.6 GFLOP for square products (256 x 1024 x 256: 29 here and there;
-  // 502 x 251 x 1255: 41 against 55 on the FP64 tensor cores, 1255 x 502 x 251: 46 against
-  // 63) and far later for a short K, whose outputs dominate (4096 x 960 x 64: 165 against 75).
+  // lines cross near 0.6 GFLOP for square products (events around one call, which add some 8:
+  // 448 x 448 x 448 taken by the FP64 tensor cores in 36, 512 x 512 x 512 41 here against 50
+  // there; 502 x 251 x 1255 47 against 64, 1255 x 502 x 251 49 against 70, 300 x 300 x 1200 48
+  // against 47) and far later for a short K, whose outputs dominate (4096 x 960 x 64: 165
+  // against 88).
   const int64_t tiles = (int64_t)((M + GT - 1) / GT) * ((N + GT - 1) / GT) * NPL, npair = ctx->num_sms / 2;
   const double t_here = 16.0 + 15.4e-6 * ((double)M + N) * K + 14.8e-6 * M * (double)N +
                         (double)((tiles + npair - 1) / npair) * std::max(2.7, 3.2 / 1024 * K);
