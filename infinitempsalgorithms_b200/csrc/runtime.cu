@@ -7,7 +7,9 @@
 #include <vector>
 #include <cmath>
 #include <cstring>
+#include <array>
 #include <atomic>
+#include <map>
 #include <system_error>
 #include <thread>
 
@@ -627,17 +629,18 @@ void synchronize(Context* ctx) {
 namespace {
 // Large arrays of the caller's pageable memory go through page-locked chunks, filled or emptied
 // by a few threads: one thread's copies (and, into a fresh array, its page faults) take longer
-// than the transfer.  The threads only move memory: the calling thread issues every transfer and
-// event on the context's stream, whose handle may name another stream in another thread
-// (cudaStreamPerThread).  One staging area per process; a second context that finds it taken,
-// small arrays and page-locked ones use the plain copy.
-constexpr int kStageThreads = 4;
-constexpr int kStageSlots = 2 * kStageThreads;
-constexpr size_t kStageChunk = (size_t)1 << 20, kStageMin = (size_t)4 << 20;
+// than the transfer.  The calling thread issues every transfer and event on the context's
+// stream, whose handle may name another stream in another thread (cudaStreamPerThread); the
+// others move host memory and make no CUDA calls, whose first one in a thread costs some 100
+// us.  One staging area per process; a second context that finds it taken, small arrays and
+// page-locked ones use the plain copy.
+constexpr size_t kStageThreads = 4;   // with the calling one
+constexpr size_t kStageSlots = 2 * kStageThreads, kStageChunk = (size_t)1 << 20, kStageMin = (size_t)4 << 20;
 
 struct Staging {
   std::mutex mu;
   char* mem = nullptr;   // kStageSlots chunks
+  std::map<int, std::array<cudaEvent_t, kStageSlots>> events;   // of each device
 };
 Staging& staging() {
   static auto* s = new Staging;   // as long as the process, like the driver's own
@@ -653,67 +656,99 @@ bool page_locked(const void* p) {
   return a.type != cudaMemoryTypeUnregistered;
 }
 
-// One array's way through the slots: chunk i uses slot i % kStageSlots and is moved in host
-// memory by thread i % kStageThreads, in ascending order each.
+// One array's way through the slots.  Thread t moves the t-th contiguous part in host memory
+// (its own pages and its own two slots); chunk i is the (i / kStageThreads)-th of part
+// i % kStageThreads and uses slot i % kStageSlots, and the transfers go in the order of i.
 struct StagedCopy {
   char *dev, *host, *slots;
-  size_t bytes, n;
+  size_t bytes, part, n;
   bool to_device;
-  int device;
   cudaStream_t stream;
-  cudaEvent_t ev[kStageSlots] = {};
-  std::atomic<size_t> issued{0};                 // chunks whose transfer and event are queued
-  std::atomic<size_t> moved[kStageSlots] = {};   // 1 + the last chunk of the slot moved in host memory
-  std::atomic<int> failed{0};
+  cudaEvent_t* ev;
+  std::atomic<size_t> limit{0};                  // chunks below may be moved: their slot is free (or full)
+  std::atomic<size_t> moved[kStageSlots] = {};   // 1 + the last chunk of the slot that was moved
+  std::atomic<bool> stop{false};                 // all is done, or a transfer failed
+  cudaError_t error = cudaSuccess;               // (the calling thread's from here)
+  size_t issued = 0, done = 0;                   // transfers queued and completed
+  size_t mine = 0;                               // the calling thread's next chunk
 
+  size_t offset(size_t i) const { return i % kStageThreads * part + i / kStageThreads * kStageChunk; }
+  size_t len(size_t i) const {
+    const size_t end = std::min(bytes, (i % kStageThreads + 1) * part), o = offset(i);
+    return o < end ? std::min(kStageChunk, end - o) : 0;
+  }
   char* slot(size_t i) const { return slots + i % kStageSlots * kStageChunk; }
-  size_t len(size_t i) const { return std::min(kStageChunk, bytes - i * kStageChunk); }
-  cudaError_t fail(cudaError_t e) {
-    if (e != cudaSuccess) {
-      int none = 0;
-      failed.compare_exchange_strong(none, (int)e);
-    }
-    return e;
-  }
-  template <class F>
-  bool wait(F&& ready) const {   // false: another thread failed
-    while (!ready()) {
-      if (failed.load()) return false;
-      std::this_thread::yield();
-    }
-    return failed.load() == 0;
-  }
-  // the host memory's side
   void move(size_t i) {
-    const size_t s = i % kStageSlots;
-    if (to_device) {
-      if (i >= kStageSlots) {   // the slot's last transfer has left it
-        if (!wait([&] { return issued.load() > i - kStageSlots; })) return;
-        if (fail(cudaEventSynchronize(ev[s])) != cudaSuccess) return;
-      }
-      std::memcpy(slot(i), host + i * kStageChunk, len(i));
-    } else {
-      if (!wait([&] { return issued.load() > i; })) return;
-      if (fail(cudaEventSynchronize(ev[s])) != cudaSuccess) return;
-      std::memcpy(host + i * kStageChunk, slot(i), len(i));
+    if (const size_t k = len(i)) {
+      if (to_device) std::memcpy(slot(i), host + offset(i), k);
+      else std::memcpy(host + offset(i), slot(i), k);
     }
-    moved[s].store(i + 1);
+    moved[i % kStageSlots].store(i + 1);
   }
   void work(size_t t) {
-    if (fail(cudaSetDevice(device)) != cudaSuccess) return;
-    for (size_t i = t; i < n && !failed.load(); i += kStageThreads) move(i);
+    for (size_t i = t; i < n; i += kStageThreads) {
+      while (limit.load() <= i) {
+        if (stop.load()) return;
+        std::this_thread::yield();
+      }
+      move(i);
+    }
+    // A core that goes idle with the chunks in its cache makes their transfer wait for it (4 MiB
+    // to the device 750 us, 250 with the threads kept until the transfers are done)
+    while (!stop.load()) std::this_thread::yield();
   }
-  // the stream's side, by the calling thread
-  void issue(size_t i) {
-    const size_t s = i % kStageSlots;
-    const size_t need = to_device ? i + 1 : (i >= kStageSlots ? i - kStageSlots + 1 : 0);
-    if (!wait([&] { return moved[s].load() >= need; })) return;
-    char* d = dev + i * kStageChunk;
-    if (fail(to_device ? cudaMemcpyAsync(d, slot(i), len(i), cudaMemcpyHostToDevice, stream)
-                       : cudaMemcpyAsync(slot(i), d, len(i), cudaMemcpyDeviceToHost, stream)) != cudaSuccess)
+  bool ok(cudaError_t e) {
+    if (e == cudaSuccess) return true;
+    error = e;
+    stop.store(true);
+    return false;
+  }
+  void issue() {
+    const size_t i = issued, k = len(i);
+    char* d = dev + offset(i);
+    if (k && !ok(to_device ? cudaMemcpyAsync(d, slot(i), k, cudaMemcpyHostToDevice, stream)
+                           : cudaMemcpyAsync(slot(i), d, k, cudaMemcpyDeviceToHost, stream)))
       return;
-    if (fail(cudaEventRecord(ev[s], stream)) != cudaSuccess) return;
-    issued.store(i + 1);
+    if (ok(cudaEventRecord(ev[i % kStageSlots], stream))) ++issued;
+  }
+  // notes the transfers that have completed
+  void poll() {
+    while (done < issued) {
+      const cudaError_t e = cudaEventQuery(ev[done % kStageSlots]);
+      if (e == cudaErrorNotReady) {
+        cudaGetLastError();
+        break;
+      }
+      if (!ok(e)) return;
+      ++done;
+    }
+    limit.store(to_device ? done + kStageSlots : done);
+  }
+  // The calling thread: transfers whose host side is ready, its own part, completions.
+  void run(size_t first_missing) {
+    limit.store(to_device ? kStageSlots : 0);
+    size_t left = 0;   // chunks of the calling thread (and of threads that did not start)
+    auto own = [&](size_t i) { return i % kStageThreads == 0 || i % kStageThreads >= first_missing; };
+    for (size_t i = 0; i < n; ++i) left += own(i);
+    while (error == cudaSuccess && (issued < n || left > 0)) {
+      const size_t ready = to_device ? issued + 1 : (issued < kStageSlots ? 0 : issued - kStageSlots + 1);
+      if (issued < n && moved[issued % kStageSlots].load() == ready) {
+        issue();
+        continue;
+      }
+      poll();
+      while (mine < n && !own(mine)) ++mine;
+      if (mine < n && mine < limit.load()) {
+        move(mine++);
+        --left;
+      } else {
+        std::this_thread::yield();
+      }
+    }
+    while (error == cudaSuccess && done < n) poll();
+    for (size_t t = 1; t < first_missing && !to_device && error == cudaSuccess; ++t)   // the others' last chunks
+      while (moved[(n - kStageThreads + t) % kStageSlots].load() != n - kStageThreads + t + 1) std::this_thread::yield();
+    stop.store(true);
   }
 };
 
@@ -728,39 +763,37 @@ bool staged_copy(Context* ctx, void* dev, void* host, size_t bytes, bool to_devi
     s.mem = nullptr;
     return false;
   }
+  auto known = s.events.find(ctx->device);
+  if (known == s.events.end()) {
+    std::array<cudaEvent_t, kStageSlots> ev{};
+    for (auto& e : ev) IMPS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    known = s.events.emplace(ctx->device, ev).first;
+  }
   StagedCopy c;
   c.dev = static_cast<char*>(dev);
   c.host = static_cast<char*>(host);
   c.slots = s.mem;
+  c.ev = known->second.data();
   c.bytes = bytes;
-  c.n = (bytes + kStageChunk - 1) / kStageChunk;
+  c.part = ((bytes + kStageThreads - 1) / kStageThreads + 4095) / 4096 * 4096;
+  c.n = kStageThreads * ((c.part + kStageChunk - 1) / kStageChunk);
   c.to_device = to_device;
-  c.device = ctx->device;
   c.stream = ctx->stream;
-  for (auto& e : c.ev) c.fail(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   std::thread th[kStageThreads];
-  for (int t = 0; t < kStageThreads; ++t) {
+  size_t started = 1;
+  for (; started < kStageThreads; ++started) {
     try {
-      th[t] = std::thread(&StagedCopy::work, &c, (size_t)t);
+      th[started] = std::thread(&StagedCopy::work, &c, started);
     } catch (const std::system_error&) {
-      break;   // no thread to be had
+      break;   // no thread to be had: the calling one takes the part
     }
   }
-  // the chunks of threads that did not start are the calling thread's
-  for (size_t i = 0; i < c.n && !c.failed.load(); ++i) {
-    const bool mine = !th[i % kStageThreads].joinable();
-    if (mine && to_device) c.move(i);
-    c.issue(i);
-    if (mine && !to_device) c.move(i);
-  }
+  c.run(started);
   for (auto& t : th)
     if (t.joinable()) t.join();
-  // every transfer has left the slots before the next array uses them
-  const cudaError_t w = cudaStreamSynchronize(ctx->stream);
-  for (auto e : c.ev)
-    if (e) cudaEventDestroy(e);
-  IMPS_CUDA((cudaError_t)c.failed.load());
-  IMPS_CUDA(w);
+  // (without an error every transfer is done and has left the slots)
+  if (c.error != cudaSuccess) cudaStreamSynchronize(ctx->stream);
+  IMPS_CUDA(c.error);
   return true;
 }
 }  // namespace
