@@ -137,7 +137,8 @@ int imps_ctx_set_wait_limit(imps_ctx* ctx, int64_t cycles);
  * the current size, with the scratch that only makes products faster (partial sums
  * and residue planes, 5.2 GiB at most) and the blocks of destroyed states and
  * environments kept for the next ones (256 MiB at most).  A cap gives both back and
- * keeps neither until it is lifted; imps_ctx_trim gives them back once.  Object
+ * keeps neither until it is lifted; imps_ctx_trim gives them back once; an
+ * allocation of any context that does not fit takes those of idle contexts.  Object
  * storage (states, environments, MPOs) and the cached int8 operand splits are not
  * counted.  No reference counterpart (Julia's GC owns the reference's arrays). */
 int imps_ctx_set_workspace_limit(imps_ctx* ctx, int64_t bytes);

@@ -145,6 +145,7 @@ int imps_ctx_create(int device, imps_ctx** out) {
     delete h;
     return r;
   }
+  imps::register_context(&h->c);
   *out = h;
   return IMPS_OK;
 }
@@ -152,6 +153,7 @@ int imps_ctx_create(int device, imps_ctx** out) {
 int imps_ctx_destroy(imps_ctx* h) {
   if (!h) return IMPS_OK;
   imps::Context& c = h->c;
+  imps::unregister_context(&c);
   cudaSetDevice(c.device);
   cudaStreamSynchronize(c.stream);
   for (auto& p : c.pending) {
@@ -212,6 +214,7 @@ int imps_ctx_set_wait_limit(imps_ctx* h, int64_t cycles) {
 int imps_ctx_set_workspace_limit(imps_ctx* h, int64_t bytes) {
   if (!h || bytes < 0) return IMPS_INVALID_ARG;
   h->c.workspace_limit = (size_t)bytes;
+  imps::RunningCall running(&h->c);
   cudaSetDevice(h->c.device);
   if (bytes > 0) h->c.trim();
   h->c.pool->keep(bytes == 0);
@@ -228,6 +231,7 @@ int imps_ctx_trim(imps_ctx* h) {
 
 int imps_ctx_workspace_bytes(imps_ctx* h, int64_t* bytes) {
   if (!h || !bytes) return IMPS_INVALID_ARG;
+  imps::RunningCall running(&h->c);
   size_t total = 0;
   for (const auto& kv : h->c.scratch) total += kv.second.bytes;
   for (const auto& kv : h->c.optional) total += kv.second.bytes;

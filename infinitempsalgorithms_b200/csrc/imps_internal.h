@@ -80,8 +80,12 @@ class BlockPool {
 };
 
 // The device is out of memory: frees the idle blocks of all pools and the scratch that the
-// running call's context can do without.
+// running call's context, and every context without a call, can do without.
 void give_back_idle();
+// Contexts known to give_back_idle, from their creation to their end.
+struct Context;
+void register_context(Context* ctx);
+void unregister_context(Context* ctx);
 
 struct DevBuf {
   void* ptr = nullptr;
@@ -235,6 +239,10 @@ struct Context {
   // it.  Kept between calls; given back when a cap is set or when any other allocation of the
   // context does not fit, and replaced when a call needs more, so no graph may hold it.
   std::map<std::string, DevBuf> optional;
+  // held while an entry point runs (calls of one context from several threads take turns), so
+  // that an allocation of another context may take the scratch of an idle one
+  std::recursive_mutex call_mu;
+  int calls = 0;   // entry points running, 0 or nested ones of the thread that holds call_mu
   int no_scratch = 0;   // > 0: a call that must not allocate is running, or the map is in use
   struct Count {
     int& n;
@@ -277,7 +285,7 @@ struct Context {
 // The context whose entry point runs on this thread, while alive: only its own thread may
 // take its scratch from it.
 struct RunningCall {
-  Context* old;
+  Context *ctx, *old;
   explicit RunningCall(Context* ctx);
   ~RunningCall();
 };

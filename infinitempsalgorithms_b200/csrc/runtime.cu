@@ -555,13 +555,44 @@ void BlockPool::trim_all() {
 }
 
 static thread_local Context* g_running = nullptr;
-RunningCall::RunningCall(Context* ctx) : old(g_running) { g_running = ctx; }
-RunningCall::~RunningCall() { g_running = old; }
+RunningCall::RunningCall(Context* c) : ctx(c), old(g_running) {
+  if (ctx) {
+    ctx->call_mu.lock();
+    ctx->calls++;
+  }
+  g_running = ctx;
+}
+RunningCall::~RunningCall() {
+  g_running = old;
+  if (ctx) {
+    ctx->calls--;
+    ctx->call_mu.unlock();
+  }
+}
+
+static std::set<Context*>& contexts() {   // under pools_mu
+  static auto* s = new std::set<Context*>;
+  return *s;
+}
+void register_context(Context* ctx) {
+  std::lock_guard<std::mutex> lock(pools_mu());
+  contexts().insert(ctx);
+}
+void unregister_context(Context* ctx) {
+  std::lock_guard<std::mutex> lock(pools_mu());
+  contexts().erase(ctx);
+}
 
 void give_back_idle() {
   BlockPool::trim_all();
   Context* c = g_running;
   if (c && c->no_scratch == 0 && !c->optional.empty() && !c->capturing()) c->release_optional();
+  std::lock_guard<std::mutex> lock(pools_mu());
+  for (Context* o : contexts()) {
+    if (o == c || !o->call_mu.try_lock()) continue;
+    if (o->calls == 0 && !o->optional.empty() && !o->capturing()) o->release_optional();
+    o->call_mu.unlock();
+  }
 }
 
 double* Context::pinned(size_t bytes) {
